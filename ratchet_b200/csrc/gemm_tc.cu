@@ -55,10 +55,10 @@ __host__ __device__ constexpr int conv_warps(int bn) { return bn >= 128 ? 8 : 4;
 
 // Two CTAs share an SM (half of its shared memory and at most half of its tensor memory each), so one
 // CTA's pipeline fill and epilogue overlap the other's main loop.
-template <int BN, int WK, int STAGES, class Out>
+template <int BN, int WK, int STAGES, class Out, bool RAGGED>
 __global__ void __launch_bounds__(WK == WK_F16 ? kThreadsTc : kThreadsTc + conv_warps(BN) * 32, 2)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const QuantArgs qa,
-               const GemmEpilogue<Out> epi, Out* out, int M, int N, int K, int* status, int splits, float* __restrict__ partial, uint32_t idesc) {
+               const GemmEpilogue<Out, RAGGED> epi, Out* out, int M, int N, int K, int* status, int splits, float* __restrict__ partial, uint32_t idesc) {
     rcu_kernel_entry_wait_only();
     constexpr int A_BYTES = TM * TK * 2;          // 16 KiB
     constexpr int B_BYTES = BN * TK * 2;
@@ -154,14 +154,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
         const bool ok = mbar_wait(accum_bar, 0, abort_flag, status);
         tc_fence_after();
         if (ok) {
-            // every stage has been read: their memory turns the pieces around.  N is a multiple of 4 (checked by the host)
+            // every stage has been read: their memory turns the pieces around
             float4* turn = reinterpret_cast<float4*>(smem) + q * kTurnQuads;
             const int row0 = m0 + q * 32, r = lane >> 3;
 #pragma unroll 1
             for (int c = 0; c < BN; c += 32) {
                 const int col = n0 + c + (lane & 7) * 4;
                 const bool in = col < N, whole = splits == 1;      // not whole: a K slice leaves f32 partial sums, the summing kernel does the rest
-                const float4 bias = in && whole ? epi.bias4(col) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 bias = in && whole ? epi.bias4(col, N) : make_float4(0.f, 0.f, 0.f, 0.f);
                 float4 resid[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
@@ -174,7 +174,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
                 turn_piece(turn, v, [&](int i, int piece_row, const float4& x) {
                     const int row = row0 + piece_row;
                     if (!in || row >= M) return;
-                    if (whole) epi.store4(out, (size_t)row * N + col, x, bias, resid[i], col);
+                    if (whole) epi.store4(out, (size_t)row * N + col, x, bias, resid[i], col, N);
                     else *reinterpret_cast<float4*>(partial + ((size_t)sp * M + row) * N + col) = x;
                 });
             }
@@ -335,13 +335,13 @@ __global__ void __launch_bounds__(256) sum_k_slices_kernel(const float* __restri
     epi.store8(out, i, acc, (int)(i % (size_t)N));
 }
 
-template <int BN, int WK, class Out = __half>
-rcu_status launch_tc(rcu_device* dev, const CUtensorMap& xmap, const CUtensorMap& wmap, const QuantArgs& qa, const GemmEpilogue<Out>& epi, void* out,
+template <int BN, int WK, class Out = __half, bool RAGGED = false>
+rcu_status launch_tc(rcu_device* dev, const CUtensorMap& xmap, const CUtensorMap& wmap, const QuantArgs& qa, const GemmEpilogue<Out, RAGGED>& epi, void* out,
                      int M, int N, int K, int batch = 1, bool bf16 = false) {
     constexpr int STAGE = TM * TK * 2 + BN * TK * 2;
     constexpr int STAGES = (100 * 1024) / STAGE;     // two CTAs per SM
     const size_t smem = (size_t)STAGES * STAGE + 1024 + 512;
-    auto kern = gemm_tc_kernel<BN, WK, STAGES, Out>;
+    auto kern = gemm_tc_kernel<BN, WK, STAGES, Out, RAGGED>;
     RCU_CUDA(dev, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const uint32_t idesc = umma_idesc_f16(TM, BN, bf16);
     dim3 grid((N + BN - 1) / BN, (M + TM - 1) / TM, batch);
@@ -355,19 +355,21 @@ rcu_status launch_tc(rcu_device* dev, const CUtensorMap& xmap, const CUtensorMap
         splits = (int)std::min<long long>(4, (2ll * dev->sm_count) / tiles);
         while (splits > 1 && (((nk + splits - 1) / splits + 3) & ~3) * (splits - 1) >= nk) --splits;     // every slice gets k-steps
     }
-    if (splits > 1) {
-        void* partial = nullptr;
-        rcu_status st = rcu_alloc(dev, (uint64_t)splits * M * N * 4, &partial);
-        if (st != RCU_OK) return st;
-        grid.z = splits;
-        rcu_launch(dev, kern, grid, threads, smem, xmap, wmap, qa, GemmEpilogue<Out>{nullptr, nullptr, 1.f, 0}, (Out*)out, M, N, K, dev->d_status, splits,
-                   (float*)partial, idesc);
-        dev->launches++;
-        const size_t MN = (size_t)M * N;
-        rcu_launch(dev, sum_k_slices_kernel<Out>, (unsigned)((MN / 8 + 255) / 256), 256, 0, (const float*)partial, epi, (Out*)out, MN, N, splits);
-        rcu_free(dev, partial);      // the pool reuses blocks in stream order
-        RCU_LAUNCH_CHECK(dev);
-        return RCU_OK;
+    if constexpr (!RAGGED) {           // slices need N % 8 == 0
+        if (splits > 1) {
+            void* partial = nullptr;
+            rcu_status st = rcu_alloc(dev, (uint64_t)splits * M * N * 4, &partial);
+            if (st != RCU_OK) return st;
+            grid.z = splits;
+            rcu_launch(dev, kern, grid, threads, smem, xmap, wmap, qa, GemmEpilogue<Out>{nullptr, nullptr, 1.f, 0}, (Out*)out, M, N, K, dev->d_status, splits,
+                       (float*)partial, idesc);
+            dev->launches++;
+            const size_t MN = (size_t)M * N;
+            rcu_launch(dev, sum_k_slices_kernel<Out>, (unsigned)((MN / 8 + 255) / 256), 256, 0, (const float*)partial, epi, (Out*)out, MN, N, splits);
+            rcu_free(dev, partial);      // the pool reuses blocks in stream order
+            RCU_LAUNCH_CHECK(dev);
+            return RCU_OK;
+        }
     }
     rcu_launch(dev, kern, grid, threads, smem, xmap, wmap, qa, epi, (Out*)out, M, N, K, dev->d_status, 1, nullptr, idesc);
     RCU_LAUNCH_CHECK(dev);
@@ -393,8 +395,9 @@ bool make_map_f16_sw128(CUtensorMap* map, const void* base, uint64_t rows, uint6
 bool rcu_gemm_tc_eligible(int lhs_dt, int act_dt, uint64_t M, uint64_t N, uint64_t K) {
     if (act_dt != RCU_F16) return false;
     if (!(lhs_dt == RCU_F16 || lhs_dt == RCU_Q8_0H || lhs_dt == RCU_Q4_KH)) return false;
-    // small problems stay on the SIMT kernel; K rows must be 16-byte multiples for the tensor maps
-    if (M < 32 || N < 64 || K < 64 || K % 8 != 0 || N % 8 != 0) return false;
+    // small problems stay on the SIMT kernel; K rows must be 16-byte multiples for the tensor maps.  Any N: output rows that do not start
+    // on four elements (a vocabulary of 32001) are stored element by element, 610 -> 40 us at M = 33 for 32001 x 3072 f16 weights
+    if (M < 2 || N < 64 || K < 64 || K % 8 != 0) return false;
     if (M > 0x7fffffffull || N > 0x7fffffffull || K > 0x7fffffffull) return false;
     return true;
 }
@@ -464,7 +467,9 @@ rcu_status rcu_gemm_tc_dispatch(rcu_device* dev, int lhs_dt, const void* w, int 
     if (!maps)
         st = rcu_fail(dev, RCU_ERR_CUDA, "gemm_tc: cuTensorMapEncodeTiled failed (M=%llu N=%llu K=%llu)", (unsigned long long)M,
                       (unsigned long long)N, (unsigned long long)K);
-#define RCU_TC(BN_, WK_) launch_tc<BN_, WK_>(dev, xmap, wmap, qa, GemmEpilogue<__half>{(const __half*)bias, nullptr, 1.f, 0}, y, (int)M, (int)N, (int)K)
+#define RCU_TC(BN_, WK_)                                                                                                                                  \
+    (N & 3 ? launch_tc<BN_, WK_, __half, true>(dev, xmap, wmap, qa, GemmEpilogue<__half, true>{(const __half*)bias, nullptr, 1.f, 0}, y, (int)M, (int)N, (int)K) \
+           : launch_tc<BN_, WK_>(dev, xmap, wmap, qa, GemmEpilogue<__half>{(const __half*)bias, nullptr, 1.f, 0}, y, (int)M, (int)N, (int)K))
     if (st == RCU_OK) {
         if (wk == WK_F16) st = bn == 256 ? RCU_TC(256, WK_F16) : bn == 128 ? RCU_TC(128, WK_F16) : RCU_TC(64, WK_F16);
         else if (wk == WK_Q8) st = bn == 128 ? RCU_TC(128, WK_Q8) : RCU_TC(64, WK_Q8);
@@ -475,14 +480,14 @@ rcu_status rcu_gemm_tc_dispatch(rcu_device* dev, int lhs_dt, const void* w, int 
 }
 
 // `batch` independent products out[b] = X[b] . W[b]^T with X [batch, M, pitch_x] and W [batch, N, pitch_w] f16, both K-major
-// (K <= pitch, pitches multiples of 8), out [batch, M, N] f16 contiguous with N a multiple of 4.  The attention products
+// (K <= pitch, pitches multiples of 8), out [batch, M, N] f16 contiguous.  The attention products
 // of an f16 model (whisper/mha.rs:95-110: q.k^T over 6 heads, then weights.v) take this; blockIdx.z is the problem.
 rcu_status rcu_gemm_tc_batched_f16(rcu_device* dev, const void* w, const void* x, void* y, uint64_t M, uint64_t N, uint64_t K, uint64_t batch,
                                    uint64_t pitch_w, uint64_t pitch_x) {
-    if (M < 32 || N < 64 || K < 64 || N % 4 != 0 || pitch_w % 8 != 0 || pitch_x % 8 != 0 || batch == 0 || batch > 65535) return RCU_ERR_UNSUPPORTED;
+    if (M < 32 || N < 64 || K < 64 || pitch_w % 8 != 0 || pitch_x % 8 != 0 || batch == 0 || batch > 65535) return RCU_ERR_UNSUPPORTED;
     if (M > 0x7fffffffull || N > 0x7fffffffull || K > 0x7fffffffull) return RCU_ERR_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) return RCU_ERR_UNSUPPORTED;
-    if (reinterpret_cast<uintptr_t>(y) & ((N % 8 == 0) ? 15 : 7)) return RCU_ERR_UNSUPPORTED;
+    if (N % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & 7)) return RCU_ERR_UNSUPPORTED;
     DevGuard g(dev->ordinal);
     const uint64_t tiles128 = ((M + TM - 1) / TM) * ((N + 127) / 128) * batch;
     const int bn = (tiles128 >= (uint64_t)dev->sm_count && N >= 128) ? 128 : 64;
@@ -491,8 +496,11 @@ rcu_status rcu_gemm_tc_batched_f16(rcu_device* dev, const void* w, const void* x
         return rcu_fail(dev, RCU_ERR_CUDA, "gemm_tc: cuTensorMapEncodeTiled failed (batched M=%llu N=%llu K=%llu)", (unsigned long long)M,
                         (unsigned long long)N, (unsigned long long)K);
     QuantArgs qa{nullptr, nullptr, nullptr};
-    return bn == 128 ? launch_tc<128, WK_F16>(dev, xmap, wmap, qa, GemmEpilogue<__half>{nullptr, nullptr, 1.f, 0}, y, (int)M, (int)N, (int)K, (int)batch)
-                     : launch_tc<64, WK_F16>(dev, xmap, wmap, qa, GemmEpilogue<__half>{nullptr, nullptr, 1.f, 0}, y, (int)M, (int)N, (int)K, (int)batch);
+    const GemmEpilogue<__half> epi{nullptr, nullptr, 1.f, 0};
+    const GemmEpilogue<__half, true> ragged{nullptr, nullptr, 1.f, 0};
+    const int m = (int)M, n = (int)N, k = (int)K, b = (int)batch;
+    if (N & 3) return bn == 128 ? launch_tc<128, WK_F16, __half, true>(dev, xmap, wmap, qa, ragged, y, m, n, k, b) : launch_tc<64, WK_F16, __half, true>(dev, xmap, wmap, qa, ragged, y, m, n, k, b);
+    return bn == 128 ? launch_tc<128, WK_F16>(dev, xmap, wmap, qa, epi, y, m, n, k, b) : launch_tc<64, WK_F16>(dev, xmap, wmap, qa, epi, y, m, n, k, b);
 }
 
 // A Linear with 16-bit operands and a chosen output (rcu_linear): out = x . W^T (+ bias) rounded to the operands' type, or

@@ -80,9 +80,9 @@ __device__ __forceinline__ void umma2_commit_both(uint64_t* bar) {
                  : "memory");
 }
 
-template <class Out>
+template <class Out, bool RAGGED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads2, 1)
-gemm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const GemmEpilogue<Out> epi,
+gemm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const GemmEpilogue<Out, RAGGED> epi,
                 Out* out, int M, int N, int K, int tiles_m, int n_tiles, int* status, uint32_t idesc) {
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
@@ -186,9 +186,9 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
             const int r = lane >> 3, quad = lane & 7;
 #pragma unroll 1
             for (int c = c0; c < c0 + kTileN2 / 2; c += 32) {
-                const int col = n0 + c + quad * 4;              // N is a multiple of 8
+                const int col = n0 + c + quad * 4;
                 const bool in = col < N;
-                const float4 bias = in ? epi.bias4(col) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 bias = in ? epi.bias4(col, N) : make_float4(0.f, 0.f, 0.f, 0.f);
                 float4 resid[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
@@ -200,7 +200,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
                 tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * kAccCols + c), v);
                 turn_piece(mine, v, [&](int i, int piece_row, const float4& x) {
                     const int row = row0 + piece_row;
-                    if (in && row < M) epi.store4(out, (size_t)row * N + col, x, bias, resid[i], col);
+                    if (in && row < M) epi.store4(out, (size_t)row * N + col, x, bias, resid[i], col, N);
                 });
             }
             // this warp has read its part of the buffer: tell the leader's MMA thread
@@ -234,21 +234,21 @@ bool make_map_f16_sw128_rows(CUtensorMap* map, const void* base, uint64_t rows, 
 bool rcu_gemm_tc2_eligible(rcu_device* dev, uint64_t M, uint64_t N, uint64_t K) {
     static const int mode = [] { const char* e = getenv("RCU_GEMM_PAIR"); return e ? atoi(e) : 1; }();
     if (mode == 0) return false;
-    if (M < 256 || N < 256 || K < 64 || K % 8 != 0 || N % 8 != 0) return false;
+    if (M < 256 || N < 256 || K < 64 || K % 8 != 0) return false;
     const uint64_t tiles = ((M + 255) / 256) * ((N + 255) / 256);
     return tiles >= (uint64_t)dev->sm_count / 4;
 }
 
 namespace {
-template <class Out>
-rcu_status launch_pair(rcu_device* dev, const CUtensorMap& xmap, const CUtensorMap& wmap, const GemmEpilogue<Out>& epi, void* y, uint64_t M, uint64_t N,
+template <class Out, bool RAGGED = false>
+rcu_status launch_pair(rcu_device* dev, const CUtensorMap& xmap, const CUtensorMap& wmap, const GemmEpilogue<Out, RAGGED>& epi, void* y, uint64_t M, uint64_t N,
                        uint64_t K, bool bf16) {
     const int tiles_m = (int)((M + 255) / 256), tiles_n = (int)((N + 255) / 256);
     const int n_tiles = tiles_m * tiles_n;
     const int n_pairs = std::min(n_tiles, dev->sm_count / 2);
     const size_t smem = (size_t)kStages2 * kStageBytes2 + 1024 + 256;
-    RCU_CUDA(dev, cudaFuncSetAttribute(gemm_tc2_kernel<Out>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    gemm_tc2_kernel<Out><<<2 * n_pairs, kThreads2, smem, dev->stream>>>(xmap, wmap, epi, (Out*)y, (int)M, (int)N, (int)K, tiles_m, n_tiles,
+    RCU_CUDA(dev, cudaFuncSetAttribute(gemm_tc2_kernel<Out, RAGGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    gemm_tc2_kernel<Out, RAGGED><<<2 * n_pairs, kThreads2, smem, dev->stream>>>(xmap, wmap, epi, (Out*)y, (int)M, (int)N, (int)K, tiles_m, n_tiles,
                                                                        dev->d_status, umma_idesc_f16(2 * TM, kTileN2, bf16));
     RCU_LAUNCH_CHECK(dev);
     return RCU_OK;
@@ -265,5 +265,6 @@ rcu_status rcu_gemm_tc2_launch(rcu_device* dev, const void* w, const void* x, co
     if (t.out_dt == RCU_F32) return launch_pair<float>(dev, xmap, wmap, GemmEpilogue<float>{(const float*)bias, t.resid, t.alpha, t.act}, y, M, N, K, t.bf16);
     if (t.out_dt == RCU_BF16)
         return launch_pair<__nv_bfloat16>(dev, xmap, wmap, GemmEpilogue<__nv_bfloat16>{(const __nv_bfloat16*)bias, nullptr, 1.f, t.act}, y, M, N, K, t.bf16);
+    if (N & 3) return launch_pair<__half>(dev, xmap, wmap, GemmEpilogue<__half, true>{(const __half*)bias, nullptr, 1.f, t.act}, y, M, N, K, t.bf16);
     return launch_pair<__half>(dev, xmap, wmap, GemmEpilogue<__half>{(const __half*)bias, nullptr, 1.f, t.act}, y, M, N, K, t.bf16);
 }

@@ -177,7 +177,7 @@ gemm_tc_f32_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
 #pragma unroll
                     for (int j = 0; j < 32; j += 4) {
                         const int col = n0 + c + j;
-                        if (col + 4 <= N) {
+                        if (col + 4 <= N && (N & 3) == 0) {
                             float4 o = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
                             if (bias) {
                                 const float4 b = *reinterpret_cast<const float4*>(bias + col);
@@ -288,7 +288,8 @@ bool make_map_f32_sw128(CUtensorMap* map, const void* base, uint64_t batches, ui
 bool rcu_gemm_tc_f32_eligible(int lhs_dt, int act_dt, uint64_t M, uint64_t N, uint64_t K) {
     if (act_dt != RCU_F32 || lhs_dt != RCU_F32) return false;
     // small problems stay on the SIMT kernel; rows must be 16-byte multiples for the tensor maps
-    if (M < 32 || N < 64 || K < 32 || K % 4 != 0 || N % 4 != 0) return false;
+    // (two rows already pay: 222 -> 24 us for 3072 x 3072 against the SIMT kernel)
+    if (M < 2 || N < 64 || K < 32 || K % 4 != 0) return false;
     if (M > 0x7fffffffull || N > 0x7fffffffull || K > 0x7fffffffull) return false;
     static const bool off = [] { const char* e = std::getenv("RCU_GEMM_F32_TC"); return e && std::atoi(e) == 0; }();
     return !off;
@@ -299,7 +300,7 @@ rcu_status rcu_gemm_tc_f32_dispatch(rcu_device* dev, const void* w, const void* 
     if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(bias)) & 15)
         return RCU_ERR_UNSUPPORTED;
     // tensor-map strides are multiples of 16 bytes; the grid's z extent is limited
-    if (batches < 1 || batches > 65535 || (batches > 1 && ((M * K) % 4 != 0 || (N * K) % 4 != 0 || (M * N) % 4 != 0 || bias || bias_rows))) return RCU_ERR_UNSUPPORTED;
+    if (batches < 1 || batches > 65535 || (batches > 1 && ((M * K) % 4 != 0 || (N * K) % 4 != 0 || bias || bias_rows))) return RCU_ERR_UNSUPPORTED;
     DevGuard g(dev->ordinal);
     // Tile height: 64 token rows when M fits one such tile (half of a 128-row tile would be padding).  Cutting larger
     // M into 64-row tiles to put a CTA on every SM was measured and is slower (Whisper-tiny's 1500 x 384 x 384
@@ -318,7 +319,7 @@ rcu_status rcu_gemm_tc_f32_dispatch(rcu_device* dev, const void* w, const void* 
     uint64_t splits = 1, best = ~0ull;
     for (int cand : {64, 128}) {
         const uint64_t tiles_c = mt * ((N + cand - 1) / cand);
-        const uint64_t sp_max = (batches == 1 && M * N % 4 == 0) ? std::max<uint64_t>(1, std::min<uint64_t>(8, nk / kMinBlocksPerSplit)) : 1;
+        const uint64_t sp_max = (batches == 1 && N % 4 == 0) ? std::max<uint64_t>(1, std::min<uint64_t>(8, nk / kMinBlocksPerSplit)) : 1;
         for (uint64_t sp = 1; sp <= sp_max; ++sp) {
             const uint64_t kbps_c = (nk + sp - 1) / sp;
             const uint64_t rounds = (tiles_c * sp * batches + sms - 1) / sms;
@@ -330,7 +331,7 @@ rcu_status rcu_gemm_tc_f32_dispatch(rcu_device* dev, const void* w, const void* 
     if (!make_map_f32_sw128(&xmap, x, batches, M, K, (uint32_t)tmr) || !make_map_f32_sw128(&wmap, w, batches, N, K, (uint32_t)bn))
         return rcu_fail(dev, RCU_ERR_CUDA, "gemm_tc_f32: cuTensorMapEncodeTiled failed (M=%llu N=%llu K=%llu x%llu)", (unsigned long long)M,
                         (unsigned long long)N, (unsigned long long)K, (unsigned long long)batches);
-    if (splits > 1 && M * N % 4 == 0) {
+    if (splits > 1) {
         const uint64_t kbps = (nk + splits - 1) / splits;
         splits = (nk + kbps - 1) / kbps;
         void* part = nullptr;

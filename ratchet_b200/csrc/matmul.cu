@@ -13,6 +13,9 @@ rcu_status rcu_gemv_dispatch(rcu_device* dev, int lhs_dt, const void* w, int act
 rcu_status rcu_gemm_tc_dispatch(rcu_device* dev, int lhs_dt, const void* w, int act_dt, const void* x, const void* bias,
                                 void* y, uint64_t M, uint64_t N, uint64_t K);
 bool rcu_gemm_tc_eligible(int lhs_dt, int act_dt, uint64_t M, uint64_t N, uint64_t K);
+// few token rows (any number for Q8_0F weights with f16 activations): weights unpacked in registers
+rcu_status rcu_gemm_rows_dispatch(rcu_device* dev, int lhs_dt, const void* w, int act_dt, const void* x, const void* bias, void* y, uint64_t M, uint64_t N,
+                                  uint64_t K);
 // f32 Linear on the tensor cores (split-TF32, f32-level accuracy)
 rcu_status rcu_gemm_tc_f32_dispatch(rcu_device* dev, const void* w, const void* x, const void* bias, void* y, uint64_t M, uint64_t N,
                                     uint64_t K, uint64_t batches, const void* bias_rows = nullptr);
@@ -109,6 +112,15 @@ template <class FP> struct LoadQ4K {
         return rnd<FP>(fmaf(qv, delta, -mn));
     }
 };
+
+// Whether the register kernel (gemm_rows.cu) takes a Linear.  Up to sixteen token rows it is at or ahead of the tcgen05 kernels (us, K = 3072,
+// 16 rows against 33 there: f16 N = 3072 7 / 12, N = 32001 39 / 41; Q8_0H 7 / 15, 38 / 52; Q4_KH 7 / 15, 51 / 54).  Up to 32 rows codes still
+// gain where the matrix is small (Q8_0H N = 9216, 32 rows: 15 / 21; Q4_KH N = 32001: 68 / 54), f16 weights do not (19 / 13).  Q8_0F under
+// f16 activations has no other tensor-core kernel: its scales do not fit f16 tiles.
+bool takes_rows_kernel(int dt, uint64_t M, uint64_t N, uint64_t K) {
+    if (dt == RCU_Q8_0F) return true;
+    return M <= 16 || (M <= 32 && dt != RCU_F16 && N * K <= (1ull << 26));
+}
 
 constexpr int BM = 64, BN = 64, BK = 16;
 
@@ -241,7 +253,12 @@ rcu_status rcu_matmul(rcu_device* dev, const rcu_tensor* lhs, const rcu_tensor* 
         if (dt_is_q4k(lhs->dt)) return rcu_gemv_q4k_dispatch(dev, lhs->dt, lhs->data, rhs->dt, rhs->data, bptr, dst->data, d.m, d.k);
         return rcu_gemv_dispatch(dev, lhs->dt, lhs->data, rhs->dt, rhs->data, bptr, dst->data, d.m, d.k);
     }
-    // Linear convention W[N,K] . x[M,K]^T -> [M,N]: tensor-core path when the shape qualifies
+    // Linear convention W[N,K] . x[M,K]^T -> [M,N]: the register kernel for few token rows, then the tcgen05 kernels when the shape qualifies
+    const uint64_t tokens = d.rstack * d.n;
+    if (!tl && tr && td && d.lstack == 1 && takes_rows_kernel(lhs->dt, tokens, d.m, d.k)) {
+        st = rcu_gemm_rows_dispatch(dev, lhs->dt, lhs->data, rhs->dt, rhs->data, bptr, dst->data, tokens, d.m, d.k);
+        if (st != RCU_ERR_UNSUPPORTED) return st;
+    }
     if (!tl && tr && td && d.lstack == 1 && rcu_gemm_tc_eligible(lhs->dt, rhs->dt, d.rstack * d.n, d.m, d.k)) {
         st = rcu_gemm_tc_dispatch(dev, lhs->dt, lhs->data, rhs->dt, rhs->data, bptr, dst->data, d.rstack * d.n, d.m, d.k);
         if (st != RCU_ERR_UNSUPPORTED) return st;
@@ -291,7 +308,7 @@ rcu_status rcu_matmul(rcu_device* dev, const rcu_tensor* lhs, const rcu_tensor* 
     // kernel never reads the padding: the maps give the true K and fill beyond it with zeros), and an
     // untransposed B is transposed first.
     if (!tl && !td && !bias && lhs->dt == RCU_F16 && rhs->dt == RCU_F16 && d.lstack == d.rstack && d.dstack == d.lstack &&
-        d.m >= 128 && d.n >= 64 && d.k >= 64 && d.n % 4 == 0 && d.m * d.n * d.k * d.lstack >= (1ull << 24)) {
+        d.m >= 128 && d.n >= 64 && d.k >= 64 && d.m * d.n * d.k * d.lstack >= (1ull << 24)) {
         const uint64_t b = d.lstack, kp = (d.k + 7) & ~7ull;
         void* scratch[3] = {nullptr, nullptr, nullptr};
         const void* aptr = lhs->data;

@@ -172,8 +172,10 @@ template <class Put> __device__ __forceinline__ void turn_piece(float4* turn, co
 
 // What the epilogue of a tensor-core GEMM does with an accumulator: Out = f16 / bf16: round(acc + bias);
 // Out = f32: residual + alpha * (acc + bias), the residual stream of a model that keeps it in 32 bits
-// (`resid` may be the output itself: every element is read by the thread that writes it).
-template <class Out> struct GemmEpilogue {
+// (`resid` may be the output itself: every element is read by the thread that writes it).  RAGGED: the number of columns is no multiple of
+// 4, so rows do not start on four elements and bias4 / store4 go element by element (a form of its own: as a run-time test it cost
+// the whole-row GEMMs 1 %).
+template <class Out, bool RAGGED = false> struct GemmEpilogue {
     const Out* bias;          // per output column, nullable
     const float* resid;       // f32 output only, nullable
     float alpha;
@@ -189,10 +191,14 @@ template <class Out> struct GemmEpilogue {
     }
     // four consecutive columns whose bias, and residual (f32 output), the caller has loaded; `col` a multiple of 4
     struct alignas(4 * sizeof(Out)) Quad { Out v[4]; };
-    __device__ __forceinline__ float4 bias4(int col) const {
+    __device__ __forceinline__ float4 bias4(int col, int N) const {
+        if (RAGGED && bias) {
+            return make_float4(to_f32<Out>(bias[col]), col + 1 < N ? to_f32<Out>(bias[col + 1]) : 0.f, col + 2 < N ? to_f32<Out>(bias[col + 2]) : 0.f,
+                               col + 3 < N ? to_f32<Out>(bias[col + 3]) : 0.f);
+        }
         return bias ? make_float4(to_f32<Out>(bias[col]), to_f32<Out>(bias[col + 1]), to_f32<Out>(bias[col + 2]), to_f32<Out>(bias[col + 3])) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    __device__ __forceinline__ void store4(Out* out, size_t idx, const float4& acc, const float4& b, const float4& r, int col) const {
+    __device__ __forceinline__ void store4(Out* out, size_t idx, const float4& acc, const float4& b, const float4& r, int col, int N) const {
         float v[4] = {acc.x + b.x, acc.y + b.y, acc.z + b.z, acc.w + b.w};
         if (col < act.cols) {
             if (act.kind == RCU_ACT_RELU_SQUARED) {      // without branches: the others are dear enough to hide them
@@ -211,6 +217,12 @@ template <class Out> struct GemmEpilogue {
             v[1] = resid ? fmaf(alpha, v[1], r.y) : alpha * v[1];
             v[2] = resid ? fmaf(alpha, v[2], r.z) : alpha * v[2];
             v[3] = resid ? fmaf(alpha, v[3], r.w) : alpha * v[3];
+        }
+        if (RAGGED) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (col + e < N) out[idx + e] = from_f32<Out>(v[e]);
+            return;
         }
         Quad q;
 #pragma unroll
