@@ -26,6 +26,7 @@
 #include <cstdio>
 
 #include "common.cuh"
+#include "half_chains.cuh"
 
 namespace {
 
@@ -162,15 +163,17 @@ bool multi_broadcast(const rcu_lazy* x, const rcu_lazy* y, uint32_t* rank, uint6
 // opposite) — each group in the order the op lists them.  Meeting a node that is still open means the
 // graph has a cycle.
 // ------------------------------------------------------------------------------------------------
-rcu_status execution_order(rcu_lazy* root, std::vector<rcu_lazy*>* order) {
+// pending: tensors that are resolved count as leaves (what they were computed from is done with).
+rcu_status execution_order(rcu_lazy* root, std::vector<rcu_lazy*>* order, bool pending) {
     enum Mark : char { kOpen = 1, kDone = 2 };
     struct Frame {
         rcu_lazy* node;
         std::vector<rcu_lazy*> srcs;   // in visiting order
         size_t next;
     };
-    auto open_frame = [](rcu_lazy* n) {
+    auto open_frame = [pending](rcu_lazy* n) {
         Frame f{n, {}, 0};
+        if (pending && n->resolved()) return f;
         f.srcs.reserve(n->srcs.size());
         for (rcu_lazy* s : n->srcs)
             if (s->srcs.empty()) f.srcs.push_back(s);
@@ -337,6 +340,8 @@ rcu_status run_node(rcu_lazy* n) {
     }
 }
 
+#include "graph_fusion.cuh"
+
 // ------------------------------------------------------------------------------------------------
 // resolve (tensor.rs:795-859 + allocator.rs:209-340)
 // ------------------------------------------------------------------------------------------------
@@ -352,7 +357,7 @@ rcu_status resolve(rcu_lazy* out) {
     rcu_device* dev = out->dev;
     if (out->resolved()) return RCU_OK;
     std::vector<rcu_lazy*> order;
-    rcu_status st = execution_order(out, &order);
+    rcu_status st = execution_order(out, &order, true);
     if (st != RCU_OK) return st;
     const size_t n = order.size();
     std::unordered_map<uint64_t, size_t> index;
@@ -362,6 +367,18 @@ rcu_status resolve(rcu_lazy* out) {
     const bool no_reuse = (dev->debug_flags & RCU_DEBUG_NO_REUSE) != 0;
     const bool profile = (dev->debug_flags & RCU_DEBUG_PROFILE) != 0;
     const bool log = (dev->debug_flags & RCU_DEBUG_LOG) != 0;
+
+    // subgraphs that run as one kernel; a node they pass over gets neither buffer nor kernel, nor does a cache that only appends
+    const fusion::Pass fused(dev, no_reuse ? std::vector<rcu_lazy*>{} : order);
+    auto bufferless = [&](const rcu_lazy* t) {
+        if (fused.absorbed(t)) return true;
+        const fusion::Op* op = fused.find(t);
+        return op && op->kind == fusion::APPEND;
+    };
+    auto sources = [&](const rcu_lazy* t) -> const std::vector<rcu_lazy*>& {
+        const fusion::Op* op = fused.find(t);
+        return op ? op->srcs : t->srcs;
+    };
 
     // how many references to each node come from inside this graph
     std::unordered_map<uint64_t, uint32_t> internal_refs;
@@ -375,7 +392,7 @@ rcu_status resolve(rcu_lazy* out) {
     for (size_t i = 0; i < n; ++i) {
         rcu_lazy* t = order[i];
         owner[i] = i;
-        if (t->resolved() || t->srcs.empty()) continue;
+        if (t->resolved() || t->srcs.empty() || fused.absorbed(t) || fused.find(t)) continue;
         rcu_lazy* s0 = t->srcs[0];
         if (t->kind == K_VIEW) {
             owner[i] = owner[index[s0->id]];
@@ -393,7 +410,7 @@ rcu_status resolve(rcu_lazy* out) {
     uint64_t naive = 0;
     for (size_t i = 0; i < n; ++i) {
         rcu_lazy* t = order[i];
-        if (t->resolved()) continue;
+        if (t->resolved() || bufferless(t)) continue;
         if (t->kind != K_VIEW) naive += t->nbytes();
         const size_t o = owner[i];
         if (order[o]->resolved()) continue;   // in place on (or view of) an already resolved tensor
@@ -410,8 +427,8 @@ rcu_status resolve(rcu_lazy* out) {
     }
     for (size_t i = 0; i < n; ++i) {
         rcu_lazy* t = order[i];
-        if (t->resolved()) continue;
-        for (rcu_lazy* s : t->srcs) {
+        if (t->resolved() || fused.absorbed(t)) continue;
+        for (rcu_lazy* s : sources(t)) {
             const size_t si = index[s->id];
             if (order[si]->resolved() && owner[si] == si) continue;
             auto it = plan_of.find(owner[si]);
@@ -457,15 +474,17 @@ rcu_status resolve(rcu_lazy* out) {
     const uint64_t launches0 = dev->launches;
     for (size_t i = 0; i < n; ++i) {
         rcu_lazy* t = order[i];
-        if (t->resolved()) continue;
+        if (t->resolved() || fused.absorbed(t)) continue;
+        const fusion::Op* op = fused.find(t);
         const size_t o = owner[i];
-        if (o == i) t->storage = objects[plans[plan_of[o]].object].storage;
+        if (bufferless(t)) {
+        } else if (o == i) t->storage = objects[plans[plan_of[o]].object].storage;
         else t->storage = order[o]->storage;
-        if (!t->storage) return rcu_fail(dev, RCU_ERR_INVALID_ARG, "resolve: tensor %llu has no storage", (unsigned long long)t->id);   // TensorError::NoStorage
+        if (!t->storage && !bufferless(t)) return rcu_fail(dev, RCU_ERR_INVALID_ARG, "resolve: tensor %llu has no storage", (unsigned long long)t->id);   // TensorError::NoStorage
         if (t->kind == K_VIEW || t->kind == K_CONST) continue;
         if (inplace[i]) ++n_inplace;
         if (log) {
-            std::fprintf(stderr, "[rcu] node %llu %s %s [", (unsigned long long)t->id, kind_name(t->kind), dt_name(t->dt));
+            std::fprintf(stderr, "[rcu] node %llu %s %s [", (unsigned long long)t->id, op ? fusion::name_of(op->kind) : kind_name(t->kind), dt_name(t->dt));
             for (uint32_t a = 0; a < t->rank; ++a) std::fprintf(stderr, a ? ", %llu" : "%llu", (unsigned long long)t->shape[a]);
             std::fprintf(stderr, "]%s\n", inplace[i] ? " in place" : "");
         }
@@ -475,13 +494,13 @@ rcu_status resolve(rcu_lazy* out) {
             if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) return rcu_fail(dev, RCU_ERR_CUDA, "resolve: cudaEventCreate");
             cudaEventRecord(e0, dev->stream);
         }
-        st = run_node(t);
+        st = op ? fusion::run(dev, t, *op) : run_node(t);
         if (st != RCU_OK) return st;
         if (profile) {
             cudaEventRecord(e1, dev->stream);
             uint64_t bytes = t->nbytes();
-            for (rcu_lazy* s : t->srcs) bytes += s->nbytes();
-            std::string key = std::string(kind_name(t->kind)) + " " + dt_name(t->srcs.empty() ? t->dt : t->srcs[0]->dt);
+            for (rcu_lazy* s : sources(t)) bytes += s->nbytes();
+            std::string key = std::string(op ? fusion::name_of(op->kind) : kind_name(t->kind)) + " " + dt_name(t->srcs.empty() ? t->dt : t->srcs[0]->dt);
             timed.push_back(TimedNode{std::move(key), bytes, e0, e1});
         }
         ++launched;
@@ -981,7 +1000,7 @@ uint64_t rcu_lazy_id(const rcu_lazy* t) { return t ? t->id : 0; }
 rcu_status rcu_lazy_execution_order(rcu_lazy* t, uint64_t* ids, uint32_t capacity, uint32_t* n_nodes) {
     if (!t || !n_nodes || (capacity && !ids)) return RCU_ERR_INVALID_ARG;
     std::vector<rcu_lazy*> order;
-    const rcu_status st = execution_order(t, &order);
+    const rcu_status st = execution_order(t, &order, false);
     if (st != RCU_OK) return st;
     *n_nodes = (uint32_t)order.size();
     for (size_t i = 0; i < order.size() && i < capacity; ++i) ids[i] = order[i]->id;

@@ -1,0 +1,394 @@
+// Subgraphs of an f16 prompt that the resolver runs as one kernel (included by graph.cu).
+//
+// Only nodes that nothing outside the graph holds, and that a single op consumes, are passed over: they get no buffer and no kernel.
+// What is recognised (T > 1 positions; single tokens keep one kernel per op):
+//   attention    permute(softmax(f32(scores [+ mask])) v), scores = f16(scale * f32(q) f32(k)^T) with keys and values that a cache returns or
+//                that are given (phi3/attn.rs:119-157), or (dk q)(dk k^T) in f16 (whisper/mha.rs:92-127); permutes of views of
+//                q, k and v become strides, and a cache that only feeds the attention is appended to but not copied out
+//   heads        cast(rope(cast(permute(view(slice))))), and permute(view(slice)) in front of a cache: straight into the cache's rows
+//   norm         cast(norm(cast x));   act: cast(gelu or silu(cast x));   glu: up * cast(silu(cast gate)) of the halves of one tensor
+// A subgraph whose sizes or alignment a kernel does not take stays as it is.
+#pragma once
+
+namespace fusion {
+
+enum Kind { NONE = 0, ATTENTION, HEADS, APPEND, NORM, ACT, GLU };
+
+// element (position t, head h, feature d) of a [1, heads, T, D] operand at base[offset + h * head + t * row + d]
+struct Heads {
+    rcu_lazy* base = nullptr;
+    uint64_t offset = 0, head = 0, row = 0;
+    HeadRows rows() const { return HeadRows{(const char*)base->storage->ptr + offset * 2, head, row}; }
+};
+
+struct Op {
+    Kind kind = NONE;
+    std::vector<rcu_lazy*> srcs;        // what the kernel reads
+    Heads q, k, v;                      // HEADS and APPEND: q is the source
+    rcu_lazy *mask = nullptr, *scale = nullptr, *scale_q = nullptr, *scale_k = nullptr;
+    bool copied = false;                // APPEND: the source is an ordinary [1, H, T, D] tensor
+    HeadsRope rope;
+    uint32_t H = 0, T = 0, L = 0, D = 0, E = 0;
+};
+
+// `t` exists only for its one consumer
+inline bool inner(const rcu_lazy* t) { return !t->resolved() && t->refs.load() == 1; }
+inline bool inner(const rcu_lazy* t, int kind, int32_t dt) { return inner(t) && t->kind == kind && t->dt == dt; }
+inline bool permutes(const rcu_lazy* t, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    return t->rank == 4 && t->u[0] == a && t->u[1] == b && t->u[2] == c && t->u[3] == d;
+}
+
+struct Pass {
+    const rcu_device* dev;
+    std::unordered_map<uint64_t, Op> ops;           // by the id of the node whose result they produce
+    std::unordered_set<uint64_t> passed;            // nodes without a kernel or buffer
+
+    bool absorbed(const rcu_lazy* t) const { return passed.count(t->id) != 0; }
+    const Op* find(const rcu_lazy* t) const {
+        auto it = ops.find(t->id);
+        return it == ops.end() ? nullptr : &it->second;
+    }
+
+    // The operand [1, H, T, D] `x` as strides into the tensor behind its permute, view and slice, where these are its own; `seen` receives
+    // the nodes passed over.  time_last: x is [1, H, D, T].
+    static Heads strides(rcu_lazy* x, bool time_last, std::vector<rcu_lazy*>* seen) {
+        const uint64_t H = x->shape[1], T = x->shape[time_last ? 3 : 2], D = x->shape[time_last ? 2 : 3];
+        const bool perm = inner(x, K_PERMUTE, RCU_F16) && (time_last ? permutes(x, 0, 2, 3, 1) : permutes(x, 0, 2, 1, 3));
+        if (!perm) {
+            if (time_last) return Heads{};
+            return Heads{x, 0, T * D, D};
+        }
+        rcu_lazy* y = x->srcs[0];                    // [1, T, H, D]
+        seen->push_back(x);
+        if (!inner(y, K_VIEW, RCU_F16)) return Heads{y, 0, D, H * D};
+        rcu_lazy* z = y->srcs[0];
+        seen->push_back(y);
+        if (inner(z, K_SLICE, RCU_F16) && z->rank == 3 && z->shape[0] == 1 && z->shape[1] == T && z->shape[2] == H * D) {
+            rcu_lazy* w = z->srcs[0];
+            if (w->rank == 3 && w->shape[0] == 1 && w->shape[1] == T && z->a[0] == 0 && z->a[1] == 0) {
+                seen->push_back(z);
+                return Heads{w, z->a[2], D, w->shape[2]};
+            }
+        }
+        return Heads{z, 0, D, H * D};
+    }
+
+    static bool vectors(const Heads& h) { return h.base && h.offset % 8 == 0 && h.head % 8 == 0 && h.row % 8 == 0 && aligned(h.base); }
+
+    // whether the kernels' 16-byte accesses fit: pool blocks do, a tensor over memory of the caller's may not
+    static bool aligned(const rcu_lazy* t) {
+        while (!t->resolved() && t->kind == K_VIEW) t = t->srcs[0];
+        return !t->resolved() || (reinterpret_cast<uintptr_t>(t->storage->ptr) & 15) == 0;
+    }
+
+    // a cache that returns [1, H, L, D] and feeds only the attention: its tensor's rows in place
+    Heads from_cache(rcu_lazy* x, std::vector<rcu_lazy*>* appends) const {
+        if (!inner(x, K_CACHE, RCU_F16) || x->rank != 4 || x->u[0] != 2) return Heads{};
+        rcu_lazy* c = x->srcs[0];
+        if (!c->resolved() || c->rank != 4 || c->shape[0] != 1 || !aligned(c) || owners(c) != 1) return Heads{};
+        appends->push_back(x);
+        return Heads{c, 0, c->shape[2] * c->shape[3], c->shape[3]};
+    }
+
+    // caches of this graph that write to the memory of `c`
+    const std::vector<rcu_lazy*>* order;
+    int owners(const rcu_lazy* c) const {
+        const char *a = (const char*)c->storage->ptr, *b = a + c->nbytes();
+        int n = 0;
+        for (const rcu_lazy* t : *order) {
+            if (t->kind != K_CACHE && t->kind != K_INDEX_WRITE) continue;
+            if (t->resolved() || !t->srcs[0]->resolved()) continue;
+            const char* p = (const char*)t->srcs[0]->storage->ptr;
+            if (p < b && p + t->srcs[0]->nbytes() > a) ++n;
+        }
+        return n;
+    }
+
+    bool attention(rcu_lazy* root) {
+        if (root->dt != RCU_F16 || root->rank != 4 || !permutes(root, 0, 2, 1, 3) || root->shape[0] != 1) return false;
+        std::vector<rcu_lazy*> seen, appends;
+        rcu_lazy* pv = root->srcs[0];
+        if (!inner(pv, K_MATMUL, RCU_F16) || pv->srcs.size() != 2 || pv->flags[0] || pv->flags[1] || pv->flags[2]) return false;
+        rcu_lazy *w = pv->srcs[0], *v = pv->srcs[1];
+        if (!inner(w, K_CAST, RCU_F16) || v->rank != 4 || w->rank != 4 || w->shape[0] != 1 || v->shape[0] != 1 || v->shape[1] != w->shape[1]) return false;
+        rcu_lazy* sm = w->srcs[0];
+        if (!inner(sm, K_SOFTMAX, RCU_F32) || sm->u[0] != 3) return false;
+        rcu_lazy* full = sm->srcs[0];
+        if (!inner(full, K_CAST, RCU_F32)) return false;
+        seen.insert(seen.end(), {pv, w, sm, full});
+        Op op;
+        op.kind = ATTENTION;
+        op.H = (uint32_t)w->shape[1];
+        op.T = (uint32_t)w->shape[2];
+        op.L = (uint32_t)w->shape[3];
+        op.E = (uint32_t)v->shape[3];
+        if (op.T < 2 || w->shape[2] > 0x7fffffffull || w->shape[3] > 0x7fffffffull) return false;
+        rcu_lazy* z = full->srcs[0];
+        if (inner(z, K_BINARY, RCU_F16) && z->op == RCU_ADD) {
+            rcu_lazy *x = z->srcs[0], *m = z->srcs[1];
+            const uint32_t r = m->rank;
+            if (m->dt != RCU_F16 || r < 2 || m->shape[r - 2] != op.T || m->shape[r - 1] != op.L || m->numel() != (uint64_t)op.T * op.L) return false;
+            op.mask = m;
+            seen.push_back(z);
+            z = x;
+        }
+        rcu_lazy *q, *k;
+        if (inner(z, K_CAST, RCU_F16)) {            // f16(scale * f32(q) f32(k)^T)
+            rcu_lazy* mul = z->srcs[0];
+            if (!inner(mul, K_BINARY, RCU_F32) || mul->op != RCU_MUL || mul->srcs[1]->numel() != 1 || mul->srcs[1]->dt != RCU_F32) return false;
+            rcu_lazy* qk = mul->srcs[0];
+            if (!inner(qk, K_MATMUL, RCU_F32) || qk->srcs.size() != 2 || qk->flags[0] || !qk->flags[1] || qk->flags[2]) return false;
+            rcu_lazy *q32 = qk->srcs[0], *k32 = qk->srcs[1];
+            if (!inner(q32, K_CAST, RCU_F32) || !inner(k32, K_CAST, RCU_F32)) return false;
+            q = q32->srcs[0];
+            k = k32->srcs[0];
+            if (q->dt != RCU_F16 || k->dt != RCU_F16) return false;
+            op.scale = mul->srcs[1];
+            seen.insert(seen.end(), {z, mul, qk, q32, k32});
+            if (q->rank != 4 || k->rank != 4 || q->shape[0] != 1 || q->shape[1] != op.H || q->shape[2] != op.T || k->shape[0] != 1 || k->shape[1] != op.H ||
+                k->shape[2] != op.L || k->shape[3] != q->shape[3])
+                return false;
+            op.D = (uint32_t)q->shape[3];
+            op.q = strides(q, false, &seen);
+            op.k = from_cache(k, &appends);
+            if (!op.k.base) op.k = strides(k, false, &seen);
+        } else if (inner(z, K_MATMUL, RCU_F16) && !op.mask && z->srcs.size() == 2 && !z->flags[0] && !z->flags[1] && !z->flags[2]) {     // (q dk)(k^T dk)
+            rcu_lazy *qm = z->srcs[0], *km = z->srcs[1];
+            for (rcu_lazy* t : {qm, km})
+                if (!inner(t, K_BINARY, RCU_F16) || t->op != RCU_MUL || t->srcs[1]->numel() != 1 || t->srcs[1]->dt != RCU_F16 || t->rank != 4) return false;
+            q = qm->srcs[0];
+            k = km->srcs[0];
+            op.scale_q = qm->srcs[1];
+            op.scale_k = km->srcs[1];
+            seen.insert(seen.end(), {z, qm, km});
+            if (q->rank != 4 || k->rank != 4 || q->shape[0] != 1 || q->shape[1] != op.H || q->shape[2] != op.T || k->shape[0] != 1 || k->shape[1] != op.H ||
+                k->shape[3] != op.L || k->shape[2] != q->shape[3])
+                return false;
+            op.D = (uint32_t)q->shape[3];
+            op.q = strides(q, false, &seen);
+            op.k = strides(k, true, &seen);
+        } else {
+            return false;
+        }
+        if (v->shape[2] != op.L) return false;
+        op.v = from_cache(v, &appends);
+        if (!op.v.base) op.v = strides(v, false, &seen);
+        if (!vectors(op.q) || !vectors(op.k) || !vectors(op.v)) return false;
+        AttentionArgs a{};
+        a.q = HeadRows{nullptr, op.q.head, op.q.row};
+        a.k = HeadRows{nullptr, op.k.head, op.k.row};
+        a.v = HeadRows{nullptr, op.v.head, op.v.row};
+        a.H = (int)op.H; a.T = (int)op.T; a.L = (int)op.L; a.D = (int)op.D; a.E = (int)op.E;
+        a.mask = op.mask ? (const __half*)16 : nullptr;
+        if (!rcu_attention_f16_takes(dev, a)) return false;
+        for (rcu_lazy* t : seen)
+            if (absorbed(t) || find(t)) return false;
+        op.srcs = {op.q.base, op.k.base, op.v.base};
+        for (rcu_lazy* t : {op.mask, op.scale, op.scale_q, op.scale_k})
+            if (t) op.srcs.push_back(t);
+        for (rcu_lazy* t : appends) {
+            op.srcs.push_back(t);                    // runs before the attention; holds no buffer
+            append(t);
+        }
+        for (rcu_lazy* t : seen) passed.insert(t->id);
+        ops.emplace(root->id, std::move(op));
+        return true;
+    }
+
+    // q or k behind its slice, view, permute and rope, from the node that casts back to f16
+    bool rotated(rcu_lazy* root, Op* op, std::vector<rcu_lazy*>* seen) const {
+        if (root->kind != K_CAST || root->dt != RCU_F16 || root->rank != 4 || root->shape[0] != 1 || root->shape[2] < 2) return false;
+        rcu_lazy* rope = root->srcs[0];
+        if (!inner(rope, K_ROPE, RCU_F32)) return false;
+        rcu_lazy* up = rope->srcs[0];
+        if (!inner(up, K_CAST, RCU_F32) || up->srcs[0]->dt != RCU_F16) return false;
+        seen->insert(seen->end(), {rope, up});
+        op->H = (uint32_t)root->shape[1];
+        op->T = (uint32_t)root->shape[2];
+        op->D = (uint32_t)root->shape[3];
+        op->q = strides(up->srcs[0], false, seen);
+        op->rope.dim = rope->u[0];
+        op->rope.base = rope->f[1];
+        op->rope.offset = rope->u[1];
+        return vectors(op->q) && op->D % 8 == 0 && op->rope.dim % 16 == 0 && (uint64_t)op->T * op->D <= 0x7fffffffull;
+    }
+
+    bool free_of(const std::vector<rcu_lazy*>& seen) const {
+        for (rcu_lazy* t : seen)
+            if (absorbed(t) || find(t)) return false;
+        return true;
+    }
+
+    bool heads(rcu_lazy* root) {
+        Op op;
+        std::vector<rcu_lazy*> seen;
+        if (!rotated(root, &op, &seen) || !free_of(seen)) return false;
+        op.kind = HEADS;
+        op.srcs = {op.q.base};
+        for (rcu_lazy* t : seen) passed.insert(t->id);
+        ops.emplace(root->id, std::move(op));
+        return true;
+    }
+
+    // the cache node `t` only appends: from where its source's heads come from, if these are its own
+    void append(rcu_lazy* t) {
+        Op op;
+        op.kind = APPEND;
+        rcu_lazy* x = t->srcs[1];
+        std::vector<rcu_lazy*> seen;
+        bool direct = false;
+        if (inner(x) && x->shape[2] > 1) {
+            seen.push_back(x);
+            if (x->kind == K_CAST) {
+                direct = rotated(x, &op, &seen);
+            } else if (x->kind == K_PERMUTE && permutes(x, 0, 2, 1, 3)) {
+                seen.clear();
+                op.H = (uint32_t)x->shape[1];
+                op.T = (uint32_t)x->shape[2];
+                op.D = (uint32_t)x->shape[3];
+                op.q = strides(x, false, &seen);
+                direct = vectors(op.q) && op.D % 8 == 0 && (uint64_t)op.T * op.D <= 0x7fffffffull;
+            }
+            direct = direct && free_of(seen);
+        }
+        if (direct) {
+            for (rcu_lazy* s : seen) passed.insert(s->id);
+            op.srcs = {t->srcs[0], op.q.base};
+        } else {
+            op = Op{};
+            op.kind = APPEND;
+            op.copied = true;
+            op.srcs = {t->srcs[0], x};
+        }
+        ops.emplace(t->id, std::move(op));
+    }
+
+    // cast(op(cast x)) of an f16 tensor: the op, null if it is another graph
+    rcu_lazy* between_casts(rcu_lazy* root, int kind, std::vector<rcu_lazy*>* seen) const {
+        if (root->kind != K_CAST || root->dt != RCU_F16) return nullptr;
+        rcu_lazy* t = root->srcs[0];
+        if (!inner(t, kind, RCU_F32)) return nullptr;
+        rcu_lazy* up = t->srcs[0];
+        if (!inner(up, K_CAST, RCU_F32) || up->srcs[0]->dt != RCU_F16) return nullptr;
+        seen->insert(seen->end(), {t, up});
+        return t;
+    }
+
+    static uint64_t rows_of(const rcu_lazy* t) { return t->numel() / t->shape[t->rank - 1]; }
+
+    bool norm(rcu_lazy* root) {
+        std::vector<rcu_lazy*> seen;
+        rcu_lazy* t = between_casts(root, K_NORM, &seen);
+        const uint64_t N = root->shape[root->rank - 1];
+        if (!t || t->op == RCU_GROUP_NORM || N % 8 || N > 8192 || rows_of(root) < 2 || rows_of(root) > 0x7fffffffull || !free_of(seen)) return false;
+        for (size_t i = 1; i < t->srcs.size(); ++i)
+            if (t->srcs[i]->dt != RCU_F32 || t->srcs[i]->numel() != N || !aligned(t->srcs[i])) return false;
+        if (!aligned(seen[1]->srcs[0])) return false;
+        Op op;
+        op.kind = NORM;
+        op.srcs = t->srcs;
+        op.srcs[0] = seen[1]->srcs[0];
+        for (rcu_lazy* s : seen) passed.insert(s->id);
+        ops.emplace(root->id, std::move(op));
+        return true;
+    }
+
+    bool act(rcu_lazy* root) {
+        std::vector<rcu_lazy*> seen;
+        rcu_lazy* t = between_casts(root, K_UNARY, &seen);
+        if (!t || (t->op != RCU_GELU && t->op != RCU_SILU) || root->numel() % 8 || rows_of(root) < 2 || !aligned(seen[1]->srcs[0]) || !free_of(seen)) return false;
+        Op op;
+        op.kind = ACT;
+        op.srcs = {seen[1]->srcs[0]};
+        for (rcu_lazy* s : seen) passed.insert(s->id);
+        ops.emplace(root->id, std::move(op));
+        return true;
+    }
+
+    // up * cast(silu(cast gate)), gate and up the halves of one tensor's last dimension
+    bool glu(rcu_lazy* root) {
+        if (root->kind != K_BINARY || root->op != RCU_MUL || root->dt != RCU_F16) return false;
+        rcu_lazy *up = root->srcs[0], *a = root->srcs[1];
+        if (!inner(up, K_SLICE, RCU_F16) || !inner(a, K_CAST, RCU_F16)) return false;
+        std::vector<rcu_lazy*> seen{up, a};
+        rcu_lazy* t = between_casts(a, K_UNARY, &seen);
+        if (!t || (t->op != RCU_GELU && t->op != RCU_SILU)) return false;
+        rcu_lazy* gate = seen.back()->srcs[0];
+        if (!inner(gate, K_SLICE, RCU_F16) || gate->srcs[0] != up->srcs[0] || gate->rank != up->rank) return false;
+        seen.push_back(gate);
+        const rcu_lazy* x = up->srcs[0];
+        const uint32_t r = x->rank;
+        const uint64_t F = root->shape[root->rank - 1];
+        if (r != up->rank || x->shape[r - 1] != 2 * F || F % 8 || F > 0x7fffffffull || gate->a[r - 1] != 0 || up->a[r - 1] != F || up->shape[r - 1] != F || gate->shape[r - 1] != F) return false;
+        for (uint32_t i = 0; i + 1 < r; ++i)
+            if (gate->a[i] || up->a[i] || gate->shape[i] != x->shape[i] || up->shape[i] != x->shape[i]) return false;
+        if (rows_of(root) < 2 || root->numel() * 2 != x->numel() || !aligned(x) || !free_of(seen)) return false;
+        Op op;
+        op.kind = GLU;
+        op.srcs = {up->srcs[0]};
+        for (rcu_lazy* s : seen) passed.insert(s->id);
+        ops.emplace(root->id, std::move(op));
+        return true;
+    }
+
+    // consumers before what they consume, so that a chain is recognised from its end
+    Pass(const rcu_device* d, const std::vector<rcu_lazy*>& o) : dev(d), order(&o) {
+        for (size_t i = o.size(); i-- > 0;) {
+            rcu_lazy* t = o[i];
+            if (t->resolved() || absorbed(t) || find(t)) continue;
+            if (t->kind == K_PERMUTE) attention(t);
+            else if (t->kind == K_CAST) heads(t) || norm(t) || act(t);
+            else if (t->kind == K_BINARY) glu(t);
+        }
+    }
+};
+
+inline const char* name_of(Kind k) {
+    static const char* names[] = {"", "attention", "heads", "cache", "norm chain", "act chain", "glu chain"};
+    return names[k];
+}
+
+rcu_status run(rcu_device* dev, rcu_lazy* t, const Op& op) {
+    auto data = [](const rcu_lazy* x) { return x ? x->storage->ptr : nullptr; };
+    switch (op.kind) {
+        case ATTENTION: {
+            AttentionArgs a{};
+            a.q = op.q.rows();
+            a.k = op.k.rows();
+            a.v = op.v.rows();
+            a.out = t->storage->ptr;
+            a.H = (int)op.H; a.T = (int)op.T; a.L = (int)op.L; a.D = (int)op.D; a.E = (int)op.E;
+            a.scale32[0] = (const float*)data(op.scale);
+            a.scale16[0] = (const __half*)data(op.scale_q);
+            a.scale16[1] = (const __half*)data(op.scale_k);
+            a.mask = (const __half*)data(op.mask);
+            return rcu_attention_f16(dev, a);
+        }
+        case HEADS:
+            return rcu_heads_half(dev, op.q.rows(), HeadRows{t->storage->ptr, (uint64_t)op.T * op.D, op.D}, op.H, op.T, op.D, op.rope);
+        case APPEND: {
+            rcu_lazy* c = op.srcs[0];
+            rcu_tensor cd = c->desc();
+            if (op.copied) {
+                rcu_tensor sd = op.srcs[1]->desc();
+                return rcu_cache(dev, &cd, &sd, t->u[0], t->u[1], nullptr);
+            }
+            const uint64_t D = c->shape[3];
+            return rcu_heads_half(dev, op.q.rows(), HeadRows{(char*)c->storage->ptr + t->u[1] * D * 2, c->shape[2] * D, D}, op.H, op.T, op.D, op.rope);
+        }
+        case NORM: {
+            const rcu_lazy* n = t->srcs[0];
+            const uint64_t N = t->shape[t->rank - 1];
+            const bool bias = op.srcs.size() > 2 && n->op == RCU_LAYER_NORM;
+            return rcu_norm_half(dev, n->op, data(op.srcs[0]), data(op.srcs[1]), bias ? data(op.srcs[2]) : nullptr, n->f[0], t->storage->ptr, t->numel() / N, N);
+        }
+        case ACT: return rcu_act_half(dev, t->srcs[0]->op, data(op.srcs[0]), t->storage->ptr, t->numel());
+        case GLU: {
+            const uint64_t F = t->shape[t->rank - 1];
+            return rcu_glu_half(dev, t->srcs[1]->srcs[0]->op, data(op.srcs[0]), t->storage->ptr, t->numel() / F, F);
+        }
+        default: return rcu_fail(dev, RCU_ERR_UNSUPPORTED, "resolve: fused op %d", op.kind);
+    }
+}
+
+}  // namespace fusion
