@@ -12,11 +12,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "_obj")
 LIB = os.path.join(HERE, "libratchet_cuda.so")
+GRAPH_LIB = os.path.join(HERE, "_graph.so")          # the Python type over the lazy graph (csrc/pygraph.c): plain C, no CUDA
 CORE_LIB = os.path.join(HERE, "libratchet_cuda_core.so")
 NOT_CORE = {"decode.cu", "comm.cu", "gguf.cu"}
 
@@ -64,7 +66,20 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if force:
         for f in glob.glob(os.path.join(OBJ, "*.o")):
             os.remove(f)
+    build_graph_module()
     return _link(LIB, _sources(), verbose)
+
+
+def build_graph_module() -> str:
+    src = os.path.join(CSRC, "pygraph.c")
+    if _stale(GRAPH_LIB, [src] + _headers()):
+        part = f"{GRAPH_LIB}.{os.getpid()}"
+        cmd = [os.environ.get("CC", "cc"), "-O2", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"], src, "-o", part, "-ldl"]
+        proc = subprocess.run(cmd, capture_output=True, text=True)
+        if proc.returncode != 0:
+            raise RuntimeError(f"{' '.join(cmd)} failed:\n{proc.stdout}\n{proc.stderr}")
+        os.replace(part, GRAPH_LIB)
+    return GRAPH_LIB
 
 
 def _sources(core: bool = False):
@@ -89,6 +104,7 @@ def _link(lib: str, sources, verbose: bool) -> str:
 def ensure_runtime() -> str:
     """Path of a library that is newer than its sources: the full one where it has been built, else the core library,
     built first if need be."""
+    build_graph_module()
     if not _stale(LIB, _sources() + _headers()):
         return LIB
     if _stale(CORE_LIB, _sources(core=True) + _headers()):

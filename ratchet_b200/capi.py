@@ -264,8 +264,18 @@ def lib(path: str = None) -> C.CDLL:
             fn = getattr(handle, name)  # AttributeError here = the library does not export a declared symbol
             fn.restype = res
             fn.argtypes = args
+        graph_module().bind(path)
         _lib = handle
     return _lib
+
+
+def graph_module():
+    """The extension module whose ``Node`` is the base of ``Tensor``, built on the first use in a fresh checkout."""
+    from . import _build
+    if not os.path.exists(_build.GRAPH_LIB):
+        _build.build_graph_module()
+    from . import _graph
+    return _graph
 
 
 def dtype_nbytes(dt: int, numel: int) -> int:

@@ -40,13 +40,27 @@ inline bool permutes(const rcu_lazy* t, uint32_t a, uint32_t b, uint32_t c, uint
 
 struct Pass {
     const rcu_device* dev;
-    std::unordered_map<uint64_t, Op> ops;           // by the id of the node whose result they produce
-    std::unordered_set<uint64_t> passed;            // nodes without a kernel or buffer
+    const Order& order;
+    static constexpr int kPlain = -1, kPassed = -2;
+    std::deque<Op> ops;
+    std::vector<int> role;                          // by position in the order: the op whose result the node is, or no kernel nor buffer (kPassed)
+    std::vector<rcu_lazy*> writers;                 // nodes that write into a tensor which is there already
 
-    bool absorbed(const rcu_lazy* t) const { return passed.count(t->id) != 0; }
+    int role_of(const rcu_lazy* t) const {
+        const uint32_t at = order.at(t);
+        return at == Order::kNone ? kPlain : role[at];
+    }
+    bool absorbed(const rcu_lazy* t) const { return role_of(t) == kPassed; }
     const Op* find(const rcu_lazy* t) const {
-        auto it = ops.find(t->id);
-        return it == ops.end() ? nullptr : &it->second;
+        const int r = role_of(t);
+        return r < 0 ? nullptr : &ops[r];
+    }
+    void pass(const std::vector<rcu_lazy*>& seen) {
+        for (const rcu_lazy* t : seen) role[order.at(t)] = kPassed;
+    }
+    void give(const rcu_lazy* root, Op&& op) {
+        role[order.at(root)] = (int)ops.size();
+        ops.push_back(std::move(op));
     }
 
     // The operand [1, H, T, D] `x` as strides into the tensor behind its permute, view and slice, where these are its own; `seen` receives
@@ -91,13 +105,10 @@ struct Pass {
     }
 
     // caches of this graph that write to the memory of `c`
-    const std::vector<rcu_lazy*>* order;
     int owners(const rcu_lazy* c) const {
         const char *a = (const char*)c->storage->ptr, *b = a + c->nbytes();
         int n = 0;
-        for (const rcu_lazy* t : *order) {
-            if (t->kind != K_CACHE && t->kind != K_INDEX_WRITE) continue;
-            if (t->resolved() || !t->srcs[0]->resolved()) continue;
+        for (const rcu_lazy* t : writers) {
             const char* p = (const char*)t->srcs[0]->storage->ptr;
             if (p < b && p + t->srcs[0]->nbytes() > a) ++n;
         }
@@ -190,8 +201,8 @@ struct Pass {
             op.srcs.push_back(t);                    // runs before the attention; holds no buffer
             append(t);
         }
-        for (rcu_lazy* t : seen) passed.insert(t->id);
-        ops.emplace(root->id, std::move(op));
+        pass(seen);
+        give(root, std::move(op));
         return true;
     }
 
@@ -225,8 +236,8 @@ struct Pass {
         if (!rotated(root, &op, &seen) || !free_of(seen)) return false;
         op.kind = HEADS;
         op.srcs = {op.q.base};
-        for (rcu_lazy* t : seen) passed.insert(t->id);
-        ops.emplace(root->id, std::move(op));
+        pass(seen);
+        give(root, std::move(op));
         return true;
     }
 
@@ -252,7 +263,7 @@ struct Pass {
             direct = direct && free_of(seen);
         }
         if (direct) {
-            for (rcu_lazy* s : seen) passed.insert(s->id);
+            pass(seen);
             op.srcs = {t->srcs[0], op.q.base};
         } else {
             op = Op{};
@@ -260,7 +271,7 @@ struct Pass {
             op.copied = true;
             op.srcs = {t->srcs[0], x};
         }
-        ops.emplace(t->id, std::move(op));
+        give(t, std::move(op));
     }
 
     // cast(op(cast x)) of an f16 tensor: the op, null if it is another graph
@@ -288,8 +299,8 @@ struct Pass {
         op.kind = NORM;
         op.srcs = t->srcs;
         op.srcs[0] = seen[1]->srcs[0];
-        for (rcu_lazy* s : seen) passed.insert(s->id);
-        ops.emplace(root->id, std::move(op));
+        pass(seen);
+        give(root, std::move(op));
         return true;
     }
 
@@ -300,8 +311,8 @@ struct Pass {
         Op op;
         op.kind = ACT;
         op.srcs = {seen[1]->srcs[0]};
-        for (rcu_lazy* s : seen) passed.insert(s->id);
-        ops.emplace(root->id, std::move(op));
+        pass(seen);
+        give(root, std::move(op));
         return true;
     }
 
@@ -326,15 +337,18 @@ struct Pass {
         Op op;
         op.kind = GLU;
         op.srcs = {up->srcs[0]};
-        for (rcu_lazy* s : seen) passed.insert(s->id);
-        ops.emplace(root->id, std::move(op));
+        pass(seen);
+        give(root, std::move(op));
         return true;
     }
 
     // consumers before what they consume, so that a chain is recognised from its end
-    Pass(const rcu_device* d, const std::vector<rcu_lazy*>& o) : dev(d), order(&o) {
-        for (size_t i = o.size(); i-- > 0;) {
-            rcu_lazy* t = o[i];
+    Pass(const rcu_device* d, const Order& o, bool on) : dev(d), order(o), role(o.nodes.size(), kPlain) {
+        if (!on) return;
+        for (rcu_lazy* t : o.nodes)
+            if ((t->kind == K_CACHE || t->kind == K_INDEX_WRITE) && !t->resolved() && t->srcs[0]->resolved()) writers.push_back(t);
+        for (size_t i = o.nodes.size(); i-- > 0;) {
+            rcu_lazy* t = o.nodes[i];
             if (t->resolved() || absorbed(t) || find(t)) continue;
             if (t->kind == K_PERMUTE) attention(t);
             else if (t->kind == K_CAST) heads(t) || norm(t) || act(t);
