@@ -20,3 +20,13 @@ struct AttentionArgs {
 // RCU_ERR_UNSUPPORTED: sizes or alignments the kernel does not take (nothing has been launched)
 rcu_status rcu_attention_f16(rcu_device* dev, const AttentionArgs& a);
 bool rcu_attention_f16_takes(const rcu_device* dev, const AttentionArgs& a);
+
+// The same in f32, the factors of queries and keys as f32 tensors of one element
+struct Attention32Args {
+    HeadRows q, k, v;
+    void* out;                      // [T, H, E] f32
+    int H, T, L, D, E;
+    const float* scale[2];          // nullable
+};
+rcu_status rcu_attention_f32(rcu_device* dev, const Attention32Args& a);
+bool rcu_attention_f32_takes(const rcu_device* dev, const Attention32Args& a);

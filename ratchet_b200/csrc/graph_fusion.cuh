@@ -1,10 +1,11 @@
-// Subgraphs of an f16 prompt that the resolver runs as one kernel (included by graph.cu).
+// Subgraphs of a prompt that the resolver runs as one kernel (included by graph.cu).
 //
 // Only nodes that nothing outside the graph holds, and that a single op consumes, are passed over: they get no buffer and no kernel.
 // What is recognised (T > 1 positions; single tokens keep one kernel per op):
 //   attention    permute(softmax(f32(scores [+ mask])) v), scores = f16(scale * f32(q) f32(k)^T) with keys and values that a cache returns or
 //                that are given (phi3/attn.rs:119-157), or (dk q)(dk k^T) in f16 (whisper/mha.rs:92-127); permutes of views of
 //                q, k and v become strides, and a cache that only feeds the attention is appended to but not copied out
+//   attention32  permute(softmax((dk q)(dk k)^T) v) in f32 (the same with f32 activations, whose casts are no nodes)
 //   heads        cast(rope(cast(permute(view(slice))))), and permute(view(slice)) in front of a cache: straight into the cache's rows
 //   norm         cast(norm(cast x));   act: cast(gelu or silu(cast x));   glu: up * cast(silu(cast gate)) of the halves of one tensor
 // A subgraph whose sizes or alignment a kernel does not take stays as it is.
@@ -12,7 +13,7 @@
 
 namespace fusion {
 
-enum Kind { NONE = 0, ATTENTION, HEADS, APPEND, NORM, ACT, GLU };
+enum Kind { NONE = 0, ATTENTION, ATTENTION32, HEADS, APPEND, NORM, ACT, GLU };
 
 // element (position t, head h, feature d) of a [1, heads, T, D] operand at base[offset + h * head + t * row + d]
 struct Heads {
@@ -65,19 +66,19 @@ struct Pass {
 
     // The operand [1, H, T, D] `x` as strides into the tensor behind its permute, view and slice, where these are its own; `seen` receives
     // the nodes passed over.  time_last: x is [1, H, D, T].
-    static Heads strides(rcu_lazy* x, bool time_last, std::vector<rcu_lazy*>* seen) {
+    static Heads strides(rcu_lazy* x, bool time_last, std::vector<rcu_lazy*>* seen, int32_t dt = RCU_F16) {
         const uint64_t H = x->shape[1], T = x->shape[time_last ? 3 : 2], D = x->shape[time_last ? 2 : 3];
-        const bool perm = inner(x, K_PERMUTE, RCU_F16) && (time_last ? permutes(x, 0, 2, 3, 1) : permutes(x, 0, 2, 1, 3));
+        const bool perm = inner(x, K_PERMUTE, dt) && (time_last ? permutes(x, 0, 2, 3, 1) : permutes(x, 0, 2, 1, 3));
         if (!perm) {
             if (time_last) return Heads{};
             return Heads{x, 0, T * D, D};
         }
         rcu_lazy* y = x->srcs[0];                    // [1, T, H, D]
         seen->push_back(x);
-        if (!inner(y, K_VIEW, RCU_F16)) return Heads{y, 0, D, H * D};
+        if (!inner(y, K_VIEW, dt)) return Heads{y, 0, D, H * D};
         rcu_lazy* z = y->srcs[0];
         seen->push_back(y);
-        if (inner(z, K_SLICE, RCU_F16) && z->rank == 3 && z->shape[0] == 1 && z->shape[1] == T && z->shape[2] == H * D) {
+        if (inner(z, K_SLICE, dt) && z->rank == 3 && z->shape[0] == 1 && z->shape[1] == T && z->shape[2] == H * D) {
             rcu_lazy* w = z->srcs[0];
             if (w->rank == 3 && w->shape[0] == 1 && w->shape[1] == T && z->a[0] == 0 && z->a[1] == 0) {
                 seen->push_back(z);
@@ -204,6 +205,62 @@ struct Pass {
         pass(seen);
         give(root, std::move(op));
         return true;
+    }
+
+    // the same in f32, without casts, mask or cache
+    bool attention32(rcu_lazy* root) {
+        if (root->dt != RCU_F32 || root->rank != 4 || !permutes(root, 0, 2, 1, 3) || root->shape[0] != 1) return false;
+        std::vector<rcu_lazy*> seen;
+        auto product = [&](rcu_lazy* t) { return inner(t, K_MATMUL, RCU_F32) && t->srcs.size() == 2 && !t->flags[0] && !t->flags[1] && !t->flags[2]; };
+        rcu_lazy* pv = root->srcs[0];
+        if (!product(pv)) return false;
+        rcu_lazy *w = pv->srcs[0], *v = pv->srcs[1];
+        if (!inner(w, K_SOFTMAX, RCU_F32) || w->u[0] != 3 || w->rank != 4 || w->shape[0] != 1) return false;
+        rcu_lazy* z = w->srcs[0];
+        if (!product(z)) return false;
+        seen.insert(seen.end(), {pv, w, z});
+        Op op;
+        op.kind = ATTENTION32;
+        const uint64_t H = w->shape[1], T = w->shape[2], L = w->shape[3];
+        if (H > 65535 || T > 0x7fffffffull || L > 0x7fffffffull) return false;
+        op.H = (uint32_t)H;
+        op.T = (uint32_t)T;
+        op.L = (uint32_t)L;
+        rcu_lazy* side[2] = {z->srcs[0], z->srcs[1]};
+        for (int i = 0; i < 2; ++i) {
+            rcu_lazy* t = side[i];
+            if (!inner(t, K_BINARY, RCU_F32) || t->op != RCU_MUL || t->rank != 4 || t->srcs[1]->numel() != 1 || t->srcs[1]->dt != RCU_F32 || t->srcs[0]->rank != 4)
+                return false;
+            (i ? op.scale_k : op.scale_q) = t->srcs[1];
+            side[i] = t->srcs[0];
+            seen.push_back(t);
+        }
+        rcu_lazy *q = side[0], *k = side[1];
+        if (q->shape[0] != 1 || q->shape[1] != H || q->shape[2] != T || k->shape[0] != 1 || k->shape[1] != H || k->shape[3] != L || k->shape[2] != q->shape[3] ||
+            v->dt != RCU_F32 || v->rank != 4 || v->shape[0] != 1 || v->shape[1] != H || v->shape[2] != L || q->shape[3] > 64 || v->shape[3] > 64)
+            return false;
+        op.D = (uint32_t)q->shape[3];
+        op.E = (uint32_t)v->shape[3];
+        op.q = strides(q, false, &seen, RCU_F32);
+        op.k = strides(k, true, &seen, RCU_F32);
+        op.v = strides(v, false, &seen, RCU_F32);
+        for (const Heads* h : {&op.q, &op.k, &op.v})
+            if (!h->base || h->offset % 4 || !aligned(h->base)) return false;
+        if (!rcu_attention_f32_takes(dev, args32(op)) || !free_of(seen)) return false;
+        op.srcs = {op.q.base, op.k.base, op.v.base, op.scale_q, op.scale_k};
+        pass(seen);
+        give(root, std::move(op));
+        return true;
+    }
+
+    // sizes and pitches; no addresses
+    static Attention32Args args32(const Op& op) {
+        Attention32Args a{};
+        a.q = HeadRows{nullptr, op.q.head, op.q.row};
+        a.k = HeadRows{nullptr, op.k.head, op.k.row};
+        a.v = HeadRows{nullptr, op.v.head, op.v.row};
+        a.H = (int)op.H; a.T = (int)op.T; a.L = (int)op.L; a.D = (int)op.D; a.E = (int)op.E;
+        return a;
     }
 
     // q or k behind its slice, view, permute and rope, from the node that casts back to f16
@@ -350,7 +407,7 @@ struct Pass {
         for (size_t i = o.nodes.size(); i-- > 0;) {
             rcu_lazy* t = o.nodes[i];
             if (t->resolved() || absorbed(t) || find(t)) continue;
-            if (t->kind == K_PERMUTE) attention(t);
+            if (t->kind == K_PERMUTE) attention(t) || attention32(t);
             else if (t->kind == K_CAST) heads(t) || norm(t) || act(t);
             else if (t->kind == K_BINARY) glu(t);
         }
@@ -358,7 +415,7 @@ struct Pass {
 };
 
 inline const char* name_of(Kind k) {
-    static const char* names[] = {"", "attention", "heads", "cache", "norm chain", "act chain", "glu chain"};
+    static const char* names[] = {"", "attention", "attention", "heads", "cache", "norm chain", "act chain", "glu chain"};
     return names[k];
 }
 
@@ -377,6 +434,17 @@ rcu_status run(rcu_device* dev, rcu_lazy* t, const Op& op) {
             a.scale16[1] = (const __half*)data(op.scale_k);
             a.mask = (const __half*)data(op.mask);
             return rcu_attention_f16(dev, a);
+        }
+        case ATTENTION32: {
+            Attention32Args a = Pass::args32(op);
+            auto at = [&](HeadRows& r, const Heads& h) { r.data = (const float*)h.base->storage->ptr + h.offset; };
+            at(a.q, op.q);
+            at(a.k, op.k);
+            at(a.v, op.v);
+            a.out = t->storage->ptr;
+            a.scale[0] = (const float*)data(op.scale_q);
+            a.scale[1] = (const float*)data(op.scale_k);
+            return rcu_attention_f32(dev, a);
         }
         case HEADS:
             return rcu_heads_half(dev, op.q.rows(), HeadRows{t->storage->ptr, (uint64_t)op.T * op.D, op.D}, op.H, op.T, op.D, op.rope);
