@@ -199,8 +199,6 @@ attention_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant
                 const unsigned char* line = ms + (2 * b + w) * kBlockQ + rw * 128;
 #pragma unroll
                 for (int c = 0; c < 8; ++c) mv[c] = *reinterpret_cast<const uint4*>(line + ((c ^ (rw & 7)) << 4));
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&m_empty[b]);
             }
             ok = __all_sync(0xffffffffu, mbar_wait_spin(&s_full[w][b], (n >> 1) & 1, &abort_flag, a.status));
             if (!ok) break;
@@ -267,7 +265,13 @@ attention_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant
             tmem_st_32x32(t + 64 * b, pw);
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&p_full[w][b]);
+            if (lane == 0) {
+                mbar_arrive(&p_full[w][b]);
+                // The mask's piece is given back here and not behind its loads: the weights stored above depend on every value of it, so the
+                // loads are over.  Given back at once, a piece was now and then replaced before the last warps had it (a load needs nothing
+                // but its own value to wait for): keys of one 16-byte chunk lost their weight in 1 to 5 % of the passes over 199 positions.
+                if (MASK) mbar_arrive(&m_empty[b]);
+            }
         }
         if (ok) {
             ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[w], (tiles - 1) & 1, &abort_flag, a.status));
