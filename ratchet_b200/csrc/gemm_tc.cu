@@ -55,10 +55,10 @@ __host__ __device__ constexpr int conv_warps(int bn) { return bn >= 128 ? 8 : 4;
 
 // Two CTAs share an SM (half of its shared memory and at most half of its tensor memory each), so one
 // CTA's pipeline fill and epilogue overlap the other's main loop.
-template <int BN, int WK, int STAGES, class Out, bool RAGGED>
+template <int BN, int WK, int STAGES, class Out, int MODE>
 __global__ void __launch_bounds__(WK == WK_F16 ? kThreadsTc : kThreadsTc + conv_warps(BN) * 32, 2)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const QuantArgs qa,
-               const GemmEpilogue<Out, RAGGED> epi, Out* out, int M, int N, int K, int* status, int splits, float* __restrict__ partial, uint32_t idesc) {
+               const GemmEpilogue<Out, MODE> epi, Out* out, int M, int N, int K, int* status, int splits, float* __restrict__ partial, uint32_t idesc) {
     rcu_kernel_entry_wait_only();
     constexpr int A_BYTES = TM * TK * 2;          // 16 KiB
     constexpr int B_BYTES = BN * TK * 2;
@@ -162,15 +162,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
                 const int col = n0 + c + (lane & 7) * 4;
                 const bool in = col < N, whole = splits == 1;      // not whole: a K slice leaves f32 partial sums, the summing kernel does the rest
                 const float4 bias = in && whole ? epi.bias4(col, N) : make_float4(0.f, 0.f, 0.f, 0.f);
-                float4 resid[8];
+                typename GemmEpilogue<Out, MODE>::Resid resid[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const int row = row0 + 4 * i + r;
-                    resid[i] = sizeof(Out) == 4 && whole && epi.resid && in && row < M ? *reinterpret_cast<const float4*>(epi.resid + (size_t)row * N + col)
-                                                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+                    resid[i] = epi.resid4((size_t)row * N + col, whole && in && row < M);
                 }
+                const uint32_t at = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c;
                 float v[32];
-                tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c, v);
+                tmem_ld_32x32(at, v);
                 turn_piece(turn, v, [&](int i, int piece_row, const float4& x) {
                     const int row = row0 + piece_row;
                     if (!in || row >= M) return;
@@ -318,8 +318,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
 }
 
 // out[m, n] = epilogue(sum over slices, in order, of partial[s, m, n]); eight outputs per thread
-template <class Out>
-__global__ void __launch_bounds__(256) sum_k_slices_kernel(const float* __restrict__ partial, const GemmEpilogue<Out> epi, Out* out, size_t MN, int N,
+template <class Out, int MODE>
+__global__ void __launch_bounds__(256) sum_k_slices_kernel(const float* __restrict__ partial, const GemmEpilogue<Out, MODE> epi, Out* out, size_t MN, int N,
                                                           int splits) {
     rcu_kernel_entry();
     const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
@@ -335,13 +335,13 @@ __global__ void __launch_bounds__(256) sum_k_slices_kernel(const float* __restri
     epi.store8(out, i, acc, (int)(i % (size_t)N));
 }
 
-template <int BN, int WK, class Out = __half, bool RAGGED = false>
-rcu_status launch_tc(rcu_device* dev, const CUtensorMap& xmap, const CUtensorMap& wmap, const QuantArgs& qa, const GemmEpilogue<Out, RAGGED>& epi, void* out,
+template <int BN, int WK, class Out = __half, int MODE = EPI_PLAIN>
+rcu_status launch_tc(rcu_device* dev, const CUtensorMap& xmap, const CUtensorMap& wmap, const QuantArgs& qa, const GemmEpilogue<Out, MODE>& epi, void* out,
                      int M, int N, int K, int batch = 1, bool bf16 = false) {
     constexpr int STAGE = TM * TK * 2 + BN * TK * 2;
     constexpr int STAGES = (100 * 1024) / STAGE;     // two CTAs per SM
     const size_t smem = (size_t)STAGES * STAGE + 1024 + 512;
-    auto kern = gemm_tc_kernel<BN, WK, STAGES, Out, RAGGED>;
+    auto kern = gemm_tc_kernel<BN, WK, STAGES, Out, MODE>;
     RCU_CUDA(dev, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const uint32_t idesc = umma_idesc_f16(TM, BN, bf16);
     dim3 grid((N + BN - 1) / BN, (M + TM - 1) / TM, batch);
@@ -355,17 +355,17 @@ rcu_status launch_tc(rcu_device* dev, const CUtensorMap& xmap, const CUtensorMap
         splits = (int)std::min<long long>(4, (2ll * dev->sm_count) / tiles);
         while (splits > 1 && (((nk + splits - 1) / splits + 3) & ~3) * (splits - 1) >= nk) --splits;     // every slice gets k-steps
     }
-    if constexpr (!RAGGED) {           // slices need N % 8 == 0
+    if constexpr (MODE != EPI_RAGGED) {           // slices need N % 8 == 0
         if (splits > 1) {
             void* partial = nullptr;
             rcu_status st = rcu_alloc(dev, (uint64_t)splits * M * N * 4, &partial);
             if (st != RCU_OK) return st;
             grid.z = splits;
-            rcu_launch(dev, kern, grid, threads, smem, xmap, wmap, qa, GemmEpilogue<Out>{nullptr, nullptr, 1.f, 0}, (Out*)out, M, N, K, dev->d_status, splits,
+            rcu_launch(dev, kern, grid, threads, smem, xmap, wmap, qa, GemmEpilogue<Out, MODE>{nullptr, nullptr, 1.f, 0}, (Out*)out, M, N, K, dev->d_status, splits,
                        (float*)partial, idesc);
             dev->launches++;
             const size_t MN = (size_t)M * N;
-            rcu_launch(dev, sum_k_slices_kernel<Out>, (unsigned)((MN / 8 + 255) / 256), 256, 0, (const float*)partial, epi, (Out*)out, MN, N, splits);
+            rcu_launch(dev, sum_k_slices_kernel<Out, MODE>, (unsigned)((MN / 8 + 255) / 256), 256, 0, (const float*)partial, epi, (Out*)out, MN, N, splits);
             rcu_free(dev, partial);      // the pool reuses blocks in stream order
             RCU_LAUNCH_CHECK(dev);
             return RCU_OK;
@@ -407,18 +407,31 @@ bool rcu_gemm_tc2_eligible(rcu_device* dev, uint64_t M, uint64_t N, uint64_t K);
 rcu_status rcu_gemm_tc2_launch(rcu_device* dev, const void* w, const void* x, const void* bias, void* y, uint64_t M, uint64_t N, uint64_t K,
                                const TcLinear& t);
 
+// Beyond this many token rows quantised weights are converted once per product (below)
+constexpr uint64_t kFusedMaxM = 256;
+
+// The Linear of an f16 graph with what follows it (TcLinear: chained, or glu): whether the tensor-core kernels take it.  A gate and its up
+// columns meet in one tile of the pair kernel only, so that form wants f16 weights, or as many rows as have them converted.  An activation
+// is left to that kernel too, whose epilogues run behind the next tile's products: in the one-CTA kernel four warps work it out with nothing
+// to hide it (501 x 1536 x 384 with gelu: 17.1 us, the product and act_half_kernel 7.7 + 3.6).
+bool rcu_gemm_tc_chain_takes(rcu_device* dev, int w_dt, uint64_t M, uint64_t N, uint64_t K, bool glu, bool act) {
+    if (w_dt == RCU_BF16) return glu && N % 16 == 0 && rcu_gemm_tc2_eligible(dev, M, N, K) && M <= 0x7fffffffull && N <= 0x7fffffffull && K <= 0x7fffffffull;
+    if (!rcu_gemm_tc_eligible(w_dt, RCU_F16, M, N, K) || N % 8 != 0) return false;
+    if (!glu && !act) return M > 32;               // fewer rows: gemm_rows.cu
+    return N % 16 == 0 && (w_dt == RCU_F16 || M > kFusedMaxM) && rcu_gemm_tc2_eligible(dev, M, N, K);
+}
+
 rcu_status rcu_gemm_tc_dispatch(rcu_device* dev, int lhs_dt, const void* w, int act_dt, const void* x, const void* bias, void* y,
-                                uint64_t M, uint64_t N, uint64_t K) {
+                                uint64_t M, uint64_t N, uint64_t K, const TcLinear& t) {
     if (!rcu_gemm_tc_eligible(lhs_dt, act_dt, M, N, K)) return RCU_ERR_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(w)) & 15) return RCU_ERR_UNSUPPORTED;
     DevGuard g(dev->ordinal);
-    if (lhs_dt == RCU_F16 && rcu_gemm_tc2_eligible(dev, M, N, K)) return rcu_gemm_tc2_launch(dev, w, x, bias, y, M, N, K, TcLinear{});
+    if (lhs_dt == RCU_F16 && rcu_gemm_tc2_eligible(dev, M, N, K)) return rcu_gemm_tc2_launch(dev, w, x, bias, y, M, N, K, t);
     // Quantised weights.  The fused kernel converts a weight tile once per 128-row token tile, i.e.
     // M/128 times over the whole problem, and it is the one-CTA kernel.  Beyond kFusedMaxM token rows it
     // is cheaper to convert the matrix once into pooled f16 scratch (which stays in L2) and run the f16
     // kernels on it (M = 512, N = 8192, K = 3072, Q4_K: 34 us against 46 us fused).  RCU_GEMM_FUSED=0/1
     // forces either path.
-    constexpr uint64_t kFusedMaxM = 256;
     if (lhs_dt != RCU_F16) {
         const char* force = getenv("RCU_GEMM_FUSED");
         const bool fused = force ? atoi(force) != 0 : M <= kFusedMaxM;
@@ -429,7 +442,7 @@ rcu_status rcu_gemm_tc_dispatch(rcu_device* dev, int lhs_dt, const void* w, int 
             rcu_tensor src{lhs_dt, 2, {N, K, 1, 1}, const_cast<void*>(w)};
             rcu_tensor dst{RCU_F16, 2, {N, K, 1, 1}, scratch};
             st = rcu_dequantize(dev, &src, &dst);
-            if (st == RCU_OK) st = rcu_gemm_tc_dispatch(dev, RCU_F16, scratch, act_dt, x, bias, y, M, N, K);
+            if (st == RCU_OK) st = rcu_gemm_tc_dispatch(dev, RCU_F16, scratch, act_dt, x, bias, y, M, N, K, t);
             rcu_free(dev, scratch);   // the pool reuses blocks in stream order
             return st;
         }
@@ -467,8 +480,9 @@ rcu_status rcu_gemm_tc_dispatch(rcu_device* dev, int lhs_dt, const void* w, int 
     if (!maps)
         st = rcu_fail(dev, RCU_ERR_CUDA, "gemm_tc: cuTensorMapEncodeTiled failed (M=%llu N=%llu K=%llu)", (unsigned long long)M,
                       (unsigned long long)N, (unsigned long long)K);
+    const GemmEpilogue<__half, EPI_RESID> added{(const __half*)bias, nullptr, 1.f, {}, t.bias32, (const __half*)t.resid16, -1};
 #define RCU_TC(BN_, WK_)                                                                                                                                  \
-    (N & 3 ? launch_tc<BN_, WK_, __half, true>(dev, xmap, wmap, qa, GemmEpilogue<__half, true>{(const __half*)bias, nullptr, 1.f, 0}, y, (int)M, (int)N, (int)K) \
+    (t.chained() ? launch_tc<BN_, WK_, __half, EPI_RESID>(dev, xmap, wmap, qa, added, y, (int)M, (int)N, (int)K) : N & 3 ? launch_tc<BN_, WK_, __half, EPI_RAGGED>(dev, xmap, wmap, qa, GemmEpilogue<__half, EPI_RAGGED>{(const __half*)bias, nullptr, 1.f, 0}, y, (int)M, (int)N, (int)K) \
            : launch_tc<BN_, WK_>(dev, xmap, wmap, qa, GemmEpilogue<__half>{(const __half*)bias, nullptr, 1.f, 0}, y, (int)M, (int)N, (int)K))
     if (st == RCU_OK) {
         if (wk == WK_F16) st = bn == 256 ? RCU_TC(256, WK_F16) : bn == 128 ? RCU_TC(128, WK_F16) : RCU_TC(64, WK_F16);
@@ -497,9 +511,9 @@ rcu_status rcu_gemm_tc_batched_f16(rcu_device* dev, const void* w, const void* x
                         (unsigned long long)N, (unsigned long long)K);
     QuantArgs qa{nullptr, nullptr, nullptr};
     const GemmEpilogue<__half> epi{nullptr, nullptr, 1.f, 0};
-    const GemmEpilogue<__half, true> ragged{nullptr, nullptr, 1.f, 0};
+    const GemmEpilogue<__half, EPI_RAGGED> ragged{nullptr, nullptr, 1.f, 0};
     const int m = (int)M, n = (int)N, k = (int)K, b = (int)batch;
-    if (N & 3) return bn == 128 ? launch_tc<128, WK_F16, __half, true>(dev, xmap, wmap, qa, ragged, y, m, n, k, b) : launch_tc<64, WK_F16, __half, true>(dev, xmap, wmap, qa, ragged, y, m, n, k, b);
+    if (N & 3) return bn == 128 ? launch_tc<128, WK_F16, __half, EPI_RAGGED>(dev, xmap, wmap, qa, ragged, y, m, n, k, b) : launch_tc<64, WK_F16, __half, EPI_RAGGED>(dev, xmap, wmap, qa, ragged, y, m, n, k, b);
     return bn == 128 ? launch_tc<128, WK_F16>(dev, xmap, wmap, qa, epi, y, m, n, k, b) : launch_tc<64, WK_F16>(dev, xmap, wmap, qa, epi, y, m, n, k, b);
 }
 
@@ -528,4 +542,27 @@ rcu_status rcu_gemm_tc_linear(rcu_device* dev, const void* w, const void* x, con
     if (t.out_dt == RCU_BF16) return RCU_TC(__nv_bfloat16, (GemmEpilogue<__nv_bfloat16>{(const __nv_bfloat16*)bias, nullptr, 1.f, t.act}));
     return RCU_TC(__half, (GemmEpilogue<__half>{(const __half*)bias, nullptr, 1.f, t.act}));
 #undef RCU_TC
+}
+
+rcu_status rcu_gemm_tc_dispatch(rcu_device* dev, int lhs_dt, const void* w, int act_dt, const void* x, const void* bias, void* y, uint64_t M, uint64_t N, uint64_t K) {
+    return rcu_gemm_tc_dispatch(dev, lhs_dt, w, act_dt, x, bias, y, M, N, K, TcLinear{});
+}
+
+rcu_status rcu_gemm_tc_chain(rcu_device* dev, int w_dt, const void* w, const void* x, void* y, uint64_t M, uint64_t N, uint64_t K, const LinearChain& c) {
+    if (!rcu_gemm_tc_chain_takes(dev, w_dt, M, N, K, c.glu >= 0, c.op >= 0)) return RCU_ERR_UNSUPPORTED;
+    if ((c.glu >= 0 && (c.bias || c.bias32 || c.resid || c.op >= 0)) || (c.op >= 0 && c.resid)) return RCU_ERR_UNSUPPORTED;
+    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(c.resid)) & 15) return RCU_ERR_UNSUPPORTED;
+    DevGuard g(dev->ordinal);
+    TcLinear t;
+    t.bias32 = c.bias32;
+    t.resid16 = c.resid;
+    t.chain_op = c.op;
+    t.glu = c.glu;
+    if (w_dt == RCU_BF16) {
+        t.bf16 = true;
+        t.out_dt = RCU_BF16;
+        t.x_pitch = c.x_pitch;
+        return t.x_pitch % 8 ? RCU_ERR_UNSUPPORTED : rcu_gemm_tc2_launch(dev, w, x, nullptr, y, M, N, K, t);
+    }
+    return rcu_gemm_tc_dispatch(dev, w_dt, w, RCU_F16, x, c.bias, y, M, N, K, t);
 }

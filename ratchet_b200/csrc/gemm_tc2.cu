@@ -27,6 +27,9 @@
 // memory is freed, so neither touches the other's shared memory after it has exited.
 #include <cuda.h>
 
+#include <type_traits>
+
+#include "lm_math.cuh"
 #include "tc_common.cuh"
 
 namespace {
@@ -80,10 +83,22 @@ __device__ __forceinline__ void umma2_commit_both(uint64_t* bar) {
                  : "memory");
 }
 
-template <class Out, bool RAGGED>
+// glu_value: a gate and an up value as the graph's own kernels have them - f16: half_chains.cu (silu rounded before the product),
+// bf16: glu_kernel of stream_ops.cu
+template <class Out> __device__ __forceinline__ float glu_value(int act, float gate, float up) {
+    gate = rnd<Out>(gate);
+    up = rnd<Out>(up);
+    if constexpr (std::is_same<Out, __half>::value) return up * rnd<Out>(chain_act(act, gate));
+    else return (act == RCU_GELU ? lm::gelu_tanh(gate) : lm::silu(gate)) * up;
+}
+
+// GLU: W holds N gate rows, then N up rows; a tile's first CTA brings 128 gate rows, the second their up rows, and the output tile is 128
+// columns wide.  Written separately, the product and its gate cost 55 MB of traffic more at 1000 x 2 x 8192 (12.9 us of the kernel that read
+// it), 185 MB at 4096 x 2 x 5632 (33.9 us).
+template <class Out, int MODE, bool GLU>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads2, 1)
-gemm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const GemmEpilogue<Out, RAGGED> epi,
-                Out* out, int M, int N, int K, int tiles_m, int n_tiles, int* status, uint32_t idesc) {
+gemm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const GemmEpilogue<Out, MODE> epi,
+                Out* out, int M, int N, int K, int tiles_m, int n_tiles, int* status, uint32_t idesc, int glu_act) {
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages2 * kStageBytes2);   // leader's are the ones in use
@@ -118,6 +133,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
     tc_fence_before();
     cluster_sync_all();            // barriers of both CTAs initialised before anyone signals them
     tc_fence_after();
+    rcu_kernel_entry_wait_only();  // nothing before this touches global memory: the set-up overlaps the kernel before
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
@@ -126,7 +142,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
             bool ok = true;
             for (int t = pair; t < n_tiles && ok; t += n_pairs) {
                 const int m0 = (t % tiles_m) * 2 * TM + (int)rank * TM;
-                const int n0 = (t / tiles_m) * kTileN2 + (int)rank * (kTileN2 / 2);
+                const int n0 = GLU ? (t / tiles_m) * (kTileN2 / 2) + (int)rank * N : (t / tiles_m) * kTileN2 + (int)rank * (kTileN2 / 2);
                 for (int k = 0; k < nk; ++k, ++it) {
                     const int s = it % kStages2;
                     if (it >= kStages2 && !mbar_wait(&empty[s], ((it / kStages2) - 1) & 1, abort_flag, status)) { ok = false; break; }
@@ -181,27 +197,65 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
             if (!ok) break;
             tc_fence_after();
             const int row0 = (t % tiles_m) * 2 * TM + (int)rank * TM + q * 32;
-            const int n0 = (t / tiles_m) * kTileN2;
+            const int n0 = (t / tiles_m) * (GLU ? kTileN2 / 2 : kTileN2);
             float4* mine = turn[warp - 2];
             const int r = lane >> 3, quad = lane & 7;
+            if constexpr (GLU) {
+#pragma unroll 1
+                for (int c = c0 / 2; c < c0 / 2 + kTileN2 / 4; c += 32) {
+                    const int col = n0 + c + quad * 4;
+                    const uint32_t at = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * kAccCols + c);
+                    turn_piece8(
+                        mine,
+                        [&](int c8, float* v) {
+                            float u[8];
+                            tmem_ld_32x8(at + 8 * c8, v);
+                            tmem_ld_32x8(at + kTileN2 / 2 + 8 * c8, u);
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) v[e] = glu_value<Out>(glu_act, v[e], u[e]);
+                        },
+                        [&](int i, int piece_row, const float4& x) {
+                            const int row = row0 + piece_row;
+                            if (col >= N || row >= M) return;
+                            typename GemmEpilogue<Out, MODE>::Quad o;
+                            o.v[0] = from_f32<Out>(x.x);
+                            o.v[1] = from_f32<Out>(x.y);
+                            o.v[2] = from_f32<Out>(x.z);
+                            o.v[3] = from_f32<Out>(x.w);
+                            *reinterpret_cast<decltype(o)*>(out + (size_t)row * N + col) = o;
+                        });
+                }
+            } else {
 #pragma unroll 1
             for (int c = c0; c < c0 + kTileN2 / 2; c += 32) {
                 const int col = n0 + c + quad * 4;
                 const bool in = col < N;
                 const float4 bias = in ? epi.bias4(col, N) : make_float4(0.f, 0.f, 0.f, 0.f);
-                float4 resid[8];
+                typename GemmEpilogue<Out, MODE>::Resid resid[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const int row = row0 + 4 * i + r;
-                    resid[i] = sizeof(Out) == 4 && epi.resid && in && row < M ? *reinterpret_cast<const float4*>(epi.resid + (size_t)row * N + col)
-                                                                             : make_float4(0.f, 0.f, 0.f, 0.f);
+                    resid[i] = epi.resid4((size_t)row * N + col, in && row < M);
                 }
-                float v[32];
-                tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * kAccCols + c), v);
-                turn_piece(mine, v, [&](int i, int piece_row, const float4& x) {
+                const uint32_t at = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * kAccCols + c);
+                auto put = [&](int i, int piece_row, const float4& x) {
                     const int row = row0 + piece_row;
                     if (in && row < M) epi.store4(out, (size_t)row * N + col, x, bias, resid[i], col, N);
-                });
+                };
+                if constexpr (MODE == EPI_ACT) {
+                    turn_piece8(
+                        mine,
+                        [&](int c8, float* v) {
+                            tmem_ld_32x8(at + 8 * c8, v);
+                            epi.finish8(v, n0 + c + 8 * c8, N);
+                        },
+                        put);
+                } else {
+                    float v[32];
+                    tmem_ld_32x32(at, v);
+                    turn_piece(mine, v, put);
+                }
+            }
             }
             // this warp has read its part of the buffer: tell the leader's MMA thread
             tc_fence_before();
@@ -240,16 +294,18 @@ bool rcu_gemm_tc2_eligible(rcu_device* dev, uint64_t M, uint64_t N, uint64_t K) 
 }
 
 namespace {
-template <class Out, bool RAGGED = false>
-rcu_status launch_pair(rcu_device* dev, const CUtensorMap& xmap, const CUtensorMap& wmap, const GemmEpilogue<Out, RAGGED>& epi, void* y, uint64_t M, uint64_t N,
-                       uint64_t K, bool bf16) {
-    const int tiles_m = (int)((M + 255) / 256), tiles_n = (int)((N + 255) / 256);
+// `N`: rows of W; with a gate the output has half as many columns
+template <class Out, int MODE = EPI_PLAIN, bool GLU = false>
+rcu_status launch_pair(rcu_device* dev, const CUtensorMap& xmap, const CUtensorMap& wmap, const GemmEpilogue<Out, MODE>& epi, void* y, uint64_t M, uint64_t N,
+                       uint64_t K, const TcLinear& t) {
+    const int tiles_m = (int)((M + 255) / 256), tiles_n = (int)((N + 255) / 256);      // a tile of gates takes 256 rows of W too
     const int n_tiles = tiles_m * tiles_n;
     const int n_pairs = std::min(n_tiles, dev->sm_count / 2);
     const size_t smem = (size_t)kStages2 * kStageBytes2 + 1024 + 256;
-    RCU_CUDA(dev, cudaFuncSetAttribute(gemm_tc2_kernel<Out, RAGGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    gemm_tc2_kernel<Out, RAGGED><<<2 * n_pairs, kThreads2, smem, dev->stream>>>(xmap, wmap, epi, (Out*)y, (int)M, (int)N, (int)K, tiles_m, n_tiles,
-                                                                       dev->d_status, umma_idesc_f16(2 * TM, kTileN2, bf16));
+    auto kern = gemm_tc2_kernel<Out, MODE, GLU>;
+    RCU_CUDA(dev, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    RCU_CUDA(dev, rcu_launch(dev, kern, 2 * n_pairs, kThreads2, smem, xmap, wmap, epi, (Out*)y, (int)M, (int)(GLU ? N / 2 : N), (int)K, tiles_m, n_tiles, dev->d_status,
+                             umma_idesc_f16(2 * TM, kTileN2, t.bf16), t.glu));
     RCU_LAUNCH_CHECK(dev);
     return RCU_OK;
 }
@@ -262,9 +318,13 @@ rcu_status rcu_gemm_tc2_launch(rcu_device* dev, const void* w, const void* x, co
         !make_map_f16_sw128_rows(&wmap, w, N, K, kTileN2 / 2, K, t.bf16))
         return rcu_fail(dev, RCU_ERR_CUDA, "gemm_tc2: cuTensorMapEncodeTiled failed (M=%llu N=%llu K=%llu)", (unsigned long long)M,
                         (unsigned long long)N, (unsigned long long)K);
-    if (t.out_dt == RCU_F32) return launch_pair<float>(dev, xmap, wmap, GemmEpilogue<float>{(const float*)bias, t.resid, t.alpha, t.act}, y, M, N, K, t.bf16);
-    if (t.out_dt == RCU_BF16)
-        return launch_pair<__nv_bfloat16>(dev, xmap, wmap, GemmEpilogue<__nv_bfloat16>{(const __nv_bfloat16*)bias, nullptr, 1.f, t.act}, y, M, N, K, t.bf16);
-    if (N & 3) return launch_pair<__half>(dev, xmap, wmap, GemmEpilogue<__half, true>{(const __half*)bias, nullptr, 1.f, t.act}, y, M, N, K, t.bf16);
-    return launch_pair<__half>(dev, xmap, wmap, GemmEpilogue<__half>{(const __half*)bias, nullptr, 1.f, t.act}, y, M, N, K, t.bf16);
+#define RCU_PAIR(OUT_, MODE_, GLU_, ...) launch_pair<OUT_, MODE_, GLU_>(dev, xmap, wmap, GemmEpilogue<OUT_, MODE_>{(const OUT_*)bias, __VA_ARGS__}, y, M, N, K, t)
+    if (t.glu >= 0) return t.bf16 ? RCU_PAIR(__nv_bfloat16, EPI_PLAIN, true, nullptr, 1.f, {}) : RCU_PAIR(__half, EPI_PLAIN, true, nullptr, 1.f, {});
+    if (t.out_dt == RCU_F32) return RCU_PAIR(float, EPI_PLAIN, false, t.resid, t.alpha, t.act);
+    if (t.out_dt == RCU_BF16) return RCU_PAIR(__nv_bfloat16, EPI_PLAIN, false, nullptr, 1.f, t.act);
+    if (t.chain_op >= 0) return RCU_PAIR(__half, EPI_ACT, false, nullptr, 1.f, {}, t.bias32, nullptr, t.chain_op);
+    if (t.chained()) return RCU_PAIR(__half, EPI_RESID, false, nullptr, 1.f, {}, t.bias32, (const __half*)t.resid16, -1);
+    if (N & 3) return RCU_PAIR(__half, EPI_RAGGED, false, nullptr, 1.f, t.act);
+    return RCU_PAIR(__half, EPI_PLAIN, false, nullptr, 1.f, t.act);
+#undef RCU_PAIR
 }

@@ -501,6 +501,7 @@ rcu_status resolve(rcu_lazy* out) {
     // run
     struct TimedNode { std::string key; uint64_t bytes; cudaEvent_t e0, e1; };
     std::vector<TimedNode> timed;
+    fusion::RopeTables rope_tables(dev);
     uint32_t launched = 0, n_inplace = 0;
     const uint64_t launches0 = dev->launches;
     for (size_t i = 0; i < n; ++i) {
@@ -525,7 +526,7 @@ rcu_status resolve(rcu_lazy* out) {
             if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) return rcu_fail(dev, RCU_ERR_CUDA, "resolve: cudaEventCreate");
             cudaEventRecord(e0, dev->stream);
         }
-        st = op ? fusion::run(dev, t, *op) : run_node(t);
+        st = op ? fusion::run(dev, t, *op, &rope_tables) : run_node(t);
         if (st != RCU_OK) return st;
         if (profile) {
             cudaEventRecord(e1, dev->stream);

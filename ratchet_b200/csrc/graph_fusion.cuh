@@ -7,13 +7,15 @@
 //                q, k and v become strides, and a cache that only feeds the attention is appended to but not copied out
 //   attention32  permute(softmax((dk q)(dk k)^T) v) in f32 (the same with f32 activations, whose casts are no nodes)
 //   heads        cast(rope(cast(permute(view(slice))))), and permute(view(slice)) in front of a cache: straight into the cache's rows
+//   linear       a product with its bias's cast, gelu or silu between casts or the addition to the residual behind it; the product of a glu
+//                (bf16's too)
 //   norm         cast(norm(cast x));   act: cast(gelu or silu(cast x));   glu: up * cast(silu(cast gate)) of the halves of one tensor
 // A subgraph whose sizes or alignment a kernel does not take stays as it is.
 #pragma once
 
 namespace fusion {
 
-enum Kind { NONE = 0, ATTENTION, ATTENTION32, HEADS, APPEND, NORM, ACT, GLU };
+enum Kind { NONE = 0, ATTENTION, ATTENTION32, HEADS, APPEND, NORM, ACT, GLU, LINEAR };
 
 // element (position t, head h, feature d) of a [1, heads, T, D] operand at base[offset + h * head + t * row + d]
 struct Heads {
@@ -30,6 +32,10 @@ struct Op {
     bool copied = false;                // APPEND: the source is an ordinary [1, H, T, D] tensor
     HeadsRope rope;
     uint32_t H = 0, T = 0, L = 0, D = 0, E = 0;
+    rcu_lazy *w = nullptr, *x = nullptr, *bias = nullptr, *bias32 = nullptr, *resid = nullptr;      // LINEAR
+    int act = -1, glu = -1;
+    uint32_t x_col = 0;
+    uint64_t M = 0, N = 0, K = 0;
 };
 
 // `t` exists only for its one consumer
@@ -40,7 +46,7 @@ inline bool permutes(const rcu_lazy* t, uint32_t a, uint32_t b, uint32_t c, uint
 }
 
 struct Pass {
-    const rcu_device* dev;
+    rcu_device* dev;
     const Order& order;
     static constexpr int kPlain = -1, kPassed = -2;
     std::deque<Op> ops;
@@ -344,6 +350,86 @@ struct Pass {
 
     static uint64_t rows_of(const rcu_lazy* t) { return t->numel() / t->shape[t->rank - 1]; }
 
+    // the product `mm` (x W^T + bias in f16) as a LINEAR op, its bias's cast passed over
+    bool product(const rcu_lazy* mm, bool glu, bool act, Op* op, std::vector<rcu_lazy*>* seen) const {
+        if (mm->kind != K_MATMUL || mm->dt != RCU_F16 || mm->resolved() || mm->flags[0] || !mm->flags[1] || !mm->flags[2]) return false;
+        rcu_lazy *w = mm->srcs[0], *x = mm->srcs[1];
+        if (w->rank != 2 || x->dt != RCU_F16 || x->rank < 2) return false;
+        op->kind = LINEAR;
+        op->w = w;
+        op->x = x;
+        op->N = w->shape[0];
+        op->K = w->shape[1];
+        op->M = x->numel() / x->shape[x->rank - 1];
+        if (x->shape[x->rank - 1] != op->K || mm->numel() != op->M * op->N || !aligned(w) || !aligned(x) || !rcu_gemm_tc_chain_takes(dev, w->dt, op->M, op->N, op->K, glu, act)) return false;
+        op->srcs = {w, x};
+        if (mm->srcs.size() < 3) return true;
+        rcu_lazy* b = mm->srcs[2];
+        if (glu || b->numel() != op->N) return false;
+        if (inner(b, K_CAST, RCU_F16) && b->srcs[0]->dt == RCU_F32) {
+            seen->push_back(b);
+            op->bias32 = b->srcs[0];
+        } else {
+            op->bias = b;
+        }
+        op->srcs.push_back(op->bias32 ? op->bias32 : op->bias);
+        return true;
+    }
+
+    // a product whose bias is cast, one in front of an addition, or one in front of an activation between casts
+    bool linear(rcu_lazy* root) {
+        Op op;
+        std::vector<rcu_lazy*> seen;
+        if (root->kind == K_MATMUL) {
+            if (!product(root, false, false, &op, &seen) || !op.bias32) return false;
+        } else if (root->kind == K_BINARY && root->op == RCU_ADD && root->dt == RCU_F16) {
+            for (int i = 0; i < 2 && !op.resid; ++i) {
+                rcu_lazy *g = root->srcs[i], *r = root->srcs[1 - i];
+                if (!inner(g, K_MATMUL, RCU_F16) || g == r || r->dt != RCU_F16 || r->rank != g->rank || root->rank != g->rank || !aligned(r)) continue;
+                if (!std::equal(g->shape, g->shape + g->rank, r->shape)) continue;
+                op = Op{};
+                seen.assign(1, g);
+                if (product(g, false, false, &op, &seen)) op.resid = r;
+            }
+            if (!op.resid) return false;
+            op.srcs.push_back(op.resid);
+        } else {
+            rcu_lazy* t = between_casts(root, K_UNARY, &seen);
+            if (!t || (t->op != RCU_GELU && t->op != RCU_SILU)) return false;
+            rcu_lazy* g = seen[1]->srcs[0];
+            if (!inner(g, K_MATMUL, RCU_F16) || !product(g, false, true, &op, &seen)) return false;
+            seen.push_back(g);
+            op.act = t->op;
+        }
+        if (!free_of(seen)) return false;
+        pass(seen);
+        give(root, std::move(op));
+        return true;
+    }
+
+    // glu of a bf16 product that nothing else reads
+    bool glu_rows(rcu_lazy* root) {
+        rcu_lazy* l = root->srcs[0];
+        if (root->dt != RCU_BF16 || !inner(l, K_LINEAR, RCU_BF16) || l->flags[0] || l->flags[1] || (l->op != RCU_ACT_NONE && l->u[1] > 0) || l->f[0] != 1.0f) return false;
+        Op op;
+        op.kind = LINEAR;
+        op.w = l->srcs[0];
+        op.x = l->srcs[1];
+        op.N = op.w->shape[0];
+        op.K = op.w->shape[1];
+        op.x_col = l->u[0];
+        op.M = l->numel() / op.N;
+        op.glu = root->op;
+        const uint64_t pitch = op.x->shape[op.x->rank - 1];
+        if (op.w->dt != RCU_BF16 || op.x->dt != RCU_BF16 || pitch % 8 || op.x_col % 8 || !aligned(op.w) || !aligned(op.x) || absorbed(l) || find(l) ||
+            !rcu_gemm_tc_chain_takes(dev, RCU_BF16, op.M, op.N, op.K, true, false))
+            return false;
+        op.srcs = {op.w, op.x};
+        pass({l});
+        give(root, std::move(op));
+        return true;
+    }
+
     bool norm(rcu_lazy* root) {
         std::vector<rcu_lazy*> seen;
         rcu_lazy* t = between_casts(root, K_NORM, &seen);
@@ -392,15 +478,22 @@ struct Pass {
             if (gate->a[i] || up->a[i] || gate->shape[i] != x->shape[i] || up->shape[i] != x->shape[i]) return false;
         if (rows_of(root) < 2 || root->numel() * 2 != x->numel() || !aligned(x) || !free_of(seen)) return false;
         Op op;
-        op.kind = GLU;
-        op.srcs = {up->srcs[0]};
+        rcu_lazy* p = up->srcs[0];
+        if (p->kind == K_MATMUL && !p->resolved() && p->refs.load() == 2 && !absorbed(p) && !find(p) && product(p, true, false, &op, &seen)) {       // gate and up are all that reads it
+            op.glu = t->op;
+            seen.push_back(p);
+        } else {
+            op = Op{};
+            op.kind = GLU;
+            op.srcs = {p};
+        }
         pass(seen);
         give(root, std::move(op));
         return true;
     }
 
     // consumers before what they consume, so that a chain is recognised from its end
-    Pass(const rcu_device* d, const Order& o, bool on) : dev(d), order(o), role(o.nodes.size(), kPlain) {
+    Pass(rcu_device* d, const Order& o, bool on) : dev(d), order(o), role(o.nodes.size(), kPlain) {
         if (!on) return;
         for (rcu_lazy* t : o.nodes)
             if ((t->kind == K_CACHE || t->kind == K_INDEX_WRITE) && !t->resolved() && t->srcs[0]->resolved()) writers.push_back(t);
@@ -408,18 +501,50 @@ struct Pass {
             rcu_lazy* t = o.nodes[i];
             if (t->resolved() || absorbed(t) || find(t)) continue;
             if (t->kind == K_PERMUTE) attention(t) || attention32(t);
-            else if (t->kind == K_CAST) heads(t) || norm(t) || act(t);
-            else if (t->kind == K_BINARY) glu(t);
+            else if (t->kind == K_CAST) heads(t) || norm(t) || linear(t) || act(t);
+            else if (t->kind == K_BINARY) glu(t) || linear(t);
+            else if (t->kind == K_MATMUL) linear(t);
+            else if (t->kind == K_GLU) glu_rows(t);
         }
     }
 };
 
 inline const char* name_of(Kind k) {
-    static const char* names[] = {"", "attention", "attention", "heads", "cache", "norm chain", "act chain", "glu chain"};
+    static const char* names[] = {"", "attention", "attention", "heads", "cache", "norm chain", "act chain", "glu chain", "linear chain"};
     return names[k];
 }
 
-rcu_status run(rcu_device* dev, rcu_lazy* t, const Op& op) {
+// cos and sin of a prompt's angles, worked out once for all the layers of a resolve
+struct RopeTables {
+    rcu_device* dev;
+    struct Entry { HeadsRope rope; uint32_t T; void* table; };
+    std::vector<Entry> made;
+    explicit RopeTables(rcu_device* d) : dev(d) {}
+    ~RopeTables() {
+        for (Entry& e : made) rcu_free(dev, e.table);          // the pool reuses blocks in stream order
+    }
+    rcu_status of(HeadsRope* rope, uint32_t T) {
+        if (rope->dim == 0) return RCU_OK;
+        for (Entry& e : made)
+            if (e.T == T && e.rope.dim == rope->dim && e.rope.base == rope->base && e.rope.offset == rope->offset) {
+                rope->table = e.table;
+                return RCU_OK;
+            }
+        Entry e{*rope, T, nullptr};
+        rcu_status st = rcu_alloc(dev, (uint64_t)T * rope->dim * 4, &e.table);
+        if (st != RCU_OK) return st;
+        made.push_back(e);
+        rope->table = e.table;
+        return rcu_heads_angles(dev, *rope, T, e.table);
+    }
+};
+
+rcu_status run(rcu_device* dev, rcu_lazy* t, const Op& op, RopeTables* tables) {
+    HeadsRope rope = op.rope;
+    if (op.kind == HEADS || (op.kind == APPEND && !op.copied)) {
+        const rcu_status st = tables->of(&rope, op.T);
+        if (st != RCU_OK) return st;
+    }
     auto data = [](const rcu_lazy* x) { return x ? x->storage->ptr : nullptr; };
     switch (op.kind) {
         case ATTENTION: {
@@ -447,7 +572,7 @@ rcu_status run(rcu_device* dev, rcu_lazy* t, const Op& op) {
             return rcu_attention_f32(dev, a);
         }
         case HEADS:
-            return rcu_heads_half(dev, op.q.rows(), HeadRows{t->storage->ptr, (uint64_t)op.T * op.D, op.D}, op.H, op.T, op.D, op.rope);
+            return rcu_heads_half(dev, op.q.rows(), HeadRows{t->storage->ptr, (uint64_t)op.T * op.D, op.D}, op.H, op.T, op.D, rope);
         case APPEND: {
             rcu_lazy* c = op.srcs[0];
             rcu_tensor cd = c->desc();
@@ -456,7 +581,7 @@ rcu_status run(rcu_device* dev, rcu_lazy* t, const Op& op) {
                 return rcu_cache(dev, &cd, &sd, t->u[0], t->u[1], nullptr);
             }
             const uint64_t D = c->shape[3];
-            return rcu_heads_half(dev, op.q.rows(), HeadRows{(char*)c->storage->ptr + t->u[1] * D * 2, c->shape[2] * D, D}, op.H, op.T, op.D, op.rope);
+            return rcu_heads_half(dev, op.q.rows(), HeadRows{(char*)c->storage->ptr + t->u[1] * D * 2, c->shape[2] * D, D}, op.H, op.T, op.D, rope);
         }
         case NORM: {
             const rcu_lazy* n = t->srcs[0];
@@ -468,6 +593,16 @@ rcu_status run(rcu_device* dev, rcu_lazy* t, const Op& op) {
         case GLU: {
             const uint64_t F = t->shape[t->rank - 1];
             return rcu_glu_half(dev, t->srcs[1]->srcs[0]->op, data(op.srcs[0]), t->storage->ptr, t->numel() / F, F);
+        }
+        case LINEAR: {
+            LinearChain c;
+            c.bias = data(op.bias);
+            c.bias32 = (const float*)data(op.bias32);
+            c.resid = data(op.resid);
+            c.op = op.act;
+            c.glu = op.glu;
+            c.x_pitch = op.x->shape[op.x->rank - 1];
+            return rcu_gemm_tc_chain(dev, op.w->dt, op.w->storage->ptr, (const char*)op.x->storage->ptr + op.x_col * 2, t->storage->ptr, op.M, op.N, op.K, c);
         }
         default: return rcu_fail(dev, RCU_ERR_UNSUPPORTED, "resolve: fused op %d", op.kind);
     }

@@ -13,11 +13,6 @@ namespace {
 
 struct alignas(16) Half8 { __half v[8]; };
 
-__device__ __forceinline__ float chain_act(int act, float x) {
-    if (act == RCU_GELU) return (0.5f * x) * (1.0f + tanhf((0.7978846f * x) * (1.0f + (0.044715f * x) * x)));      // the f32 form of unary gelu
-    return x / (1.0f + expf(-x));
-}
-
 // CTA = one row of up to 256 * 8 * PER features, kept in registers
 template <int PER>
 __global__ void __launch_bounds__(256)
@@ -92,22 +87,36 @@ __global__ void __launch_bounds__(256) glu_half_kernel(const __half* __restrict_
     }
 }
 
+// Thread = one rotation pair of one position (as rcu_rope, cpu/rope.rs:38-41).  Some 200 double-precision operations, so that a prompt of 1000
+// tokens takes 4 us; inside the rotation of every layer's queries and keys they were most of its 13 us.
+__global__ void __launch_bounds__(128) heads_angles_kernel(float2* __restrict__ table, int n, int half, float ln_base, int offset) {
+    rcu_kernel_entry();
+    const int idx = blockIdx.x * 128 + threadIdx.x;
+    if (idx >= n) return;
+    const int s = idx / half, i = idx - s * half;
+    const float ex = -(float)i * ln_base / (float)half;
+    const float inv = (float)exp((double)ex), th = (float)(s + offset) * inv;
+    double sd, cd;
+    sincos((double)th, &sd, &cd);
+    table[idx] = make_float2((float)cd, (float)sd);
+}
+
 // Thread = eight consecutive rotation pairs of one position: their angles once, then every head this thread visits
 __global__ void __launch_bounds__(128)
-heads_rope_kernel(const __half* __restrict__ x, __half* __restrict__ out, size_t xh, size_t xr, size_t oh, size_t orow, int H, int T, int D, int dim, float ln_base, int offset) {
+heads_rope_kernel(const __half* __restrict__ x, __half* __restrict__ out, size_t xh, size_t xr, size_t oh, size_t orow, int H, int T, int D, int dim, const float2* __restrict__ table) {
     rcu_kernel_entry();
     const int half = dim >> 1, hv = half / 8, idx = blockIdx.x * 128 + threadIdx.x;
     if (idx < T * hv) {
         const int s = idx / hv, i0 = (idx - s * hv) * 8;
         float sn[8], cs[8];
+        const float4* row = reinterpret_cast<const float4*>(table + (size_t)s * half + i0);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {            // as rcu_rope (cpu/rope.rs:38-41)
-            const float ex = -(float)(i0 + e) * ln_base / (float)half;
-            const float inv = (float)exp((double)ex), th = (float)(s + offset) * inv;
-            double sd, cd;
-            sincos((double)th, &sd, &cd);
-            sn[e] = (float)sd;
-            cs[e] = (float)cd;
+        for (int e = 0; e < 4; ++e) {
+            const float4 v = row[e];
+            cs[2 * e] = v.x;
+            sn[2 * e] = v.y;
+            cs[2 * e + 1] = v.z;
+            sn[2 * e + 1] = v.w;
         }
 #pragma unroll 2
         for (int h = blockIdx.y; h < H; h += gridDim.y) {
@@ -176,6 +185,14 @@ rcu_status rcu_glu_half(rcu_device* dev, int act, const void* x, void* out, uint
     return RCU_OK;
 }
 
+rcu_status rcu_heads_angles(rcu_device* dev, const HeadsRope& rope, uint32_t tokens, void* table) {
+    const uint64_t n = (uint64_t)tokens * (rope.dim / 2);
+    if (rope.dim % 16 || n == 0 || n > 0x7fffffffull) return RCU_ERR_UNSUPPORTED;
+    RCU_CUDA(dev, rcu_launch(dev, heads_angles_kernel, (unsigned)((n + 127) / 128), 128, 0, (float2*)table, (int)n, (int)(rope.dim / 2), logf(rope.base), (int)rope.offset));
+    RCU_LAUNCH_CHECK(dev);
+    return RCU_OK;
+}
+
 rcu_status rcu_heads_half(rcu_device* dev, const HeadRows& src, const HeadRows& dst, uint32_t H, uint32_t T, uint32_t D, const HeadsRope& rope) {
     if (D % 8 || D == 0 || H == 0 || T == 0 || (src.head | src.row | dst.head | dst.row) % 8 || !aligned16({src.data, dst.data}) || (uint64_t)T * D > 0x7fffffffull)
         return RCU_ERR_UNSUPPORTED;
@@ -185,11 +202,11 @@ rcu_status rcu_heads_half(rcu_device* dev, const HeadRows& src, const HeadRows& 
         RCU_CUDA(dev, rcu_launch(dev, heads_copy_kernel, (unsigned)grid_for((uint64_t)H * T * (D / 8), 256, dev->sm_count * 16), 256, 0, x, o, (size_t)src.head, (size_t)src.row,
                                  (size_t)dst.head, (size_t)dst.row, (int)H, (int)T, (int)(D / 8)));
     } else {
-        if (rope.dim % 16 || rope.dim > D) return RCU_ERR_UNSUPPORTED;
+        if (rope.dim % 16 || rope.dim > D || !rope.table) return RCU_ERR_UNSUPPORTED;
         const int per_row = std::max<int>(rope.dim / 16, (D - rope.dim) / 8), gx = ((int)T * per_row + 127) / 128;
         const int want = (dev->sm_count * 16 + gx - 1) / gx;
         RCU_CUDA(dev, rcu_launch(dev, heads_rope_kernel, dim3(gx, (unsigned)std::max(1, std::min<int>((int)H, want))), 128, 0, x, o, (size_t)src.head, (size_t)src.row,
-                                 (size_t)dst.head, (size_t)dst.row, (int)H, (int)T, (int)D, (int)rope.dim, logf(rope.base), (int)rope.offset));
+                                 (size_t)dst.head, (size_t)dst.row, (int)H, (int)T, (int)D, (int)rope.dim, (const float2*)rope.table));
     }
     RCU_LAUNCH_CHECK(dev);
     return RCU_OK;

@@ -2,6 +2,14 @@
 #pragma once
 #include "attention.cuh"
 
+#ifdef __CUDACC__
+// gelu or silu between two casts
+__device__ __forceinline__ float chain_act(int act, float x) {
+    if (act == RCU_GELU) return (0.5f * x) * (1.0f + tanhf((0.7978846f * x) * (1.0f + (0.044715f * x) * x)));      // the f32 form of unary gelu
+    return x / (1.0f + expf(-x));
+}
+#endif
+
 // out = f16(norm(f32(x)))  (nn's LayerNorm / RMSNorm: cast, norm, cast); scale and bias f32
 rcu_status rcu_norm_half(rcu_device* dev, int kind, const void* x, const void* scale, const void* bias, float eps, void* out, uint64_t rows, uint64_t N);
 // out = f16(act(f32(x)))
@@ -13,5 +21,20 @@ struct HeadsRope {
     uint32_t dim = 0;
     float base = 0.f;
     uint32_t offset = 0;
+    const void* table = nullptr;        // of rcu_heads_angles for these tokens
 };
+// [tokens][dim / 2] cos, sin as floats
+rcu_status rcu_heads_angles(rcu_device* dev, const HeadsRope& rope, uint32_t tokens, void* table);
 rcu_status rcu_heads_half(rcu_device* dev, const HeadRows& src, const HeadRows& dst, uint32_t heads, uint32_t tokens, uint32_t D, const HeadsRope& rope);
+
+// A Linear with what follows it in the graph, on the tensor cores (gemm_tc.cu, gemm_tc2.cu): f16, out = f16(x W^T + bias), then gelu or silu between
+// casts, or the addition to a residual; or (f16 and bf16) out = up * act(gate) of a product whose columns are gate, then up.
+struct LinearChain {
+    const void* bias = nullptr;         // in the activations' type
+    const float* bias32 = nullptr;      // in f32, to be rounded to it
+    const void* resid = nullptr;
+    int op = -1, glu = -1;              // RCU_GELU, RCU_SILU
+    uint64_t x_pitch = 0;               // of the activations' rows, 0: K
+};
+bool rcu_gemm_tc_chain_takes(rcu_device* dev, int w_dt, uint64_t M, uint64_t N, uint64_t K, bool glu, bool act);
+rcu_status rcu_gemm_tc_chain(rcu_device* dev, int w_dt, const void* w, const void* x, void* y, uint64_t M, uint64_t N, uint64_t K, const LinearChain& c);

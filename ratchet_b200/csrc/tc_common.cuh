@@ -4,7 +4,10 @@
 #pragma once
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "bulk_async.cuh"   // mbarrier + tensor-map helpers
+#include "half_chains.cuh"
 
 namespace tc {
 
@@ -87,6 +90,16 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t* r)
         "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+// 32 lanes x 8 consecutive f32 columns of tensor memory -> 8 registers per thread
+__device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, float* v) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\ttcgen05.wait::ld.sync.aligned;"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 // 16 registers per thread -> 32 lanes x 16 columns of tensor memory
 __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t* r) {
@@ -179,16 +192,65 @@ template <class Put> __device__ __forceinline__ void turn_piece(float4* turn, co
     __syncwarp();
 }
 
+// turn_piece for values that are finished on the way: load8(c, values) brings columns 8 c .. 8 c + 7 of this lane's row, in a loop
+template <class Load8, class Put> __device__ __forceinline__ void turn_piece8(float4* turn, Load8 load8, Put put) {
+    const int lane = threadIdx.x & 31, r = lane >> 3, quad = lane & 7;
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {
+        float v[8];
+        load8(c, v);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) turn[lane * 8 + ((2 * c + h) ^ (lane & 7))] = make_float4(v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) put(i, 4 * i + r, turn[(4 * i + r) * 8 + (quad ^ ((4 * i + r) & 7))]);
+    __syncwarp();
+}
+
 // What the epilogue of a tensor-core GEMM does with an accumulator: Out = f16 / bf16: round(acc + bias);
 // Out = f32: residual + alpha * (acc + bias), the residual stream of a model that keeps it in 32 bits
 // (`resid` may be the output itself: every element is read by the thread that writes it).  RAGGED: the number of columns is no multiple of
 // 4, so rows do not start on four elements and bias4 / store4 go element by element (a form of its own: as a run-time test it cost
-// the whole-row GEMMs 1 %).
-template <class Out, bool RAGGED = false> struct GemmEpilogue {
+// the whole-row GEMMs 1 %).  RESID, ACT: what an f16 graph puts behind a Linear, with its
+// roundings - a bias that is cast from f32, then an addition to the residual, or gelu / silu between casts; forms of their own for the same
+// reason.  ACT's values are finished on the way out of tensor memory, eight columns at a time in a loop (finish8): unrolled over a
+// whole piece the two activations are 30 KB of instructions that a CTA runs once or twice, and the GEMM of 501 x 384 x 384 took 16 us
+// for 7.7.
+enum { EPI_PLAIN = 0, EPI_RAGGED = 1, EPI_RESID = 2, EPI_ACT = 3 };
+template <class Out, int MODE = EPI_PLAIN> struct GemmEpilogue {
+    static constexpr bool RAGGED = MODE == EPI_RAGGED, RESID = MODE == EPI_RESID, ACT = MODE == EPI_ACT;
+    struct alignas(4 * sizeof(Out)) Quad { Out v[4]; };
+    using Resid = typename std::conditional<RESID, Quad, float4>::type;
     const Out* bias;          // per output column, nullable
     const float* resid;       // f32 output only, nullable
     float alpha;
     LinearAct act;            // after the bias
+    const float* bias32 = nullptr;      // RESID, ACT: a bias to be rounded to Out first, nullable
+    const Out* resid16 = nullptr;       // RESID: added after the rounding, nullable
+    int chain_op = -1;                  // ACT: RCU_GELU or RCU_SILU of the rounded sum
+    __device__ __forceinline__ float added(float v, float r) const {
+        v = rnd<Out>(v);
+        return resid16 ? v + r : v;
+    }
+    __device__ __forceinline__ void finish8(float* v, int col, int N) const {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            float b = 0.f;
+            if (col + e < N) b = bias32 ? rnd<Out>(bias32[col + e]) : bias ? to_f32<Out>(bias[col + e]) : 0.f;
+            v[e] = chain_act(chain_op, rnd<Out>(v[e] + b));
+        }
+    }
+    // what store4 adds to four columns; `idx` a multiple of 4
+    __device__ __forceinline__ Resid resid4(size_t idx, bool in) const {
+        if constexpr (RESID) {
+            Quad q{};
+            if (in && resid16) q = *reinterpret_cast<const Quad*>(resid16 + idx);
+            return q;
+        } else {
+            return sizeof(Out) == 4 && in && resid ? *reinterpret_cast<const float4*>(resid + idx) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
     __device__ __forceinline__ float value(float acc, int col) const {
         const float v = acc + (bias ? to_f32<Out>(bias[col]) : 0.f);
         return col < act.cols ? act(v) : v;
@@ -199,16 +261,21 @@ template <class Out, bool RAGGED = false> struct GemmEpilogue {
         return from_f32<Out>(v);
     }
     // four consecutive columns whose bias, and residual (f32 output), the caller has loaded; `col` a multiple of 4
-    struct alignas(4 * sizeof(Out)) Quad { Out v[4]; };
     __device__ __forceinline__ float4 bias4(int col, int N) const {
+        if (ACT) return make_float4(0.f, 0.f, 0.f, 0.f);          // finish8 has added it
+        if (RESID && bias32) return make_float4(rnd<Out>(bias32[col]), rnd<Out>(bias32[col + 1]), rnd<Out>(bias32[col + 2]), rnd<Out>(bias32[col + 3]));
         if (RAGGED && bias) {
             return make_float4(to_f32<Out>(bias[col]), col + 1 < N ? to_f32<Out>(bias[col + 1]) : 0.f, col + 2 < N ? to_f32<Out>(bias[col + 2]) : 0.f,
                                col + 3 < N ? to_f32<Out>(bias[col + 3]) : 0.f);
         }
         return bias ? make_float4(to_f32<Out>(bias[col]), to_f32<Out>(bias[col + 1]), to_f32<Out>(bias[col + 2]), to_f32<Out>(bias[col + 3])) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    __device__ __forceinline__ void store4(Out* out, size_t idx, const float4& acc, const float4& b, const float4& r, int col, int N) const {
+    __device__ __forceinline__ void store4(Out* out, size_t idx, const float4& acc, const float4& b, const Resid& r, int col, int N) const {
         float v[4] = {acc.x + b.x, acc.y + b.y, acc.z + b.z, acc.w + b.w};
+        if constexpr (RESID) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = added(v[e], to_f32<Out>(r.v[e]));
+        }
         if (col < act.cols) {
             if (act.kind == RCU_ACT_RELU_SQUARED) {      // without branches: the others are dear enough to hide them
 #pragma unroll
@@ -221,7 +288,7 @@ template <class Out, bool RAGGED = false> struct GemmEpilogue {
                 for (int e = 0; e < 4; ++e) v[e] = col + e < act.cols ? act(v[e]) : v[e];
             }
         }
-        if (sizeof(Out) == 4) {
+        if constexpr (sizeof(Out) == 4) {
             v[0] = resid ? fmaf(alpha, v[0], r.x) : alpha * v[0];
             v[1] = resid ? fmaf(alpha, v[1], r.y) : alpha * v[1];
             v[2] = resid ? fmaf(alpha, v[2], r.z) : alpha * v[2];
@@ -241,7 +308,15 @@ template <class Out, bool RAGGED = false> struct GemmEpilogue {
     // eight consecutive columns, 16-byte aligned
     __device__ __forceinline__ void store8(Out* out, size_t idx, const float* acc, int col) const {
         __align__(16) Out h[8];
-        if (sizeof(Out) == 4 && resid) {
+        if constexpr (RESID || ACT) {
+            __align__(16) Out r[8] = {};
+            if (RESID && resid16) *reinterpret_cast<uint4*>(r) = *reinterpret_cast<const uint4*>(resid16 + idx);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float b = bias32 ? rnd<Out>(bias32[col + e]) : bias ? to_f32<Out>(bias[col + e]) : 0.f;
+                h[e] = from_f32<Out>(ACT ? chain_act(chain_op, rnd<Out>(acc[e] + b)) : added(acc[e] + b, to_f32<Out>(r[e])));
+            }
+        } else if (sizeof(Out) == 4 && resid) {
             __align__(16) float r[8];
             *reinterpret_cast<float4*>(r) = *reinterpret_cast<const float4*>(resid + idx);
             *reinterpret_cast<float4*>(r + 4) = *reinterpret_cast<const float4*>(resid + idx + 4);
@@ -267,4 +342,11 @@ struct TcLinear {
     const float* resid = nullptr;
     float alpha = 1.f;
     LinearAct act = {};
+    // f16 output: what an f16 graph has behind the product (GemmEpilogue's RESID, ACT)
+    const float* bias32 = nullptr;
+    const void* resid16 = nullptr;
+    int chain_op = -1;
+    // out [M, N / 2] = up * act(gate) of rows that hold gate, then up, rounded as the graph's own kernels round; glu: RCU_GELU or RCU_SILU
+    int glu = -1;
+    bool chained() const { return bias32 || resid16 || chain_op >= 0; }
 };
