@@ -1,4 +1,4 @@
-// f32 Linear on the tensor cores with f32-level accuracy (split-TF32):
+// f32 Linear of many tiles on the tensor cores with f32-level accuracy (split-TF32; gemm_parts_f32.cu takes what has few):
 //   out[M, N] = X[M, K] . W[N, K]^T (+ bias), everything f32.
 //
 // ratchet runs f32 models (Phi-2 and Whisper checkpoints as shipped, ops/matmul/gemm.rs) and its CPU
@@ -57,16 +57,13 @@ __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t adesc, uint6
         : "memory");
 }
 
-// TMR = token rows of a tile, 128 or 64.  With 64 the accumulator rows sit in the first 16 lanes of each 32-lane
-// quarter of tensor memory (row r in lane 32 (r / 16) + r % 16); a tile costs half the shared-memory traffic on the
-// activation side, which is what small M (Phi-2's 64 rows) and grids that do not fill the SMs want.
-template <int BN, int STAGES, int TMR>
+template <int BN, int STAGES>
 __global__ void __launch_bounds__(kThreadsF32, 1)
 gemm_tc_f32_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const float* __restrict__ bias,
                    const float* __restrict__ bias_rows,
                    float* __restrict__ out, int M, int N, int K, int kb_per_split, int* status) {
     rcu_kernel_entry_wait_only();
-    constexpr int A_BYTES = TMR * TK32 * 4;       // 16 or 8 KiB
+    constexpr int A_BYTES = TM * TK32 * 4;        // 16 KiB
     constexpr int B_BYTES = BN * TK32 * 4;
     constexpr int RAW = A_BYTES + B_BYTES;        // hi tiles (A then B); the lo tiles follow in the same order
     constexpr int STAGE = 2 * RAW;
@@ -80,7 +77,7 @@ gemm_tc_f32_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m0 = blockIdx.y * TMR, n0 = blockIdx.x * BN;
+    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * BN;
     // blockIdx.z is either the problem of a batch (attention heads: third coordinate of both maps) or, when
     // kb_per_split > 0, the slice of K this CTA sums: slice z covers k-blocks [z * kb_per_split, ...) of the
     // one problem and writes its partial result to slab z of `out`.
@@ -122,7 +119,7 @@ gemm_tc_f32_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_tf32(TMR, BN);
+            constexpr uint32_t idesc = umma_idesc_tf32(TM, BN);
             for (int it = 0; it < nk; ++it) {
                 const int s = it % STAGES;
                 if (!mbar_wait_spin(&full[s], (it / STAGES) & 1, abort_flag, status)) break;
@@ -148,7 +145,7 @@ gemm_tc_f32_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
         const int q = warp & 3;
         const bool ok = mbar_wait(accum_bar, 0, abort_flag, status);
         tc_fence_after();
-        const int row = TMR == 128 ? m0 + q * 32 + lane : (lane < 16 ? m0 + q * 16 + lane : M);   // 64-row tiles: 16 rows per quarter
+        const int row = m0 + q * 32 + lane;
         if (ok) {
 #pragma unroll 1
             for (int c = 0; c < BN; c += 32) {
@@ -248,27 +245,24 @@ sum_splits_kernel(const float4* __restrict__ part, int splits, size_t slab4, con
     }
 }
 
-template <int BN, int TMR>
+template <int BN>
 rcu_status launch_f32(rcu_device* dev, const CUtensorMap& xmap, const CUtensorMap& wmap, const void* bias, const void* bias_rows, void* out,
                       int M, int N, int K, int batches, int kb_per_split) {
-    constexpr int STAGE = 2 * (TMR * TK32 * 4 + BN * TK32 * 4);
+    constexpr int STAGE = 2 * (TM * TK32 * 4 + BN * TK32 * 4);
     constexpr int STAGES = (192 * 1024) / STAGE > 8 ? 8 : (192 * 1024) / STAGE;
     const size_t smem = (size_t)STAGES * STAGE + 1024 + 512;
-    auto kern = gemm_tc_f32_kernel<BN, STAGES, TMR>;
+    auto kern = gemm_tc_f32_kernel<BN, STAGES>;
     RCU_CUDA(dev, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dim3 grid((N + BN - 1) / BN, (M + TMR - 1) / TMR, batches);
+    dim3 grid((N + BN - 1) / BN, (M + TM - 1) / TM, batches);
     rcu_launch(dev, kern, grid, kThreadsF32, smem, xmap, wmap, (const float*)bias, (const float*)bias_rows, (float*)out, M, N, K, kb_per_split, dev->d_status);
     RCU_LAUNCH_CHECK(dev);
     return RCU_OK;
 }
 
-rcu_status launch_f32_any(rcu_device* dev, int bn, int tmr, const CUtensorMap& xmap, const CUtensorMap& wmap, const void* bias, const void* bias_rows,
+rcu_status launch_f32_any(rcu_device* dev, int bn, const CUtensorMap& xmap, const CUtensorMap& wmap, const void* bias, const void* bias_rows,
                           void* out, int M, int N, int K, int batches, int kb_per_split) {
-    if (tmr == 64)
-        return bn == 128 ? launch_f32<128, 64>(dev, xmap, wmap, bias, bias_rows, out, M, N, K, batches, kb_per_split)
-                         : launch_f32<64, 64>(dev, xmap, wmap, bias, bias_rows, out, M, N, K, batches, kb_per_split);
-    return bn == 128 ? launch_f32<128, 128>(dev, xmap, wmap, bias, bias_rows, out, M, N, K, batches, kb_per_split)
-                     : launch_f32<64, 128>(dev, xmap, wmap, bias, bias_rows, out, M, N, K, batches, kb_per_split);
+    return bn == 128 ? launch_f32<128>(dev, xmap, wmap, bias, bias_rows, out, M, N, K, batches, kb_per_split)
+                     : launch_f32<64>(dev, xmap, wmap, bias, bias_rows, out, M, N, K, batches, kb_per_split);
 }
 
 // [batches, rows, K] f32 row-major, box = 1 x box_rows x 32 elements, 128-byte swizzle
@@ -288,12 +282,15 @@ bool make_map_f32_sw128(CUtensorMap* map, const void* base, uint64_t batches, ui
 bool rcu_gemm_tc_f32_eligible(int lhs_dt, int act_dt, uint64_t M, uint64_t N, uint64_t K) {
     if (act_dt != RCU_F32 || lhs_dt != RCU_F32) return false;
     // small problems stay on the SIMT kernel; rows must be 16-byte multiples for the tensor maps
-    // (two rows already pay: 222 -> 24 us for 3072 x 3072 against the SIMT kernel)
     if (M < 2 || N < 64 || K < 32 || K % 4 != 0) return false;
     if (M > 0x7fffffffull || N > 0x7fffffffull || K > 0x7fffffffull) return false;
     static const bool off = [] { const char* e = std::getenv("RCU_GEMM_F32_TC"); return e && std::atoi(e) == 0; }();
     return !off;
 }
+
+// gemm_parts_f32.cu
+rcu_status rcu_gemm_parts_f32_dispatch(rcu_device* dev, const void* w, const void* x, const void* bias, void* y, uint64_t M, uint64_t N, uint64_t K, uint64_t batches,
+                                       const void* bias_rows);
 
 rcu_status rcu_gemm_tc_f32_dispatch(rcu_device* dev, const void* w, const void* x, const void* bias, void* y, uint64_t M, uint64_t N,
                                     uint64_t K, uint64_t batches, const void* bias_rows) {
@@ -302,18 +299,16 @@ rcu_status rcu_gemm_tc_f32_dispatch(rcu_device* dev, const void* w, const void* 
     // tensor-map strides are multiples of 16 bytes; the grid's z extent is limited
     if (batches < 1 || batches > 65535 || (batches > 1 && ((M * K) % 4 != 0 || (N * K) % 4 != 0 || bias || bias_rows))) return RCU_ERR_UNSUPPORTED;
     DevGuard g(dev->ordinal);
-    // Tile height: 64 token rows when M fits one such tile (half of a 128-row tile would be padding).  Cutting larger
-    // M into 64-row tiles to put a CTA on every SM was measured and is slower (Whisper-tiny's 1500 x 384 x 384
-    // Linear and the unfolded conv1d): the weight side of a tile costs the same and is then paid twice as often.
+    const rcu_status parts = rcu_gemm_parts_f32_dispatch(dev, w, x, bias, y, M, N, K, batches, bias_rows);
+    if (parts != RCU_ERR_UNSUPPORTED) return parts;
     const uint64_t sms = (uint64_t)dev->sm_count;
-    const int tmr = M <= 64 ? 64 : 128;
     // Tile width and K slices together.  A CTA spends about 0.7 us per 32-wide k-block almost regardless of the tile's
     // width (twelve small MMAs issued by one thread, the lo pass, the barrier hops between them), so what counts is
     // how many k-blocks a CTA runs one after the other and how many rounds of CTAs the grid needs; the width adds a
     // little through shared-memory traffic.  Slices of K (blockIdx.z; every slice writes a partial result to pooled
     // scratch and one pass sums the slices in order: deterministic) are taken whenever they shorten that chain, with a
     // charge for the summing pass.
-    const uint64_t mt = (M + tmr - 1) / tmr, nk = (K + TK32 - 1) / TK32;
+    const uint64_t mt = (M + TM - 1) / TM, nk = (K + TK32 - 1) / TK32;
     constexpr uint64_t kMinBlocksPerSplit = 24, kFixed = 600, kSumCharge = 4;
     int bn = 64;
     uint64_t splits = 1, best = ~0ull;
@@ -323,12 +318,12 @@ rcu_status rcu_gemm_tc_f32_dispatch(rcu_device* dev, const void* w, const void* 
         for (uint64_t sp = 1; sp <= sp_max; ++sp) {
             const uint64_t kbps_c = (nk + sp - 1) / sp;
             const uint64_t rounds = (tiles_c * sp * batches + sms - 1) / sms;
-            const uint64_t cost = (rounds * kbps_c + (sp > 1 ? kSumCharge : 0)) * (kFixed + (uint64_t)(tmr + cand));
+            const uint64_t cost = (rounds * kbps_c + (sp > 1 ? kSumCharge : 0)) * (kFixed + (uint64_t)(TM + cand));
             if (cost < best) { best = cost; bn = cand; splits = sp; }
         }
     }
     CUtensorMap xmap, wmap;
-    if (!make_map_f32_sw128(&xmap, x, batches, M, K, (uint32_t)tmr) || !make_map_f32_sw128(&wmap, w, batches, N, K, (uint32_t)bn))
+    if (!make_map_f32_sw128(&xmap, x, batches, M, K, TM) || !make_map_f32_sw128(&wmap, w, batches, N, K, (uint32_t)bn))
         return rcu_fail(dev, RCU_ERR_CUDA, "gemm_tc_f32: cuTensorMapEncodeTiled failed (M=%llu N=%llu K=%llu x%llu)", (unsigned long long)M,
                         (unsigned long long)N, (unsigned long long)K, (unsigned long long)batches);
     if (splits > 1) {
@@ -337,7 +332,7 @@ rcu_status rcu_gemm_tc_f32_dispatch(rcu_device* dev, const void* w, const void* 
         void* part = nullptr;
         rcu_status st = rcu_alloc(dev, splits * M * N * 4, &part);
         if (st != RCU_OK) return st;
-        st = launch_f32_any(dev, bn, tmr, xmap, wmap, nullptr, nullptr, part, (int)M, (int)N, (int)K, (int)splits, (int)kbps);
+        st = launch_f32_any(dev, bn, xmap, wmap, nullptr, nullptr, part, (int)M, (int)N, (int)K, (int)splits, (int)kbps);
         if (st == RCU_OK) {
             const size_t slab4 = (size_t)(M * N / 4);
             const int grid = (int)std::min<size_t>((slab4 + 255) / 256, (size_t)dev->sm_count * 8);
@@ -348,5 +343,5 @@ rcu_status rcu_gemm_tc_f32_dispatch(rcu_device* dev, const void* w, const void* 
         rcu_free(dev, part);      // the pool reuses blocks in stream order
         return st;
     }
-    return launch_f32_any(dev, bn, tmr, xmap, wmap, bias, bias_rows, y, (int)M, (int)N, (int)K, (int)batches, 0);
+    return launch_f32_any(dev, bn, xmap, wmap, bias, bias_rows, y, (int)M, (int)N, (int)K, (int)batches, 0);
 }

@@ -101,6 +101,12 @@ __device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, float* v) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
+// 8 registers per thread -> 32 lanes x 8 columns of tensor memory, not waited for (tcgen05.wait::st)
+__device__ __forceinline__ void tmem_st_32x8_start(uint32_t taddr, const uint32_t* r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]),
+                 "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
 // 16 registers per thread -> 32 lanes x 16 columns of tensor memory
 __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t* r) {
     asm volatile(
