@@ -28,6 +28,7 @@ constexpr int kBlockQ = kTileQ * 128, kBlockK = kTileK * 128;       // bytes of 
 struct Args {
     __half* out;
     int H, T, L, E;
+    int per;                    // queries of a CTA, one tile or two
     const float* scale32;
     const __half *scale_q, *scale_k;
     int* status;
@@ -55,8 +56,8 @@ attention_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant
     __shared__ volatile int abort_flag;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h = blockIdx.x, i0 = blockIdx.y * 2 * kTileQ;
-    const int nq = min(2 * kTileQ, a.T - i0);               // the CTA's queries
+    const int h = blockIdx.x, i0 = blockIdx.y * a.per;
+    const int nq = min(a.per, a.T - i0);               // the CTA's queries
     const int tiles = (a.L + kTileK - 1) / kTileK;
     const bool second = nq > kTileQ;                        // whether the second query tile holds any
 
@@ -330,7 +331,7 @@ constexpr size_t smem_of(int nb, int eb, bool mask) { return 1024 + (size_t)2 * 
 }  // namespace
 
 bool rcu_attention_f16_takes(const rcu_device* dev, const AttentionArgs& a) {
-    if (a.T < 2 || a.L < 1 || a.H < 1 || a.H > 0x7fffffff / 128 || a.T > 65535 * 2 * kTileQ || a.L > (1 << 30)) return false;
+    if (a.T < 2 || a.L < 1 || a.H < 1 || a.H > 0x7fffffff / 128 || a.T > 65535 * kTileQ || a.L > (1 << 30)) return false;
     if (a.D < 8 || a.D > 128 || a.D % 8 || a.E < 8 || a.E > 128 || a.E % 8) return false;
     for (const HeadRows* t : {&a.q, &a.k, &a.v})
         if (t->head % 8 || t->row % 8 || t->head == 0 || t->row == 0) return false;
@@ -365,8 +366,10 @@ rcu_status rcu_attention_f16(rcu_device* dev, const AttentionArgs& a) {
         if (padded) rcu_free(dev, padded);
         return rcu_fail(dev, RCU_ERR_CUDA, "attention: cuTensorMapEncodeTiled failed (T=%d L=%d H=%d D=%d)", a.T, a.L, a.H, a.D);
     }
-    const Args t{(__half*)a.out, a.H, a.T, a.L, a.E, a.scale32[0], a.scale16[0], a.scale16[1], dev->d_status};
-    const dim3 grid(a.H, (a.T + 2 * kTileQ - 1) / (2 * kTileQ));
+    // two tiles take turns on the tensor cores and in the softmax; where they leave most SMs idle one is better (6 heads of 501 positions: 12 CTAs)
+    const int per = 2 * a.H * ((a.T + 2 * kTileQ - 1) / (2 * kTileQ)) <= dev->sm_count ? kTileQ : 2 * kTileQ;
+    const Args t{(__half*)a.out, a.H, a.T, a.L, a.E, per, a.scale32[0], a.scale16[0], a.scale16[1], dev->d_status};
+    const dim3 grid(a.H, (a.T + per - 1) / per);
     const size_t smem = smem_of(nb, eb, mask);
     void (*kern)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, Args);
 #define RCU_ATT(NB_, EB_) kern = mask ? attention_kernel<NB_, EB_, true> : attention_kernel<NB_, EB_, false>

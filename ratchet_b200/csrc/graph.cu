@@ -278,7 +278,8 @@ const char* dt_name(int dt) {
 // ------------------------------------------------------------------------------------------------
 // op dispatch
 // ------------------------------------------------------------------------------------------------
-rcu_status run_node(rcu_lazy* n) {
+// converted: srcs[0] of a product in its activations' type (nullable)
+rcu_status run_node(rcu_lazy* n, void* converted) {
     rcu_device* dev = n->dev;
     rcu_tensor dst = n->desc();
     auto S = [&](size_t i) { return n->srcs[i]->desc(); };
@@ -288,6 +289,10 @@ rcu_status run_node(rcu_lazy* n) {
         case K_CAST: { rcu_tensor x = S(0); return rcu_cast(dev, &x, &dst); }
         case K_MATMUL: {
             rcu_tensor l = S(0), r = S(1), bias;
+            if (converted) {
+                l.dt = rcu_activation_dtype(l.dt);
+                l.data = converted;
+            }
             if (n->srcs.size() > 2) bias = S(2);
             // weights that were uploaded and waited for cannot be written by anything in flight: the GEMV may start early
             const bool before = dev->const_weights;
@@ -382,6 +387,64 @@ struct Plan {
     uint64_t size;
     bool exclusive;           // output / externally referenced: never shared
     int object = -1;
+};
+
+// Weights of this resolve's Linears that are converted ahead of them (rcu_linear_converts): small matrices, where a conversion is all launch; a large
+// one stays beside its product, which then finds it in L2.
+struct Converted {
+    static constexpr uint64_t kNumel = 1ull << 20, kTotal = 64ull << 20;      // weights of one matrix; bytes of all of them
+    rcu_device* dev;
+    void* block = nullptr;
+    std::vector<std::pair<const rcu_lazy*, void*>> made;
+    explicit Converted(rcu_device* d) : dev(d) {}
+    ~Converted() {
+        if (block) rcu_free(dev, block);          // the pool reuses blocks in stream order
+    }
+    void* of(const rcu_lazy* w) const {
+        for (auto& m : made)
+            if (m.first == w) return m.second;
+        return nullptr;
+    }
+    static const rcu_lazy* weight(const rcu_lazy* t, const fusion::Op* op) {
+        const bool fused = op && op->kind == fusion::LINEAR;
+        if (!fused && (op || t->kind != K_MATMUL || t->flags[0] || !t->flags[1] || !t->flags[2])) return nullptr;
+        const rcu_lazy *w = fused ? op->w : t->srcs[0], *x = fused ? op->x : t->srcs[1];
+        if (!dt_is_q8(w->dt) || w->rank != 2 || !w->resolved() || w->numel() > kNumel || x->shape[x->rank - 1] != w->shape[1] || !fusion::Pass::aligned(w)) return nullptr;
+        return rcu_linear_converts(w->dt, x->dt, x->numel() / w->shape[1], w->shape[0], w->shape[1]) ? w : nullptr;
+    }
+    rcu_status make(const std::vector<rcu_lazy*>& order, const fusion::Pass& fused) {
+        uint64_t total = 0;
+        for (rcu_lazy* t : order) {
+            if (t->resolved() || fused.absorbed(t)) continue;
+            const rcu_lazy* w = weight(t, fused.find(t));
+            if (!w || of(w)) continue;
+            const uint64_t bytes = align256(w->numel() * dt_esize(rcu_activation_dtype(w->dt)));
+            if (total + bytes > kTotal) break;
+            made.emplace_back(w, (void*)total);
+            total += bytes;
+        }
+        if (made.size() < 2) {
+            made.clear();
+            return RCU_OK;
+        }
+        const rcu_status st = rcu_alloc(dev, total, &block);
+        if (st != RCU_OK) {
+            made.clear();                          // beside their products, as large ones
+            return RCU_OK;
+        }
+        for (auto& m : made) m.second = (char*)block + (uint64_t)m.second;
+        for (const int dt : {RCU_Q8_0H, RCU_Q8_0F}) {
+            std::vector<DequantItem> items;
+            for (size_t i = 0; i <= made.size(); ++i) {
+                if (i < made.size() && made[i].first->dt == dt) items.push_back(DequantItem{made[i].first->storage->ptr, made[i].second, made[i].first->numel()});
+                if (items.empty() || (items.size() < (size_t)kDequantItems && i < made.size())) continue;
+                const rcu_status s2 = rcu_dequantize_items(dev, dt, items.data(), (int)items.size());
+                if (s2 != RCU_OK) return s2;
+                items.clear();
+            }
+        }
+        return RCU_OK;
+    }
 };
 
 rcu_status resolve(rcu_lazy* out) {
@@ -502,6 +565,8 @@ rcu_status resolve(rcu_lazy* out) {
     struct TimedNode { std::string key; uint64_t bytes; cudaEvent_t e0, e1; };
     std::vector<TimedNode> timed;
     fusion::RopeTables rope_tables(dev);
+    Converted converted(dev);
+    if (!no_reuse && !profile && (st = converted.make(order, fused)) != RCU_OK) return st;
     uint32_t launched = 0, n_inplace = 0;
     const uint64_t launches0 = dev->launches;
     for (size_t i = 0; i < n; ++i) {
@@ -526,7 +591,8 @@ rcu_status resolve(rcu_lazy* out) {
             if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) return rcu_fail(dev, RCU_ERR_CUDA, "resolve: cudaEventCreate");
             cudaEventRecord(e0, dev->stream);
         }
-        st = op ? fusion::run(dev, t, *op, &rope_tables) : run_node(t);
+        void* cw = converted.made.empty() ? nullptr : op ? (op->kind == fusion::LINEAR ? converted.of(op->w) : nullptr) : t->kind == K_MATMUL ? converted.of(t->srcs[0]) : nullptr;
+        st = op ? fusion::run(dev, t, *op, &rope_tables, cw) : run_node(t, cw);
         if (st != RCU_OK) return st;
         if (profile) {
             cudaEventRecord(e1, dev->stream);

@@ -539,7 +539,7 @@ struct RopeTables {
     }
 };
 
-rcu_status run(rcu_device* dev, rcu_lazy* t, const Op& op, RopeTables* tables) {
+rcu_status run(rcu_device* dev, rcu_lazy* t, const Op& op, RopeTables* tables, void* converted) {
     HeadsRope rope = op.rope;
     if (op.kind == HEADS || (op.kind == APPEND && !op.copied)) {
         const rcu_status st = tables->of(&rope, op.T);
@@ -602,7 +602,7 @@ rcu_status run(rcu_device* dev, rcu_lazy* t, const Op& op, RopeTables* tables) {
             c.op = op.act;
             c.glu = op.glu;
             c.x_pitch = op.x->shape[op.x->rank - 1];
-            return rcu_gemm_tc_chain(dev, op.w->dt, op.w->storage->ptr, (const char*)op.x->storage->ptr + op.x_col * 2, t->storage->ptr, op.M, op.N, op.K, c);
+            return rcu_gemm_tc_chain(dev, converted ? RCU_F16 : op.w->dt, converted ? converted : op.w->storage->ptr, (const char*)op.x->storage->ptr + op.x_col * 2, t->storage->ptr, op.M, op.N, op.K, c);
         }
         default: return rcu_fail(dev, RCU_ERR_UNSUPPORTED, "resolve: fused op %d", op.kind);
     }

@@ -38,3 +38,14 @@ struct LinearChain {
 };
 bool rcu_gemm_tc_chain_takes(rcu_device* dev, int w_dt, uint64_t M, uint64_t N, uint64_t K, bool glu, bool act);
 rcu_status rcu_gemm_tc_chain(rcu_device* dev, int w_dt, const void* w, const void* x, void* y, uint64_t M, uint64_t N, uint64_t K, const LinearChain& c);
+
+// The Linears of a resolve whose weights are converted once per product (gemm_tc.cu, matmul.cu), converted together: small matrices, in one launch
+struct DequantItem {
+    const void* src;                    // Q8_0 segments
+    void* dst;
+    uint64_t numel;
+};
+constexpr int kDequantItems = 32;       // of one launch
+rcu_status rcu_dequantize_items(rcu_device* dev, int dt, const DequantItem* items, int n);
+// whether a Linear over M rows of activations converts its weights of this type in a launch of its own
+bool rcu_linear_converts(int w_dt, int act_dt, uint64_t M, uint64_t N, uint64_t K);
