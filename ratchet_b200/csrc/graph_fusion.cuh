@@ -105,8 +105,10 @@ struct Pass {
     // a cache that returns [1, H, L, D] and feeds only the attention: its tensor's rows in place
     Heads from_cache(rcu_lazy* x, std::vector<rcu_lazy*>* appends) const {
         if (!inner(x, K_CACHE, RCU_F16) || x->rank != 4 || x->u[0] != 2) return Heads{};
+        const rcu_lazy* src = x->srcs[1];
         rcu_lazy* c = x->srcs[0];
         if (!c->resolved() || c->rank != 4 || c->shape[0] != 1 || !aligned(c) || owners(c) != 1) return Heads{};
+        if (src->shape[0] != 1 || src->shape[1] != c->shape[1] || src->shape[3] != c->shape[3]) return Heads{};      // rcu_cache refuses it
         appends->push_back(x);
         return Heads{c, 0, c->shape[2] * c->shape[3], c->shape[3]};
     }

@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 from ratchet_b200 import callers, capi, nn
+from ratchet_b200.capi import RatchetCudaError
 
 pytestmark = pytest.mark.gpu
 F16 = np.float16
@@ -120,6 +121,33 @@ def test_scores_beyond_f16_behave_as_in_the_graph(dev):
     assert any(n.startswith("attention") for n in names)
     assert np.array_equal(np.isnan(got), np.isnan(want))
     close(np.nan_to_num(got), np.nan_to_num(want), "large")
+
+
+# what a source has where the cache has one batch entry, two heads of 64
+@pytest.mark.parametrize("B,H,D", [(1, 1, 64), (1, 4, 64), (1, 2, 32), (1, 2, 128), (2, 2, 64)])
+@pytest.mark.parametrize("rotated", [False, True])
+def test_a_source_that_differs_from_its_cache_is_refused(dev, B, H, D, rotated):
+    T, h, d = 40, 2, 64
+    g = np.random.Generator(np.random.PCG64(H * D))
+    held = [tensor(dev, g.standard_normal((1, h, 48, d)).astype(F16)) for _ in range(2)]
+    before = [c.to_numpy() for c in held]
+    q = tensor(dev, g.standard_normal((1, h, T, d)).astype(F16))
+    scale, rows = tensor(dev, np.array([0.125], np.float32)), g.standard_normal((B, T, H * D)).astype(F16)
+
+    def source():
+        s = tensor(dev, rows).view([B, T, H, D]).permute([0, 2, 1, 3])
+        return s.full().rope(32, 10000.0, 0).half() if rotated else s
+
+    k = held[0].cache(source(), 2, 0)
+    v = held[1].cache(source(), 2, 0)
+    z = q.full().matmul(k.full(), False, True).mul(scale).half()
+    del k
+    out = z.full().softmax(3).half().matmul(v, False, False).permute([0, 2, 1, 3])
+    del z, v
+    with pytest.raises(RatchetCudaError, match="source differs from cache"):
+        out.resolve()
+    for c, b in zip(held, before):
+        assert np.array_equal(c.to_numpy(), b)
 
 
 def test_held_tensors_are_computed(dev):
