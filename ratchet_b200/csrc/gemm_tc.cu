@@ -407,8 +407,14 @@ bool rcu_gemm_tc2_eligible(rcu_device* dev, uint64_t M, uint64_t N, uint64_t K);
 rcu_status rcu_gemm_tc2_launch(rcu_device* dev, const void* w, const void* x, const void* bias, void* y, uint64_t M, uint64_t N, uint64_t K,
                                const TcLinear& t);
 
-// Beyond this many token rows quantised weights are converted once per product (below)
+// Quantised weights.  The fused kernel converts a weight tile once per 128-row token tile, i.e. M/128 times over the whole problem, and it is the
+// one-CTA kernel.  Beyond kFusedMaxM token rows it is cheaper to convert the matrix once into pooled f16 scratch (which stays in L2) and
+// run the f16 kernels on it (M = 512, N = 8192, K = 3072, Q4_K: 34 us against 46 us fused).  RCU_GEMM_FUSED=0/1 forces either path.
 constexpr uint64_t kFusedMaxM = 256;
+static bool converts_once(uint64_t M) {
+    const char* force = getenv("RCU_GEMM_FUSED");
+    return force ? atoi(force) == 0 : M > kFusedMaxM;
+}
 
 // The Linear of an f16 graph with what follows it (TcLinear: chained, or glu): whether the tensor-core kernels take it.  A gate and its up
 // columns meet in one tile of the pair kernel only, so that form wants f16 weights, or as many rows as have them converted.  An activation
@@ -418,7 +424,7 @@ bool rcu_gemm_tc_chain_takes(rcu_device* dev, int w_dt, uint64_t M, uint64_t N, 
     if (w_dt == RCU_BF16) return glu && N % 16 == 0 && rcu_gemm_tc2_eligible(dev, M, N, K) && M <= 0x7fffffffull && N <= 0x7fffffffull && K <= 0x7fffffffull;
     if (!rcu_gemm_tc_eligible(w_dt, RCU_F16, M, N, K) || N % 8 != 0) return false;
     if (!glu && !act) return M > 32;               // fewer rows: gemm_rows.cu
-    return N % 16 == 0 && (w_dt == RCU_F16 || M > kFusedMaxM) && rcu_gemm_tc2_eligible(dev, M, N, K);
+    return N % 16 == 0 && (w_dt == RCU_F16 || converts_once(M)) && rcu_gemm_tc2_eligible(dev, M, N, K);
 }
 
 rcu_status rcu_gemm_tc_dispatch(rcu_device* dev, int lhs_dt, const void* w, int act_dt, const void* x, const void* bias, void* y,
@@ -427,26 +433,18 @@ rcu_status rcu_gemm_tc_dispatch(rcu_device* dev, int lhs_dt, const void* w, int 
     if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(w)) & 15) return RCU_ERR_UNSUPPORTED;
     DevGuard g(dev->ordinal);
     if (lhs_dt == RCU_F16 && rcu_gemm_tc2_eligible(dev, M, N, K)) return rcu_gemm_tc2_launch(dev, w, x, bias, y, M, N, K, t);
-    // Quantised weights.  The fused kernel converts a weight tile once per 128-row token tile, i.e.
-    // M/128 times over the whole problem, and it is the one-CTA kernel.  Beyond kFusedMaxM token rows it
-    // is cheaper to convert the matrix once into pooled f16 scratch (which stays in L2) and run the f16
-    // kernels on it (M = 512, N = 8192, K = 3072, Q4_K: 34 us against 46 us fused).  RCU_GEMM_FUSED=0/1
-    // forces either path.
-    if (lhs_dt != RCU_F16) {
-        const char* force = getenv("RCU_GEMM_FUSED");
-        const bool fused = force ? atoi(force) != 0 : M <= kFusedMaxM;
-        if (!fused) {
-            void* scratch = nullptr;
-            rcu_status st = rcu_alloc(dev, N * K * 2, &scratch);
-            if (st != RCU_OK) return st;
-            rcu_tensor src{lhs_dt, 2, {N, K, 1, 1}, const_cast<void*>(w)};
-            rcu_tensor dst{RCU_F16, 2, {N, K, 1, 1}, scratch};
-            st = rcu_dequantize(dev, &src, &dst);
-            if (st == RCU_OK) st = rcu_gemm_tc_dispatch(dev, RCU_F16, scratch, act_dt, x, bias, y, M, N, K, t);
-            rcu_free(dev, scratch);   // the pool reuses blocks in stream order
-            return st;
-        }
+    if (lhs_dt != RCU_F16 && converts_once(M)) {
+        void* scratch = nullptr;
+        rcu_status st = rcu_alloc(dev, N * K * 2, &scratch);
+        if (st != RCU_OK) return st;
+        rcu_tensor src{lhs_dt, 2, {N, K, 1, 1}, const_cast<void*>(w)};
+        rcu_tensor dst{RCU_F16, 2, {N, K, 1, 1}, scratch};
+        st = rcu_dequantize(dev, &src, &dst);
+        if (st == RCU_OK) st = rcu_gemm_tc_dispatch(dev, RCU_F16, scratch, act_dt, x, bias, y, M, N, K, t);
+        rcu_free(dev, scratch);   // the pool reuses blocks in stream order
+        return st;
     }
+    if (t.glu >= 0 || t.chain_op >= 0) return RCU_ERR_UNSUPPORTED;      // the one-CTA kernel stores every column, as the product gives it
     // tile width: enough CTAs to cover the SMs when M is small
     const uint64_t tiles128 = ((M + TM - 1) / TM) * ((N + 127) / 128);
     int bn = tiles128 >= (uint64_t)dev->sm_count ? 128 : 64;
@@ -569,6 +567,6 @@ rcu_status rcu_gemm_tc_chain(rcu_device* dev, int w_dt, const void* w, const voi
 
 bool rcu_gemm_tc_f32_eligible(int lhs_dt, int act_dt, uint64_t M, uint64_t N, uint64_t K);
 bool rcu_linear_converts(int w_dt, int act_dt, uint64_t M, uint64_t N, uint64_t K) {
-    if (w_dt == RCU_Q8_0H && act_dt == RCU_F16) return M > kFusedMaxM && rcu_gemm_tc_eligible(w_dt, act_dt, M, N, K) && !getenv("RCU_GEMM_FUSED");
+    if (w_dt == RCU_Q8_0H && act_dt == RCU_F16) return M > kFusedMaxM && converts_once(M) && rcu_gemm_tc_eligible(w_dt, act_dt, M, N, K);
     return w_dt == RCU_Q8_0F && act_dt == RCU_F32 && rcu_gemm_tc_f32_eligible(RCU_F32, RCU_F32, M, N, K);
 }

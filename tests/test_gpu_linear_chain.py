@@ -104,3 +104,24 @@ def test_a_product_that_is_kept_is_computed(dev):
     z = h.full().gelu().cast(capi.F16).add(h)
     del h
     assert np.isfinite(z.resolve().to_numpy()).all()
+
+
+# rows on either side of the rule that the switch overrides, as many columns as the pair kernel wants
+@pytest.mark.parametrize("fused", ["0", "1"])
+@pytest.mark.parametrize("M,F,K", [(256, 4752, 64), (600, 1600, 512)])
+@pytest.mark.parametrize("what", ["gate", "gelu", "resid"])
+def test_with_the_conversion_forced(dev, monkeypatch, fused, M, F, K, what):
+    monkeypatch.setenv("RCU_GEMM_FUSED", fused)
+    g = np.random.Generator(np.random.PCG64(M))
+    w, x, r = weight(dev, g, "q8_0h", 2 * F, K), g.standard_normal((1, M, K)).astype(F16), g.standard_normal((1, M, 2 * F)).astype(F16)
+
+    def build():
+        h = nn.Linear(w).schedule(tensor(dev, x))
+        if what == "gelu":
+            return h.full().gelu().cast(capi.F16)
+        if what == "resid":
+            return h.add(tensor(dev, r))
+        return h.slice([(0, 1), (0, M), (F, 2 * F)]).mul(h.slice([(0, 1), (0, M), (0, F)]).full().silu().cast(capi.F16))
+
+    (got, _), (want, _) = both(dev, build)
+    assert np.array_equal(got, want)
