@@ -499,7 +499,8 @@ rcu_status rcu_gemm_tc_batched_f16(rcu_device* dev, const void* w, const void* x
     if (M < 32 || N < 64 || K < 64 || pitch_w % 8 != 0 || pitch_x % 8 != 0 || batch == 0 || batch > 65535) return RCU_ERR_UNSUPPORTED;
     if (M > 0x7fffffffull || N > 0x7fffffffull || K > 0x7fffffffull) return RCU_ERR_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) return RCU_ERR_UNSUPPORTED;
-    if (N % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & 7)) return RCU_ERR_UNSUPPORTED;
+    // rows that start on four columns are stored by fours, and slices of K are summed by eights
+    if (N % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & (N % 8 == 0 ? 15 : 7))) return RCU_ERR_UNSUPPORTED;
     DevGuard g(dev->ordinal);
     const uint64_t tiles128 = ((M + TM - 1) / TM) * ((N + 127) / 128) * batch;
     const int bn = (tiles128 >= (uint64_t)dev->sm_count && N >= 128) ? 128 : 64;

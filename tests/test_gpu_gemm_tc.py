@@ -64,6 +64,20 @@ def test_gemm_tc_batched_f16(dev, b, M, K, N, trans_rhs):
     check(y.to_numpy(), ref, 1e-2, f"batched f16 {b}x{M}x{K}x{N}")
 
 
+# outputs that start on 8 bytes only: columns in eights and a K that is cut into slices, eights without slices, fours
+@pytest.mark.parametrize("b,M,K,N", [(1, 256, 1024, 64), (2, 130, 128, 72), (1, 256, 1024, 68)])
+def test_gemm_tc_batched_f16_into_an_output_between_vectors(dev, b, M, K, N):
+    from ratchet_b200 import capi
+    rng = np.random.Generator(np.random.PCG64(K + N))
+    a, w = rng.standard_normal((b, M, K)).astype(np.float16), (rng.standard_normal((b, K, N)) * 0.1).astype(np.float16)
+    held = dev.zeros(capi.F16, (b * M * N + 16,))
+    out = dev.wrap(capi.F16, (b, M, N), held.ptr + 8)
+    dev.matmul(dev.from_numpy(a), dev.from_numpy(w), None, out=out)
+    check(out.to_numpy(), a.astype(np.float64) @ w.astype(np.float64), 1e-2, f"{b}x{M}x{K}x{N}")
+    edge = held.to_numpy()
+    assert not edge[:4].any() and not edge[4 + b * M * N:].any()
+
+
 @pytest.mark.parametrize("kind", ["Q8_0H", "Q4_KH"])
 @pytest.mark.parametrize("M,N,K", [(128, 512, 768), (512, 256, 3072), (77, 96, 512), (64, 512, 2048), (48, 1024, 4096)])
 def test_gemm_tc_quantised(dev, kind, M, N, K):
