@@ -172,7 +172,9 @@ gemm_rows_kernel(const RowsWeights w, const __half* __restrict__ x, const __half
     };
 #pragma unroll
     for (int p = 0; p < PF; ++p) fetch(p, warp + p * kRowsWarps);
-    if (early) asm volatile("griddepcontrol.wait;" ::: "memory");       // the weights stay as they are; x may be the predecessor's output
+    // early: the weights stay as they are (the resolver knows; a caller's rcu_set_constant_weights speaks of matrix-vector products only); x may
+    // be the predecessor's output
+    if (early) asm volatile("griddepcontrol.wait;" ::: "memory");
 
     float acc[RT][NT][4];
 #pragma unroll
@@ -245,7 +247,7 @@ rcu_status launch_rows(rcu_device* dev, const RowsWeights& w, const void* x, con
     constexpr int ROWS = RT * 16;
     const dim3 grid((N + ROWS - 1) / ROWS, (M + NT * 8 - 1) / (NT * 8));
     RCU_CUDA(dev, rcu_launch(dev, gemm_rows_kernel<WT, NT, RT, PF>, grid, kRowsWarps * 32, 0, w, (const __half*)x, (const __half*)bias, (__half*)y, M, N, K,
-                             dev->const_weights ? 1 : 0));
+                             dev->resident_weights ? 1 : 0));
     RCU_LAUNCH_CHECK(dev);
     return RCU_OK;
 }

@@ -294,10 +294,12 @@ rcu_status run_node(rcu_lazy* n, void* converted) {
                 l.data = converted;
             }
             if (n->srcs.size() > 2) bias = S(2);
-            // weights that were uploaded and waited for cannot be written by anything in flight: the GEMV may start early
+            // weights that were uploaded and waited for cannot be written by anything in flight: the product may start early on them
             const bool before = dev->const_weights;
-            if (n->srcs[0]->resident_const) dev->const_weights = true;
+            dev->resident_weights = n->srcs[0]->resident_const;
+            if (dev->resident_weights) dev->const_weights = true;
             const rcu_status st = rcu_matmul(dev, &l, &r, n->srcs.size() > 2 ? &bias : nullptr, n->flags[0], n->flags[1], n->flags[2], &dst);
+            dev->resident_weights = false;
             dev->const_weights = before;
             return st;
         }

@@ -76,3 +76,31 @@ def test_q8_0f_at_any_number_of_rows(dev, M, N, K):
                                         ("f32", 2, 64, 32), ("f32", 31, 67, 128), ("f32", 65, 130, 2048), ("f32", 200, 129, 96)])
 def test_any_number_of_features(dev, kind, M, N, K):
     run(dev, kind, M, N, K, with_bias=True)
+
+
+# the promise is about matrix-vector products: a matrix written right before it is multiplied by a few rows is read as written
+@pytest.mark.parametrize("kind,M", [("f16", 8), ("f16", 2), ("q8_0f", 20), ("q8_0f", 100)])
+def test_weights_that_were_just_written_under_constant_weights(dev, kind, M):
+    from ratchet_b200 import capi
+    N, K = 2048, 1024
+    g = np.random.Generator(np.random.PCG64(M))
+    x = dev.from_numpy(g.standard_normal((M, K)).astype(np.float16))
+    dense = [(g.standard_normal((N, K)) * 0.05).astype(np.float32) for _ in range(2)]
+    if kind == "f16":
+        sources = [dev.from_quantized(orc.quantize_q8(d.astype(np.float16)), capi.Q8_0H, (N, K)) for d in dense]
+        w, write = dev.empty(capi.F16, (N, K)), dev.dequantize
+    else:
+        sources = [dev.from_numpy(d) for d in dense]
+        w, write = dev.empty(capi.Q8_0F, (N, K)), dev.quantize
+    want = []
+    for s in sources:
+        write(s, w)
+        want.append(dev.matmul(w, x, None, False, True, True).to_numpy())
+    assert not np.array_equal(*want)
+    dev.set_constant_weights(True)
+    try:
+        for i in range(60):
+            write(sources[i % 2], w)
+            assert np.array_equal(dev.matmul(w, x, None, False, True, True).to_numpy(), want[i % 2])
+    finally:
+        dev.set_constant_weights(False)
