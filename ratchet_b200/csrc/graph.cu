@@ -295,8 +295,9 @@ rcu_status run_node(rcu_lazy* n, void* converted) {
             }
             if (n->srcs.size() > 2) bias = S(2);
             // weights that were uploaded and waited for cannot be written by anything in flight: the product may start early on them
+            // (converted ones have just been written)
             const bool before = dev->const_weights;
-            dev->resident_weights = n->srcs[0]->resident_const;
+            dev->resident_weights = n->srcs[0]->resident_const && !converted;
             if (dev->resident_weights) dev->const_weights = true;
             const rcu_status st = rcu_matmul(dev, &l, &r, n->srcs.size() > 2 ? &bias : nullptr, n->flags[0], n->flags[1], n->flags[2], &dst);
             dev->resident_weights = false;
@@ -406,6 +407,11 @@ struct Converted {
         for (auto& m : made)
             if (m.first == w) return m.second;
         return nullptr;
+    }
+    // for the product of node `t`: another one over the same weights, of fewer rows or without the Linear convention, reads them as stored
+    void* of(const rcu_lazy* t, const fusion::Op* op) const {
+        const rcu_lazy* w = made.empty() ? nullptr : weight(t, op);
+        return w ? of(w) : nullptr;
     }
     static const rcu_lazy* weight(const rcu_lazy* t, const fusion::Op* op) {
         const bool fused = op && op->kind == fusion::LINEAR;
@@ -593,7 +599,7 @@ rcu_status resolve(rcu_lazy* out) {
             if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) return rcu_fail(dev, RCU_ERR_CUDA, "resolve: cudaEventCreate");
             cudaEventRecord(e0, dev->stream);
         }
-        void* cw = converted.made.empty() ? nullptr : op ? (op->kind == fusion::LINEAR ? converted.of(op->w) : nullptr) : t->kind == K_MATMUL ? converted.of(t->srcs[0]) : nullptr;
+        void* cw = converted.of(t, op);
         st = op ? fusion::run(dev, t, *op, &rope_tables, cw) : run_node(t, cw);
         if (st != RCU_OK) return st;
         if (profile) {
