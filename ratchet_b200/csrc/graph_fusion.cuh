@@ -371,8 +371,10 @@ struct Pass {
         if (inner(b, K_CAST, RCU_F16) && b->srcs[0]->dt == RCU_F32) {
             seen->push_back(b);
             op->bias32 = b->srcs[0];
-        } else {
+        } else if (b->dt == RCU_F16) {
             op->bias = b;
+        } else {
+            return false;                // rcu_matmul refuses it
         }
         op->srcs.push_back(op->bias32 ? op->bias32 : op->bias);
         return true;

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from ratchet_b200 import capi, nn
+from ratchet_b200.capi import RatchetCudaError
 
 pytestmark = pytest.mark.gpu
 F16 = np.float16
@@ -125,3 +126,18 @@ def test_with_the_conversion_forced(dev, monkeypatch, fused, M, F, K, what):
 
     (got, _), (want, _) = both(dev, build)
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("M", [20, 64, 600])
+@pytest.mark.parametrize("what", ["alone", "gelu", "resid"])
+def test_a_bias_of_another_type_is_refused(dev, M, what):
+    g = np.random.Generator(np.random.PCG64(M))
+    N, K = 3328, 128
+    w, x = weight(dev, g, "f16", N, K), tensor(dev, g.standard_normal((1, M, K)).astype(F16))
+    h = w.gemm(x, tensor(dev, g.standard_normal(N).astype(np.float32)), False, True, True)
+    if what == "gelu":
+        h = h.full().gelu().cast(capi.F16)
+    if what == "resid":
+        h = h.add(tensor(dev, g.standard_normal((1, M, N)).astype(F16)))
+    with pytest.raises(RatchetCudaError, match="DType mismatch: bias"):
+        h.resolve()
