@@ -286,7 +286,8 @@ struct Pass {
         op->rope.dim = rope->u[0];
         op->rope.base = rope->f[1];
         op->rope.offset = rope->u[1];
-        return vectors(op->q) && op->D % 8 == 0 && op->rope.dim % 16 == 0 && (uint64_t)op->T * op->D <= 0x7fffffffull;
+        // (rcu_rope refuses no features, and more than there are)
+        return vectors(op->q) && op->D % 8 == 0 && op->rope.dim > 0 && op->rope.dim <= op->D && op->rope.dim % 16 == 0 && (uint64_t)op->T * op->D <= 0x7fffffffull;
     }
 
     bool free_of(const std::vector<rcu_lazy*>& seen) const {

@@ -150,6 +150,25 @@ def test_a_source_that_differs_from_its_cache_is_refused(dev, B, H, D, rotated):
         assert np.array_equal(c.to_numpy(), b)
 
 
+@pytest.mark.parametrize("dim", [0, 15, 80])
+@pytest.mark.parametrize("cached", [False, True])
+def test_a_rotation_of_no_features_or_too_many_is_refused(dev, dim, cached):
+    T, H, D = 24, 2, 64
+    g = np.random.Generator(np.random.PCG64(dim))
+    q, v, rows = (tensor(dev, g.standard_normal(s).astype(F16)) for s in ((1, H, T, D), (1, H, T, D), (1, T, H * D)))
+    k = rows.view([1, T, H, D]).permute([0, 2, 1, 3]).full().rope(dim, 10000.0, 0).half()
+    if cached:
+        held = tensor(dev, np.zeros((1, H, 32, D), F16))
+        z = q.full().matmul(held.cache(k, 2, 0).full(), False, True).mul(tensor(dev, np.array([0.125], np.float32))).half()
+        del k
+        out = z.full().softmax(3).half().matmul(v, False, False).permute([0, 2, 1, 3])
+        del z
+    else:
+        out = k
+    with pytest.raises(RatchetCudaError, match="rope: dim must be even"):
+        out.resolve()
+
+
 def test_held_tensors_are_computed(dev):
     """A score matrix or a cache's result that the caller keeps is there afterwards: no fusion passes over it."""
     T, H, D = 40, 2, 64
