@@ -458,6 +458,7 @@ struct Converted {
 rcu_status resolve(rcu_lazy* out) {
     rcu_device* dev = out->dev;
     if (out->resolved()) return RCU_OK;
+    DevGuard guard(dev->ordinal);                // of the fused kernels' launches, copies and attributes: the ops' entry points have one each
     Order nodes;
     rcu_status st = execution_order(out, &nodes, true);
     if (st != RCU_OK) return st;

@@ -219,3 +219,18 @@ def test_activation_and_gate_between_casts(dev, shape):
 
     (got, _, names), (want, _, _) = both(dev, gate)
     assert any(n.startswith("glu chain") for n in names) == (F % 8 == 0) and np.array_equal(got, want, equal_nan=True)
+
+
+def test_a_prompt_on_a_device_that_is_not_the_current_one():
+    import torch
+    from ratchet_b200 import Device
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs 2 GPUs")
+    torch.cuda.set_device(0)
+    other, x = Device(1), np.random.Generator(np.random.PCG64(4)).standard_normal((1, 40, 128)).astype(F16)
+    try:
+        mha = callers.WhisperMHA(*[nn.Linear(tensor(other, np.eye(128, dtype=F16))) for _ in range(4)], 2, tensor(other, np.array([0.35], F16)))
+        assert np.isfinite(mha.schedule(nn.RMSNorm(tensor(other, np.ones(128, np.float32)), 1e-5).schedule(tensor(other, x))).resolve().to_numpy()).all()
+        assert torch.cuda.current_device() == 0
+    finally:
+        other.close()

@@ -59,3 +59,12 @@ def test_builders_validate_without_a_device():
     assert lib.rcu_lazy_binary(0, a, h, C.byref(out)) == capi.ERR_INVALID_ARG      # dtype mismatch
     for t in (a, b, h):
         lib.rcu_lazy_release(t)
+
+
+def test_a_resolve_makes_its_device_the_current_one():
+    """The fused kernels' entry points leave that to the resolver, which has to do it before the first of them (and before it converts weights)."""
+    import os
+    from ratchet_b200 import _build
+    with open(os.path.join(_build.CSRC, "graph.cu")) as f:
+        body = f.read().split("rcu_status resolve(rcu_lazy* out) {")[1]
+    assert 0 < body.find("DevGuard") < min(body.find(s) for s in ("converted.make", "fusion::run", "cudaEventCreate"))
