@@ -51,7 +51,8 @@ struct Pass {
     static constexpr int kPlain = -1, kPassed = -2;
     std::deque<Op> ops;
     std::vector<int> role;                          // by position in the order: the op whose result the node is, or no kernel nor buffer (kPassed)
-    std::vector<rcu_lazy*> writers;                 // nodes that write into a tensor which is there already
+    struct Written { const rcu_lazy* t; const char *begin, *end; };      // begin null: not resolved
+    std::vector<Written> written;                   // tensors that a node of this graph writes into, once per node
 
     int role_of(const rcu_lazy* t) const {
         const uint32_t at = order.at(t);
@@ -62,12 +63,21 @@ struct Pass {
         const int r = role_of(t);
         return r < 0 ? nullptr : &ops[r];
     }
-    void pass(const std::vector<rcu_lazy*>& seen) {
+    // `root` becomes the op, the nodes behind it are passed over: unless one of them has a part already, or a node that comes between where
+    // they stood and where the op runs may write into what the op reads (a cache's rows that the op's own appends write are not in `reads`)
+    bool give(const rcu_lazy* root, Op&& op, const std::vector<rcu_lazy*>& seen, const std::vector<rcu_lazy*>& reads) {
+        for (const rcu_lazy* t : seen)
+            if (absorbed(t) || find(t)) return false;
+        for (const rcu_lazy* t : reads)
+            if (t && writes_to(t) > 0) return false;
         for (const rcu_lazy* t : seen) role[order.at(t)] = kPassed;
-    }
-    void give(const rcu_lazy* root, Op&& op) {
         role[order.at(root)] = (int)ops.size();
         ops.push_back(std::move(op));
+        return true;
+    }
+    bool give(const rcu_lazy* root, Op&& op, const std::vector<rcu_lazy*>& seen) {
+        const std::vector<rcu_lazy*> reads = op.srcs;
+        return give(root, std::move(op), seen, reads);
     }
 
     // The operand [1, H, T, D] `x` as strides into the tensor behind its permute, view and slice, where these are its own; `seen` receives
@@ -96,9 +106,15 @@ struct Pass {
 
     static bool vectors(const Heads& h) { return h.base && h.offset % 8 == 0 && h.head % 8 == 0 && h.row % 8 == 0 && aligned(h.base); }
 
+    // the tensor whose memory `t` is
+    static const rcu_lazy* viewed(const rcu_lazy* t) {
+        while (!t->resolved() && t->kind == K_VIEW) t = t->srcs[0];
+        return t;
+    }
+
     // whether the kernels' 16-byte accesses fit: pool blocks do, a tensor over memory of the caller's may not
     static bool aligned(const rcu_lazy* t) {
-        while (!t->resolved() && t->kind == K_VIEW) t = t->srcs[0];
+        t = viewed(t);
         return !t->resolved() || (reinterpret_cast<uintptr_t>(t->storage->ptr) & 15) == 0;
     }
 
@@ -107,20 +123,18 @@ struct Pass {
         if (!inner(x, K_CACHE, RCU_F16) || x->rank != 4 || x->u[0] != 2) return Heads{};
         const rcu_lazy* src = x->srcs[1];
         rcu_lazy* c = x->srcs[0];
-        if (!c->resolved() || c->rank != 4 || c->shape[0] != 1 || !aligned(c) || owners(c) != 1) return Heads{};
+        if (!c->resolved() || c->rank != 4 || c->shape[0] != 1 || !aligned(c) || writes_to(c) != 1) return Heads{};
         if (src->shape[0] != 1 || src->shape[1] != c->shape[1] || src->shape[3] != c->shape[3]) return Heads{};      // rcu_cache refuses it
         appends->push_back(x);
         return Heads{c, 0, c->shape[2] * c->shape[3], c->shape[3]};
     }
 
-    // caches of this graph that write to the memory of `c`
-    int owners(const rcu_lazy* c) const {
-        const char *a = (const char*)c->storage->ptr, *b = a + c->nbytes();
+    // nodes of this graph that write into the memory of `t`
+    int writes_to(const rcu_lazy* t) const {
+        t = viewed(t);
+        const char *begin = t->resolved() ? (const char*)t->storage->ptr : nullptr, *end = begin ? begin + t->nbytes() : nullptr;
         int n = 0;
-        for (const rcu_lazy* t : writers) {
-            const char* p = (const char*)t->srcs[0]->storage->ptr;
-            if (p < b && p + t->srcs[0]->nbytes() > a) ++n;
-        }
+        for (const Written& w : written) n += w.t == t || (begin && w.begin && begin < w.end && w.begin < end);
         return n;
     }
 
@@ -153,6 +167,7 @@ struct Pass {
             z = x;
         }
         rcu_lazy *q, *k;
+        bool k_cached = false;
         if (inner(z, K_CAST, RCU_F16)) {            // f16(scale * f32(q) f32(k)^T)
             rcu_lazy* mul = z->srcs[0];
             if (!inner(mul, K_BINARY, RCU_F32) || mul->op != RCU_MUL || mul->srcs[1]->numel() != 1 || mul->srcs[1]->dt != RCU_F32) return false;
@@ -171,7 +186,8 @@ struct Pass {
             op.D = (uint32_t)q->shape[3];
             op.q = strides(q, false, &seen);
             op.k = from_cache(k, &appends);
-            if (!op.k.base) op.k = strides(k, false, &seen);
+            k_cached = op.k.base != nullptr;
+            if (!k_cached) op.k = strides(k, false, &seen);
         } else if (inner(z, K_MATMUL, RCU_F16) && !op.mask && z->srcs.size() == 2 && !z->flags[0] && !z->flags[1] && !z->flags[2]) {     // (q dk)(k^T dk)
             rcu_lazy *qm = z->srcs[0], *km = z->srcs[1];
             for (rcu_lazy* t : {qm, km})
@@ -192,7 +208,8 @@ struct Pass {
         }
         if (v->shape[2] != op.L) return false;
         op.v = from_cache(v, &appends);
-        if (!op.v.base) op.v = strides(v, false, &seen);
+        const bool v_cached = op.v.base != nullptr;
+        if (!v_cached) op.v = strides(v, false, &seen);
         if (!vectors(op.q) || !vectors(op.k) || !vectors(op.v)) return false;
         AttentionArgs a{};
         a.q = HeadRows{nullptr, op.q.head, op.q.row};
@@ -201,17 +218,15 @@ struct Pass {
         a.H = (int)op.H; a.T = (int)op.T; a.L = (int)op.L; a.D = (int)op.D; a.E = (int)op.E;
         a.mask = op.mask ? (const __half*)16 : nullptr;
         if (!rcu_attention_f16_takes(dev, a)) return false;
-        for (rcu_lazy* t : seen)
-            if (absorbed(t) || find(t)) return false;
+        std::vector<rcu_lazy*> reads = {op.q.base, op.mask, op.scale, op.scale_q, op.scale_k};
+        if (!k_cached) reads.push_back(op.k.base);
+        if (!v_cached) reads.push_back(op.v.base);
         op.srcs = {op.q.base, op.k.base, op.v.base};
         for (rcu_lazy* t : {op.mask, op.scale, op.scale_q, op.scale_k})
             if (t) op.srcs.push_back(t);
-        for (rcu_lazy* t : appends) {
-            op.srcs.push_back(t);                    // runs before the attention; holds no buffer
-            append(t);
-        }
-        pass(seen);
-        give(root, std::move(op));
+        op.srcs.insert(op.srcs.end(), appends.begin(), appends.end());       // these run before the attention and hold no buffer
+        if (!give(root, std::move(op), seen, reads)) return false;
+        for (rcu_lazy* t : appends) append(t);
         return true;
     }
 
@@ -254,11 +269,9 @@ struct Pass {
         op.v = strides(v, false, &seen, RCU_F32);
         for (const Heads* h : {&op.q, &op.k, &op.v})
             if (!h->base || h->offset % 4 || !aligned(h->base)) return false;
-        if (!rcu_attention_f32_takes(dev, args32(op)) || !free_of(seen)) return false;
+        if (!rcu_attention_f32_takes(dev, args32(op))) return false;
         op.srcs = {op.q.base, op.k.base, op.v.base, op.scale_q, op.scale_k};
-        pass(seen);
-        give(root, std::move(op));
-        return true;
+        return give(root, std::move(op), seen);
     }
 
     // sizes and pitches; no addresses
@@ -290,21 +303,13 @@ struct Pass {
         return vectors(op->q) && op->D % 8 == 0 && op->rope.dim > 0 && op->rope.dim <= op->D && op->rope.dim % 16 == 0 && (uint64_t)op->T * op->D <= 0x7fffffffull;
     }
 
-    bool free_of(const std::vector<rcu_lazy*>& seen) const {
-        for (rcu_lazy* t : seen)
-            if (absorbed(t) || find(t)) return false;
-        return true;
-    }
-
     bool heads(rcu_lazy* root) {
         Op op;
         std::vector<rcu_lazy*> seen;
-        if (!rotated(root, &op, &seen) || !free_of(seen)) return false;
+        if (!rotated(root, &op, &seen)) return false;
         op.kind = HEADS;
         op.srcs = {op.q.base};
-        pass(seen);
-        give(root, std::move(op));
-        return true;
+        return give(root, std::move(op), seen);
     }
 
     // the cache node `t` only appends: from where its source's heads come from, if these are its own
@@ -326,18 +331,17 @@ struct Pass {
                 op.q = strides(x, false, &seen);
                 direct = vectors(op.q) && op.D % 8 == 0 && (uint64_t)op.T * op.D <= 0x7fffffffull;
             }
-            direct = direct && free_of(seen);
         }
         if (direct) {
-            pass(seen);
+            const std::vector<rcu_lazy*> reads = {op.q.base};
             op.srcs = {t->srcs[0], op.q.base};
-        } else {
-            op = Op{};
-            op.kind = APPEND;
-            op.copied = true;
-            op.srcs = {t->srcs[0], x};
+            if (give(t, Op(op), seen, reads)) return;
         }
-        give(t, std::move(op));
+        op = Op{};
+        op.kind = APPEND;
+        op.copied = true;
+        op.srcs = {t->srcs[0], x};
+        give(t, std::move(op), {}, {});
     }
 
     // cast(op(cast x)) of an f16 tensor: the op, null if it is another graph
@@ -406,10 +410,7 @@ struct Pass {
             seen.push_back(g);
             op.act = t->op;
         }
-        if (!free_of(seen)) return false;
-        pass(seen);
-        give(root, std::move(op));
-        return true;
+        return give(root, std::move(op), seen);
     }
 
     // glu of a bf16 product that nothing else reads
@@ -426,20 +427,18 @@ struct Pass {
         op.M = l->numel() / op.N;
         op.glu = root->op;
         const uint64_t pitch = op.x->shape[op.x->rank - 1];
-        if (op.w->dt != RCU_BF16 || op.x->dt != RCU_BF16 || pitch % 8 || op.x_col % 8 || !aligned(op.w) || !aligned(op.x) || absorbed(l) || find(l) ||
+        if (op.w->dt != RCU_BF16 || op.x->dt != RCU_BF16 || pitch % 8 || op.x_col % 8 || !aligned(op.w) || !aligned(op.x) ||
             !rcu_gemm_tc_chain_takes(dev, RCU_BF16, op.M, op.N, op.K, true, false))
             return false;
         op.srcs = {op.w, op.x};
-        pass({l});
-        give(root, std::move(op));
-        return true;
+        return give(root, std::move(op), {l});
     }
 
     bool norm(rcu_lazy* root) {
         std::vector<rcu_lazy*> seen;
         rcu_lazy* t = between_casts(root, K_NORM, &seen);
         const uint64_t N = root->shape[root->rank - 1];
-        if (!t || t->op == RCU_GROUP_NORM || N % 8 || N > 8192 || rows_of(root) < 2 || rows_of(root) > 0x7fffffffull || !free_of(seen)) return false;
+        if (!t || t->op == RCU_GROUP_NORM || N % 8 || N > 8192 || rows_of(root) < 2 || rows_of(root) > 0x7fffffffull) return false;
         for (size_t i = 1; i < t->srcs.size(); ++i)
             if (t->srcs[i]->dt != RCU_F32 || t->srcs[i]->numel() != N || !aligned(t->srcs[i])) return false;
         if (!aligned(seen[1]->srcs[0])) return false;
@@ -447,21 +446,17 @@ struct Pass {
         op.kind = NORM;
         op.srcs = t->srcs;
         op.srcs[0] = seen[1]->srcs[0];
-        pass(seen);
-        give(root, std::move(op));
-        return true;
+        return give(root, std::move(op), seen);
     }
 
     bool act(rcu_lazy* root) {
         std::vector<rcu_lazy*> seen;
         rcu_lazy* t = between_casts(root, K_UNARY, &seen);
-        if (!t || (t->op != RCU_GELU && t->op != RCU_SILU) || root->numel() % 8 || rows_of(root) < 2 || !aligned(seen[1]->srcs[0]) || !free_of(seen)) return false;
+        if (!t || (t->op != RCU_GELU && t->op != RCU_SILU) || root->numel() % 8 || rows_of(root) < 2 || !aligned(seen[1]->srcs[0])) return false;
         Op op;
         op.kind = ACT;
         op.srcs = {seen[1]->srcs[0]};
-        pass(seen);
-        give(root, std::move(op));
-        return true;
+        return give(root, std::move(op), seen);
     }
 
     // up * cast(silu(cast gate)), gate and up the halves of one tensor's last dimension
@@ -481,7 +476,7 @@ struct Pass {
         if (r != up->rank || x->shape[r - 1] != 2 * F || F % 8 || F > 0x7fffffffull || gate->a[r - 1] != 0 || up->a[r - 1] != F || up->shape[r - 1] != F || gate->shape[r - 1] != F) return false;
         for (uint32_t i = 0; i + 1 < r; ++i)
             if (gate->a[i] || up->a[i] || gate->shape[i] != x->shape[i] || up->shape[i] != x->shape[i]) return false;
-        if (rows_of(root) < 2 || root->numel() * 2 != x->numel() || !aligned(x) || !free_of(seen)) return false;
+        if (rows_of(root) < 2 || root->numel() * 2 != x->numel() || !aligned(x)) return false;
         Op op;
         rcu_lazy* p = up->srcs[0];
         if (p->kind == K_MATMUL && !p->resolved() && p->refs.load() == 2 && !absorbed(p) && !find(p) && product(p, true, false, &op, &seen)) {       // gate and up are all that reads it
@@ -492,16 +487,20 @@ struct Pass {
             op.kind = GLU;
             op.srcs = {p};
         }
-        pass(seen);
-        give(root, std::move(op));
-        return true;
+        return give(root, std::move(op), seen);
     }
 
     // consumers before what they consume, so that a chain is recognised from its end
     Pass(rcu_device* d, const Order& o, bool on) : dev(d), order(o), role(o.nodes.size(), kPlain) {
         if (!on) return;
-        for (rcu_lazy* t : o.nodes)
-            if ((t->kind == K_CACHE || t->kind == K_INDEX_WRITE) && !t->resolved() && t->srcs[0]->resolved()) writers.push_back(t);
+        for (const rcu_lazy* t : o.nodes) {
+            if (t->resolved()) continue;
+            const bool first = t->kind == K_CACHE || t->kind == K_INDEX_WRITE, third = t->kind == K_LIGHTNING, fourth = t->kind == K_LATENT_APPEND || t->kind == K_KV_APPEND;
+            if (!first && !third && !fourth) continue;
+            const rcu_lazy* w = viewed(t->srcs[first ? 0 : third ? 2 : 3]);
+            const char* begin = w->resolved() ? (const char*)w->storage->ptr : nullptr;
+            written.push_back(Written{w, begin, begin ? begin + w->nbytes() : nullptr});
+        }
         for (size_t i = o.nodes.size(); i-- > 0;) {
             rcu_lazy* t = o.nodes[i];
             if (t->resolved() || absorbed(t) || find(t)) continue;

@@ -169,6 +169,54 @@ def test_a_rotation_of_no_features_or_too_many_is_refused(dev, dim, cached):
         out.resolve()
 
 
+# who appends: two caches; both to one; both to one, the second through a view; one whose rows are the queries
+@pytest.mark.parametrize("caches", ["apart", "one", "view", "late view", "queries"])
+def test_attention_over_caches_that_share_memory(dev, caches):
+    T, H, D, cap = 70, 2, 64, 70 if caches == "queries" else 80
+    g = np.random.Generator(np.random.PCG64(9))
+    arrays = [g.standard_normal((1, H, n, D)).astype(F16) for n in (T, T, T, cap, cap)]
+    scale = tensor(dev, np.array([0.125], np.float32))
+
+    def build():
+        q, ks, vs, kc, vc = (tensor(dev, a) for a in arrays)
+        held = [kc, vc]
+        if caches in ("one", "view"):
+            vc = kc if caches == "one" else kc.view([1, H, cap, D])
+            held = [kc]
+        if caches == "late view":                     # a view made before its tensor was there
+            kc = kc.mul(tensor(dev, np.array([1.0], F16)))
+            vc = kc.view([1, H, cap, D])
+            kc.resolve()
+            held = [kc]
+        if caches == "queries":
+            q = kc
+        z = q.full().matmul(kc.cache(ks, 2, 0).full(), False, True).mul(scale).half()
+        return z.full().softmax(3).half().matmul(vc.cache(vs, 2, 0), False, False).permute([0, 2, 1, 3]), held
+
+    (got, held, names), (want, held0, _) = both(dev, build)
+    assert any(n.startswith("attention") for n in names), names
+    close(got, want, caches)
+    for a, b in zip(held, held0):
+        assert np.array_equal(a, b)
+
+
+def test_an_operand_that_is_written_before_the_op_runs(dev):
+    """x W^T + r, where computing r appends to x: the product sees x as it was, as it does with one kernel per op."""
+    T, d = 64, 128
+    g = np.random.Generator(np.random.PCG64(10))
+    x, w, new = g.standard_normal((1, T, d)).astype(F16), (g.standard_normal((d, d)) / 11).astype(F16), g.standard_normal((1, T, d)).astype(F16)
+
+    def build():
+        held, wt = tensor(dev, x), tensor(dev, w)
+        h = wt.gemm(held, None, False, True, True)
+        r = held.cache(tensor(dev, new), 1, 0)
+        return h.add(r), [held]
+
+    (got, held, _), (want, held0, _) = both(dev, build)
+    assert np.array_equal(got, want) and np.array_equal(held[0], held0[0]) and np.array_equal(held[0], new)
+    close(got, x[0].astype(np.float64) @ w.astype(np.float64).T + new, "product", 1e-2)
+
+
 def test_held_tensors_are_computed(dev):
     """A score matrix or a cache's result that the caller keeps is there afterwards: no fusion passes over it."""
     T, H, D = 40, 2, 64
