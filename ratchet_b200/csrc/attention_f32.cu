@@ -233,7 +233,7 @@ attention_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                 tmem_ld_32x32(t + 128 + c, x);
                 tmem_ld_32x32(t + 192 + c, y);
 #pragma unroll
-                for (int j = 0; j < 32; ++j) acc[c + j] = fmaf(acc[c + j], corr, x[j] + y[j]);
+                for (int j = 0; j < 32; ++j) acc[c + j] = fmaf(acc[c + j], corr, main_and_small(x[j], y[j]));
             }
         };
         bool ok = true;
@@ -254,7 +254,7 @@ attention_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                 tmem_ld_32x32(t + c, s + c);
                 tmem_ld_32x32(t + 64 + c, y);
 #pragma unroll
-                for (int j = 0; j < 32; ++j) s[c + j] += y[j];
+                for (int j = 0; j < 32; ++j) s[c + j] = main_and_small(s[c + j], y[j]);
             }
             const int left = a.L - (first + n) * kTileK;
             if (left < kTileK) {

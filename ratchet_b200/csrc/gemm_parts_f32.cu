@@ -86,12 +86,12 @@ struct Walk {
     }
 };
 
-// two values into their three parts, packed (the first in the lower half)
+// Two values into their three parts, packed (the first in the lower half).  An infinity is its own leading part and leaves NaN for the others, as
+// NaN does (cvt keeps a NaN whose payload lies in the bits that are cut off): main_and_small has the rest.
 __device__ __forceinline__ void split3(float x, float y, uint32_t (&p)[3]) {
-    const uint32_t xb = __float_as_uint(x), yb = __float_as_uint(y);
-    p[0] = __byte_perm(xb, yb, 0x7632);
-    x -= __uint_as_float(xb & 0xffff0000u);
-    y -= __uint_as_float(yb & 0xffff0000u);
+    asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(p[0]) : "f"(y), "f"(x));
+    x -= __uint_as_float(p[0] << 16);
+    y -= __uint_as_float(p[0] & 0xffff0000u);
     const __nv_bfloat162 b = __floats2bfloat162_rn(x, y);
     p[1] = *reinterpret_cast<const uint32_t*>(&b);
     x -= __uint_as_float(p[1] << 16);
@@ -219,7 +219,7 @@ gemm_parts_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
                     tmem_ld_32x8(at + T, y);
                     tmem_ld_32x8(at + 2 * T, z);
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) acc[j + e] += x[e] + (y[e] + z[e]);
+                    for (int e = 0; e < 8; ++e) acc[j + e] += main_and_small(x[e], y[e] + z[e]);
                 }
                 tc_fence_before();
                 __syncwarp();

@@ -91,6 +91,10 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t* r)
         : "memory");
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
+// The sum of a product over operands in three bf16 parts: the leading parts' and the small ones'.  The latter is NaN exactly where an operand
+// is infinite or NaN (its remainders are), and then the leading parts alone are what f32 arithmetic gives; fminf takes the number.
+__device__ __forceinline__ float main_and_small(float main, float small) { return main + fminf(small, 3.402823466e+38f); }
+
 // 32 lanes x 8 consecutive f32 columns of tensor memory -> 8 registers per thread
 __device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, float* v) {
     uint32_t r[8];

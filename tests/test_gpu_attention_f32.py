@@ -56,8 +56,7 @@ def test_against_64_bits_and_the_unfused_graph(dev, T, H, D):
     want = ((p / p.sum(-1, keepdims=True)) @ v).transpose(1, 0, 2).reshape(1, T, d)
     n = np.linalg.norm(want)
     err, err0 = np.linalg.norm(got - want) / n, np.linalg.norm(chain - want) / n
-    print(f"T={T} H={H} D={D}: {err:.2e}, one kernel per op {err0:.2e}")
-    assert err <= err0 + 2.0 ** -24
+    assert err <= err0 + 2.0 ** -24, (err, err0)
 
 
 def test_infinities_and_nan(dev):
@@ -77,3 +76,36 @@ def test_infinities_and_nan(dev):
         finally:
             dev.set_debug()
     assert np.array_equal(np.isfinite(res[0]), np.isfinite(res[1])) and not np.isfinite(res[1]).all()
+
+
+@pytest.mark.parametrize("T", [20, 300])
+def test_infinite_operands_as_in_f32(dev, T):
+    """A key that no query can see (a score of minus infinity has no weight), one that takes everything (NaN), infinite values."""
+    from ratchet_b200 import Tensor
+    D = 64
+    g = np.random.Generator(np.random.PCG64(T))
+    q, k, v = (g.standard_normal((1, 1, T, D)).astype(np.float32) for _ in range(3))
+    q[..., 0] = np.abs(q[..., 0]) + 0.5
+    q[0, 0, 3, 0] *= -1                                  # to this query the first key is plus infinity
+    k[0, 0, 1, 0], v[0, 0, 5, 7], v[0, 0, 6, 8] = -np.inf, np.inf, -np.inf
+    t = lambda a: Tensor.from_data(np.ascontiguousarray(a, np.float32), device=dev)
+    one = t(np.array([1.0]))
+    heads = lambda a: t(a.transpose(0, 2, 1, 3))
+    a, b = heads(q).permute([0, 2, 1, 3]).mul(one), heads(k).permute([0, 2, 3, 1]).mul(one)
+    dev.set_debug(profile=True)
+    try:
+        dev.profile_report()
+        got = a.matmul(b).softmax(3).matmul(heads(v).permute([0, 2, 1, 3])).permute([0, 2, 1, 3])
+        del a, b
+        got = got.resolve().to_numpy()[0, :, 0].astype(np.float64)
+        assert "attention" in dev.profile_report()
+    finally:
+        dev.set_debug()
+    with np.errstate(invalid="ignore"):
+        s = q[0, 0].astype(np.float64) @ k[0, 0].astype(np.float64).T
+        p = np.exp(s - s.max(-1, keepdims=True))
+        want = (p / p.sum(-1, keepdims=True)) @ v[0, 0].astype(np.float64)
+    assert np.isnan(want[3]).all() and np.isfinite(np.delete(want[0], [7, 8])).all() and want[0, 7] == np.inf and want[0, 8] == -np.inf
+    fine = np.isfinite(want)
+    assert np.array_equal(got[~fine], want[~fine], equal_nan=True)
+    assert np.linalg.norm(np.where(fine, got - want, 0)) < 1e-5 * np.linalg.norm(np.where(fine, want, 0))

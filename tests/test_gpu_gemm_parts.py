@@ -44,12 +44,24 @@ def test_batched_f32(dev, B, M, N, K):
     assert np.linalg.norm(got - want) <= (2.0 ** -23 + 16 * 2.0 ** -24) * np.linalg.norm(want)
 
 
-def test_large_values_and_nan(dev):
-    """Values near the type's largest stay finite; infinities and NaN reach the tokens and features that they meet."""
-    w, x = np.zeros((64, 64), np.float32), np.ones((1, 20, 64), np.float32)
-    np.fill_diagonal(w, 1.0)
-    w[3, 3], x[0, 5, 7], x[0, 6, 8] = 3.4e38, np.nan, np.inf
-    got = nn.Linear(tensor(dev, w)).schedule(tensor(dev, x)).resolve().to_numpy()[0]
-    fine = np.ones(20, bool)
-    fine[5:7] = False
-    assert np.isfinite(got[fine]).all() and abs(got[0, 3] / 3.4e38 - 1) < 1e-6 and not np.isfinite(got[5, 7]) and not np.isfinite(got[6, 8])
+# token rows that the FMA pipe, and that split TF32 took before; one tile per CTA and tiles that are cut
+@pytest.mark.parametrize("M,N,K", [(2, 64, 64), (20, 100, 300), (31, 128, 2560), (64, 128, 512), (200, 72, 256)])
+def test_infinities_and_nan_as_in_f32(dev, M, N, K):
+    """Values near the type's largest stay finite; infinities and NaN give what f32 arithmetic gives, sign by sign, and only where they meet."""
+    g = np.random.Generator(np.random.PCG64(M + K))
+    # whole numbers and halves, many of whose remainders are zero, beside numbers of 24 bits
+    x, w = (np.where(g.random(s) < 0.5, g.integers(1, 5, s) * g.choice([-0.5, 0.5], s), g.standard_normal(s)).astype(np.float32) for s in ((1, M, K), (N, K)))
+    x[0, 0, 3], x[0, 1, 5], w[7, 9], w[8, 2] = np.inf, -np.inf, np.inf, np.nan
+    w[11, 3] = 0.0
+    w.view(np.uint32)[9, 1] = 0x7f800001                     # NaN in the bits that no leading part holds
+    w[20], x[0, :, 30] = 0.0, 1.0
+    w[20, 30] = 3.4e38
+    with np.errstate(invalid="ignore"):
+        want = x[0].astype(np.float64) @ w.astype(np.float64).T
+        want[:, 9] = np.nan
+    got = nn.Linear(tensor(dev, w)).schedule(tensor(dev, x)).resolve().to_numpy()[0].astype(np.float64)
+    fine = np.isfinite(want)
+    assert np.isinf(want).sum() > N and np.isnan(want).sum() > 2 * M - 2
+    assert np.array_equal(got[~fine], want[~fine], equal_nan=True)
+    assert np.linalg.norm(np.where(fine, got - want, 0)[:, :20]) <= (2.0 ** -23 + 16 * 2.0 ** -24) * np.linalg.norm(np.where(fine, want, 0)[:, :20])
+    assert np.abs(got[2:, 20] / want[2:, 20] - 1).max(initial=0) < 1e-6
