@@ -375,8 +375,7 @@ rcu_status launch_f32(rcu_device* dev, const void* w, const void* x, const void*
     cut.runs = tiles % sms != 0 && even < whole ? (int)runs : 0;
     void* partial = nullptr;
     if (cut.runs) {
-        const rcu_status st = rcu_alloc(dev, (runs + tiles) * (uint64_t)(T * kRowsW) * 4, &partial);
-        if (st != RCU_OK) return st;
+        if (rcu_alloc(dev, (runs + tiles) * (uint64_t)(T * kRowsW) * 4, &partial) != RCU_OK) cut.runs = 0;      // no room: whole tiles need none
     }
     const unsigned grid = cut.runs ? (unsigned)cut.runs : (unsigned)std::min(tiles, sms);
     cudaError_t e = cudaFuncSetAttribute(gemm_parts_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(T));
@@ -399,9 +398,10 @@ rcu_status rcu_gemm_parts_f32_dispatch(rcu_device* dev, const void* w, const voi
                                        const void* bias_rows) {
     // Up to 64 tokens, and wherever the tiles leave room on the SMs.  With more tiles than that the 128 x 128 tiles of the split-TF32 kernel
     // need fewer bytes of shared memory per product (us here / there: 1500 x 1536 x 384, 288 tiles, 20.2 / 16.3; 512 x 3072 x 3072, 192, 74 / 66;
-    // 1500 x 384 x 1536, 72, 21.3 / 23.3; 128 x 3072 x 3072, 48, 25.1 / 26.2; 64 x 10240 x 2560 33 / 49)
+    // 1500 x 384 x 1536, 72, 21.3 / 23.3; 128 x 3072 x 3072, 48, 25.1 / 26.2; 64 x 10240 x 2560 33 / 49).  Rows that do not start on four columns
+    // come here at any size: the FMA pipe, which they would go to otherwise, is as exact as this and the split-TF32 kernel is not.
     const uint64_t tiles = batches * ((M + 63) / 64) * ((N + kRowsW - 1) / kRowsW);
-    if (M > 64 && tiles > (uint64_t)dev->sm_count) return RCU_ERR_UNSUPPORTED;
+    if (M > 64 && N % 4 == 0 && tiles > (uint64_t)dev->sm_count) return RCU_ERR_UNSUPPORTED;
     // Tiles of 32 tokens where they leave room on the SMs too and K is short: a CTA's chain of units is what counts then, and theirs are shorter
     // (33 x 64 x 256: 9.8 us with tiles of 64)
     const bool narrow = K <= 8 * kUnitK && batches * ((M + 31) / 32) * ((N + kRowsW - 1) / kRowsW) <= (uint64_t)dev->sm_count;

@@ -174,7 +174,7 @@ gemm_tc_f32_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
 #pragma unroll
                     for (int j = 0; j < 32; j += 4) {
                         const int col = n0 + c + j;
-                        if (col + 4 <= N && (N & 3) == 0) {
+                        if (col + 4 <= N) {
                             float4 o = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
                             if (bias) {
                                 const float4 b = *reinterpret_cast<const float4*>(bias + col);
@@ -301,6 +301,7 @@ rcu_status rcu_gemm_tc_f32_dispatch(rcu_device* dev, const void* w, const void* 
     DevGuard g(dev->ordinal);
     const rcu_status parts = rcu_gemm_parts_f32_dispatch(dev, w, x, bias, y, M, N, K, batches, bias_rows);
     if (parts != RCU_ERR_UNSUPPORTED) return parts;
+    if (N % 4 != 0) return RCU_ERR_UNSUPPORTED;
     const uint64_t sms = (uint64_t)dev->sm_count;
     // Tile width and K slices together.  A CTA spends about 0.7 us per 32-wide k-block almost regardless of the tile's
     // width (twelve small MMAs issued by one thread, the lo pass, the barrier hops between them), so what counts is
@@ -314,7 +315,7 @@ rcu_status rcu_gemm_tc_f32_dispatch(rcu_device* dev, const void* w, const void* 
     uint64_t splits = 1, best = ~0ull;
     for (int cand : {64, 128}) {
         const uint64_t tiles_c = mt * ((N + cand - 1) / cand);
-        const uint64_t sp_max = (batches == 1 && N % 4 == 0) ? std::max<uint64_t>(1, std::min<uint64_t>(8, nk / kMinBlocksPerSplit)) : 1;
+        const uint64_t sp_max = batches == 1 ? std::max<uint64_t>(1, std::min<uint64_t>(8, nk / kMinBlocksPerSplit)) : 1;
         for (uint64_t sp = 1; sp <= sp_max; ++sp) {
             const uint64_t kbps_c = (nk + sp - 1) / sp;
             const uint64_t rounds = (tiles_c * sp * batches + sms - 1) / sms;

@@ -35,6 +35,16 @@ def test_linear_f32(dev, M, N, K):
     assert np.linalg.norm(got - want) <= (2.0 ** -23 + 16 * 2.0 ** -24) * np.linalg.norm(want)
 
 
+# more tiles than SMs and rows that do not start on four features: as exact as where there are few (and as the FMA pipe)
+@pytest.mark.parametrize("M,N,K", [(450, 2501, 10240), (129, 9999, 260), (600, 2050, 64)])
+def test_many_tiles_of_odd_features(dev, M, N, K):
+    g = np.random.Generator(np.random.PCG64(N))
+    x, w, b = g.standard_normal((1, M, K), np.float32), g.standard_normal((N, K), np.float32) * np.float32(0.05), g.standard_normal(N, np.float32)
+    got = nn.Linear(tensor(dev, w), tensor(dev, b)).schedule(tensor(dev, x)).resolve().to_numpy()[0].astype(np.float64)
+    want = x[0].astype(np.float64) @ w.astype(np.float64).T + b
+    assert np.linalg.norm(got - want) <= (2.0 ** -23 + 16 * 2.0 ** -24) * np.linalg.norm(want)
+
+
 @pytest.mark.parametrize("B,M,N,K", [(3, 40, 72, 64), (2, 100, 64, 300), (5, 17, 128, 36)])
 def test_batched_f32(dev, B, M, N, K):
     g = np.random.Generator(np.random.PCG64(B))
