@@ -67,18 +67,19 @@ static int as_float(PyObject* o, float* out) {
     return 1;
 }
 
-/* int(entry) of a list or tuple; entries beyond `cap` are counted, not stored (no rank is that large: the library refuses) */
-static int as_words(PyObject* seq, uint64_t* out, Py_ssize_t cap, Py_ssize_t* n) {
-    PyObject* f = PySequence_Fast(seq, "a sequence of whole numbers is expected");
+/* Whole numbers of a sequence (`convert`: int(entry) of any); entries beyond `cap` are counted, not stored (no rank is that large: the library
+ * refuses).  A tuple of its own: converting an entry may run code that changes a list. */
+static int as_words(PyObject* seq, int convert, uint64_t* out, Py_ssize_t cap, Py_ssize_t* n) {
+    PyObject* f = PySequence_Tuple(seq);
     if (!f) return 0;
-    *n = PySequence_Fast_GET_SIZE(f);
+    *n = PyTuple_GET_SIZE(f);
     int ok = 1;
     for (Py_ssize_t i = 0; ok && i < *n && i < cap; ++i) {
-        PyObject* o = PySequence_Fast_GET_ITEM(f, i);
+        PyObject* o = PyTuple_GET_ITEM(f, i);
         if (PyLong_Check(o)) {
             out[i] = PyLong_AsUnsignedLongLongMask(o);
         } else {
-            PyObject* w = PyNumber_Long(o);
+            PyObject* w = convert ? PyNumber_Long(o) : PyNumber_Index(o);
             if (!w) { ok = 0; break; }
             out[i] = PyLong_AsUnsignedLongLongMask(w);
             Py_DECREF(w);
@@ -319,14 +320,14 @@ METHOD(view) {
     ARGS("view", 1, 1, "shape");
     uint64_t s[RCU_MAX_RANK];
     Py_ssize_t rank;
-    if (!as_words(v[0], s, RCU_MAX_RANK, &rank)) return NULL;
+    if (!as_words(v[0], 1, s, RCU_MAX_RANK, &rank)) return NULL;
     DONE(p_view(self->h, (uint32_t)rank, s, &out));
 }
 METHOD(broadcast_to) {
     ARGS("broadcast_to", 1, 1, "shape");
     uint64_t s[RCU_MAX_RANK];
     Py_ssize_t rank;
-    if (!as_words(v[0], s, RCU_MAX_RANK, &rank)) return NULL;
+    if (!as_words(v[0], 1, s, RCU_MAX_RANK, &rank)) return NULL;
     DONE(p_broadcast(self->h, (uint32_t)rank, s, &out));
 }
 METHOD(permute) {
@@ -336,7 +337,7 @@ METHOD(permute) {
     Py_ssize_t rank;
     rcu_tensor t;
     info(self, &t);
-    if (!as_words(v[0], s, RCU_MAX_RANK, &rank)) return NULL;
+    if (!as_words(v[0], 0, s, RCU_MAX_RANK, &rank)) return NULL;
     if (rank != (Py_ssize_t)t.rank) return PyObject_CallMethod((PyObject*)self, "_permute_rank", NULL);
     for (Py_ssize_t i = 0; i < rank; ++i) p[i] = (uint32_t)s[i];
     DONE(p_permute(self->h, p, &out));

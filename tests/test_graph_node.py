@@ -1,6 +1,7 @@
 """The native base of ``Tensor``: arguments by position and name, errors, lifetime - on graphs without a device."""
 import ctypes as C
 
+import numpy as np
 import pytest
 
 from ratchet_b200 import Tensor, capi
@@ -38,7 +39,7 @@ def test_builders_take_names_and_positions():
 @pytest.mark.parametrize("call, error", [
     (lambda x: x.view([5]), RatchetCudaError), (lambda x: x.view([1] * 9), RatchetCudaError), (lambda x: x.permute([0, 1]), RatchetCudaError),
     (lambda x: x.slice([(0, 1)]), RatchetCudaError), (lambda x: x.slice([(0, 3), (0, 3), (0, 8)]), RatchetCudaError), (lambda x: x.softmax(-1), RatchetCudaError),
-    (lambda x: x.add(3), TypeError), (lambda x: x.matmul(), TypeError), (lambda x: x.matmul(x, trans=True), TypeError), (lambda x: x.add(x, other=x), TypeError),
+    (lambda x: x.permute([0, 1.0, 2]), TypeError), (lambda x: x.view(6), TypeError), (lambda x: x.add(3), TypeError), (lambda x: x.matmul(), TypeError), (lambda x: x.matmul(x, trans=True), TypeError), (lambda x: x.add(x, other=x), TypeError),
 ])
 def test_refusals(call, error):
     with pytest.raises(error):
@@ -56,3 +57,16 @@ def test_a_handle_is_one_reference():
     assert x._h is None and x.shape() == ()
     with pytest.raises(RatchetCudaError):
         x.gelu()
+
+
+def test_a_sequence_that_changes_while_it_is_read():
+    x, shape = leaf(2, 3, 8), []
+
+    class Entry:
+        def __int__(self):
+            shape.clear()
+            return 6
+
+    shape += [Entry(), 8]
+    assert x.view(shape).shape() == (6, 8)
+    assert x.view(np.array([6, 8])).shape() == (6, 8)
