@@ -18,7 +18,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "_obj")
 LIB = os.path.join(HERE, "libratchet_cuda.so")
-GRAPH_LIB = os.path.join(HERE, "_graph.so")          # the Python type over the lazy graph (csrc/pygraph.c): plain C, no CUDA
+# the Python type over the lazy graph (csrc/pygraph.c): plain C, no CUDA; one file per interpreter
+GRAPH_LIB = os.path.join(HERE, "_graph" + sysconfig.get_config_var("EXT_SUFFIX"))
 CORE_LIB = os.path.join(HERE, "libratchet_cuda_core.so")
 NOT_CORE = {"decode.cu", "comm.cu", "gguf.cu"}
 
@@ -72,10 +73,14 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
 def build_graph_module() -> str:
     src = os.path.join(CSRC, "pygraph.c")
-    if _stale(GRAPH_LIB, [src] + _headers()):
+    sources = [f for f in [src, os.path.join(HERE, "..", "include", "ratchet_cuda.h")] if os.path.exists(f)]
+    if _stale(GRAPH_LIB, sources):
         part = f"{GRAPH_LIB}.{os.getpid()}"
         cmd = [os.environ.get("CC", "cc"), "-O2", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"], src, "-o", part, "-ldl"]
-        proc = subprocess.run(cmd, capture_output=True, text=True)
+        try:
+            proc = subprocess.run(cmd, capture_output=True, text=True)
+        except OSError as e:
+            raise RuntimeError(f"{cmd[0]}: {e}") from e
         if proc.returncode != 0:
             raise RuntimeError(f"{' '.join(cmd)} failed:\n{proc.stdout}\n{proc.stderr}")
         os.replace(part, GRAPH_LIB)
@@ -104,7 +109,6 @@ def _link(lib: str, sources, verbose: bool) -> str:
 def ensure_runtime() -> str:
     """Path of a library that is newer than its sources: the full one where it has been built, else the core library,
     built first if need be."""
-    build_graph_module()
     if not _stale(LIB, _sources() + _headers()):
         return LIB
     if _stale(CORE_LIB, _sources(core=True) + _headers()):

@@ -7,7 +7,9 @@ compute call needs the library and a B200, and raises :class:`RatchetCudaError` 
 from __future__ import annotations
 
 import ctypes as C
+import importlib
 import os
+import types
 
 import numpy as np
 
@@ -264,18 +266,39 @@ def lib(path: str = None) -> C.CDLL:
             fn = getattr(handle, name)  # AttributeError here = the library does not export a declared symbol
             fn.restype = res
             fn.argtypes = args
-        graph_module().bind(path)
+        if hasattr(graph_module(), "bind"):          # not the stand-in
+            graph_module().bind(path)
         _lib = handle
     return _lib
 
 
+_graph_module = None
+
+
 def graph_module():
-    """The extension module whose ``Node`` is the base of ``Tensor``, built on the first use in a fresh checkout."""
-    from . import _build
-    if not os.path.exists(_build.GRAPH_LIB):
-        _build.build_graph_module()
-    from . import _graph
-    return _graph
+    """The extension module whose ``Node`` is the base of ``Tensor``, built first where it is missing or older than its source.  A
+    package that is imported for something else needs no C compiler for it: where the module cannot be built, a stand-in whose ``Node``
+    says so when it is made."""
+    global _graph_module
+    if _graph_module is None:
+        from . import _build
+        try:
+            _build.build_graph_module()
+            importlib.invalidate_caches()
+            _graph_module = importlib.import_module("._graph", __package__)
+        except (ImportError, OSError, RuntimeError) as e:
+            _graph_module = _without_graphs(str(e))
+    return _graph_module
+
+
+def _without_graphs(why: str):
+    class Node:
+        __slots__ = ()
+
+        def __new__(cls, *args, **kw):
+            raise RatchetCudaError(ERR_CUDA, f"the tensor graph's module could not be built: {why}")
+
+    return types.SimpleNamespace(Node=Node)
 
 
 def dtype_nbytes(dt: int, numel: int) -> int:

@@ -33,6 +33,7 @@ FUNCTIONS(X)
 #undef X
 
 static PyObject *s_handle, *s_check;
+static int bound;
 
 /* ------------------------------------------------------------------------------------------------ arguments */
 static int as_node(PyObject* o, rcu_lazy** out) {          /* None: no tensor */
@@ -174,6 +175,10 @@ static PyObject* node_new(PyTypeObject* type, PyObject* args, PyObject* kw) {
     static char* names[] = {"dev", "handle", NULL};
     PyObject *dev, *handle;
     if (!PyArg_ParseTupleAndKeywords(args, kw, "OO", names, &dev, &handle)) return NULL;
+    if (!bound) {                                          /* no handle can come from anywhere else, and no method could run */
+        PyErr_SetString(PyExc_RuntimeError, "the runtime library has not been loaded (capi.lib())");
+        return NULL;
+    }
     PyObject* value = PyLong_Check(handle) || handle == Py_None ? Py_NewRef(handle) : PyObject_GetAttrString(handle, "value");     /* a c_void_p */
     if (!value) return NULL;
     void* h = value == Py_None ? NULL : PyLong_AsVoidPtr(value);
@@ -446,6 +451,7 @@ static PyObject* bind(PyObject* module, PyObject* path) {
     }
     FUNCTIONS(X)
 #undef X
+    bound = 1;
     Py_RETURN_NONE;
 }
 

@@ -1,10 +1,15 @@
 """The native base of ``Tensor``: arguments by position and name, errors, lifetime - on graphs without a device."""
 import ctypes as C
+import os
+import shutil
+import subprocess
+import sys
+import sysconfig
 
 import numpy as np
 import pytest
 
-from ratchet_b200 import Tensor, capi
+from ratchet_b200 import Tensor, _build, capi
 from ratchet_b200.capi import RatchetCudaError
 
 
@@ -70,3 +75,44 @@ def test_a_sequence_that_changes_while_it_is_read():
     shape += [Entry(), 8]
     assert x.view(shape).shape() == (6, 8)
     assert x.view(np.array([6, 8])).shape() == (6, 8)
+
+
+def run(code, folder=None, **env):
+    return subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, env={**os.environ, **env}, timeout=300,
+                          cwd=folder or os.path.join(_build.HERE, ".."))
+
+
+def test_no_tensor_before_the_library_is_loaded():
+    p = run("from ratchet_b200 import Tensor\ntry: Tensor(None, 16)\nexcept RuntimeError as e: print(e)")
+    assert p.returncode == 0 and "has not been loaded" in p.stdout, p.stderr
+
+
+@pytest.fixture
+def checkout(tmp_path):
+    """The package's sources without anything built."""
+    pkg = tmp_path / "ratchet_b200"
+    shutil.copytree(_build.HERE, pkg, ignore=shutil.ignore_patterns("*.so", "_obj", "__pycache__"))
+    shutil.copytree(os.path.join(_build.HERE, "..", "include"), tmp_path / "include")
+    return tmp_path
+
+
+def test_importing_needs_no_compiler(checkout):
+    code = "import ratchet_b200 as r\nfrom ratchet_b200 import gguf, nn, callers, models\n" \
+           "assert r.__file__.startswith(%r)\ntry: r.Tensor(None, 16)\nexcept r.RatchetCudaError as e: print(e)" % str(checkout)
+    p = run(code, checkout, CC="no-such-compiler")
+    assert p.returncode == 0 and "could not be built" in p.stdout, p.stderr
+
+
+def test_the_module_is_as_new_as_its_source(checkout):
+    """Built on the first import under this interpreter's name, left alone by the second, built again after a change of the header."""
+    built = checkout / "ratchet_b200" / ("_graph" + sysconfig.get_config_var("EXT_SUFFIX"))
+    code = "import ratchet_b200 as r; assert r.__file__.startswith(%r) and r.Tensor.__base__.__module__ == 'ratchet_b200._graph'" % str(checkout)
+    assert os.path.basename(_build.GRAPH_LIB) == built.name
+    for change, again in ((False, True), (False, False), (True, True)):
+        if built.exists():
+            os.utime(built, (1e9, 1e9))
+        for f in (checkout / "include" / "ratchet_cuda.h", checkout / "ratchet_b200" / "csrc" / "pygraph.c"):
+            os.utime(f, (1e9 - 10, 1e9 + 10 if change else 1e9 - 10))
+        p = run(code, checkout)
+        assert p.returncode == 0, p.stderr
+        assert (os.path.getmtime(built) != 1e9) == again
