@@ -416,7 +416,7 @@ struct Pass {
     // glu of a bf16 product that nothing else reads
     bool glu_rows(rcu_lazy* root) {
         rcu_lazy* l = root->srcs[0];
-        if (root->dt != RCU_BF16 || !inner(l, K_LINEAR, RCU_BF16) || l->flags[0] || l->flags[1] || (l->op != RCU_ACT_NONE && l->u[1] > 0) || l->f[0] != 1.0f) return false;
+        if (root->dt != RCU_BF16 || !inner(l, K_LINEAR, RCU_BF16) || l->flags[0] || l->flags[1] || l->op != RCU_ACT_NONE || l->f[0] != 1.0f) return false;
         Op op;
         op.kind = LINEAR;
         op.w = l->srcs[0];
@@ -427,7 +427,7 @@ struct Pass {
         op.M = l->numel() / op.N;
         op.glu = root->op;
         const uint64_t pitch = op.x->shape[op.x->rank - 1];
-        if (op.w->dt != RCU_BF16 || op.x->dt != RCU_BF16 || pitch % 8 || op.x_col % 8 || !aligned(op.w) || !aligned(op.x) ||
+        if (l->u[1] > op.N || op.w->dt != RCU_BF16 || op.x->dt != RCU_BF16 || pitch % 8 || op.x_col % 8 || !aligned(op.w) || !aligned(op.x) ||
             !rcu_gemm_tc_chain_takes(dev, RCU_BF16, op.M, op.N, op.K, true, false))
             return false;
         op.srcs = {op.w, op.x};

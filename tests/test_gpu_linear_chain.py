@@ -141,3 +141,14 @@ def test_a_bias_of_another_type_is_refused(dev, M, what):
         h = h.add(tensor(dev, g.standard_normal((1, M, N)).astype(F16)))
     with pytest.raises(RatchetCudaError, match="DType mismatch: bias"):
         h.resolve()
+
+
+@pytest.mark.parametrize("kw", [{"act_cols": 3096}, {"act": "softcap", "act_cols": 0}])
+def test_what_linear_refuses_is_refused_in_front_of_a_gate(dev, kw):
+    """More activated columns than there are; a softcap without its parameter."""
+    from ratchet_b200 import Tensor
+    g = np.random.Generator(np.random.PCG64(5))
+    w = Tensor.from_data(capi.to_bf16(g.standard_normal((3088, 256)).astype(np.float32)), device=dev, dt=capi.BF16)
+    x = tensor(dev, g.standard_normal((1000, 256)).astype(np.float32)).cast(capi.BF16)
+    with pytest.raises(RatchetCudaError, match="linear: "):
+        w.linear(x, **kw).glu("gelu").resolve()
