@@ -460,9 +460,8 @@ def whisper_encoder_bench(dev, torch, stream, mode="f32"):
     what = {"f32": "f32 activations and weights",
             "q8f": "f32 activations, Q8_0F Linear weights (dequantised into pooled scratch, then the f32 tensor-core GEMM)",
             "q8h": "f16 activations, Q8_0H Linear weights (tcgen05 f16 GEMM)"}[mode]
-    score_mb = 6 * n_ctx * n_ctx * (2 if mode == "q8h" else 4) * 3 / 1e6
     return {"us_per_forward": us, "device_us_per_forward": dev_us, "kernels_per_forward": int(launches), "tflops": flops / us * 1e-6,
-            "note": what + f"; mixed launch- and compute-bound ({score_mb:.0f} MB of 1500x1500 score matrices per layer pass through L2)"}
+            "note": what + "; mixed launch- and compute-bound (attention in one pass, no score matrices in memory)"}
 
 
 def phi3_decode_bytes(c):
