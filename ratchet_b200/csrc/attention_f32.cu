@@ -357,12 +357,14 @@ constexpr size_t kSmem = 1024 + 6 * kBlockQ + 12 * kBlockK;
 
 }  // namespace
 
+bool rcu_f32_tensor_cores();      // gemm_tc_f32.cu
+
 bool rcu_attention_f32_takes(const rcu_device* dev, const Attention32Args& a) {
     if (a.T < 2 || a.L < 1 || a.H < 1 || a.H > 65535 || a.T > 65535 * 2 * kTileQ || a.L > (1 << 30)) return false;
     if (a.D < 4 || a.D > kCols || a.D % 4 || a.E < 4 || a.E > kCols || a.E % 4) return false;
     for (const HeadRows* t : {&a.q, &a.k, &a.v})
         if (t->head % 4 || t->row % 4) return false;
-    return kSmem + 1024 <= (size_t)dev->smem_optin;
+    return rcu_f32_tensor_cores() && kSmem + 1024 <= (size_t)dev->smem_optin;
 }
 
 rcu_status rcu_attention_f32(rcu_device* dev, const Attention32Args& a) {

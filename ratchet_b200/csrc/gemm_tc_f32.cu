@@ -279,13 +279,18 @@ bool make_map_f32_sw128(CUtensorMap* map, const void* base, uint64_t batches, ui
 
 }  // namespace
 
+// RCU_GEMM_F32_TC=0 keeps f32 products, and attention in one pass over them, off the tensor cores
+bool rcu_f32_tensor_cores() {
+    static const bool on = [] { const char* e = std::getenv("RCU_GEMM_F32_TC"); return !e || std::atoi(e) != 0; }();
+    return on;
+}
+
 bool rcu_gemm_tc_f32_eligible(int lhs_dt, int act_dt, uint64_t M, uint64_t N, uint64_t K) {
     if (act_dt != RCU_F32 || lhs_dt != RCU_F32) return false;
     // small problems stay on the SIMT kernel; rows must be 16-byte multiples for the tensor maps
     if (M < 2 || N < 64 || K < 32 || K % 4 != 0) return false;
     if (M > 0x7fffffffull || N > 0x7fffffffull || K > 0x7fffffffull) return false;
-    static const bool off = [] { const char* e = std::getenv("RCU_GEMM_F32_TC"); return e && std::atoi(e) == 0; }();
-    return !off;
+    return rcu_f32_tensor_cores();
 }
 
 // gemm_parts_f32.cu

@@ -110,3 +110,23 @@ def test_infinite_operands_as_in_f32(dev, T):
     assert np.array_equal(got[~fine], want[~fine], equal_nan=True)
     got, want = (np.where(fine, a, 0) for a in (got, want))
     assert np.linalg.norm(got - want) < 1e-5 * np.linalg.norm(want)
+
+
+def test_the_switch_that_keeps_f32_off_the_tensor_cores():
+    import os
+    import subprocess
+    import sys
+    code = """
+import numpy as np
+from ratchet_b200 import Device, Tensor
+dev = Device(0)
+q, k, v = (Tensor.from_data(np.ones((1, 40, 1, 64), np.float32), device=dev) for _ in range(3))
+s = Tensor.from_data(np.ones(1, np.float32), device=dev)
+o = q.permute([0, 2, 1, 3]).mul(s).matmul(k.permute([0, 2, 3, 1]).mul(s)).softmax(3).matmul(v.permute([0, 2, 1, 3])).permute([0, 2, 1, 3])
+dev.set_debug(profile=True)
+assert (o.resolve().to_numpy() == 1).all()
+print("attention" in dev.profile_report())
+"""
+    for switch, fused in (("1", "True"), ("0", "False")):
+        p = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, env={**os.environ, "RCU_GEMM_F32_TC": switch})
+        assert p.returncode == 0 and p.stdout.strip() == fused, (switch, p.stdout, p.stderr)
