@@ -289,6 +289,9 @@ bool rcu_gemm_tc_f32_eligible(int lhs_dt, int act_dt, uint64_t M, uint64_t N, ui
     if (act_dt != RCU_F32 || lhs_dt != RCU_F32) return false;
     // small problems stay on the SIMT kernel; rows must be 16-byte multiples for the tensor maps
     if (M < 2 || N < 64 || K < 32 || K % 4 != 0) return false;
+    // One or two steps of the FMA pipe along K and few features: a launch's length is what counts, and the SIMT kernel has the least to set up (us,
+    // SIMT / gemm_parts: 31 x 512 x 32 4.0 / 4.9, 31 x 4096 x 36 4.9 / 5.5; but 31 x 32768 x 32 10.7 / 7.0, 8 x 512 x 36 4.8 / 4.5, 31 x 512 x 60 6.1 / 5.3)
+    if (N <= 4096 && (K <= 32 ? M < (N % 4 ? 65 : 48) : K < 48 && M > 16 && M < 48)) return false;
     if (M > 0x7fffffffull || N > 0x7fffffffull || K > 0x7fffffffull) return false;
     return rcu_f32_tensor_cores();
 }
