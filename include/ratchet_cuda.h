@@ -139,8 +139,9 @@ rcu_status rcu_set_wait_limit_ns(rcu_device* dev, uint64_t nanoseconds);
  * ratchet-nn/src/linear.rs:10-24).  The GEMV kernels are then launched as programmatic dependents of their
  * predecessor and request their first weight rows while it drains; activations, bias and output are touched only
  * after the predecessor has completed, as always.  Off by default: through rcu_matmul the predecessor may be the
- * kernel that produced the weights.  The lazy resolver switches it on by itself for weights that were uploaded with
- * rcu_lazy_from_host (resident before the call returned).  No counterpart in the reference. */
+ * kernel that produced the weights.  Products of more than one vector read their weights after the predecessor whatever is promised
+ * here.  The lazy resolver needs no promise for weights that were uploaded with rcu_lazy_from_host (resident before the call
+ * returned): its matrix-vector products, and those of a few rows, start early on these.  No counterpart in the reference. */
 rcu_status rcu_set_constant_weights(rcu_device* dev, int on);
 
 /* ------------------------------------------------------------------ layouts (dtype/blocks.rs) */

@@ -2,8 +2,8 @@
 //   softmax(scale * q k^T [+ mask]) v        (phi3/attn.rs:120-157, whisper/mha.rs:92-127)
 // asks for, in one kernel and without its score matrices in memory.  The resolver (graph_fusion.cuh) sends such subgraphs here.
 //
-// CTA = 256 queries of one head, in two tiles of 128 that take turns, as in window_tc.cu: TMA brings the queries once, then 64 keys,
-// their values and the mask's 256 x 64 piece per stage; one warp issues S = Q K^T and O += P V with P read from tensor memory; eight warps hold a
+// CTA = 256 queries of one head, in two tiles of 128 that take turns, as in window_tc.cu, or one tile of 128 where few CTAs would be left: TMA
+// brings the queries once, then 64 keys, their values and the mask's 256 x 64 piece per stage; one warp issues S = Q K^T and O += P V with P read from tensor memory; eight warps hold a
 // query per thread.  With a mask the scores are rounded where the graph rounds them (f16 after the scale, f16 after the mask), so that
 // a row whose keys are all masked with the type's lowest value averages over them as it does there; without one they stay f32.
 // Weights enter the product in f16, which is the type the graph casts them to; their sum is taken in f32 before that.
@@ -268,9 +268,10 @@ attention_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(&p_full[w][b]);
-                // The mask's piece is given back here and not behind its loads: the weights stored above depend on every value of it, so the
-                // loads are over.  Given back at once, a piece was now and then replaced before the last warps had it (a load needs nothing
-                // but its own value to wait for): keys of one 16-byte chunk lost their weight in 1 to 5 % of the passes over 199 positions.
+                // The mask's piece is given back here, behind the store of weights that depend on every value of it: its loads are over.  Given
+                // back right behind the loads, keys of one 16-byte chunk lost their weight in 1 to 5 % of the passes over 199 positions - as if
+                // the next piece had come before the last load.  Why is not established (the reads are ordinary ones, the refill is TMA's, and an
+                // arrive speaks of accesses of one kind); values that have been used are what this ring and the others rest on.
                 if (MASK) mbar_arrive(&m_empty[b]);
             }
         }

@@ -329,7 +329,8 @@ struct WarpState {
     bool alive;
 };
 
-// The slot just read goes back to the requester.
+// The slot just read goes back to the requester: its values have been multiplied, so every load from it is over (bulk copies refill it, and an
+// arrive alone is not what holds them back from loads that are still out; attention_tc.cu has the case).
 __device__ __forceinline__ void release_slot(const Params& p, const Ranges& rg, WarpState& ws, uint64_t* empty) {
     __syncwarp();
     if ((threadIdx.x & 31) == 0) gemvq8::mbar_arrive(&empty[ws.slot]);

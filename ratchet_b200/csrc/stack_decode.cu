@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(kThreads) rows_mma_kernel(const __grid_constan
                     else lm::mma(c0, w, x.x, x.y);
                 }
             }
-            __syncwarp();                               // every lane has read the slot
+            __syncwarp();                               // every lane has read the slot: its fragments have entered their products
             if (lane == 0 && ok && pu < units) request();
             if (ok && ++slot == slots) { slot = 0; phase ^= 1; }
             i += parts;

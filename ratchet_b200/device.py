@@ -203,7 +203,8 @@ class Device:
 
     def set_constant_weights(self, on: bool = True) -> None:
         """Promise that nothing in flight writes the weight operands of the GEMVs that follow (a loaded model's
-        Linear weights): they are then launched as programmatic dependents and start fetching weights early."""
+        Linear weights): they are then launched as programmatic dependents and start fetching weights early.  Products of more than one
+        vector are not concerned."""
         self.check(self._lib.rcu_set_constant_weights(self.handle, int(bool(on))))
 
     def set_wait_limit_ns(self, ns: int) -> None:
