@@ -80,6 +80,8 @@ struct Args {
     int* status;
 };
 
+// CARE: infinite operands give what f32 arithmetic gives (main_and_small), not NaN
+template <bool CARE>
 __global__ void __launch_bounds__(kThreadsA, 1)
 attention_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, const Args a) {
     rcu_kernel_entry_wait_only();
@@ -233,7 +235,7 @@ attention_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                 tmem_ld_32x32(t + 128 + c, x);
                 tmem_ld_32x32(t + 192 + c, y);
 #pragma unroll
-                for (int j = 0; j < 32; ++j) acc[c + j] = fmaf(acc[c + j], corr, main_and_small(x[j], y[j]));
+                for (int j = 0; j < 32; ++j) acc[c + j] = fmaf(acc[c + j], corr, CARE ? main_and_small(x[j], y[j]) : x[j] + y[j]);
             }
         };
         bool ok = true;
@@ -254,7 +256,7 @@ attention_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                 tmem_ld_32x32(t + c, s + c);
                 tmem_ld_32x32(t + 64 + c, y);
 #pragma unroll
-                for (int j = 0; j < 32; ++j) s[c + j] = main_and_small(s[c + j], y[j]);
+                for (int j = 0; j < 32; ++j) s[c + j] = CARE ? main_and_small(s[c + j], y[j]) : s[c + j] + y[j];
             }
             const int left = a.L - (first + n) * kTileK;
             if (left < kTileK) {
@@ -406,9 +408,12 @@ rcu_status rcu_attention_f32(rcu_device* dev, const Attention32Args& a) {
     } else {
         const Args t{runs > 1 ? (float*)part : (float*)a.out, runs > 1 ? (float2*)((char*)part + part_bytes) : nullptr, a.H, a.T, a.L, a.E, per, dev->d_status};
         e = rcu_launch(dev, split_heads_kernel, dim3((unsigned)grid_for(std::max(T, L) * H * 8, 256, dev->sm_count * 8), 3), 256, 0, s);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+        // Fewer than 32 positions have their products on the FMA pipe with one kernel per op, and infinities with them; from 32 on those products
+        // are split too and give NaN.  The minimum on every value costs 4 % of the kernel (36.4 us for 35.1, 6 heads of 1500 positions).
+        const auto kern = a.T < 32 ? attention_f32_kernel<true> : attention_f32_kernel<false>;
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
         if (e == cudaSuccess)
-            e = rcu_launch(dev, attention_f32_kernel, dim3(a.H, (a.T + 2 * kTileQ - 1) / (2 * kTileQ), runs), kThreadsA, kSmem, qm, km, vm, t);
+            e = rcu_launch(dev, kern, dim3(a.H, (a.T + 2 * kTileQ - 1) / (2 * kTileQ), runs), kThreadsA, kSmem, qm, km, vm, t);
         if (e == cudaSuccess && runs > 1)
             e = rcu_launch(dev, merge_kernel, (unsigned)grid_for(th * (a.E / 4), 256, dev->sm_count * 8), 256, 0, (const float*)part, t.ml, (float*)a.out, (size_t)th, a.E, runs);
         dev->launches += runs > 1 ? 3 : 2;

@@ -78,15 +78,15 @@ def test_infinities_and_nan(dev):
     assert np.array_equal(np.isfinite(res[0]), np.isfinite(res[1])) and not np.isfinite(res[1]).all()
 
 
-@pytest.mark.parametrize("T", [20, 300])
+@pytest.mark.parametrize("T", [2, 20, 31])
 def test_infinite_operands_as_in_f32(dev, T):
-    """A key that no query can see (a score of minus infinity has no weight), one that takes everything (NaN), infinite values."""
+    """Few positions: a key that no query can see (a score of minus infinity has no weight), one that takes everything (NaN), infinite values."""
     from ratchet_b200 import Tensor
-    D = 64
+    D, L = 64, 200
     g = np.random.Generator(np.random.PCG64(T))
-    q, k, v = (g.standard_normal((1, 1, T, D)).astype(np.float32) for _ in range(3))
+    q, k, v = (g.standard_normal((1, 1, n, D)).astype(np.float32) for n in (T, L, L))
     q[..., 0] = np.abs(q[..., 0]) + 0.5
-    q[0, 0, 3, 0] *= -1                                  # to this query the first key is plus infinity
+    q[0, 0, 1, 0] *= -1                                  # to this query the second key is plus infinity
     k[0, 0, 1, 0], v[0, 0, 5, 7], v[0, 0, 6, 8] = -np.inf, np.inf, -np.inf
     t = lambda a: Tensor.from_data(np.ascontiguousarray(a, np.float32), device=dev)
     one = t(np.array([1.0]))
@@ -105,7 +105,7 @@ def test_infinite_operands_as_in_f32(dev, T):
         s = q[0, 0].astype(np.float64) @ k[0, 0].astype(np.float64).T
         p = np.exp(s - s.max(-1, keepdims=True))
         want = (p / p.sum(-1, keepdims=True)) @ v[0, 0].astype(np.float64)
-    assert np.isnan(want[3]).all() and np.isfinite(np.delete(want[0], [7, 8])).all() and want[0, 7] == np.inf and want[0, 8] == -np.inf
+    assert np.isnan(want[1]).all() and np.isfinite(np.delete(want[0], [7, 8])).all() and want[0, 7] == np.inf and want[0, 8] == -np.inf
     fine = np.isfinite(want)
     assert np.array_equal(got[~fine], want[~fine], equal_nan=True)
     got, want = (np.where(fine, a, 0) for a in (got, want))
