@@ -8,9 +8,11 @@
 // A CTA computes a 64 (Cout) x 64 (Lout) output tile; input channels are consumed 8 at a time
 // through shared memory (input window and filter slab), each thread owning a 4 x 4 register tile.
 //
-// f32 problems large enough for the tensor cores take another route: the input is unfolded into
+// f32 problems large enough for the tensor cores take another route, one batch entry after the other: the input is unfolded into
 // col[Lout, 3*Cin] (col[l, 3*ci + t] = x[ci, l*stride + t - pad], zero outside the input) and the product
-// y[Cout, Lout] = w[Cout, 3*Cin] . col^T runs on the split-TF32 tcgen05 GEMM with the bias added per row.
+// y[Cout, Lout] = w[Cout, 3*Cin] . col^T runs on the f32 tcgen05 GEMMs with the bias added per row.
+#include <algorithm>
+
 #include "common.cuh"
 
 rcu_status rcu_gemm_tc_f32_dispatch(rcu_device* dev, const void* w, const void* x, const void* bias, void* y, uint64_t M, uint64_t N,
@@ -114,6 +116,20 @@ unfold_k3_kernel(const float* __restrict__ x, float* __restrict__ col, int Cin, 
     }
 }
 
+// Outputs of 32 channels and more whose rows start on four positions are unfolded at any batch (384 input channels: 1.0e-7 from 64 bits, the
+// direct kernel's chains 3.2e-7).  Others where unfolding and the product take less than the direct kernel, in us: its CTAs walk the input
+// channels at 0.25 us each and share the SMs from about 200 on (stride 2, whose windows are twice as wide: 0.37); the other route pays its
+// launches per batch entry, then the product at 150 TFLOP/s and the unfolded copy.  Measured, direct / unfolded: 1 x [16, 1001] -> [31, 1001]
+// 6.9 / 8.3, 1 x [80, 1001] -> [31, 1001] 25 / 12, 32 x [16, 1001] -> [32, 1001] 15 / 246, 32 x [80, 2999] -> [384, 2999] 833 / 525, 8 x [384, 3000]
+// -> [31, 1500] 195 / 143.
+bool unfolds(uint64_t B, uint64_t Cin, uint64_t Cout, uint64_t Lout, uint32_t stride) {
+    const double ctas = (double)((Lout + TLO - 1) / TLO) * (double)((Cout + TCO - 1) / TCO) * (double)B;
+    if (Cout >= 32 && Lout % 4 == 0) return true;
+    const double direct = 2.5 + (double)Cin * (stride == 2 ? std::max(0.37, 0.002 * ctas) : std::max(0.25, 0.0011 * ctas));
+    const double flops = 2.0 * (double)std::max<uint64_t>(Cout, 64) * (double)Lout * 3.0 * (double)Cin, copied = (double)Lout * 3.0 * (double)Cin * 8.0;
+    return (double)B * (7.0 + 0.045 * (double)std::min<uint64_t>(Cin, 100) + flops * (1e6 / 150e12) + copied * (1e6 / 6e12)) < direct;
+}
+
 }  // namespace
 
 extern "C" rcu_status rcu_conv1d(rcu_device* dev, const rcu_tensor* x, const rcu_tensor* w, const rcu_tensor* bias,
@@ -134,7 +150,10 @@ extern "C" rcu_status rcu_conv1d(rcu_device* dev, const rcu_tensor* x, const rcu
     dim3 grid((unsigned)((Lout + TLO - 1) / TLO), (unsigned)((Cout + TCO - 1) / TCO), (unsigned)B);
     RCU_REQUIRE(dev, grid.y <= 65535 && grid.z <= 65535, "conv1d: too many channels / batches");
     const void* bp = bias ? bias->data : nullptr;
-    if (rcu_gemm_tc_f32_eligible(w->dt, x->dt, Cout, Lout, 3 * Cin) && Cin <= 65535ull * 32 && Lin <= 0x3fffffffull) {
+    // the GEMMs want every entry's output, and the weights, on 16 bytes
+    const bool aligned = ((reinterpret_cast<uintptr_t>(dst->data) | reinterpret_cast<uintptr_t>(w->data)) & 15) == 0 && (B == 1 || Cout * Lout % 4 == 0);
+    if (rcu_gemm_tc_f32_eligible(w->dt, x->dt, Cout, Lout, 3 * Cin) && Cin <= 65535ull * 32 && Lin <= 0x3fffffffull && aligned &&
+        unfolds(B, Cin, Cout, Lout, stride)) {
         void* col = nullptr;
         rcu_status st = rcu_alloc(dev, Lout * 3 * Cin * 4, &col);
         if (st != RCU_OK) return st;

@@ -565,6 +565,20 @@ def test_conv1d_unfolded_batches(dev, batch, cin, lin, cout, stride, pad):
     assert_close(nb.to_numpy(), orc.conv1d_k3(x, w, None, stride, pad), 1e-4, "conv1d unfolded, no bias")
 
 
+# few channels in a batch, entries that do not start on 16 bytes, and on either side of the estimate: one launch, or several per entry
+@pytest.mark.parametrize("batch,cin,lin,cout,stride,launches", [(9, 16, 100, 8, 1, 1), (3, 80, 1001, 31, 1, 1), (2, 80, 1001, 32, 1, 1), (1, 80, 1001, 31, 1, None),
+                                                                (3, 16, 130, 32, 2, 1), (1, 384, 201, 9, 2, None), (2, 384, 2998, 34, 1, None)])
+def test_conv1d_direct_or_unfolded(dev, batch, cin, lin, cout, stride, launches):
+    g = rng(18)
+    x, w = g.standard_normal((batch, cin, lin)).astype(np.float32), (g.standard_normal((cout, cin, 3)) * 0.05).astype(np.float32)
+    b = g.standard_normal(cout).astype(np.float32)
+    args = dev.from_numpy(x), dev.from_numpy(w), dev.from_numpy(b)
+    before = dev.launches
+    got = dev.conv1d(*args, stride, 1)
+    assert (dev.launches - before == launches) if launches else dev.launches - before > batch
+    assert_close(got.to_numpy(), orc.conv1d_k3(x, w, b, stride, 1), 1e-4, "conv1d")
+
+
 def test_allocator_reuses_blocks(dev):
     from ratchet_b200 import capi
     a = dev.empty(capi.F32, (123457,))
