@@ -150,13 +150,12 @@ extern "C" rcu_status rcu_conv1d(rcu_device* dev, const rcu_tensor* x, const rcu
     dim3 grid((unsigned)((Lout + TLO - 1) / TLO), (unsigned)((Cout + TCO - 1) / TCO), (unsigned)B);
     RCU_REQUIRE(dev, grid.y <= 65535 && grid.z <= 65535, "conv1d: too many channels / batches");
     const void* bp = bias ? bias->data : nullptr;
+    void* col = nullptr;
     // the GEMMs want every entry's output, and the weights, on 16 bytes
     const bool aligned = ((reinterpret_cast<uintptr_t>(dst->data) | reinterpret_cast<uintptr_t>(w->data)) & 15) == 0 && (B == 1 || Cout * Lout % 4 == 0);
     if (rcu_gemm_tc_f32_eligible(w->dt, x->dt, Cout, Lout, 3 * Cin) && Cin <= 65535ull * 32 && Lin <= 0x3fffffffull && aligned &&
-        unfolds(B, Cin, Cout, Lout, stride)) {
-        void* col = nullptr;
-        rcu_status st = rcu_alloc(dev, Lout * 3 * Cin * 4, &col);
-        if (st != RCU_OK) return st;
+        unfolds(B, Cin, Cout, Lout, stride) && rcu_alloc(dev, Lout * 3 * Cin * 4, &col) == RCU_OK) {       // without room: the direct kernel
+        rcu_status st = RCU_OK;
         const dim3 ugrid((unsigned)((Lout + 31) / 32), (unsigned)((Cin + 31) / 32));
         for (uint64_t b = 0; b < B && st == RCU_OK; ++b) {
             const float* xb = (const float*)x->data + b * Cin * Lin;

@@ -269,12 +269,11 @@ rcu_status rcu_matmul(rcu_device* dev, const rcu_tensor* lhs, const rcu_tensor* 
     }
     // Quantised weights with f32 activations (Q8_0F / Q4_KF Linear, the quantised Whisper graphs): the
     // weights are dequantised once into pooled scratch (bit-exact, as the CPU path does for every
-    // quantised op) and the product runs on the f32 tensor-core kernel.
+    // quantised op) and the product runs on the f32 tensor-core kernel.  Where the pool has no room for that (four bytes a weight), the SIMT
+    // kernel reads the codes.
+    void* wf = nullptr;
     if (!tl && tr && td && d.lstack == 1 && (lhs->dt == RCU_Q8_0F || lhs->dt == RCU_Q4_KF) && rhs->dt == RCU_F32 &&
-        rcu_gemm_tc_f32_eligible(RCU_F32, RCU_F32, d.rstack * d.n, d.m, d.k)) {
-        void* wf = nullptr;
-        st = rcu_alloc(dev, d.m * d.k * 4, &wf);
-        if (st != RCU_OK) return st;
+        rcu_gemm_tc_f32_eligible(RCU_F32, RCU_F32, d.rstack * d.n, d.m, d.k) && rcu_alloc(dev, d.m * d.k * 4, &wf) == RCU_OK) {
         rcu_tensor wsrc{lhs->dt, 2, {d.m, d.k, 1, 1}, lhs->data};
         rcu_tensor wdst{RCU_F32, 2, {d.m, d.k, 1, 1}, wf};
         st = rcu_dequantize(dev, &wsrc, &wdst);
@@ -289,9 +288,9 @@ rcu_status rcu_matmul(rcu_device* dev, const rcu_tensor* lhs, const rcu_tensor* 
         const void* wptr = rhs->data;
         void* scratch = nullptr;
         st = RCU_OK;
-        if (!tr) {
-            st = rcu_alloc(dev, d.rstack * d.k * d.n * 4, &scratch);
-            if (st != RCU_OK) return st;
+        if (!tr && rcu_alloc(dev, d.rstack * d.k * d.n * 4, &scratch) != RCU_OK) {
+            st = RCU_ERR_UNSUPPORTED;            // no room for the transpose: the SIMT kernel needs none
+        } else if (!tr) {
             rcu_tensor src{RCU_F32, 3, {d.rstack, d.k, d.n, 1}, rhs->data};
             rcu_tensor tdst{RCU_F32, 3, {d.rstack, d.n, d.k, 1}, scratch};
             const uint32_t perm[3] = {0, 2, 1};
@@ -335,7 +334,7 @@ rcu_status rcu_matmul(rcu_device* dev, const rcu_tensor* lhs, const rcu_tensor* 
         if (st == RCU_OK) st = rcu_gemm_tc_batched_f16(dev, wptr, aptr, dst->data, d.m, d.n, d.k, b, kp, kp);
         for (void* s : scratch)
             if (s) rcu_free(dev, s);     // the pool reuses blocks in stream order
-        if (st != RCU_ERR_UNSUPPORTED) return st;
+        if (st != RCU_ERR_UNSUPPORTED && st != RCU_ERR_OOM) return st;      // without room for the copies: the SIMT kernel needs none
     }
     const uint64_t numel = t_numel(lhs);
     uint64_t off[4];
