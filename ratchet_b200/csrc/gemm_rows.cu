@@ -13,14 +13,15 @@
 // the tokens in an accumulator of their own, which enters the sum through an f32 fma with the block's scale.  This form serves any
 // number of token rows (blockIdx.y).
 //
-// Measured on B200 (us, K = 3072, 2 / 16 / 32 rows; before: the SIMT kernel, which unpacks every weight anew for each 64-row tile and
-// multiplies on the FMA pipe):
-//             N = 3072                            N = 9216                              N = 32001
-//   Q8_0H   183 / 188 / 14 ->  7 /  7 /  8     253 / 236 / 20 ->  7 / 11 / 15      568 / 578 / 592 -> 23 / 38 /  -
-//   Q8_0F   201 / 204 / 209 -> 7 /  7 / 12     272 / 275 / 332 -> 9 / 15 / 28      608 / 619 / 636 -> 37 / 62 / 111
-//   Q4_KH   303 / 314 / 15 ->  6 /  7 / 11     422 / 409 / 23 -> 10 / 16 / 20      791 / 809 / 853 -> 32 / 51 /  -
-//   f16     184 / 185 / 10 ->  6 /  7 /  -     258 / 254 / 13 -> 10 / 11 /  -      611 / 612 / 611 -> 33 / 39 /  -
-// Q8_0F at 2048 rows, N = K = 3072: 1405 -> 498.  What is left to the bytes of W (Q8_0H, 9216 x 3072: 4.6 us) is a CTA's start, its first
+// Measured on B200 (us, K = 3072, 2 / 16 / 32 rows, weights that rotate through more than L2, from a CUDA graph; before: the SIMT kernel, which
+// unpacks every weight anew for each 64-row tile and multiplies on the FMA pipe; 32 rows of Q8_0H, Q4_KH and f16 at N = 32001 are not this kernel's):
+//             N = 3072                              N = 9216                               N = 32001
+//   Q8_0H   213 / 209 / 13 -> 5.3 / 6.6 / 8.9    253 / 251 / 20 ->  8.6 / 13 / 17     570 / 581 / 593 -> 25 / 39 /  -
+//   Q8_0F   239 / 242 / 240 -> 8.5 / 8.4 / 14    277 / 282 / 288 -> 11 / 20 / 39      609 / 621 / 635 -> 40 / 65 / 116
+//   Q4_KH   322 / 335 / 14 -> 6.5 / 7.6 / 11     445 / 446 / 22 ->  10 / 17 / 21      827 / 855 / 994 -> 32 / 52 /  -
+//   f16     265 / 266 / 10 -> 7.1 / 7.6 /  -     271 / 271 / 16 ->  12 / 13 /  -      610 / 611 / 610 -> 38 / 43 /  -
+// Weights that are known to be resident are requested before the predecessor has ended: 1.0 to 1.4 us less (Q8_0H, N = 3072: 3.9 / 5.1 / 7.8).
+// Q8_0F at 2048 rows, N = K = 3072: 1416 -> 468.  What is left to the bytes of W (Q8_0H, 9216 x 3072: 4.6 us) is a CTA's start, its first
 // loads and the sum over its warps.
 #include "dequant.cuh"
 #include "common.cuh"
