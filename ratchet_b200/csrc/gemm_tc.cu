@@ -356,10 +356,8 @@ rcu_status launch_tc(rcu_device* dev, const CUtensorMap& xmap, const CUtensorMap
         while (splits > 1 && (((nk + splits - 1) / splits + 3) & ~3) * (splits - 1) >= nk) --splits;     // every slice gets k-steps
     }
     if constexpr (MODE != EPI_RAGGED) {           // slices need N % 8 == 0
-        if (splits > 1) {
-            void* partial = nullptr;
-            rcu_status st = rcu_alloc(dev, (uint64_t)splits * M * N * 4, &partial);
-            if (st != RCU_OK) return st;
+        void* partial = nullptr;
+        if (splits > 1 && rcu_alloc(dev, (uint64_t)splits * M * N * 4, &partial) == RCU_OK) {       // no room for the slices' sums: one slice
             grid.z = splits;
             rcu_launch(dev, kern, grid, threads, smem, xmap, wmap, qa, GemmEpilogue<Out, MODE>{nullptr, nullptr, 1.f, 0}, (Out*)out, M, N, K, dev->d_status, splits,
                        (float*)partial, idesc);
@@ -433,18 +431,17 @@ rcu_status rcu_gemm_tc_dispatch(rcu_device* dev, int lhs_dt, const void* w, int 
     if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(w)) & 15) return RCU_ERR_UNSUPPORTED;
     DevGuard g(dev->ordinal);
     if (lhs_dt == RCU_F16 && rcu_gemm_tc2_eligible(dev, M, N, K)) return rcu_gemm_tc2_launch(dev, w, x, bias, y, M, N, K, t);
-    if (lhs_dt != RCU_F16 && converts_once(M)) {
-        void* scratch = nullptr;
-        rcu_status st = rcu_alloc(dev, N * K * 2, &scratch);
-        if (st != RCU_OK) return st;
+    void* scratch = nullptr;
+    if (lhs_dt != RCU_F16 && converts_once(M) && rcu_alloc(dev, N * K * 2, &scratch) == RCU_OK) {       // no room for the matrix: fused
         rcu_tensor src{lhs_dt, 2, {N, K, 1, 1}, const_cast<void*>(w)};
         rcu_tensor dst{RCU_F16, 2, {N, K, 1, 1}, scratch};
-        st = rcu_dequantize(dev, &src, &dst);
+        rcu_status st = rcu_dequantize(dev, &src, &dst);
         if (st == RCU_OK) st = rcu_gemm_tc_dispatch(dev, RCU_F16, scratch, act_dt, x, bias, y, M, N, K, t);
         rcu_free(dev, scratch);   // the pool reuses blocks in stream order
         return st;
     }
-    if (t.glu >= 0 || t.chain_op >= 0) return RCU_ERR_UNSUPPORTED;      // the one-CTA kernel stores every column, as the product gives it
+    // the one-CTA kernel stores every column, as the product gives it
+    if (t.glu >= 0 || t.chain_op >= 0) return lhs_dt != RCU_F16 && converts_once(M) ? RCU_ERR_OOM : RCU_ERR_UNSUPPORTED;
     // tile width: enough CTAs to cover the SMs when M is small
     const uint64_t tiles128 = ((M + TM - 1) / TM) * ((N + 127) / 128);
     int bn = tiles128 >= (uint64_t)dev->sm_count ? 128 : 64;
