@@ -566,7 +566,7 @@ def test_conv1d_unfolded_batches(dev, batch, cin, lin, cout, stride, pad):
 
 
 # few channels in a batch, entries that do not start on 16 bytes, and on either side of the estimate: one launch, or several per entry
-@pytest.mark.parametrize("batch,cin,lin,cout,stride,launches", [(9, 16, 100, 8, 1, 1), (3, 80, 1001, 31, 1, 1), (2, 80, 1001, 32, 1, 1), (1, 80, 1001, 31, 1, None),
+@pytest.mark.parametrize("batch,cin,lin,cout,stride,launches", [(9, 16, 100, 8, 1, 1), (3, 80, 1001, 31, 1, 1), (3, 80, 1001, 32, 1, 1), (1, 80, 1001, 31, 1, None),
                                                                 (3, 16, 130, 32, 2, 1), (1, 384, 201, 9, 2, None), (2, 384, 2998, 34, 1, None)])
 def test_conv1d_direct_or_unfolded(dev, batch, cin, lin, cout, stride, launches):
     g = rng(18)
