@@ -403,8 +403,6 @@ rcu_status rcu_gemm_parts_f32_dispatch(rcu_device* dev, const void* w, const voi
     // come here at any size: the FMA pipe, which they would go to otherwise, is as exact as this and the split-TF32 kernel is not.
     const uint64_t tiles = batches * ((M + 63) / 64) * ((N + kRowsW - 1) / kRowsW);
     if (M > 64 && N % 4 == 0 && tiles > (uint64_t)dev->sm_count) return RCU_ERR_UNSUPPORTED;
-    // Half a unit of K and few features (below 48 tokens the FMA pipe has them): 64 x 512 x 32 4.9 / 4.2, 1000 x 512 x 32 5.5 / 4.7, 300 x 4096 x 32 6.1 / 6.0
-    if (M >= 48 && N % 4 == 0 && N <= 4096 && K <= 32) return RCU_ERR_UNSUPPORTED;
     // Tiles of 32 tokens where they leave room on the SMs too and K is short: a CTA's chain of units is what counts then, and theirs are shorter
     // (33 x 64 x 256: 9.8 us with tiles of 64)
     const bool narrow = K <= 8 * kUnitK && batches * ((M + 31) / 32) * ((N + kRowsW - 1) / kRowsW) <= (uint64_t)dev->sm_count;

@@ -19,7 +19,7 @@ rcu_status rcu_gemm_rows_dispatch(rcu_device* dev, int lhs_dt, const void* w, in
 // f32 Linear on the tensor cores (split-TF32, f32-level accuracy)
 rcu_status rcu_gemm_tc_f32_dispatch(rcu_device* dev, const void* w, const void* x, const void* bias, void* y, uint64_t M, uint64_t N,
                                     uint64_t K, uint64_t batches, const void* bias_rows = nullptr);
-bool rcu_gemm_tc_f32_eligible(int lhs_dt, int act_dt, uint64_t M, uint64_t N, uint64_t K);
+bool rcu_gemm_tc_f32_eligible(int lhs_dt, int act_dt, uint64_t M, uint64_t N, uint64_t K, uint64_t batches = 1);
 rcu_status rcu_gemm_tc_batched_f16(rcu_device* dev, const void* w, const void* x, void* y, uint64_t M, uint64_t N, uint64_t K, uint64_t batch,
                                    uint64_t pitch_w, uint64_t pitch_x);
 rcu_status rcu_copy2d_pitched(rcu_device* dev, const void* src, void* dst, size_t rows, size_t row_bytes, size_t spitch, size_t dpitch);
@@ -284,7 +284,7 @@ rcu_status rcu_matmul(rcu_device* dev, const rcu_tensor* lhs, const rcu_tensor* 
     // Batched f32 products of the attention kind, A[b, M, K] . B[b, K, N] (or B given as [b, N, K] with
     // trans_rhs): the tensor-core kernel wants both operands K-major, so an untransposed B is transposed
     // into pooled scratch first (it is the small operand of these products).
-    if (!tl && !td && !bias && d.lstack == d.rstack && d.dstack == d.lstack && rcu_gemm_tc_f32_eligible(lhs->dt, rhs->dt, d.m, d.n, d.k)) {
+    if (!tl && !td && !bias && d.lstack == d.rstack && d.dstack == d.lstack && rcu_gemm_tc_f32_eligible(lhs->dt, rhs->dt, d.m, d.n, d.k, d.lstack)) {
         const void* wptr = rhs->data;
         void* scratch = nullptr;
         st = RCU_OK;
