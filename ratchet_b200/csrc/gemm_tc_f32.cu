@@ -291,9 +291,10 @@ bool rcu_gemm_tc_f32_eligible(int lhs_dt, int act_dt, uint64_t M, uint64_t N, ui
     if (M < 2 || N < 64 || K < 32 || K % 4 != 0) return false;
     // Two or three steps of the FMA pipe along K and few tiles: a launch's length is what counts, and the SIMT kernel has the least to set up (us,
     // SIMT / gemm_parts: 31 x 512 x 32 4.0 / 4.9, 64 x 4096 x 32 4.8 / 5.1, 128 x 512 x 32 4.6 / 5.0, 31 x 4096 x 36 4.9 / 5.5; but 31 x 32768 x 32 10.7 /
-    // 7.0, 128 x 4096 x 32 7.9 / 5.2, 256 problems of 2 x 512 x 32 23 / 12, 8 x 512 x 36 4.8 / 4.5, 31 x 512 x 60 6.1 / 5.3)
+    // 7.0, 128 x 4096 x 32 7.9 / 5.2, 256 problems of 2 x 512 x 32 23 / 12, 8 x 512 x 36 4.8 / 4.5, 31 x 512 x 60 6.1 / 5.3).  Features that fill half
+    // of gemm_parts' 128 are the SIMT kernel's however many problems there are (2000 of 31 x 64 x 32 25 / 30, 36 with a transpose in front).
     const uint64_t ctas = batches * ((M + 63) / 64) * ((N + 63) / 64);
-    if (K <= 32 ? ctas <= (M <= 64 ? 128 : 64) : K < 48 && M > 16 && M < 48 && ctas <= 64) return false;
+    if (K <= 32 ? ctas <= (M <= 64 ? 128 : 64) || (N <= 64 && M <= 64) : K < 48 && M > 16 && M < 48 && ctas <= 64) return false;
     if (M > 0x7fffffffull || N > 0x7fffffffull || K > 0x7fffffffull) return false;
     return rcu_f32_tensor_cores();
 }
