@@ -28,6 +28,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <type_traits>
 
 #include "bulk_async.cuh"
 #include "grouped_step.cuh"
@@ -66,31 +67,43 @@ struct RowsArgs {
     int n_silu, n_sigmoid;          // EPI_MIXER_IN: rows below n_silu pass silu, rows from n_sigmoid on sigmoid
     int parts, slots;               // warps per team; ring slots per warp
     int* status;
-    // latent append, done by the first CTA (C == 0: none)
+    // latent append, done by a further CTA (C == 0: none)
     const float* low;               // [C + R]
-    const float *c_scale, *freqs;
+    const float* c_scale;
+    const float2* angles;           // (cos, sin) of the position's pairs
     void* ring;
     int C, R, n_freq, ring_rows;
-    float magnitude;
     const uint32_t* d_pos;
+    bool vec;                       // input vectors, scales and gates: 16-byte aligned, lengths multiples of four
 };
 
-// normalised latent and rotated key part of the current token into its ring row
+// normalised latent and rotated key part of the current token into its ring row; rows hold at most 1280 elements
 template <class T> __device__ void append_latent(const RowsArgs& a, float* scratch) {
-    float s = 0.f;
-    for (int j = threadIdx.x; j < a.C; j += kThreads) s = fmaf(a.low[j], a.low[j], s);
-    const float rstd = 1.0f / sqrtf(lm::block_sum(s, scratch) / (float)a.C + a.eps);
-    const uint32_t p = *a.d_pos;
-    T* row = reinterpret_cast<T*>(a.ring) + (size_t)(p % (uint32_t)a.ring_rows) * (a.C + a.R);
-    for (int j = threadIdx.x; j < a.C; j += kThreads) row[j] = from_f32<T>(a.low[j] * rstd * a.c_scale[j]);
+    constexpr int kMost = 1280 / kThreads;
+    float v[kMost], scale[kMost], s = 0.f;
+#pragma unroll
+    for (int i = 0; i < kMost; ++i) {
+        const int j = threadIdx.x + i * kThreads;
+        v[i] = j < a.C ? a.low[j] : 0.f;
+        scale[i] = j < a.C ? a.c_scale[j] : 0.f;
+    }
+    T* row = reinterpret_cast<T*>(a.ring) + (size_t)(*a.d_pos % (uint32_t)a.ring_rows) * (a.C + a.R);
     const float* kr = a.low + a.C;
     for (int i = threadIdx.x; i < a.n_freq; i += kThreads) {
-        const float2 cs = lm::rotary_angle(a.freqs, a.n_freq, i, p, a.magnitude);
-        const float u = kr[2 * i], v = kr[2 * i + 1];
-        row[a.C + 2 * i] = from_f32<T>(u * cs.x - v * cs.y);
-        row[a.C + 2 * i + 1] = from_f32<T>(v * cs.x + u * cs.y);
+        const float2 cs = a.angles[i];
+        const float u = kr[2 * i], w = kr[2 * i + 1];
+        row[a.C + 2 * i] = from_f32<T>(u * cs.x - w * cs.y);
+        row[a.C + 2 * i + 1] = from_f32<T>(w * cs.x + u * cs.y);
     }
     for (int j = 2 * a.n_freq + threadIdx.x; j < a.R; j += kThreads) row[a.C + j] = from_f32<T>(kr[j]);
+#pragma unroll
+    for (int i = 0; i < kMost; ++i) s = fmaf(v[i], v[i], s);
+    const float rstd = 1.0f / sqrtf(lm::block_sum(s, scratch) / (float)a.C + a.eps);
+#pragma unroll
+    for (int i = 0; i < kMost; ++i) {
+        const int j = threadIdx.x + i * kThreads;
+        if (j < a.C) row[j] = from_f32<T>(v[i] * rstd * scale[i]);
+    }
 }
 
 __host__ __device__ __forceinline__ int padded(int k) { return (k + 127) & ~127; }      // whole ring items
@@ -99,11 +112,18 @@ __device__ __forceinline__ float4 load4(const float* p, int n) {       // elemen
     if (n >= 4 && (reinterpret_cast<uintptr_t>(p) & 15) == 0) return *reinterpret_cast<const float4*>(p);
     return make_float4(n > 0 ? p[0] : 0.f, n > 1 ? p[1] : 0.f, n > 2 ? p[2] : 0.f, n > 3 ? p[3] : 0.f);
 }
+// VEC: p is 16-byte aligned and n a multiple of four.  Without the scalar path the loads of a batch leave together; with it each went its
+// own trip to L2 (7680 floats of an output projection's two inputs: 5.2 us).
+template <bool VEC> __device__ __forceinline__ float4 load4(const float* p, int n) {
+    if constexpr (VEC) return n > 0 ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+    else return load4(p, n);
+}
 
 constexpr int kKept = 4;                // quads of a vector that a thread keeps in registers
+constexpr int kBatch = 8;               // quads of a vector that is only copied, in flight at a time
 
 // The norm scales of a product's input, requested before the wait for the kernel before it (they are constant).
-struct StagedScales {
+template <bool VEC> struct StagedScales {
     float4 s1[kKept], s2[kKept];
     __device__ __forceinline__ void request(const RowsArgs& a) {
         if (a.pro == PRO_CONCAT) return;
@@ -111,21 +131,21 @@ struct StagedScales {
 #pragma unroll
         for (int i = 0; i < kKept; ++i) {
             const int j = (threadIdx.x + i * kThreads) * 4;
-            s1[i] = load4(a.s1 + j, a.ka - j);          // zero beyond the end
-            if (second) s2[i] = load4(second + j, a.ka - j);
+            s1[i] = load4<VEC>(a.s1 + j, a.ka - j);          // zero beyond the end
+            if (second) s2[i] = load4<VEC>(second + j, a.ka - j);
         }
     }
 };
 
 // x + LayerNorm(x2) * s1 + b1, and - with s2 - LayerNorm(that) * s2 + b2
-template <class Put> __device__ __forceinline__ void stage_post_norm(const RowsArgs& a, const StagedScales& sc, float* scratch, Put put) {
+template <bool VEC, class Put> __device__ __forceinline__ void stage_post_norm(const RowsArgs& a, const StagedScales<VEC>& sc, float* scratch, Put put) {
     const int step = kThreads * 4, j0 = threadIdx.x * 4, quads = (padded(a.ka) + step - 1) / step;
     float4 y[kKept], x[kKept];
 #pragma unroll
     for (int i = 0; i < kKept; ++i) {
         const int j = j0 + i * step;
-        y[i] = load4(a.x2 + j, a.ka - j);
-        x[i] = load4(a.x + j, a.ka - j);
+        y[i] = load4<VEC>(a.x2 + j, a.ka - j);
+        x[i] = load4<VEC>(a.x + j, a.ka - j);
     }
     auto total = [](const float4& w) { return (w.x + w.y) + (w.z + w.w); };
     auto square = [&](float q, const float4& w, int j, float mean) {
@@ -138,17 +158,17 @@ template <class Put> __device__ __forceinline__ void stage_post_norm(const RowsA
     float s = 0.f, q = 0.f;
 #pragma unroll
     for (int i = 0; i < kKept; ++i) s += total(y[i]);
-    for (int i = kKept; i < quads; ++i) s += total(load4(a.x2 + j0 + i * step, a.ka - (j0 + i * step)));
+    for (int i = kKept; i < quads; ++i) s += total(load4<VEC>(a.x2 + j0 + i * step, a.ka - (j0 + i * step)));
     const float mean = lm::block_sum(s, scratch) / (float)a.ka;
 #pragma unroll
     for (int i = 0; i < kKept; ++i) q = square(q, y[i], j0 + i * step, mean);
-    for (int i = kKept; i < quads; ++i) q = square(q, load4(a.x2 + j0 + i * step, a.ka - (j0 + i * step)), j0 + i * step, mean);
+    for (int i = kKept; i < quads; ++i) q = square(q, load4<VEC>(a.x2 + j0 + i * step, a.ka - (j0 + i * step)), j0 + i * step, mean);
     const float rstd = 1.0f / sqrtf(lm::block_sum(q, scratch) / (float)a.ka + a.eps);
     auto sum = [&](const float4& x, const float4& y, const float4& g, const float4& b) {
         return make_float4(x.x + fmaf((y.x - mean) * rstd, g.x, b.x), x.y + fmaf((y.y - mean) * rstd, g.y, b.y), x.z + fmaf((y.z - mean) * rstd, g.z, b.z),
                            x.w + fmaf((y.w - mean) * rstd, g.w, b.w));
     };
-    auto late = [&](int j) { return sum(load4(a.x + j, a.ka - j), load4(a.x2 + j, a.ka - j), load4(a.s1 + j, a.ka - j), load4(a.b1 + j, a.ka - j)); };
+    auto late = [&](int j) { return sum(load4<VEC>(a.x + j, a.ka - j), load4<VEC>(a.x2 + j, a.ka - j), load4<VEC>(a.s1 + j, a.ka - j), load4<VEC>(a.b1 + j, a.ka - j)); };
 #pragma unroll
     for (int i = 0; i < kKept; ++i) x[i] = sum(x[i], y[i], sc.s1[i], sc.s2[i]);       // zero beyond the end: scale and shift are
     if (a.x_out && blockIdx.x == 0) {
@@ -177,7 +197,7 @@ template <class Put> __device__ __forceinline__ void stage_post_norm(const RowsA
     auto emit = [&](float4 w, int j) {
         if (j >= padded(a.ka)) return;
         if (a.s2) {
-            const float4 g = load4(a.s2 + j, a.ka - j), b = a.b2 ? load4(a.b2 + j, a.ka - j) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 g = load4<VEC>(a.s2 + j, a.ka - j), b = a.b2 ? load4<VEC>(a.b2 + j, a.ka - j) : make_float4(0.f, 0.f, 0.f, 0.f);
             w = make_float4(fmaf((w.x - mean2) * rstd2, g.x, b.x), fmaf((w.y - mean2) * rstd2, g.y, b.y), fmaf((w.z - mean2) * rstd2, g.z, b.z),
                             fmaf((w.w - mean2) * rstd2, g.w, b.w));
         }
@@ -190,7 +210,7 @@ template <class Put> __device__ __forceinline__ void stage_post_norm(const RowsA
 
 // The input vectors of a product, normalised or gated, four elements at a time: put(piece, j, values); zeros from the end of a
 // vector to its padded length.
-template <class Put> __device__ __forceinline__ void stage_input(const RowsArgs& a, const StagedScales& sc, float* scratch, Put put) {
+template <bool VEC, class Put> __device__ __forceinline__ void stage_input(const RowsArgs& a, const StagedScales<VEC>& sc, float* scratch, Put put) {
     const int step = kThreads * 4, j0 = threadIdx.x * 4;
     if (a.pro == PRO_POST_NORM) {
         stage_post_norm(a, sc, scratch, put);
@@ -199,8 +219,8 @@ template <class Put> __device__ __forceinline__ void stage_input(const RowsArgs&
     if (a.pro == PRO_LAYER_NORM || a.pro == PRO_RMS) {
         float4 v[kKept];
 #pragma unroll
-        for (int i = 0; i < kKept; ++i) v[i] = load4(a.x + j0 + i * step, a.ka - (j0 + i * step));
-        auto quad = [&](int i) { return i < kKept ? v[i] : load4(a.x + j0 + i * step, a.ka - (j0 + i * step)); };
+        for (int i = 0; i < kKept; ++i) v[i] = load4<VEC>(a.x + j0 + i * step, a.ka - (j0 + i * step));
+        auto quad = [&](int i) { return i < kKept ? v[i] : load4<VEC>(a.x + j0 + i * step, a.ka - (j0 + i * step)); };
         const int quads = (padded(a.ka) + step - 1) / step;
         float mean = 0.f;
         if (a.pro == PRO_LAYER_NORM) {
@@ -227,7 +247,7 @@ template <class Put> __device__ __forceinline__ void stage_input(const RowsArgs&
         auto emit = [&](const float4& w, int j, const float4& s1, const float4& s2) {
             if (j >= padded(a.ka)) return;
             const float x = (w.x - mean) * rstd, y = (w.y - mean) * rstd, z = (w.z - mean) * rstd, t = (w.w - mean) * rstd;
-            const float4 b = a.b1 ? load4(a.b1 + j, a.ka - j) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 b = a.b1 ? load4<VEC>(a.b1 + j, a.ka - j) : make_float4(0.f, 0.f, 0.f, 0.f);
             put(0, j, make_float4(fmaf(x, s1.x, b.x), fmaf(y, s1.y, b.y), fmaf(z, s1.z, b.z), fmaf(t, s1.w, b.w)));
             if (a.s2) put(1, j, make_float4(x * s2.x, y * s2.y, z * s2.z, t * s2.w));
         };
@@ -235,53 +255,77 @@ template <class Put> __device__ __forceinline__ void stage_input(const RowsArgs&
         for (int i = 0; i < kKept; ++i) emit(v[i], j0 + i * step, sc.s1[i], sc.s2[i]);
         for (int i = kKept; i < quads; ++i) {
             const int j = j0 + i * step;
-            emit(quad(i), j, load4(a.s1 + j, a.ka - j), a.s2 ? load4(a.s2 + j, a.ka - j) : make_float4(0.f, 0.f, 0.f, 0.f));
+            emit(quad(i), j, load4<VEC>(a.s1 + j, a.ka - j), a.s2 ? load4<VEC>(a.s2 + j, a.ka - j) : make_float4(0.f, 0.f, 0.f, 0.f));
         }
         return;                                         // both pieces come from the norm
     }
+    // the second input's first quads travel with the first input
+    float4 second[kBatch];
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) second[i] = load4<VEC>(a.x2 + j0 + i * step, a.split ? 0 : a.kb - (j0 + i * step));
     if (a.pro == PRO_GATED_RMS) {
-        float4 v[kKept];
+        float4 v[kKept], g[kKept];
         float q = 0.f;
         auto square = [&](const float4& w) { q += (w.x * w.x + w.y * w.y) + (w.z * w.z + w.w * w.w); };
 #pragma unroll
         for (int i = 0; i < kKept; ++i) {
-            v[i] = load4(a.x + j0 + i * step, a.ka - (j0 + i * step));
-            square(v[i]);
+            v[i] = load4<VEC>(a.x + j0 + i * step, a.ka - (j0 + i * step));
+            g[i] = load4<VEC>(a.gate + j0 + i * step, a.ka - (j0 + i * step));
         }
-        for (int j = j0 + kKept * step; j < a.ka; j += step) square(load4(a.x + j, a.ka - j));
+#pragma unroll
+        for (int i = 0; i < kKept; ++i) square(v[i]);
+        for (int j = j0 + kKept * step; j < a.ka; j += step) square(load4<VEC>(a.x + j, a.ka - j));
         const float rstd = 1.0f / sqrtf(lm::block_sum(q, scratch) / (float)a.ka + a.eps);
-        auto emit = [&](const float4& w, int j, const float4& s) {
+        auto emit = [&](const float4& w, int j, const float4& s, const float4& g) {
             if (j >= padded(a.ka)) return;
-            const float4 g = load4(a.gate + j, a.ka - j);
             put(0, j, make_float4(w.x * rstd * s.x * g.x, w.y * rstd * s.y * g.y, w.z * rstd * s.z * g.z, w.w * rstd * s.w * g.w));
         };
 #pragma unroll
-        for (int i = 0; i < kKept; ++i) emit(v[i], j0 + i * step, sc.s1[i]);
-        for (int j = j0 + kKept * step; j < padded(a.ka); j += step) emit(load4(a.x + j, a.ka - j), j, load4(a.s1 + j, a.ka - j));
+        for (int i = 0; i < kKept; ++i) emit(v[i], j0 + i * step, sc.s1[i], g[i]);
+        for (int j = j0 + kKept * step; j < padded(a.ka); j += step)
+            emit(load4<VEC>(a.x + j, a.ka - j), j, load4<VEC>(a.s1 + j, a.ka - j), load4<VEC>(a.gate + j, a.ka - j));
     } else {
-#pragma unroll 4
-        for (int j = j0; j < padded(a.ka); j += step) {
-            if (a.split) {
-                auto at = [&](int i) { return i >= a.ka ? 0.f : i < a.split ? a.x[i] : a.x2[i - a.split]; };
-                put(0, j, make_float4(at(j), at(j + 1), at(j + 2), at(j + 3)));
-            } else {
-                put(0, j, load4(a.x + j, a.ka - j));
-            }
+        // x, or x[0, split) followed by x2
+        auto at = [&](int j) {
+            if constexpr (VEC) return load4<VEC>(a.split && j >= a.split ? a.x2 + (j - a.split) : a.x + j, a.ka - j);
+            if (!a.split) return load4(a.x + j, a.ka - j);
+            auto one = [&](int i) { return i >= a.ka ? 0.f : i < a.split ? a.x[i] : a.x2[i - a.split]; };
+            return make_float4(one(j), one(j + 1), one(j + 2), one(j + 3));
+        };
+        for (int j = j0; j < padded(a.ka); j += kBatch * step) {
+            float4 v[kBatch];
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) v[i] = at(j + i * step);
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i)
+                if (j + i * step < padded(a.ka)) put(0, j + i * step, v[i]);
         }
     }
-#pragma unroll 4
-    for (int j = j0; j < padded(a.kb); j += step) put(1, j, load4(a.x2 + j, a.kb - j));
+    for (int j = j0; j < padded(a.kb); j += kBatch * step) {
+        if (j != j0) {
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) second[i] = load4<VEC>(a.x2 + j + i * step, a.kb - (j + i * step));
+        }
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i)
+            if (j + i * step < padded(a.kb)) put(1, j + i * step, second[i]);
+    }
 }
 
-__device__ __forceinline__ void finish_row(const RowsArgs& a, int row, float v) {
+// What a row's epilogue adds: its bias or residual.  Asked for before the product, a trip to L2 (0.8 us) does not follow it.
+__device__ __forceinline__ float addend(const RowsArgs& a, int row) {
+    if (row >= a.na) return 0.f;
+    return a.epi == EPI_BIAS ? a.bias[row] : a.epi == EPI_RESIDUAL ? a.resid[row] : 0.f;
+}
+__device__ __forceinline__ void finish_row(const RowsArgs& a, int row, float v, float add) {
     if (row >= a.na) return;
     if (a.epi == EPI_MIXER_IN) {
         if (row < a.n_silu) v = lm::silu(v);
         else if (row >= a.n_sigmoid) v = lm::sigmoid(v);
     } else if (a.epi == EPI_RESIDUAL) {
-        v = fmaf(a.alpha, v, a.resid[row]);
+        v = fmaf(a.alpha, v, add);
     } else if (a.epi == EPI_BIAS) {
-        v += a.bias[row];
+        v += add;
     } else if (a.epi == EPI_RELU_SQUARED) {
         v = v > 0.f ? v * v : 0.f;
     } else if (a.epi == EPI_SOFTCAP) {
@@ -300,14 +344,17 @@ __global__ void __launch_bounds__(kThreads) rows_kernel(const RowsArgs a) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int parts = a.parts, teams = kWarps / parts, team = warp / parts, part = warp % parts;
     const int ua = (a.na + kRows - 1) / kRows, units = ua + (a.dual ? 0 : a.pairs);
-    const int xb = padded(a.ka);
-    StagedScales sc;
+    const int xb = padded(a.ka), grid = (int)gridDim.x - (a.C > 0);
+    if ((int)blockIdx.x == grid) {
+        append_latent<T>(a, scratch);
+        return;
+    }
+    StagedScales<false> sc;
     sc.request(a);
-    stage_input(a, sc, scratch, [&](int piece, int j, const float4& v) { *reinterpret_cast<float4*>(xs + (piece ? xb : 0) + j) = v; });
-    if (a.C > 0 && blockIdx.x == 0) append_latent<T>(a, scratch);
+    stage_input<false>(a, sc, scratch, [&](int piece, int j, const float4& v) { *reinterpret_cast<float4*>(xs + (piece ? xb : 0) + j) = v; });
     __syncthreads();
     const T *wa = reinterpret_cast<const T*>(a.wa), *wb = reinterpret_cast<const T*>(a.wb);
-    for (int u = team * gridDim.x + blockIdx.x; u < units; u += gridDim.x * teams) {
+    for (int u = team * grid + blockIdx.x; u < units; u += grid * teams) {
         float acc[kRows] = {};
         auto dot = [&](const T* w0, const T* w1, const float* x, int K) {
 #pragma unroll 8
@@ -339,8 +386,8 @@ __global__ void __launch_bounds__(kThreads) rows_kernel(const RowsArgs a) {
         }
         if (part == 0 && lane == 0) {
             if (a.dual || u < ua) {
-                finish_row(a, u * kRows, acc[0]);
-                finish_row(a, u * kRows + 1, acc[1]);
+                finish_row(a, u * kRows, acc[0], addend(a, u * kRows));
+                finish_row(a, u * kRows + 1, acc[1], addend(a, u * kRows + 1));
             } else {
                 a.out2[u - ua] = lm::gelu_tanh(acc[0]) * acc[1];
             }
@@ -366,7 +413,7 @@ __global__ void __launch_bounds__(kThreads) rows_mma_kernel(const __grid_constan
     const int xb = padded(a.ka);                        // one word per element
     const int ua = (a.na + kUnit - 1) / kUnit, units = ua + (a.dual ? 0 : (a.pairs + kUnit / 2 - 1) / (kUnit / 2));
     const int ia = (a.ka + kItem - 1) / kItem, ib = (a.kb + kItem - 1) / kItem;      // items of a piece
-    const int gt = team * gridDim.x + blockIdx.x, gteams = gridDim.x * teams;      // a last, partial round of units spreads over the SMs
+    const int grid = (int)gridDim.x - (a.C > 0), gt = team * grid + blockIdx.x, gteams = grid * teams;      // a last, partial round of units spreads over the SMs
     auto items_of = [&](int u) { return a.dual ? ia + ib : (u < ua ? ia : ib); };
     int pu = gt, pi = part, pslot = 0;                  // next item to request: unit, item, slot
     auto request = [&]() {
@@ -391,6 +438,11 @@ __global__ void __launch_bounds__(kThreads) rows_mma_kernel(const __grid_constan
     };
 
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if ((int)blockIdx.x == grid) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        append_latent<__nv_bfloat16>(a, scratch);
+        return;
+    }
     if (threadIdx.x == 0) abort_flag = 0;
     if (lane == 0) {
         for (int i = 0; i < slots; ++i) gemvq8::mbar_init(&full[warp][i], 1);
@@ -398,19 +450,34 @@ __global__ void __launch_bounds__(kThreads) rows_mma_kernel(const __grid_constan
         for (int i = 0; i < slots && pu < units; ++i) request();
     }
     __syncwarp();
-    StagedScales sc;
-    sc.request(a);
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-
-    stage_input(a, sc, scratch, [&](int piece, int j, const float4& v) {
+    // lanes that end up with rows g and g + 8 of a unit
+    const bool mine = part == 0 && (parts > 1 ? lane < 8 : (lane & 3) == 0);
+    const int g = parts > 1 ? lane : lane >> 2;
+    float add_lo = 0.f, add_hi = 0.f;
+    auto request_addends = [&](int u) {
+        if (mine && (a.dual || u < ua)) {
+            add_lo = addend(a, u * kUnit + g);
+            add_hi = addend(a, u * kUnit + g + 8);
+        }
+    };
+    auto put = [&](int piece, int j, const float4& v) {
         uint32_t h0, l0, h1, l1;
         lm::split2(v.x, v.y, h0, l0);
         lm::split2(v.z, v.w, h1, l1);
         uint32_t* f = xf + (piece ? xb : 0) + (j >> 4) * 16 + ((j & 7) >> 1) * 2 + ((j >> 3) & 1);
         f[0] = h0; f[2] = h1;                           // column 0, lanes t and t + 1
         f[8] = l0; f[10] = l1;                          // column 1
-    });
-    if (a.C > 0 && blockIdx.x == 0) append_latent<__nv_bfloat16>(a, scratch);
+    };
+    auto stage = [&](auto vec) {
+        StagedScales<decltype(vec)::value> sc;
+        sc.request(a);
+        if (a.epi == EPI_BIAS) request_addends(gt);     // constant
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (a.epi == EPI_RESIDUAL) request_addends(gt);
+        stage_input<decltype(vec)::value>(a, sc, scratch, put);
+    };
+    if (a.vec) stage(std::true_type{});
+    else stage(std::false_type{});
     __syncthreads();
 
     const int row = lane & 7;
@@ -424,6 +491,7 @@ __global__ void __launch_bounds__(kThreads) rows_mma_kernel(const __grid_constan
     for (int u = gt; u < units; u += gteams, parity ^= 1) {
         const int n = items_of(u);
         float c0[4] = {}, c1[4] = {};
+        if (u != gt) request_addends(u);
         int i = part;
         do {
             // once a wait has given up, the warp only keeps its team's barriers company
@@ -451,16 +519,12 @@ __global__ void __launch_bounds__(kThreads) rows_mma_kernel(const __grid_constan
         } while (i < n);
         // lanes 4 g: columns 0 and 1 of rows g and g + 8
         float lo = (c0[0] + c1[0]) + (c0[1] + c1[1]), hi = (c0[2] + c1[2]) + (c0[3] + c1[3]);
-        int g = lane >> 2;
-        bool mine = (lane & 3) == 0;
         if (parts > 1) {
-            if (mine) {
-                red[parity][warp][g] = lo;
-                red[parity][warp][g + 8] = hi;
+            if ((lane & 3) == 0) {
+                red[parity][warp][lane >> 2] = lo;
+                red[parity][warp][(lane >> 2) + 8] = hi;
             }
             asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(parts * 32) : "memory");
-            mine = part == 0 && lane < 8;
-            g = lane;
             if (mine) {
                 lo = hi = 0.f;
                 for (int q = 0; q < parts; ++q) {
@@ -471,8 +535,8 @@ __global__ void __launch_bounds__(kThreads) rows_mma_kernel(const __grid_constan
         }
         if (mine) {
             if (a.dual || u < ua) {
-                finish_row(a, u * kUnit + g, lo);
-                finish_row(a, u * kUnit + g + 8, hi);
+                finish_row(a, u * kUnit + g, lo, add_lo);
+                finish_row(a, u * kUnit + g + 8, hi, add_hi);
             } else {
                 const int p = (u - ua) * (kUnit / 2) + g;
                 if (p < a.pairs) a.out2[p] = lm::gelu_tanh(lo) * hi;
@@ -570,8 +634,8 @@ __global__ void __launch_bounds__(kThreads) lightning_step_kernel(const float* _
 
 // Queries into latent space: qa[h] = scale * [W_uk[h]^T q_h, rotate(q_h's rotated part)].  CTA = (head, 32 latent columns).
 template <class T>
-__global__ void __launch_bounds__(kThreads) absorb_kernel(const float* __restrict__ q, const T* __restrict__ uk, const float* __restrict__ freqs, int n_freq,
-                                                          float magnitude, const uint32_t* d_pos, float* __restrict__ qa, int D, int R, int C, float scale) {
+__global__ void __launch_bounds__(kThreads) absorb_kernel(const float* __restrict__ q, const T* __restrict__ uk, const float2* __restrict__ angles, int n_freq,
+                                                          float* __restrict__ qa, int D, int R, int C, float scale) {
     rcu_kernel_entry();
     __shared__ float part[kWarps][32];
     const int h = blockIdx.x, lane = threadIdx.x & 31, g = threadIdx.x >> 5;
@@ -593,9 +657,8 @@ __global__ void __launch_bounds__(kThreads) absorb_kernel(const float* __restric
         dst[c] = acc * scale;
     }
     if (blockIdx.y == 0) {
-        const uint32_t p = *d_pos;
         for (int i = threadIdx.x; i < n_freq; i += kThreads) {
-            const float2 cs = lm::rotary_angle(freqs, n_freq, i, p, magnitude);
+            const float2 cs = angles[i];
             const float u = qh[D + 2 * i], v = qh[D + 2 * i + 1];
             dst[C + 2 * i] = (u * cs.x - v * cs.y) * scale;
             dst[C + 2 * i + 1] = (v * cs.x + u * cs.y) * scale;
@@ -980,7 +1043,7 @@ struct rcu_stack {
     float* pool = nullptr;              // every f32 vector below
     float *x0, *xa, *xb, *mix, *act, *y, *sub, *q, *qa, *partial, *logits;
     float *angle_pool, *angle_tables, *arrived;      // (cos, sin) pairs; AngleTable[n_angles]; counters of the grouped attention
-    std::vector<float2*> run_angles;                 // per run: its pairs (null: no grouped mixer)
+    std::vector<float2*> run_angles;                 // per run: its pairs (null: a lightning mixer)
     int n_angles = 0;
     uint32_t* d_pos = nullptr;
     uint32_t position = 0, kernels_per_step = 0;
@@ -1035,7 +1098,10 @@ template <class T> rcu_status launch_rows(rcu_device* dev, RowsArgs a) {
         const int units = (a.na + kUnit - 1) / kUnit + (a.dual ? 0 : (a.pairs + kUnit / 2 - 1) / (kUnit / 2));
         const int ia = (a.ka + kItem - 1) / kItem, ib = has_b ? (a.kb + kItem - 1) / kItem : 0;
         a.parts = plan_parts(dev->sm_count, units, a.dual ? ia + ib : std::max(ia, ib));
-        const int grid = std::max(1, std::min(dev->sm_count, units));
+        const int append = a.C > 0;                          // its CTA wants an SM of its own
+        const int grid = std::max(1, std::min(dev->sm_count - append, units)) + append;
+        const uintptr_t at = (uintptr_t)a.x | (uintptr_t)a.x2 | (uintptr_t)a.s1 | (uintptr_t)a.s2 | (uintptr_t)a.b1 | (uintptr_t)a.b2 | (uintptr_t)a.gate;
+        a.vec = at % 16 == 0 && a.split % 4 == 0;             // lengths are multiples of 64
         CUtensorMap ma, mb;
         if (!make_block_map(&ma, a.wa, a.na, a.ka) || !make_block_map(&mb, has_b ? a.wb : a.wa, has_b ? (a.dual ? a.na : 2 * a.pairs) : a.na, has_b ? a.kb : a.ka))
             return rcu_fail(dev, RCU_ERR_CUDA, "stack: cuTensorMapEncodeTiled failed (%d x %d)", a.na, a.ka);
@@ -1044,7 +1110,7 @@ template <class T> rcu_status launch_rows(rcu_device* dev, RowsArgs a) {
     } else {
         const int units = (a.na + kRows - 1) / kRows + (a.dual ? 0 : a.pairs), nca = (a.ka + 255) / 256, ncb = (a.kb + 255) / 256;
         a.parts = plan_parts(dev->sm_count, units, a.dual ? nca + ncb : std::max(nca, ncb));
-        const int teams = kWarps / a.parts, grid = std::max(1, std::min(4 * dev->sm_count, (units + teams - 1) / teams));
+        const int teams = kWarps / a.parts, grid = std::max(1, std::min(4 * dev->sm_count, (units + teams - 1) / teams)) + (a.C > 0);
         if (inputs > most) return rcu_fail(dev, RCU_ERR_UNSUPPORTED, "stack: input vectors of %d + %d do not fit shared memory", a.ka, a.kb);
         RCU_CUDA(dev, cudaFuncSetAttribute(rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
         RCU_CUDA(dev, rcu_launch(dev, rows_kernel<T>, grid, kThreads, inputs, a));
@@ -1170,11 +1236,10 @@ template <class T> rcu_status run_step(rcu_stack* s, const int32_t* token, float
             STACK_TRY(launch_rows<T>(dev, in));
             RowsArgs uq = {};
             uq.wa = r.uq; uq.na = H * (D + R); uq.ka = Q; uq.pro = PRO_RMS; uq.x = s->mix; uq.s1 = (const float*)r.mix_norm; uq.eps = c.eps; uq.out = s->q;
-            uq.low = s->mix + Q; uq.c_scale = (const float*)r.kv_norm; uq.freqs = (const float*)r.freqs; uq.ring = r.state; uq.C = C; uq.R = R; uq.n_freq = nf;
-            uq.ring_rows = (int)r.ring_rows; uq.magnitude = r.rot_magnitude; uq.d_pos = s->d_pos;
+            uq.low = s->mix + Q; uq.c_scale = (const float*)r.kv_norm; uq.angles = s->run_angles[k]; uq.ring = r.state; uq.C = C; uq.R = R; uq.n_freq = nf;
+            uq.ring_rows = (int)r.ring_rows; uq.d_pos = s->d_pos;
             STACK_TRY(launch_rows<T>(dev, uq));
-            RCU_CUDA(dev, rcu_launch(dev, absorb_kernel<T>, dim3(H, (C + 31) / 32), kThreads, 0, s->q, (const T*)r.ukv, (const float*)r.freqs, nf, r.rot_magnitude,
-                                     s->d_pos, s->qa, D, R, C, r.scale));
+            RCU_CUDA(dev, rcu_launch(dev, absorb_kernel<T>, dim3(H, (C + 31) / 32), kThreads, 0, s->q, (const T*)r.ukv, s->run_angles[k], nf, s->qa, D, R, C, r.scale));
             RCU_LAUNCH_CHECK(dev);
             STACK_TRY(launch_latent_step(dev, s, r, c.weight_dt));
             const int per = 2 * kWarps, quads = (C + 3) / 4, groups = std::max(1, kThreads / quads);
@@ -1237,15 +1302,6 @@ rcu_status rcu_stack_create(rcu_device* dev, const rcu_stack_config* cfg, const 
             mix = std::max(mix, (size_t)(r.heads + r.kv_heads) * r.dim + (size_t)r.kv_heads * r.vdim);
             partial = std::max(partial, (size_t)grouped_splits(dev, r, cfg->weight_dt) * r.heads * gstep::pitch_of((int)r.vdim));
             arrived = std::max(arrived, (size_t)r.heads);
-            for (size_t t = 0; t < table_run.size() && table_of[i] < 0; ++t) {
-                const rcu_stack_run& o = runs[table_run[t]];
-                if (o.freqs == r.freqs && o.rot_pairs == r.rot_pairs && o.rot_magnitude == r.rot_magnitude) table_of[i] = (int)t;
-            }
-            if (table_of[i] < 0) {
-                table_of[i] = (int)table_run.size();
-                table_run.push_back(i);
-            }
-            pairs = std::max(pairs, (size_t)r.rot_pairs);
         } else {
             RCU_REQUIRE(dev, r.mixer == RCU_MIXER_LATENT, "stack: run %u has an unknown mixer", i);
             RCU_REQUIRE(dev, r.q_rank && r.kv_rank && r.kv_norm && r.uq && r.ukv && (r.rot_pairs == 0 || r.freqs) && 2 * r.rot_pairs <= r.rot_dim,
@@ -1256,6 +1312,17 @@ rcu_status rcu_stack_create(rcu_device* dev, const rcu_stack_config* cfg, const 
             q = std::max(q, (size_t)r.heads * (r.dim + r.rot_dim));
             qa = std::max(qa, (size_t)r.heads * (r.kv_rank + r.rot_dim));
             partial = std::max(partial, (size_t)latent_splits(r) * r.heads * partial_pitch((int)r.kv_rank));
+        }
+        if (r.mixer != RCU_MIXER_LIGHTNING) {
+            for (size_t t = 0; t < table_run.size() && table_of[i] < 0; ++t) {
+                const rcu_stack_run& o = runs[table_run[t]];
+                if (o.freqs == r.freqs && o.rot_pairs == r.rot_pairs && o.rot_magnitude == r.rot_magnitude) table_of[i] = (int)t;
+            }
+            if (table_of[i] < 0) {
+                table_of[i] = (int)table_run.size();
+                table_run.push_back(i);
+            }
+            pairs = std::max(pairs, (size_t)r.rot_pairs);
         }
         act = std::max(act, (size_t)r.ff);
         y = std::max(y, (size_t)r.heads * r.vdim);

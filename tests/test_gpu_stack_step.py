@@ -1,0 +1,37 @@
+"""The fused decode step where the staging of a product's inputs changes its form: vectors that do not start on sixteen bytes, second inputs
+of more than one batch of loads, and the token's latent written beside the query expansion."""
+import numpy as np
+import pytest
+
+from oracle import dadezen_plain as dz
+
+from . import dadezen_builders as B
+
+pytestmark = pytest.mark.gpu
+
+# the bound of the bf16 model tests (root mean square over the logits'): bf16 cached rows and 16-bit activations through two layers
+LIMIT = 4e-2
+MODELS = {
+    # a gate that starts at 2 * 63 + 64 floats: rows of whole blocks behind unaligned vectors
+    "unaligned": B.config(128, 64, [B.lightning(1, 63, 64, (0.9,), ff=192), B.latent(2, 30, 6, 32, 64, 64, 5, 0.2, ff=64)]),
+    # 8256 = 8192 + 64 activations of a feed-forward: one more than a batch takes
+    "long": B.config(64, 64, [B.lightning(2, 32, 32, (0.8, 0.99), ff=8256), B.latent(4, 16, 8, 16, 128, 192, 21, 0.25, scaling=B.YARN, ff=8192)]),
+}
+
+
+@pytest.mark.parametrize("name", sorted(MODELS))
+def test_tokens_agree_with_the_restatement(name, tmp_path):
+    from ratchet_b200 import Device
+    from ratchet_b200.models import load_model
+    cfg = MODELS[name]
+    W = B.weights(cfg, seed=5)
+    tokens = np.random.Generator(np.random.PCG64(3)).integers(0, cfg["vocab"], 40).tolist()
+    want = dz.forward(cfg, W, tokens)
+    dev = Device(0)
+    try:
+        m = load_model(B.write_model(str(tmp_path / name), cfg, W), dev, "bfloat16")
+        st = m.new_state(len(tokens))
+        got = np.concatenate([m.decode(st, t)[0].to_numpy() for t in tokens])
+    finally:
+        dev.close()
+    assert np.sqrt(((got - want) ** 2).mean(-1) / (want ** 2).mean()).max() < LIMIT
