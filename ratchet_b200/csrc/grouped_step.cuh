@@ -38,6 +38,7 @@ struct Args {
     uint32_t* arrived;                // one counter per blockIdx.y, zero between steps
     int H, G, D, E, pairs, ring_rows, window, chunk;
     float eps, scale;
+    bool ahead;                       // the ring's rows are not written by another run of the same step
 };
 
 __host__ __device__ __forceinline__ int pitch_of(int E) { return ((E + 3) & ~3) + 4; }
@@ -135,6 +136,7 @@ __global__ void __launch_bounds__(kThreads) grouped_step_mma_kernel(const Args a
     float* acc_s = reinterpret_cast<float*>(ql + kMmaHeads * ldq);        // [warps][nh][E]; the CTA's sums end up in the first [nh][E]
     __shared__ float m_s[kWarps][kMmaHeads], l_s[kWarps][kMmaHeads], weights[kMaxSplits * 16];
     __shared__ float cta_m[kMmaHeads], cta_l[kMmaHeads];
+    __shared__ __align__(16) bf16 now_k[NB * 32], now_v[EB * 64];         // the token's key and value as the ring holds them
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gr = lane >> 2, t = lane & 3;
     const int per = a.H / a.G, groups = head_groups(a.H, a.G, kMmaHeads);
     const int g = blockIdx.y / groups, hg = (blockIdx.y - g * groups) * kMmaHeads;
@@ -151,11 +153,69 @@ __global__ void __launch_bounds__(kThreads) grouped_step_mma_kernel(const Args a
     for (int h = warp; h < kMmaHeads; h += kWarps)
         for (int d = lane; d < ldq; d += 32)
             if (h >= nh || d >= a.D) qh[h * ldq + d] = ql[h * ldq + d] = __float2bfloat16_rn(0.f);
+    // What steps before this one wrote - the position, the cached rows - is complete before any kernel of this step but the first starts
+    // (embed_kernel); it is requested ahead of the wait for the kernel before, past L1, which may hold what an earlier step read.
+    if (!a.ahead) asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint32_t pos = __ldcg(a.d_pos);
+    const Visible see{a.window, a.chunk, 0};
+    const int low = see.first((int)pos), n = (int)pos - low + 1, tiles = (n + kTile - 1) / kTile;
+    const int active = min((int)gridDim.x, tiles);
+    const size_t W = (size_t)a.G * (a.D + a.E);
+    const bf16* K = reinterpret_cast<const bf16*>(a.ring) + (size_t)g * a.D;
+    const bf16* V = reinterpret_cast<const bf16*>(a.ring) + (size_t)a.G * a.D + (size_t)g * a.E;
+    uint4 k[NB][2], v[EB][4];
+    auto load = [&](int p0) {                 // rows before the current position; the others are zero until it is known (current)
+        const int base = p0 % a.ring_rows, cached = (int)pos - p0;
+        auto row = [&](int i) { return (size_t)(base + i < a.ring_rows ? base + i : base + i - a.ring_rows) * W; };
+        const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int r = i * 8 + gr;
+            const bf16* src = K + row(r);
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                const int d = b * 32 + t * 8;
+                k[b][i] = d < a.D && r < cached ? __ldcg(reinterpret_cast<const uint4*>(src + d)) : none;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = (i >> 1) * 8 + 2 * t + (i & 1);
+            const bf16* src = V + row(r);
+#pragma unroll
+            for (int c = 0; c < EB; ++c) {
+                const int e = c * 64 + gr * 8;
+                v[c][i] = e < a.E && r < cached ? __ldcg(reinterpret_cast<const uint4*>(src + e)) : none;
+            }
+        }
+    };
+    auto current = [&](int r) {               // the current position's row of a tile, from shared memory; rows behind it keep zeros, weight zero
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            if (i * 8 + gr == r)
+#pragma unroll
+                for (int b = 0; b < NB; ++b)
+                    if (b * 32 + t * 8 < a.D) k[b][i] = *reinterpret_cast<const uint4*>(now_k + b * 32 + t * 8);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if ((i >> 1) * 8 + 2 * t + (i & 1) == r)
+#pragma unroll
+                for (int c = 0; c < EB; ++c)
+                    if (c * 64 + gr * 8 < a.E) v[c][i] = *reinterpret_cast<const uint4*>(now_v + c * 64 + gr * 8);
+    };
+    const int first = (int)blockIdx.x + warp * active, step = active * kWarps;
+    const bool mine = (int)blockIdx.x < active && first < tiles;
+    if (mine) load(low + first * kTile);
+    const int merged = (int)blockIdx.x * kThreads + threadIdx.x;           // the first output quad this thread merges (clusters)
+    const float sink = CL && a.sink && merged < nh * (a.E / 4) ? a.sink[h0 + merged / (a.E / 4)] : 0.f;
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
-    const uint32_t pos = *a.d_pos;
     // the token's heads this warp prepares (two query heads; the last warp also the key and the value) and the angles, all in flight at once
-    float2 xq[2][KP], xk[KP], cs[KP];
+    float2 xq[2][KP], xk[KP], xv[EB], cs[KP];
+    const float* value = a.mix + (size_t)(a.H + a.G) * a.D + (size_t)g * a.E;
+#pragma unroll
+    for (int i = 0; i < EB; ++i)
+        xv[i] = 2 * (lane + 32 * i) < a.E && warp == kWarps - 1 ? *reinterpret_cast<const float2*>(value + 2 * (lane + 32 * i)) : make_float2(0.f, 0.f);
     const float* key = a.mix + (size_t)(a.H + g) * a.D;
 #pragma unroll
     for (int i = 0; i < KP; ++i) {
@@ -166,43 +226,7 @@ __global__ void __launch_bounds__(kThreads) grouped_step_mma_kernel(const Args a
             xq[x][i] = d < a.D && warp + x * kWarps < nh ? *reinterpret_cast<const float2*>(a.mix + (size_t)(h0 + warp + x * kWarps) * a.D + d) : make_float2(0.f, 0.f);
         xk[i] = d < a.D && warp == kWarps - 1 ? *reinterpret_cast<const float2*>(key + d) : make_float2(0.f, 0.f);
     }
-    const Visible see{a.window, a.chunk, 0};
-    const int low = see.first((int)pos), n = (int)pos - low + 1, tiles = (n + kTile - 1) / kTile;
-    const int active = min((int)gridDim.x, tiles);
     if (!CL && (int)blockIdx.x >= active) return;
-
-    const size_t W = (size_t)a.G * (a.D + a.E);
-    const bf16* K = reinterpret_cast<const bf16*>(a.ring) + (size_t)g * a.D;
-    const bf16* V = reinterpret_cast<const bf16*>(a.ring) + (size_t)a.G * a.D + (size_t)g * a.E;
-    uint4 k[NB][2], v[EB][4];
-    auto load = [&](int p0) {
-        const int base = p0 % a.ring_rows;
-        auto row = [&](int i) {               // positions beyond the current one: any row, weight zero
-            const int r = base + min(i, (int)pos - p0);
-            return (size_t)(r < a.ring_rows ? r : r - a.ring_rows) * W;
-        };
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const bf16* src = K + row(i * 8 + gr);
-#pragma unroll
-            for (int b = 0; b < NB; ++b) {
-                const int d = b * 32 + t * 8;
-                k[b][i] = d < a.D ? *reinterpret_cast<const uint4*>(src + d) : make_uint4(0u, 0u, 0u, 0u);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const bf16* src = V + row((i >> 1) * 8 + 2 * t + (i & 1));
-#pragma unroll
-            for (int c = 0; c < EB; ++c) {
-                const int e = c * 64 + gr * 8;
-                v[c][i] = e < a.E ? *reinterpret_cast<const uint4*>(src + e) : make_uint4(0u, 0u, 0u, 0u);
-            }
-        }
-    };
-    const int first = (int)blockIdx.x + warp * active, step = active * kWarps;
-    const bool mine = (int)blockIdx.x < active && first < tiles, early = mine && low + first * kTile + kTile <= (int)pos;
-    if (early) load(low + first * kTile);     // cached rows only: they travel while the queries are prepared
 
     // norm and rotation of a head in registers
     auto prepare = [&](float2(&x)[KP], const float2(&scale)[KP]) {
@@ -238,12 +262,20 @@ __global__ void __launch_bounds__(kThreads) grouped_step_mma_kernel(const Args a
 #pragma unroll
         for (int i = 0; i < KP; ++i) {
             const int d = 2 * (lane + 32 * i);
-            if (d < a.D) *reinterpret_cast<__nv_bfloat162*>(dst + (size_t)g * a.D + d) = __floats2bfloat162_rn(xk[i].x, xk[i].y);
+            if (d < a.D) {
+                const __nv_bfloat162 u = __floats2bfloat162_rn(xk[i].x, xk[i].y);
+                *reinterpret_cast<__nv_bfloat162*>(now_k + d) = u;
+                *reinterpret_cast<__nv_bfloat162*>(dst + (size_t)g * a.D + d) = u;
+            }
         }
-        const float* xv = a.mix + (size_t)(a.H + a.G) * a.D + (size_t)g * a.E;
-        for (int e = 2 * lane; e < a.E; e += 64) {
-            const float2 u = *reinterpret_cast<const float2*>(xv + e);
-            *reinterpret_cast<__nv_bfloat162*>(dst + (size_t)a.G * a.D + (size_t)g * a.E + e) = __floats2bfloat162_rn(u.x, u.y);
+#pragma unroll
+        for (int i = 0; i < EB; ++i) {
+            const int e = 2 * (lane + 32 * i);
+            if (e < a.E) {
+                const __nv_bfloat162 u = __floats2bfloat162_rn(xv[i].x, xv[i].y);
+                *reinterpret_cast<__nv_bfloat162*>(now_v + e) = u;
+                *reinterpret_cast<__nv_bfloat162*>(dst + (size_t)a.G * a.D + (size_t)g * a.E + e) = u;
+            }
         }
     }
     __syncthreads();
@@ -255,7 +287,8 @@ __global__ void __launch_bounds__(kThreads) grouped_step_mma_kernel(const Args a
         for (int j = 0; j < 8; ++j) o[c][j][0] = o[c][j][1] = o[c][j][2] = o[c][j][3] = 0.f;
     for (int tile = mine ? first : tiles; tile < tiles; tile += step) {
         const int p0 = low + tile * kTile;
-        if (tile != first || !early) load(p0);
+        if (tile != first) load(p0);
+        if (p0 + kTile > (int)pos) current((int)pos - p0);
         float s0[4] = {}, s1[4] = {};
 #pragma unroll
         for (int b = 0; b < NB; ++b)
@@ -379,7 +412,7 @@ __global__ void __launch_bounds__(kThreads) grouped_step_mma_kernel(const Args a
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();
     // every CTA merges a share of the outputs
-    for (int i = (int)blockIdx.x * kThreads + threadIdx.x; i < nh * quads; i += (int)gridDim.x * kThreads) {
+    for (int i = merged; i < nh * quads; i += (int)gridDim.x * kThreads) {
         const int h = i / quads, e = (i - h * quads) * 4;
         float M = -INFINITY, ms[kCluster], ls[kCluster];
         float4 x[kCluster];
@@ -393,7 +426,7 @@ __global__ void __launch_bounds__(kThreads) grouped_step_mma_kernel(const Args a
 #pragma unroll
         for (int j = 0; j < kCluster; ++j)
             if (j < active) M = fmaxf(M, ms[j]);
-        float l = a.sink ? expf(a.sink[h0 + h] - M) : 0.f;
+        float l = a.sink ? expf((i == merged ? sink : a.sink[h0 + h]) - M) : 0.f;
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int j = 0; j < kCluster; ++j)

@@ -574,7 +574,10 @@ struct AngleTable {
 template <class T>
 __global__ void __launch_bounds__(kThreads) embed_kernel(const int32_t* token, const T* __restrict__ table, int vocab, int width, float* x0, float* x,
                                                          const AngleTable* __restrict__ angles, int n_angles, const uint32_t* d_pos, int* status) {
-    rcu_kernel_entry();
+    // The step's first kernel lets the others start only behind its own wait: whatever steps before this one wrote (states, rings, the
+    // position) is complete when any of them begins, and may be read ahead of its wait.  (+1 us a step, against one trip to L2 or memory a mixer)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int rows = (int)gridDim.x - n_angles;
     if ((int)blockIdx.x >= rows) {
         const AngleTable t = angles[blockIdx.x - rows];
@@ -593,33 +596,43 @@ __global__ void __launch_bounds__(kThreads) embed_kernel(const int32_t* token, c
     }
 }
 
-// One token of linear attention: CTA = (head, 32 value columns), lane = column, warp = every eighth feature row.
+// One token of linear attention: CTA = (head, 32 value columns), lane = column, warp = every eighth feature row.  The state's rows come
+// from the step before: they are requested ahead of the wait (embed_kernel), so that behind it only the token's vectors travel.
 __global__ void __launch_bounds__(kThreads) lightning_step_kernel(const float* __restrict__ mix, const float* __restrict__ decay, float* __restrict__ state,
-                                                                  float* __restrict__ out, int H, int D, int E) {
-    rcu_kernel_entry();
+                                                                  float* __restrict__ out, int H, int D, int E, bool ahead) {
+    constexpr int kAhead = 16;                // rows of a warp in flight: all of a head of 128
     __shared__ float part[kWarps][32];
     const int h = blockIdx.x, lane = threadIdx.x & 31, g = threadIdx.x >> 5;
     const int e = blockIdx.y * 32 + lane;
     const float* q = mix + (size_t)h * D;
     const float* k = q + (size_t)H * D;
-    const float v = e < E ? mix[(size_t)2 * H * D + (size_t)h * E + e] : 0.f;
-    const float dec = decay[h];
     float* S = state + (size_t)h * D * E;
-    float o = 0.f;
-    if (e < E) {
-        constexpr int kAhead = 16;            // rows requested before the first of them is written back
-        for (int d0 = g; d0 < D; d0 += kWarps * kAhead) {
-            float s[kAhead];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const float dec = decay[h];
+    float s[kAhead], o = 0.f;
+    auto request = [&](int d0) {
 #pragma unroll
-            for (int i = 0; i < kAhead; ++i) s[i] = d0 + i * kWarps < D ? S[(size_t)(d0 + i * kWarps) * E + e] : 0.f;
+        for (int i = 0; i < kAhead; ++i) s[i] = e < E && d0 + i * kWarps < D ? __ldcg(S + (size_t)(d0 + i * kWarps) * E + e) : 0.f;
+    };
+    if (!ahead) asm volatile("griddepcontrol.wait;" ::: "memory");
+    request(g);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const float v = e < E ? __ldcg(mix + (size_t)2 * H * D + (size_t)h * E + e) : 0.f;
+    for (int d0 = g; d0 < D; d0 += kWarps * kAhead) {
+        if (d0 != g) request(d0);
+        float qd[kAhead], kd[kAhead];
 #pragma unroll
-            for (int i = 0; i < kAhead; ++i) {
-                const int d = d0 + i * kWarps;
-                if (d >= D) break;
-                s[i] = fmaf(dec, s[i], k[d] * v);
-                S[(size_t)d * E + e] = s[i];
-                o = fmaf(q[d], s[i], o);
-            }
+        for (int i = 0; i < kAhead; ++i) {
+            const bool in = d0 + i * kWarps < D;
+            qd[i] = in ? __ldcg(q + d0 + i * kWarps) : 0.f;
+            kd[i] = in ? __ldcg(k + d0 + i * kWarps) : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+            const int d = d0 + i * kWarps;
+            s[i] = fmaf(dec, s[i], kd[i] * v);
+            if (e < E && d < D) S[(size_t)d * E + e] = s[i];
+            o = d < D ? fmaf(qd[i], s[i], o) : o;
         }
     }
     part[g][lane] = o;
@@ -636,17 +649,30 @@ __global__ void __launch_bounds__(kThreads) lightning_step_kernel(const float* _
 template <class T>
 __global__ void __launch_bounds__(kThreads) absorb_kernel(const float* __restrict__ q, const T* __restrict__ uk, const float2* __restrict__ angles, int n_freq,
                                                           float* __restrict__ qa, int D, int R, int C, float scale) {
-    rcu_kernel_entry();
+    constexpr int kAhead = 16;                // rows of a warp in flight; weights are constant: the first ones are requested ahead of the wait
     __shared__ float part[kWarps][32];
     const int h = blockIdx.x, lane = threadIdx.x & 31, g = threadIdx.x >> 5;
     const int c = blockIdx.y * 32 + lane;
     const float* qh = q + (size_t)h * (D + R);
     float* dst = qa + (size_t)h * (C + R);
+    const T* w = uk + (size_t)h * D * C + c;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    T u[kAhead];
+    auto request = [&](int d0) {
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) u[i] = c < C && d0 + i * kWarps < D ? w[(size_t)(d0 + i * kWarps) * C] : from_f32<T>(0.f);
+    };
+    request(g);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     float acc = 0.f;
-    if (c < C) {
-        const T* w = uk + (size_t)h * D * C + c;
-#pragma unroll 8
-        for (int d = g; d < D; d += kWarps) acc = fmaf(to_f32<T>(w[(size_t)d * C]), qh[d], acc);
+    for (int d0 = g; d0 < D; d0 += kWarps * kAhead) {
+        if (d0 != g) request(d0);
+        float x[kAhead];
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) x[i] = d0 + i * kWarps < D ? __ldcg(qh + d0 + i * kWarps) : 0.f;
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i)
+            if (d0 + i * kWarps < D) acc = fmaf(to_f32<T>(u[i]), x[i], acc);
     }
     part[g][lane] = acc;
     __syncthreads();
@@ -786,8 +812,7 @@ __global__ void __launch_bounds__(kThreads) latent_step_kernel(const float* __re
 constexpr int kMmaHeads = 16;
 template <int PC>
 __global__ void __launch_bounds__(kThreads) latent_step_mma_kernel(const float* __restrict__ qa, const lm::bf16* __restrict__ ring, int ring_rows, int window,
-                                                                   const uint32_t* d_pos, float* __restrict__ partial, int H, int C, int R) {
-    rcu_kernel_entry();
+                                                                   const uint32_t* d_pos, float* __restrict__ partial, int H, int C, int R, bool ahead) {
     using lm::bf16;
     extern __shared__ __align__(16) bf16 tiles[];        // queries (value, remainder), staged rows
     __shared__ float part[kWarps][kMmaHeads][kSub + 1];
@@ -797,37 +822,67 @@ __global__ void __launch_bounds__(kThreads) latent_step_mma_kernel(const float* 
     bf16 *qh = tiles, *ql = qh + kMmaHeads * ld, *rows = ql + kMmaHeads * ld;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int h0 = blockIdx.y * kMmaHeads;
-    const int pos = (int)*d_pos, first = max(0, pos - window + 1), n = pos - first + 1;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // the position and the rows of earlier tokens were written by earlier steps: requested ahead of the wait (embed_kernel)
+    const int pos = (int)__ldcg(d_pos), first = max(0, pos - window + 1), n = pos - first + 1;
     const int per = (n + gridDim.x - 1) / gridDim.x;
     const int begin = first + min(n, (int)blockIdx.x * per), end = first + min(n, ((int)blockIdx.x + 1) * per);
-    auto stage = [&](int p0) {
-        const int np = min(kSub, end - p0), octets = wp / 8;
+    const int octets = wp / 8;
+    // rows r0 to r1 of the kSub behind p0; those from `end` on become zero
+    auto stage = [&](int p0, int r0, int r1) {
+        const int np = min(kSub, end - p0);
         if (W % 8 == 0) {
 #pragma unroll 6
-            for (int i = threadIdx.x; i < kSub * octets; i += kThreads) {
+            for (int i = r0 * octets + threadIdx.x; i < r1 * octets; i += kThreads) {
                 const int r = i / octets, c = (i - r * octets) * 8;
                 const bool in = r < np && c < W;
                 lm::cp_async16(rows + r * ld + c, ring + (in ? (size_t)((p0 + r) % ring_rows) * W + c : 0), in);
             }
             lm::cp_commit();
         } else {
-            for (int i = threadIdx.x; i < kSub * wp; i += kThreads) {
+            for (int i = r0 * wp + threadIdx.x; i < r1 * wp; i += kThreads) {
                 const int r = i / wp, c = i - r * wp;
                 rows[r * ld + c] = r < np && c < W ? ring[(size_t)((p0 + r) % ring_rows) * W + c] : __float2bfloat16_rn(0.f);
             }
         }
     };
-    if (begin < end) stage(begin);
+    // row of the current position in this CTA's first tile (kSub: not there)
+    const int now = W % 8 != 0 ? 0 : begin < end && pos - begin < kSub && pos < end ? pos - begin : kSub;
+    if (!ahead) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (begin < end) stage(begin, 0, now);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (begin < end) stage(begin, now, kSub);
     const int quads = wp / 4;
-#pragma unroll 8
-    for (int i = threadIdx.x; i < kMmaHeads * quads; i += kThreads) {
-        const int r = i / quads, c = (i - r * quads) * 4;
-        const float4 v = h0 + r < H ? load4(qa + (size_t)(h0 + r) * W + c, W - c) : make_float4(0.f, 0.f, 0.f, 0.f);
-        uint2 hi, lo;
-        lm::split2(v.x, v.y, hi.x, lo.x);
-        lm::split2(v.z, v.w, hi.y, lo.y);
-        *reinterpret_cast<uint2*>(qh + r * ld + c) = hi;
-        *reinterpret_cast<uint2*>(ql + r * ld + c) = lo;
+    if (W % 4 == 0) {                                    // a query head starts on sixteen bytes: batches of loads that leave together
+        constexpr int kFly = 10;
+        for (int i0 = threadIdx.x; i0 < kMmaHeads * quads; i0 += kFly * kThreads) {
+            float4 v[kFly];
+#pragma unroll
+            for (int x = 0; x < kFly; ++x) {
+                const int i = i0 + x * kThreads, r = i / quads, c = (i - r * quads) * 4;
+                v[x] = r < kMmaHeads && h0 + r < H && c < W ? __ldcg(reinterpret_cast<const float4*>(qa + (size_t)(h0 + r) * W + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int x = 0; x < kFly; ++x) {
+                const int i = i0 + x * kThreads, r = i / quads, c = (i - r * quads) * 4;
+                if (r >= kMmaHeads) break;
+                uint2 hi, lo;
+                lm::split2(v[x].x, v[x].y, hi.x, lo.x);
+                lm::split2(v[x].z, v[x].w, hi.y, lo.y);
+                *reinterpret_cast<uint2*>(qh + r * ld + c) = hi;
+                *reinterpret_cast<uint2*>(ql + r * ld + c) = lo;
+            }
+        }
+    } else {
+        for (int i = threadIdx.x; i < kMmaHeads * quads; i += kThreads) {
+            const int r = i / quads, c = (i - r * quads) * 4;
+            const float4 v = h0 + r < H ? load4(qa + (size_t)(h0 + r) * W + c, W - c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            uint2 hi, lo;
+            lm::split2(v.x, v.y, hi.x, lo.x);
+            lm::split2(v.z, v.w, hi.y, lo.y);
+            *reinterpret_cast<uint2*>(qh + r * ld + c) = hi;
+            *reinterpret_cast<uint2*>(ql + r * ld + c) = lo;
+        }
     }
     const int sh = threadIdx.x >> 4, sp = threadIdx.x & 15;              // this thread's (head, position) of the softmax
     float m = -INFINITY, l = 0.f, o[PC][2][4];
@@ -838,7 +893,7 @@ __global__ void __launch_bounds__(kThreads) latent_step_mma_kernel(const float* 
     for (int p0 = begin; p0 < end; p0 += kSub) {
         if (p0 != begin) {
             __syncthreads();
-            stage(p0);
+            stage(p0, 0, kSub);
         }
         lm::cp_wait<0>();
         __syncthreads();
@@ -940,6 +995,14 @@ __global__ void __launch_bounds__(kThreads) latent_values_kernel(const float* __
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const float* ph = partial + (size_t)h * pitch;
     const size_t stride = (size_t)H * pitch;
+    // the first sums of each group travel with the maxima that weigh them
+    constexpr int kFly = 16;
+    const int gi = threadIdx.x / quads, gc = (threadIdx.x - gi * quads) * 4;
+    const bool whole = groups * quads <= kThreads;       // one (group, quad) per thread
+    float4 fly[kFly];
+#pragma unroll
+    for (int i = 0; i < kFly; ++i)
+        fly[i] = whole && gi < groups && gi + i * groups < splits ? __ldcg(reinterpret_cast<const float4*>(ph + (gi + i * groups) * stride + gc)) : make_float4(0.f, 0.f, 0.f, 0.f);
     if (warp == 0) {
         const float m0 = lane < splits ? ph[lane * stride + pitch - 2] : -INFINITY, m1 = lane + 32 < splits ? ph[(lane + 32) * stride + pitch - 2] : -INFINITY;
         const float l0 = lane < splits ? ph[lane * stride + pitch - 1] : 0.f, l1 = lane + 32 < splits ? ph[(lane + 32) * stride + pitch - 1] : 0.f;
@@ -953,8 +1016,21 @@ __global__ void __launch_bounds__(kThreads) latent_values_kernel(const float* __
     for (int i = threadIdx.x; i < groups * quads; i += kThreads) {
         const int g = i / quads, c = (i - g * quads) * 4;
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        int j0 = g;
+        if (whole) {
+#pragma unroll
+            for (int x = 0; x < kFly; ++x) {
+                if (g + x * groups >= splits) break;
+                const float w = wgt[g + x * groups];
+                s.x = fmaf(w, fly[x].x, s.x);
+                s.y = fmaf(w, fly[x].y, s.y);
+                s.z = fmaf(w, fly[x].z, s.z);
+                s.w = fmaf(w, fly[x].w, s.w);
+            }
+            j0 = g + kFly * groups;
+        }
 #pragma unroll 16
-        for (int j = g; j < splits; j += groups) {
+        for (int j = j0; j < splits; j += groups) {
             const float4 v = *reinterpret_cast<const float4*>(ph + j * stride + c);
             s.x = fmaf(wgt[j], v.x, s.x);
             s.y = fmaf(wgt[j], v.y, s.y);
@@ -1045,6 +1121,7 @@ struct rcu_stack {
     float *angle_pool, *angle_tables, *arrived;      // (cos, sin) pairs; AngleTable[n_angles]; counters of the grouped attention
     std::vector<float2*> run_angles;                 // per run: its pairs (null: a lightning mixer)
     int n_angles = 0;
+    bool ahead = true;                  // no two runs share memory of their states: kernels may read theirs ahead of the wait
     uint32_t* d_pos = nullptr;
     uint32_t position = 0, kernels_per_step = 0;
     uint64_t steps = 0;
@@ -1121,18 +1198,18 @@ template <class T> rcu_status launch_rows(rcu_device* dev, RowsArgs a) {
 
 rcu_status launch_latent_step(rcu_device* dev, const rcu_stack* s, const rcu_stack_run& r, int dt) {
     const int H = (int)r.heads, C = (int)r.kv_rank, R = (int)r.rot_dim, splits = latent_splits(r);
-#define RCU_LS(KERN_, GRID_, T_)                                                                                                                 \
+#define RCU_LS(KERN_, GRID_, T_, ...)                                                                                                                 \
     do {                                                                                                                                         \
         RCU_CUDA(dev, cudaFuncSetAttribute(KERN_, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(smem, (size_t)(48 * 1024))));       \
-        RCU_CUDA(dev, rcu_launch(dev, KERN_, GRID_, kThreads, smem, s->qa, (const T_*)r.state, (int)r.ring_rows, (int)r.window, s->d_pos, s->partial, H, C, R)); \
+        RCU_CUDA(dev, rcu_launch(dev, KERN_, GRID_, kThreads, smem, s->qa, (const T_*)r.state, (int)r.ring_rows, (int)r.window, s->d_pos, s->partial, H, C, R, ##__VA_ARGS__)); \
     } while (0)
     if (dt == RCU_BF16) {
         const int wp = (C + R + 15) & ~15;
         const size_t smem = (size_t)(2 * kMmaHeads + kSub) * (wp + 8) * sizeof(lm::bf16);
         const dim3 grid(splits, (H + kMmaHeads - 1) / kMmaHeads);
-        if (wp <= 256) RCU_LS(latent_step_mma_kernel<2>, grid, lm::bf16);
-        else if (wp <= 640) RCU_LS(latent_step_mma_kernel<5>, grid, lm::bf16);
-        else RCU_LS(latent_step_mma_kernel<10>, grid, lm::bf16);
+        if (wp <= 256) RCU_LS(latent_step_mma_kernel<2>, grid, lm::bf16, s->ahead);
+        else if (wp <= 640) RCU_LS(latent_step_mma_kernel<5>, grid, lm::bf16, s->ahead);
+        else RCU_LS(latent_step_mma_kernel<10>, grid, lm::bf16, s->ahead);
     } else {
         const int WP = (C + R + 7) & ~7;
         const size_t smem = (size_t)kHeads * WP * 4 + (size_t)kSub * WP * sizeof(float);
@@ -1186,7 +1263,7 @@ template <class T> rcu_status run_step(rcu_stack* s, const int32_t* token, float
             STACK_TRY(launch_rows<T>(dev, in));
             const gstep::Args at{s->mix, (const float*)r.mix_norm, (const float*)r.kv_norm, s->run_angles[k], (const float*)r.sink, r.state, s->d_pos, s->y, s->partial,
                                  (uint32_t*)s->arrived, H, G, D, E, (int)r.rot_pairs, (int)r.ring_rows,
-                                 r.window ? (int)std::min<uint32_t>(r.window, 1u << 30) : 1 << 30, (int)std::min<uint32_t>(r.chunk, 1u << 30), c.eps, r.scale};
+                                 r.window ? (int)std::min<uint32_t>(r.window, 1u << 30) : 1 << 30, (int)std::min<uint32_t>(r.chunk, 1u << 30), c.eps, r.scale, s->ahead};
             STACK_TRY(gstep::launch(dev, c.weight_dt, at, grouped_splits(dev, r, c.weight_dt)));
             RowsArgs o = {};
             o.wa = r.out; o.na = W; o.ka = H * E; o.pro = PRO_CONCAT; o.x = s->y; o.out = s->sub;
@@ -1226,7 +1303,7 @@ template <class T> rcu_status run_step(rcu_stack* s, const int32_t* token, float
             in.na = 2 * H * D + 2 * H * E;
             in.epi = EPI_MIXER_IN; in.n_silu = 2 * H * D + H * E; in.n_sigmoid = in.n_silu;
             STACK_TRY(launch_rows<T>(dev, in));
-            RCU_CUDA(dev, rcu_launch(dev, lightning_step_kernel, dim3(H, (E + 31) / 32), kThreads, 0, s->mix, (const float*)r.decay, (float*)r.state, s->y, H, D, E));
+            RCU_CUDA(dev, rcu_launch(dev, lightning_step_kernel, dim3(H, (E + 31) / 32), kThreads, 0, s->mix, (const float*)r.decay, (float*)r.state, s->y, H, D, E, s->ahead));
             RCU_LAUNCH_CHECK(dev);
             out.pro = PRO_GATED_RMS; out.x = s->y; out.s1 = (const float*)r.mix_norm; out.gate = s->mix + 2 * H * D + H * E;
         } else {
@@ -1355,6 +1432,16 @@ rcu_status rcu_stack_create(rcu_device* dev, const rcu_stack_config* cfg, const 
     }
     for (uint32_t i = 0; i < cfg->n_runs; ++i) s->run_angles.push_back(table_of[i] < 0 ? nullptr : tables[table_of[i]].out);
     s->n_angles = (int)n_tables;
+    std::vector<std::pair<uintptr_t, uintptr_t>> held;
+    for (const rcu_stack_run& r : s->runs) {
+        const uint64_t e = dt_esize(cfg->weight_dt);
+        const uint64_t bytes = r.mixer == RCU_MIXER_LIGHTNING ? (uint64_t)r.heads * r.dim * r.vdim * 4
+                               : r.mixer == RCU_MIXER_GROUPED ? (uint64_t)r.ring_rows * r.kv_heads * (r.dim + r.vdim) * e
+                                                              : (uint64_t)r.ring_rows * (r.kv_rank + r.rot_dim) * e;
+        held.emplace_back((uintptr_t)r.state, (uintptr_t)r.state + bytes);
+    }
+    std::sort(held.begin(), held.end());
+    for (size_t i = 1; i < held.size(); ++i) s->ahead = s->ahead && held[i - 1].second <= held[i].first;
     if (n_tables) st = rcu_h2d(dev, s->angle_tables, tables.data(), n_tables * sizeof(AngleTable));
     if (st == RCU_OK) st = rcu_memset(dev, s->arrived, 0, arrived * 4);
     if (st == RCU_OK) st = rcu_sync(dev);             // the tables' host copy ends with this call
