@@ -16,8 +16,8 @@
 //                      output feature), add bias, round to f16, store rows.
 // Quantised weights (Q8_0H, Q4_KH) are dequantised inside the kernel (up to 256 token rows): TMA
 // brings the packed bytes of the weight tile into shared memory, further warps convert them to f16
-// with the CPU dequantiser's arithmetic and write the swizzled tile the MMA reads.  Larger M
-// dequantises once into pooled scratch and runs the f16 kernel.
+// with the CPU dequantiser's arithmetic and write the swizzled tile the MMA reads.  Larger M takes the
+// pair kernel, which converts on the way too, or - too few tiles for it - dequantises once into pooled scratch.
 //
 // Every mbarrier wait is bounded; a wait that gives up sets RCU_DEVFLAG_TIMEOUT and an abort word in
 // shared memory that ends all other waits of the CTA, and the CTA still frees its tensor memory.
@@ -36,14 +36,6 @@ using namespace tc;
 }  // namespace
 
 namespace {
-
-enum { WK_F16 = 0, WK_Q8 = 1, WK_Q4K = 2 };   // how the weight tile reaches shared memory
-
-struct QuantArgs {
-    const void* scales;     // Q8_0H: f16 block scales [N * K/32]; Q4_KH: 12-byte (scale, min) packs [N * K/256]
-    const __half* d;        // Q4_KH super-block scale  [N * K/256]
-    const __half* dmin;     // Q4_KH super-block min    [N * K/256]
-};
 
 // One CTA computes one 128 x BN output tile.  WK_F16: the weight tile arrives by TMA like the
 // activation tile.  WK_Q8 / WK_Q4K: TMA brings the packed bytes of the tile (BN rows x 64 int8 or
@@ -405,13 +397,25 @@ bool rcu_gemm_tc2_eligible(rcu_device* dev, uint64_t M, uint64_t N, uint64_t K);
 rcu_status rcu_gemm_tc2_launch(rcu_device* dev, const void* w, const void* x, const void* bias, void* y, uint64_t M, uint64_t N, uint64_t K,
                                const TcLinear& t);
 
-// Quantised weights.  The fused kernel converts a weight tile once per 128-row token tile, i.e. M/128 times over the whole problem, and it is the
-// one-CTA kernel.  Beyond kFusedMaxM token rows it is cheaper to convert the matrix once into pooled f16 scratch (which stays in L2) and
-// run the f16 kernels on it (M = 512, N = 8192, K = 3072, Q4_K: 34 us against 46 us fused).  RCU_GEMM_FUSED=0/1 forces either path.
+// Quantised weights.  The one-CTA kernel converts a weight tile once per 128-row token tile, i.e. M/128 times over the whole problem.  Beyond
+// kFusedMaxM token rows the pair kernel converts its tiles itself where that pays (pair_converts); otherwise the matrix is converted once into pooled
+// f16 scratch (which stays in L2) for the f16 kernels (M = 512, N = 8192, K = 3072, Q4_K: 34 us against 46 us in the one-CTA kernel).
+// RCU_GEMM_FUSED=0/1 forces the conversion or the one-CTA kernel.
 constexpr uint64_t kFusedMaxM = 256;
 static bool converts_once(uint64_t M) {
     const char* force = getenv("RCU_GEMM_FUSED");
     return force ? atoi(force) == 0 : M > kFusedMaxM;
+}
+
+// Whether the pair kernel converts the tiles itself (gemm_tc2.cu; K of whole groups of 256).  A conversion costs 8.4 ns (Q8_0H; Q4_KH 7) for each
+// 256 weight rows and 64 of K; in the kernel every round of tiles takes some 0.16 us (0.17) longer per 64 of K, the codes passing through
+// shared memory.  us converted / in the kernel, Q8_0H 9216 x 3072: 300 rows 35.8 / 30.5, 512 36.6 / 31.0, 768 (a second round) 51.0 / 53.3, 1000 56.3 /
+// 57.8, 2048 96.4 / 120.1; 16384 x 3072: 512 74.1 / 63.3, 1000 104.7 / 119.9; 5120 x 8192: 512 66.8 / 63.7; 3072 x 8192: 1000 57.1 / 63.2; Q4_KH
+// 9216 x 3072: 300 36.5 / 31.1; 16384 x 3072: 512 69.4 / 60.6; 5120 x 8192: 512 65.9 / 68.8; 32064 x 3072: 300 126.7 / 111.9.
+static bool pair_converts(rcu_device* dev, int dt, uint64_t M, uint64_t N, uint64_t K) {
+    if (K % 256 != 0 || !rcu_gemm_tc2_eligible(dev, M, N, K)) return false;
+    const uint64_t tiles_n = (N + 255) / 256, pairs = dev->sm_count / 2, rounds = ((M + 255) / 256 * tiles_n + pairs - 1) / pairs;
+    return tiles_n > (dt == RCU_Q8_0H ? 19 : 24) * rounds;
 }
 
 // The Linear of an f16 graph with what follows it (TcLinear: chained, or glu): whether the tensor-core kernels take it.  A gate and its up
@@ -431,6 +435,15 @@ rcu_status rcu_gemm_tc_dispatch(rcu_device* dev, int lhs_dt, const void* w, int 
     if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(w)) & 15) return RCU_ERR_UNSUPPORTED;
     DevGuard g(dev->ordinal);
     if (lhs_dt == RCU_F16 && rcu_gemm_tc2_eligible(dev, M, N, K)) return rcu_gemm_tc2_launch(dev, w, x, bias, y, M, N, K, t);
+    if (lhs_dt != RCU_F16 && converts_once(M) && !getenv("RCU_GEMM_FUSED") && pair_converts(dev, lhs_dt, M, N, K)) {
+        size_t at[4];
+        rcu_dtype_segments(lhs_dt, N * K, at);
+        TcLinear q = t;
+        q.wk = lhs_dt == RCU_Q8_0H ? WK_Q8 : WK_Q4K;
+        const char* base = (const char*)w;
+        q.quant = QuantArgs{base + at[1], lhs_dt == RCU_Q4_KH ? (const __half*)(base + at[3]) : nullptr, lhs_dt == RCU_Q4_KH ? (const __half*)(base + at[2]) : nullptr, base};
+        return rcu_gemm_tc2_launch(dev, nullptr, x, bias, y, M, N, K, q);
+    }
     void* scratch = nullptr;
     if (lhs_dt != RCU_F16 && converts_once(M) && rcu_alloc(dev, N * K * 2, &scratch) == RCU_OK) {       // no room for the matrix: fused
         rcu_tensor src{lhs_dt, 2, {N, K, 1, 1}, const_cast<void*>(w)};

@@ -343,6 +343,15 @@ template <class Out, int MODE = EPI_PLAIN> struct GemmEpilogue {
 
 }  // namespace tc
 
+// How the weight tile of an f16 GEMM reaches shared memory, and what the quantised forms have beside their codes
+enum { WK_F16 = 0, WK_Q8 = 1, WK_Q4K = 2 };
+struct QuantArgs {
+    const void* scales;     // Q8_0H: f16 block scales [N * K/32]; Q4_KH: 12-byte (scale, min) packs [N * K/256]
+    const __half* d;        // Q4_KH super-block scale  [N * K/256]
+    const __half* dmin;     // Q4_KH super-block min    [N * K/256]
+    const void* codes = nullptr;      // the pair kernel reads them itself
+};
+
 // Host-side description of a 16-bit tensor-core Linear beyond its sizes (rcu_linear): operand type, row pitch of the
 // activations in elements (0: K), output type and the f32 epilogue.
 struct TcLinear {
@@ -358,5 +367,7 @@ struct TcLinear {
     int chain_op = -1;
     // out [M, N / 2] = up * act(gate) of rows that hold gate, then up, rounded as the graph's own kernels round; glu: RCU_GELU or RCU_SILU
     int glu = -1;
+    int wk = WK_F16;      // quantised weights, converted in the pair kernel
+    QuantArgs quant = {};
     bool chained() const { return bias32 || resid16 || chain_op >= 0; }
 };
