@@ -43,6 +43,9 @@ struct rcu_device {
     uint64_t wait_limit_ns = 2000000000ull;
     bool const_weights = false;  // rcu_set_constant_weights: GEMVs may request weight rows before their predecessor ends
     bool resident_weights = false;   // the resolver, for one product: its weights were uploaded and waited for, so any kernel may
+    // the resolver, for one product: a Q8_0H matrix to be converted beside it, for the product after (gemm_tc2.cu sets `started`)
+    struct NextConversion { const void* codes = nullptr; const void* scales = nullptr; void* dst = nullptr; uint64_t numel = 0; bool started = false; };
+    NextConversion* next_conversion = nullptr;
     int* h_status = nullptr;     // pinned host mirror
     rcu_resolve_stats last_resolve = {};   // counters of the last lazy-graph resolve (graph.cu)
     uint32_t debug_flags = 0;    // RCU_DEBUG_* (rcu_set_debug; RCU_NO_REUSE / RCU_PROFILE in the environment at creation)

@@ -576,6 +576,10 @@ rcu_status rcu_gemm_tc_chain(rcu_device* dev, int w_dt, const void* w, const voi
     return rcu_gemm_tc_dispatch(dev, w_dt, w, RCU_F16, x, c.bias, y, M, N, K, t);
 }
 
+bool rcu_linear_converts_beside(rcu_device* dev, uint64_t M, uint64_t N, uint64_t K) {
+    return M > kFusedMaxM && converts_once(M) && rcu_gemm_tc_eligible(RCU_Q8_0H, RCU_F16, M, N, K) && rcu_gemm_tc2_eligible(dev, M, N, K) &&
+           (getenv("RCU_GEMM_FUSED") || !pair_converts(dev, RCU_Q8_0H, M, N, K));
+}
 bool rcu_gemm_tc_f32_eligible(int lhs_dt, int act_dt, uint64_t M, uint64_t N, uint64_t K, uint64_t batches = 1);
 bool rcu_linear_converts(int w_dt, int act_dt, uint64_t M, uint64_t N, uint64_t K) {
     if (w_dt == RCU_Q8_0H && act_dt == RCU_F16) return M > kFusedMaxM && converts_once(M) && rcu_gemm_tc_eligible(w_dt, act_dt, M, N, K);

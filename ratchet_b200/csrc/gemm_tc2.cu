@@ -290,7 +290,7 @@ template <class Out> __device__ __forceinline__ float glu_value(int act, float g
 template <class Out, int MODE, bool GLU, int WK>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(threads2(WK), 1)
 gemm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const GemmEpilogue<Out, MODE> epi,
-                Out* out, int M, int N, int K, int tiles_m, int n_tiles, int* status, uint32_t idesc, int glu_act, const QuantArgs qa) {
+                Out* out, int M, int N, int K, int tiles_m, int n_tiles, int* status, uint32_t idesc, int glu_act, const QuantArgs qa, bool lead) {
     constexpr int STAGES = stages2(WK), RAW = raw_bytes(WK);
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
@@ -340,6 +340,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
     cluster_sync_all();            // barriers of both CTAs initialised before anyone signals them
     tc_fence_after();
     rcu_kernel_entry_wait_only();  // nothing before this touches global memory: the set-up overlaps the kernel before
+    if (lead) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // a conversion for the next product runs beside this one
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
@@ -513,12 +514,14 @@ rcu_status launch_pair(rcu_device* dev, const CUtensorMap& xmap, const CUtensorM
     const int tiles_m = (int)((M + 255) / 256), tiles_n = (int)((N + 255) / 256);      // a tile of gates takes 256 rows of W too
     const int n_tiles = tiles_m * tiles_n;
     const int n_pairs = std::min(n_tiles, dev->sm_count / 2);
+    rcu_device::NextConversion* next = dev->next_conversion;
     constexpr size_t smem = smem2(WK);
     auto kern = gemm_tc2_kernel<Out, MODE, GLU, WK>;
     RCU_CUDA(dev, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     RCU_CUDA(dev, rcu_launch(dev, kern, 2 * n_pairs, threads2(WK), smem, xmap, wmap, epi, (Out*)y, (int)M, (int)(GLU ? N / 2 : N), (int)K, tiles_m, n_tiles, dev->d_status,
-                             umma_idesc_f16(2 * TM, kTileN2, t.bf16), t.glu, t.quant));
+                             umma_idesc_f16(2 * TM, kTileN2, t.bf16), t.glu, t.quant, next != nullptr));
     RCU_LAUNCH_CHECK(dev);
+    if (next) next->started = rcu_dequantize_beside(dev, *next) == RCU_OK;
     return RCU_OK;
 }
 }  // namespace

@@ -413,12 +413,14 @@ struct Converted {
         const rcu_lazy* w = made.empty() ? nullptr : weight(t, op);
         return w ? of(w) : nullptr;
     }
-    static const rcu_lazy* weight(const rcu_lazy* t, const fusion::Op* op) {
+    static const rcu_lazy* weight(const rcu_lazy* t, const fusion::Op* op, bool large = false) {
         const bool fused = op && op->kind == fusion::LINEAR;
         if (!fused && (op || t->kind != K_MATMUL || t->flags[0] || !t->flags[1] || !t->flags[2])) return nullptr;
         const rcu_lazy *w = fused ? op->w : t->srcs[0], *x = fused ? op->x : t->srcs[1];
-        if (!dt_is_q8(w->dt) || w->rank != 2 || !w->resolved() || w->numel() > kNumel || x->shape[x->rank - 1] != w->shape[1] || !fusion::Pass::aligned(w)) return nullptr;
-        return rcu_linear_converts(w->dt, x->dt, x->numel() / w->shape[1], w->shape[0], w->shape[1]) ? w : nullptr;
+        if (!dt_is_q8(w->dt) || w->rank != 2 || !w->resolved() || (w->numel() > kNumel) != large || x->shape[x->rank - 1] != w->shape[1] || !fusion::Pass::aligned(w)) return nullptr;
+        const uint64_t M = x->numel() / w->shape[1];
+        if (large) return w->dt == RCU_Q8_0H && x->dt == RCU_F16 && rcu_linear_converts_beside(w->dev, M, w->shape[0], w->shape[1]) ? w : nullptr;
+        return rcu_linear_converts(w->dt, x->dt, M, w->shape[0], w->shape[1]) ? w : nullptr;
     }
     rcu_status make(const std::vector<rcu_lazy*>& order, const fusion::Pass& fused) {
         uint64_t total = 0;
@@ -452,6 +454,66 @@ struct Converted {
             }
         }
         return RCU_OK;
+    }
+};
+
+// The large weights that the products of a resolve have converted: each but the first beside the product before its own (rcu_dequantize_beside), into
+// the other of two blocks.  A conversion is a pass over memory and a product bound by the tensor cores; one after the other, as a call
+// by itself has them, the conversions of a Phi-3 prompt of eight layers were 440 us (us a prompt alone / beside, 520 tokens 2323 / 2283, 1000
+// 2989 / 2748, 1250 3618 / 3433, 1500 4003 / 3908: the products' own reads are slower meanwhile).
+struct ConvertedBeside {
+    struct Item { size_t node; const rcu_lazy* w; };
+    rcu_device* dev;
+    std::vector<Item> items;
+    size_t at = 0;                                 // the item whose product comes next
+    bool ready = false;                            // its weights are converted, or on their way
+    void* block[2] = {nullptr, nullptr};
+    rcu_device::NextConversion next;
+    explicit ConvertedBeside(rcu_device* d) : dev(d) {}
+    ~ConvertedBeside() {
+        dev->next_conversion = nullptr;
+        for (void* b : block)
+            if (b) rcu_free(dev, b);               // the pool reuses blocks in stream order
+    }
+    void plan(const std::vector<rcu_lazy*>& order, const fusion::Pass& fused) {
+        uint64_t most = 0;
+        for (size_t i = 0; i < order.size(); ++i) {
+            if (order[i]->resolved() || fused.absorbed(order[i])) continue;
+            const rcu_lazy* w = Converted::weight(order[i], fused.find(order[i]), true);
+            if (!w) continue;
+            items.push_back({i, w});
+            most = std::max(most, w->numel() * 2);
+        }
+        if (items.size() < 2 || rcu_alloc(dev, most, &block[0]) != RCU_OK || rcu_alloc(dev, most, &block[1]) != RCU_OK) items.clear();      // no room: each beside its own
+    }
+    bool has(size_t node) const { return at < items.size() && items[at].node == node; }
+    // The converted weights of the next product; with it the conversion for the one after is launched.
+    rcu_status begin(void** w) {
+        if (!ready) {
+            const rcu_tensor src = items[at].w->desc();
+            rcu_tensor dst = src;
+            dst.dt = RCU_F16;
+            dst.data = block[at & 1];
+            const rcu_status st = rcu_dequantize(dev, &src, &dst);
+            if (st != RCU_OK) return st;
+        }
+        *w = block[at & 1];
+        if (++at < items.size()) {
+            uint64_t off[4];
+            const rcu_lazy* n = items[at].w;
+            rcu_dtype_segments(RCU_Q8_0H, n->numel(), off);
+            next = {n->storage->ptr, (const char*)n->storage->ptr + off[1], block[at & 1], n->numel(), false};
+            dev->next_conversion = &next;
+        }
+        return RCU_OK;
+    }
+    void end() {
+        if (dev->next_conversion) {
+            ready = next.started;
+            dev->next_conversion = nullptr;
+        } else {
+            ready = false;
+        }
     }
 };
 
@@ -576,6 +638,8 @@ rcu_status resolve(rcu_lazy* out) {
     fusion::RopeTables rope_tables(dev);
     Converted converted(dev);
     if (!no_reuse && !profile && (st = converted.make(order, fused)) != RCU_OK) return st;
+    ConvertedBeside beside(dev);
+    if (!no_reuse && !profile) beside.plan(order, fused);
     uint32_t launched = 0, n_inplace = 0;
     const uint64_t launches0 = dev->launches;
     for (size_t i = 0; i < n; ++i) {
@@ -601,7 +665,10 @@ rcu_status resolve(rcu_lazy* out) {
             cudaEventRecord(e0, dev->stream);
         }
         void* cw = converted.of(t, op);
+        const bool large = beside.has(i);
+        if (large && (st = beside.begin(&cw)) != RCU_OK) return st;
         st = op ? fusion::run(dev, t, *op, &rope_tables, cw) : run_node(t, cw);
+        if (large) beside.end();
         if (st != RCU_OK) return st;
         if (profile) {
             cudaEventRecord(e1, dev->stream);

@@ -47,5 +47,10 @@ struct DequantItem {
 };
 constexpr int kDequantItems = 32;       // of one launch
 rcu_status rcu_dequantize_items(rcu_device* dev, int dt, const DequantItem* items, int n);
+// The conversion that dev->next_conversion describes, launched beside the kernel before it, which must be one that triggers its dependents behind
+// its own wait and neither writes these weights nor uses the destination.  RCU_ERR_UNSUPPORTED: nothing was launched.
+rcu_status rcu_dequantize_beside(rcu_device* dev, const rcu_device::NextConversion& c);
 // whether a Linear over M rows of activations converts its weights of this type in a launch of its own
 bool rcu_linear_converts(int w_dt, int act_dt, uint64_t M, uint64_t N, uint64_t K);
+// ... of Q8_0H weights under f16 activations, and the product over them is the pair kernel's
+bool rcu_linear_converts_beside(rcu_device* dev, uint64_t M, uint64_t N, uint64_t K);

@@ -72,6 +72,28 @@ __global__ void __launch_bounds__(256) dequant_q8_items_kernel(const __grid_cons
     }
 }
 
+// A large matrix for the product after the next, beside the product before it: no wait at the start (rcu_dequantize_beside has the conditions).
+// The first block waits at its end instead, so that this kernel, and with it whatever waits for it, ends behind that product.  The product leaves an SM
+// room for one or two blocks, so every thread keeps eight vectors in flight.
+__global__ void __launch_bounds__(256) dequant_q8_beside_kernel(const uint2* __restrict__ q, const __half* __restrict__ d, __half* __restrict__ out, size_t n8) {
+    constexpr int kFly = 8;
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += kFly * stride) {
+        uint2 w[kFly];
+        __half s[kFly];
+#pragma unroll
+        for (int j = 0; j < kFly; ++j)
+            if (i + j * stride < n8) {
+                w[j] = __ldg(q + i + j * stride);
+                s[j] = d[(i + j * stride) >> 2];
+            }
+#pragma unroll
+        for (int j = 0; j < kFly; ++j)
+            if (i + j * stride < n8) *reinterpret_cast<uint4*>(out + (i + j * stride) * 8) = rcu_dequant::dequant8_q8(w[j].x, w[j].y, __half2half2(s[j]));
+    }
+    if (blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 using rcu_dequant::pack_byte;
 
 // Thread = (super-block b, 32-byte chunk c, quarter q of the chunk): one 8-byte load of nibble bytes
@@ -148,6 +170,15 @@ extern "C" rcu_status rcu_dequantize(rcu_device* dev, const rcu_tensor* src, rcu
         if (src->dt == RCU_Q4_KF) rcu_launch(dev, dequant_q4k_kernel<float>, grid, 256, 0, (const uint8_t*)base, (const uint8_t*)base + off[1], (const float*)(base + off[2]), (const float*)(base + off[3]), (float*)dst->data, nsub);
         else rcu_launch(dev, dequant_q4k_kernel<__half>, grid, 256, 0, (const uint8_t*)base, (const uint8_t*)base + off[1], (const __half*)(base + off[2]), (const __half*)(base + off[3]), (__half*)dst->data, nsub);
     }
+    RCU_LAUNCH_CHECK(dev);
+    return RCU_OK;
+}
+
+rcu_status rcu_dequantize_beside(rcu_device* dev, const rcu_device::NextConversion& c) {
+    if (c.numel % 32 || (reinterpret_cast<uintptr_t>(c.codes) & 7) || (reinterpret_cast<uintptr_t>(c.dst) & 15)) return RCU_ERR_UNSUPPORTED;
+    const size_t n8 = c.numel / 8;
+    const int grid = (int)std::min<size_t>((n8 + 2047) / 2048, (size_t)dev->sm_count * 8);
+    RCU_CUDA(dev, rcu_launch(dev, dequant_q8_beside_kernel, grid, 256, 0, (const uint2*)c.codes, (const __half*)c.scales, (__half*)c.dst, n8));
     RCU_LAUNCH_CHECK(dev);
     return RCU_OK;
 }
