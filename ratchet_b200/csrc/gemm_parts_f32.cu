@@ -101,11 +101,19 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t (&p)[3]) {
     p[2] = *reinterpret_cast<const uint32_t*>(&c);
 }
 
+// GROUP: the problems share their activations; the others' weights, biases and outputs
+template <bool GROUP> struct PartsGroup {};
+template <> struct PartsGroup<true> {
+    CUtensorMap w[kGroupLinears - 1];
+    float* out[kGroupLinears - 1];
+    const float* bias[kGroupLinears - 1];
+};
+
 // T: tokens of a tile
-template <int T>
+template <int T, bool GROUP = false>
 __global__ void __launch_bounds__(kThreadsF32, 1)
 gemm_parts_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const float* __restrict__ bias,
-                const float* __restrict__ bias_rows, float* __restrict__ out, float* __restrict__ partial, int M, int N, const Cut cut, int* status) {
+                const float* __restrict__ bias_rows, float* __restrict__ out, float* __restrict__ partial, int M, int N, const Cut cut, int* status, const __grid_constant__ PartsGroup<GROUP> group) {
     constexpr int R = ring_stages(T), STAGE = stage_bytes(T), PLANE = plane_bytes(T);
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
@@ -149,14 +157,20 @@ gemm_parts_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
             int it = 0;
             bool ok = true;
             while (ok && walk.next()) {
-                const int mt = walk.tile % cut.tiles_m, rest = walk.tile / cut.tiles_m, nt = rest % cut.tiles_n, b = rest / cut.tiles_n;
+                const int mt = walk.tile % cut.tiles_m, rest = walk.tile / cut.tiles_m, nt = rest % cut.tiles_n;
+                int b = rest / cut.tiles_n;
+                const CUtensorMap* wm = &wmap;
+                if constexpr (GROUP) {
+                    if (b > 0) wm = &group.w[b - 1];
+                    b = 0;
+                }
                 for (int k = walk.k0; k < walk.k0 + walk.n; ++k, ++it) {
                     const int s = it % R;
                     if (it >= R && !mbar_wait(&raw_empty[s], (it / R - 1) & 1, &abort_flag, status)) { ok = false; break; }
                     unsigned char* st = ring + s * STAGE;
                     mbar_expect_tx(&raw_full[s], STAGE);
                     for (int h = 0; h < 2; ++h) {
-                        tma_load_3d(st + h * kBoxW, &wmap, k * kUnitK + h * 32, nt * kRowsW, b, &raw_full[s]);
+                        tma_load_3d(st + h * kBoxW, wm, k * kUnitK + h * 32, nt * kRowsW, b, &raw_full[s]);
                         tma_load_3d(st + 2 * kBoxW + h * T * 128, &xmap, k * kUnitK + h * 32, mt * T, b, &raw_full[s]);
                     }
                 }
@@ -232,8 +246,14 @@ gemm_parts_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
             const int m0 = mt * T + j0, n = nt * kRowsW + row;
             if (walk.n == cut.nk) {
                 if (n < N) {
-                    const float bn = bias ? bias[n] : 0.f;
-                    float* o = out + b * M * N + (size_t)m0 * N + n;
+                    const float* bs = bias;
+                    float* ys = out + b * M * N;
+                    if constexpr (GROUP) {
+                        bs = b > 0 ? group.bias[b - 1] : bias;
+                        ys = b > 0 ? group.out[b - 1] : out;
+                    }
+                    const float bn = bs ? bs[n] : 0.f;
+                    float* o = ys + (size_t)m0 * N + n;
 #pragma unroll
                     for (int j = 0; j < C; ++j)
                         if (m0 + j < M) o[(size_t)j * N] = acc[j] + (bias_rows ? bias_rows[m0 + j] : bn);
@@ -382,7 +402,7 @@ rcu_status launch_f32(rcu_device* dev, const void* w, const void* x, const void*
     cudaError_t e = cudaFuncSetAttribute(gemm_parts_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(T));
     if (e == cudaSuccess)
         e = rcu_launch(dev, gemm_parts_kernel<T>, grid, kThreadsF32, smem_bytes(T), xmap, wmap, (const float*)bias, (const float*)bias_rows, (float*)y, (float*)partial, (int)M,
-                       (int)N, cut, dev->d_status);
+                       (int)N, cut, dev->d_status, PartsGroup<false>{});
     dev->launches++;
     if (e == cudaSuccess && cut.runs) {
         e = rcu_launch(dev, sum_runs_kernel<T>, dim3((unsigned)tiles, 8), 256, 0, (const float*)partial, (const float*)bias, (const float*)bias_rows, (float*)y, (int)M, (int)N, cut);
@@ -393,6 +413,43 @@ rcu_status launch_f32(rcu_device* dev, const void* w, const void* x, const void*
 }
 
 }  // namespace
+
+// Products over the same rows as tiles of one launch, whole ones: short K (longer ones are cut into runs by themselves) and a product's tiles less than
+// the SMs.  Whisper-tiny's three of 1500 x 384 x 384 take one of them 10 us, the encoder with its four layers 605 us before and 563 with them together.
+bool rcu_gemm_tc_f32_eligible(int lhs_dt, int act_dt, uint64_t M, uint64_t N, uint64_t K, uint64_t batches);
+rcu_status rcu_gemm_parts_f32_group(rcu_device* dev, const LinearGroup& g) {
+    constexpr int T = 64;
+    if (g.n < 2 || g.n > kGroupLinears || g.M <= T || g.K > 8 * kUnitK || g.K < 64 || g.K % 4 || g.N % 4 || g.M > 0x7fffffffull || g.N > 0x7fffffffull || !rcu_gemm_tc_f32_eligible(RCU_F32, RCU_F32, g.M, g.N, g.K, 1))
+        return RCU_ERR_UNSUPPORTED;
+    const uint64_t tiles_m = (g.M + T - 1) / T, tiles_n = (g.N + kRowsW - 1) / kRowsW, tiles = tiles_m * tiles_n;
+    if (tiles > (uint64_t)dev->sm_count) return RCU_ERR_UNSUPPORTED;
+    uintptr_t at = (uintptr_t)g.x;
+    for (int i = 0; i < g.n; ++i) at |= (uintptr_t)g.w[i] | (uintptr_t)g.out[i];
+    if (at & 15) return RCU_ERR_UNSUPPORTED;
+    DevGuard guard(dev->ordinal);
+    CUtensorMap xmap, wmap;
+    PartsGroup<true> group{};
+    bool maps = make_map_f32_sw128(&xmap, g.x, 1, g.M, g.K, T) && make_map_f32_sw128(&wmap, g.w[0], 1, g.N, g.K, kRowsW);
+    for (int i = 1; i < g.n; ++i) {
+        maps = maps && make_map_f32_sw128(&group.w[i - 1], g.w[i], 1, g.N, g.K, kRowsW);
+        group.out[i - 1] = (float*)g.out[i];
+        group.bias[i - 1] = (const float*)g.bias[i];
+    }
+    if (!maps) return rcu_fail(dev, RCU_ERR_CUDA, "gemm_parts: cuTensorMapEncodeTiled failed (group, M=%llu N=%llu K=%llu)", (unsigned long long)g.M, (unsigned long long)g.N, (unsigned long long)g.K);
+    Cut cut;
+    cut.nk = (int)((g.K + kUnitK - 1) / kUnitK);
+    cut.tiles_m = (int)tiles_m;
+    cut.tiles_n = (int)tiles_n;
+    cut.tiles = (int)(tiles * g.n);
+    cut.runs = 0;
+    const unsigned grid = (unsigned)std::min<uint64_t>(cut.tiles, dev->sm_count);
+    auto kern = gemm_parts_kernel<T, true>;
+    RCU_CUDA(dev, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(T)));
+    RCU_CUDA(dev, rcu_launch(dev, kern, grid, kThreadsF32, smem_bytes(T), xmap, wmap, (const float*)g.bias[0], (const float*)nullptr, (float*)g.out[0], (float*)nullptr, (int)g.M, (int)g.N,
+                             cut, dev->d_status, group));
+    RCU_LAUNCH_CHECK(dev);
+    return RCU_OK;
+}
 
 // RCU_ERR_UNSUPPORTED: gemm_tc_f32.cu's kernel is the faster one
 rcu_status rcu_gemm_parts_f32_dispatch(rcu_device* dev, const void* w, const void* x, const void* bias, void* y, uint64_t M, uint64_t N, uint64_t K, uint64_t batches,

@@ -37,6 +37,15 @@ using namespace tc;
 
 namespace {
 
+// GROUP: blockIdx.z is one of several products over the same activations; the others' weights, biases and outputs
+template <bool GROUP> struct TcGroup {};
+template <> struct TcGroup<true> {
+    CUtensorMap w[kGroupLinears - 1];
+    void* out[kGroupLinears - 1];
+    const void* bias[kGroupLinears - 1];
+    const float* bias32[kGroupLinears - 1];
+};
+
 // One CTA computes one 128 x BN output tile.  WK_F16: the weight tile arrives by TMA like the
 // activation tile.  WK_Q8 / WK_Q4K: TMA brings the packed bytes of the tile (BN rows x 64 int8 or
 // BN rows x 32 nibble bytes) into the tail of the stage's weight area; warps 6-9 read them into
@@ -47,10 +56,11 @@ __host__ __device__ constexpr int conv_warps(int bn) { return bn >= 128 ? 8 : 4;
 
 // Two CTAs share an SM (half of its shared memory and at most half of its tensor memory each), so one
 // CTA's pipeline fill and epilogue overlap the other's main loop.
-template <int BN, int WK, int STAGES, class Out, int MODE>
+template <int BN, int WK, int STAGES, class Out, int MODE, bool GROUP = false>
 __global__ void __launch_bounds__(WK == WK_F16 ? kThreadsTc : kThreadsTc + conv_warps(BN) * 32, 2)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const QuantArgs qa,
-               const GemmEpilogue<Out, MODE> epi, Out* out, int M, int N, int K, int* status, int splits, float* __restrict__ partial, uint32_t idesc) {
+               GemmEpilogue<Out, MODE> epi, Out* out, int M, int N, int K, int* status, int splits, float* __restrict__ partial, uint32_t idesc,
+               const __grid_constant__ TcGroup<GROUP> group) {
     rcu_kernel_entry_wait_only();
     constexpr int A_BYTES = TM * TK * 2;          // 16 KiB
     constexpr int B_BYTES = BN * TK * 2;
@@ -76,8 +86,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
     const int sp = splits > 1 ? (int)blockIdx.z : 0;
     const int it_base = sp * nk_per;
     const int nk = max(0, min(nk_all - it_base, nk_per));
-    const int bz = splits > 1 ? 0 : (int)blockIdx.z;
+    const int bz = splits > 1 || GROUP ? 0 : (int)blockIdx.z;
     out += (size_t)bz * M * N;
+    const CUtensorMap* wm = &wmap;
+    if constexpr (GROUP) {
+        const int z = (int)blockIdx.z - 1;
+        if (z >= 0) {
+            wm = &group.w[z];
+            out = (Out*)group.out[z];
+            epi.bias = (const Out*)group.bias[z];
+            epi.bias32 = group.bias32[z];
+        }
+    }
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -108,7 +128,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
                 if (WK == WK_F16) {
                     mbar_expect_tx(&full[s], STAGE);
                     tma_load_3d(st, &xmap, (it_base + it) * TK, m0, bz, &full[s]);             // activations: rows m0.., k it*64..
-                    tma_load_3d(st + A_BYTES, &wmap, (it_base + it) * TK, n0, bz, &full[s]);   // weights: rows n0..
+                    tma_load_3d(st + A_BYTES, wm, (it_base + it) * TK, n0, bz, &full[s]);   // weights: rows n0..
                 } else {
                     mbar_expect_tx(&raw_full[s], A_BYTES + RAW_BYTES);
                     tma_load_3d(st, &xmap, (it_base + it) * TK, m0, 0, &raw_full[s]);
@@ -352,7 +372,7 @@ rcu_status launch_tc(rcu_device* dev, const CUtensorMap& xmap, const CUtensorMap
         if (splits > 1 && rcu_alloc(dev, (uint64_t)splits * M * N * 4, &partial) == RCU_OK) {       // no room for the slices' sums: one slice
             grid.z = splits;
             rcu_launch(dev, kern, grid, threads, smem, xmap, wmap, qa, GemmEpilogue<Out, MODE>{nullptr, nullptr, 1.f, 0}, (Out*)out, M, N, K, dev->d_status, splits,
-                       (float*)partial, idesc);
+                       (float*)partial, idesc, TcGroup<false>{});
             dev->launches++;
             const size_t MN = (size_t)M * N;
             rcu_launch(dev, sum_k_slices_kernel<Out, MODE>, (unsigned)((MN / 8 + 255) / 256), 256, 0, (const float*)partial, epi, (Out*)out, MN, N, splits);
@@ -361,7 +381,7 @@ rcu_status launch_tc(rcu_device* dev, const CUtensorMap& xmap, const CUtensorMap
             return RCU_OK;
         }
     }
-    rcu_launch(dev, kern, grid, threads, smem, xmap, wmap, qa, epi, (Out*)out, M, N, K, dev->d_status, 1, nullptr, idesc);
+    rcu_launch(dev, kern, grid, threads, smem, xmap, wmap, qa, epi, (Out*)out, M, N, K, dev->d_status, 1, nullptr, idesc, TcGroup<false>{});
     RCU_LAUNCH_CHECK(dev);
     return RCU_OK;
 }
@@ -574,6 +594,38 @@ rcu_status rcu_gemm_tc_chain(rcu_device* dev, int w_dt, const void* w, const voi
         return t.x_pitch % 8 ? RCU_ERR_UNSUPPORTED : rcu_gemm_tc2_launch(dev, w, x, nullptr, y, M, N, K, t);
     }
     return rcu_gemm_tc_dispatch(dev, w_dt, w, RCU_F16, x, c.bias, y, M, N, K, t);
+}
+
+// Three products of 501 x 384 x 384, 24 tiles each: 7.7 us and a launch of the host's 4 us apiece (Whisper-tiny's encoder of 1001 frames, Q8_0H:
+// 292 us apart, 244 with its four layers' q, k and v together).  Sizes whose tiles fill the device, or that
+// take other kernels or slices of K alone, stay apart.
+rcu_status rcu_gemm_tc_group(rcu_device* dev, const LinearGroup& g) {
+    constexpr int BN = 64, STAGES = (100 * 1024) / (TM * TK * 2 + BN * TK * 2);
+    if (g.n < 2 || g.n > kGroupLinears || g.M <= 32 || g.N % 8 != 0 || g.K >= 16 * TK || !rcu_gemm_tc_eligible(RCU_F16, RCU_F16, g.M, g.N, g.K)) return RCU_ERR_UNSUPPORTED;
+    const uint64_t tiles = ((g.M + TM - 1) / TM) * ((g.N + BN - 1) / BN);
+    if (tiles * (g.n - 1) > (uint64_t)dev->sm_count || rcu_gemm_tc2_eligible(dev, g.M, g.N, g.K)) return RCU_ERR_UNSUPPORTED;
+    uintptr_t at = (uintptr_t)g.x;
+    for (int i = 0; i < g.n; ++i) at |= (uintptr_t)g.w[i] | (uintptr_t)g.out[i];
+    if (at & 15) return RCU_ERR_UNSUPPORTED;
+    DevGuard guard(dev->ordinal);
+    CUtensorMap xmap, wmap;
+    TcGroup<true> group{};
+    bool maps = make_map_f16_sw128(&xmap, g.x, g.M, g.K, TM) && make_map_f16_sw128(&wmap, g.w[0], g.N, g.K, BN);
+    for (int i = 1; i < g.n; ++i) {
+        maps = maps && make_map_f16_sw128(&group.w[i - 1], g.w[i], g.N, g.K, BN);
+        group.out[i - 1] = g.out[i];
+        group.bias[i - 1] = g.bias[i];
+        group.bias32[i - 1] = g.bias32[i];
+    }
+    if (!maps) return rcu_fail(dev, RCU_ERR_CUDA, "gemm_tc: cuTensorMapEncodeTiled failed (group, M=%llu N=%llu K=%llu)", (unsigned long long)g.M, (unsigned long long)g.N, (unsigned long long)g.K);
+    constexpr size_t smem = (size_t)STAGES * (TM * TK * 2 + BN * TK * 2) + 1024 + 512;
+    auto kern = gemm_tc_kernel<BN, WK_F16, STAGES, __half, EPI_RESID, true>;
+    RCU_CUDA(dev, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    RCU_CUDA(dev, rcu_launch(dev, kern, dim3((g.N + BN - 1) / BN, (g.M + TM - 1) / TM, g.n), kThreadsTc, smem, xmap, wmap, QuantArgs{nullptr, nullptr, nullptr},
+                             GemmEpilogue<__half, EPI_RESID>{(const __half*)g.bias[0], nullptr, 1.f, {}, g.bias32[0], nullptr, -1}, (__half*)g.out[0], (int)g.M, (int)g.N, (int)g.K,
+                             dev->d_status, 1, nullptr, umma_idesc_f16(TM, BN), group));
+    RCU_LAUNCH_CHECK(dev);
+    return RCU_OK;
 }
 
 bool rcu_linear_converts_beside(rcu_device* dev, uint64_t M, uint64_t N, uint64_t K) {

@@ -457,6 +457,67 @@ struct Converted {
     }
 };
 
+// Linears next to one another in the order, over the same tensor and of the same sizes, as one launch
+struct Grouped {
+    LinearGroup g;
+    bool half = false;
+    std::vector<size_t> nodes;
+    std::vector<std::pair<const char*, const char*>> reads, writes;
+
+    static std::pair<const char*, const char*> range(const void* p, uint64_t bytes) { return {(const char*)p, (const char*)p + bytes}; }
+    static bool apart(const std::pair<const char*, const char*>& a, const std::pair<const char*, const char*>& b) { return a.second <= b.first || b.second <= a.first; }
+
+    // Node `t` as a further member (its storage is not set yet); false: it does not fit
+    bool add(size_t i, const rcu_lazy* t, const fusion::Op* op, void* converted) {
+        if ((int)nodes.size() == kGroupLinears) return false;
+        const rcu_lazy *w, *x, *bias = nullptr, *bias32 = nullptr;
+        if (op) {
+            if (op->kind != fusion::LINEAR || op->act >= 0 || op->glu >= 0 || op->resid || op->x_col || t->dt != RCU_F16) return false;
+            w = op->w; x = op->x; bias = op->bias; bias32 = op->bias32;
+        } else {
+            if (t->kind != K_MATMUL || t->flags[0] || !t->flags[1] || !t->flags[2]) return false;
+            w = t->srcs[0]; x = t->srcs[1];
+            if (t->srcs.size() > 2) bias = t->srcs[2];
+        }
+        const int32_t dt = x->dt;
+        if ((dt != RCU_F16 && dt != RCU_F32) || t->dt != dt || w->rank != 2 || x->rank < 2 || !x->storage || !w->storage || (converted ? rcu_activation_dtype(w->dt) : w->dt) != dt) return false;
+        const uint64_t N = w->shape[0], K = w->shape[1], M = x->numel() / x->shape[x->rank - 1];
+        if (x->shape[x->rank - 1] != K || t->numel() != M * N) return false;
+        if (bias && (bias->dt != dt || bias->numel() != N || !bias->storage)) return false;
+        if (bias32 && (bias32->dt != RCU_F32 || bias32->numel() != N || !bias32->storage)) return false;
+        if (nodes.empty()) {
+            g.M = M; g.N = N; g.K = K;
+            g.x = x->storage->ptr;
+            half = dt == RCU_F16;
+            reads.push_back(range(g.x, M * K * dt_esize(dt)));
+        } else if (g.x != x->storage->ptr || half != (dt == RCU_F16) || g.M != M || g.N != N || g.K != K) {
+            return false;
+        }
+        const int n = g.n;
+        g.w[n] = converted ? converted : w->storage->ptr;
+        g.bias[n] = bias ? bias->storage->ptr : nullptr;
+        g.bias32[n] = bias32 ? (const float*)bias32->storage->ptr : nullptr;
+        reads.push_back(range(g.w[n], N * K * dt_esize(dt)));
+        if (bias || bias32) reads.push_back(range(bias ? g.bias[n] : g.bias32[n], N * dt_esize(bias ? dt : (int32_t)RCU_F32)));
+        nodes.push_back(i);
+        ++g.n;
+        return true;
+    }
+    // The members' outputs are in place: whether none lies in what another member reads or writes (a buffer that is free once the first member has
+    // run may be the second's)
+    bool disjoint() {
+        for (int i = 0; i < g.n; ++i) {
+            const auto w = range(g.out[i], g.M * g.N * (half ? 2 : 4));
+            for (const auto& r : reads)
+                if (!apart(w, r)) return false;
+            for (const auto& r : writes)
+                if (!apart(w, r)) return false;
+            writes.push_back(w);
+        }
+        return true;
+    }
+};
+
 // The large weights that the products of a resolve have converted: each but the first beside the product before its own (rcu_dequantize_beside), into
 // the other of two blocks.  A conversion is a pass over memory and a product bound by the tensor cores; one after the other, as a call
 // by itself has them, the conversions of a Phi-3 prompt of eight layers were 440 us (us a prompt alone / beside, 520 tokens 2323 / 2283, 1000
@@ -642,14 +703,15 @@ rcu_status resolve(rcu_lazy* out) {
     if (!no_reuse && !profile) beside.plan(order, fused);
     uint32_t launched = 0, n_inplace = 0;
     const uint64_t launches0 = dev->launches;
+    auto place = [&](size_t i) {
+        const size_t o = owner[i];
+        order[i]->storage = o == i ? objects[plans[plan_of[o]].object].storage : order[o]->storage;
+    };
     for (size_t i = 0; i < n; ++i) {
         rcu_lazy* t = order[i];
         if (t->resolved() || fused.absorbed(t)) continue;
         const fusion::Op* op = fused.find(t);
-        const size_t o = owner[i];
-        if (bufferless(t)) {
-        } else if (o == i) t->storage = objects[plans[plan_of[o]].object].storage;
-        else t->storage = order[o]->storage;
+        if (!bufferless(t)) place(i);
         if (!t->storage && !bufferless(t)) return rcu_fail(dev, RCU_ERR_INVALID_ARG, "resolve: tensor %llu has no storage", (unsigned long long)t->id);   // TensorError::NoStorage
         if (t->kind == K_VIEW || t->kind == K_CONST) continue;
         if (inplace[i]) ++n_inplace;
@@ -666,6 +728,27 @@ rcu_status resolve(rcu_lazy* out) {
         }
         void* cw = converted.of(t, op);
         const bool large = beside.has(i);
+        if (!no_reuse && !profile && !large && (t->kind == K_MATMUL || (op && op->kind == fusion::LINEAR))) {
+            Grouped group;
+            if (group.add(i, t, op, cw)) {
+                for (size_t j = i + 1; j < n; ++j) {
+                    rcu_lazy* u = order[j];
+                    if (u->resolved() || fused.absorbed(u) || u->kind == K_CONST) continue;
+                    const fusion::Op* uop = fused.find(u);
+                    if (u->kind == K_VIEW || bufferless(u) || owner[j] != j || beside.has(j) || !group.add(j, u, uop, converted.of(u, uop))) break;
+                }
+                for (int k = 0; k < group.g.n && group.g.n > 1; ++k) group.g.out[k] = objects[plans[plan_of[group.nodes[k]]].object].storage->ptr;
+                if (group.g.n > 1 && group.disjoint()) {
+                    st = group.half ? rcu_gemm_tc_group(dev, group.g) : rcu_gemm_parts_f32_group(dev, group.g);
+                    if (st == RCU_OK) {
+                        for (size_t k : group.nodes) place(k);
+                        launched += (uint32_t)group.nodes.size();
+                        continue;
+                    }
+                    if (st != RCU_ERR_UNSUPPORTED) return st;
+                }
+            }
+        }
         if (large && (st = beside.begin(&cw)) != RCU_OK) return st;
         st = op ? fusion::run(dev, t, *op, &rope_tables, cw) : run_node(t, cw);
         if (large) beside.end();

@@ -39,6 +39,21 @@ struct LinearChain {
 bool rcu_gemm_tc_chain_takes(rcu_device* dev, int w_dt, uint64_t M, uint64_t N, uint64_t K, bool glu, bool act);
 rcu_status rcu_gemm_tc_chain(rcu_device* dev, int w_dt, const void* w, const void* x, void* y, uint64_t M, uint64_t N, uint64_t K, const LinearChain& c);
 
+// Linears of the same sizes over the same rows, in one launch: the projections of an attention, each too small to fill the device.
+constexpr int kGroupLinears = 3;
+struct LinearGroup {
+    int n = 0;
+    uint64_t M = 0, N = 0, K = 0;
+    const void* x = nullptr;
+    const void* w[kGroupLinears] = {};          // in the activations' type
+    const void* bias[kGroupLinears] = {};       // likewise, nullable
+    const float* bias32[kGroupLinears] = {};    // f16 activations: in f32, to be rounded first, nullable
+    void* out[kGroupLinears] = {};
+};
+// RCU_ERR_UNSUPPORTED: nothing was launched; sizes or alignments that the kernel does not take, or products that fill the device one by one
+rcu_status rcu_gemm_tc_group(rcu_device* dev, const LinearGroup& g);            // f16
+rcu_status rcu_gemm_parts_f32_group(rcu_device* dev, const LinearGroup& g);     // f32
+
 // The Linears of a resolve whose weights are converted once per product (gemm_tc.cu, matmul.cu), converted together: small matrices, in one launch
 struct DequantItem {
     const void* src;                    // Q8_0 segments
