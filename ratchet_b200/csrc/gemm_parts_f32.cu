@@ -109,11 +109,11 @@ template <> struct PartsGroup<true> {
     const float* bias[kGroupLinears - 1];
 };
 
-// T: tokens of a tile
-template <int T, bool GROUP = false>
+// T: tokens of a tile.  RESID: a residual is added behind the bias (a form of its own: 64 x 2560 x 10240 without one stays as it is)
+template <int T, bool GROUP = false, bool RESID = false>
 __global__ void __launch_bounds__(kThreadsF32, 1)
 gemm_parts_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const float* __restrict__ bias,
-                const float* __restrict__ bias_rows, float* __restrict__ out, float* __restrict__ partial, int M, int N, const Cut cut, int* status, const __grid_constant__ PartsGroup<GROUP> group) {
+                const float* __restrict__ bias_rows, const float* __restrict__ resid, float* __restrict__ out, float* __restrict__ partial, int M, int N, const Cut cut, int* status, const __grid_constant__ PartsGroup<GROUP> group) {
     constexpr int R = ring_stages(T), STAGE = stage_bytes(T), PLANE = plane_bytes(T);
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
@@ -254,9 +254,19 @@ gemm_parts_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
                     }
                     const float bn = bs ? bs[n] : 0.f;
                     float* o = ys + (size_t)m0 * N + n;
+                    if constexpr (RESID) {           // all of a thread's are requested before the first is added
+                        const float* rs = resid + (size_t)m0 * N + n;
+                        float r[C];
 #pragma unroll
-                    for (int j = 0; j < C; ++j)
-                        if (m0 + j < M) o[(size_t)j * N] = acc[j] + (bias_rows ? bias_rows[m0 + j] : bn);
+                        for (int j = 0; j < C; ++j) r[j] = m0 + j < M ? rs[(size_t)j * N] : 0.f;
+#pragma unroll
+                        for (int j = 0; j < C; ++j)
+                            if (m0 + j < M) o[(size_t)j * N] = (acc[j] + bn) + r[j];
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < C; ++j)
+                            if (m0 + j < M) o[(size_t)j * N] = acc[j] + (bias_rows ? bias_rows[m0 + j] : bn);
+                    }
                 }
             } else {
                 float* o = partial + (size_t)(blockIdx.x + walk.tile) * (T * kRowsW) + j0 * kRowsW + row;      // every segment has a place of its own
@@ -330,9 +340,9 @@ gemm_parts_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
 }
 
 // a tile that was cut: its runs' sums in order + bias per column / per row.  CTA = (tile, eighth of its tokens); thread = feature and token parity
-template <int T>
+template <int T, bool RESID>
 __global__ void __launch_bounds__(256)
-sum_runs_kernel(const float* __restrict__ partial, const float* __restrict__ bias, const float* __restrict__ bias_rows, float* __restrict__ out, int M, int N, const Cut cut) {
+sum_runs_kernel(const float* __restrict__ partial, const float* __restrict__ bias, const float* __restrict__ bias_rows, const float* __restrict__ resid, float* __restrict__ out, int M, int N, const Cut cut) {
     rcu_kernel_entry();
     const int tile = blockIdx.x, first = cut.run_of((long long)tile * cut.nk), last = cut.run_of((long long)(tile + 1) * cut.nk - 1);
     if (first == last) return;
@@ -343,7 +353,12 @@ sum_runs_kernel(const float* __restrict__ partial, const float* __restrict__ bia
     const float bn = bias ? bias[n] : 0.f;
     constexpr int J = T / 16;
     const int j0 = blockIdx.y * (T / 8) + (threadIdx.x >> 7);
-    float v[J] = {};
+    float v[J] = {}, r[J] = {};
+    if constexpr (RESID) {
+#pragma unroll
+        for (int i = 0; i < J; ++i)
+            if (mt * T + j0 + 2 * i < M) r[i] = resid[(size_t)(mt * T + j0 + 2 * i) * N + n];
+    }
     for (int c = first; c <= last; c += 4) {             // four runs requested before the first is added
         float p[4][J];
 #pragma unroll
@@ -358,7 +373,9 @@ sum_runs_kernel(const float* __restrict__ partial, const float* __restrict__ bia
 #pragma unroll
     for (int i = 0; i < J; ++i) {
         const int m = mt * T + j0 + 2 * i;
-        if (m < M) out[b * M * N + (size_t)m * N + n] = v[i] + (bias_rows ? bias_rows[m] : bn);
+        if (m >= M) continue;
+        const float y = v[i] + (bias_rows ? bias_rows[m] : bn);
+        out[b * M * N + (size_t)m * N + n] = RESID ? y + r[i] : y;
     }
 }
 
@@ -374,8 +391,8 @@ bool make_map_f32_sw128(CUtensorMap* map, const void* base, uint64_t batches, ui
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int T>
-rcu_status launch_f32(rcu_device* dev, const void* w, const void* x, const void* bias, const void* bias_rows, void* y, uint64_t M, uint64_t N, uint64_t K, uint64_t batches) {
+template <int T, bool RESID>
+rcu_status launch_f32(rcu_device* dev, const void* w, const void* x, const void* bias, const void* bias_rows, void* y, uint64_t M, uint64_t N, uint64_t K, uint64_t batches, const void* resid = nullptr) {
     CUtensorMap xmap, wmap;
     if (!make_map_f32_sw128(&xmap, x, batches, M, K, T) || !make_map_f32_sw128(&wmap, w, batches, N, K, kRowsW))
         return rcu_fail(dev, RCU_ERR_CUDA, "gemm_parts: cuTensorMapEncodeTiled failed (M=%llu N=%llu K=%llu x%llu)", (unsigned long long)M,
@@ -399,13 +416,14 @@ rcu_status launch_f32(rcu_device* dev, const void* w, const void* x, const void*
         if (rcu_alloc(dev, (runs + tiles) * (uint64_t)(T * kRowsW) * 4, &partial) != RCU_OK) cut.runs = 0;      // no room: whole tiles need none
     }
     const unsigned grid = cut.runs ? (unsigned)cut.runs : (unsigned)std::min(tiles, sms);
-    cudaError_t e = cudaFuncSetAttribute(gemm_parts_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(T));
+    auto kern = gemm_parts_kernel<T, false, RESID>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(T));
     if (e == cudaSuccess)
-        e = rcu_launch(dev, gemm_parts_kernel<T>, grid, kThreadsF32, smem_bytes(T), xmap, wmap, (const float*)bias, (const float*)bias_rows, (float*)y, (float*)partial, (int)M,
+        e = rcu_launch(dev, kern, grid, kThreadsF32, smem_bytes(T), xmap, wmap, (const float*)bias, (const float*)bias_rows, (const float*)resid, (float*)y, (float*)partial, (int)M,
                        (int)N, cut, dev->d_status, PartsGroup<false>{});
     dev->launches++;
     if (e == cudaSuccess && cut.runs) {
-        e = rcu_launch(dev, sum_runs_kernel<T>, dim3((unsigned)tiles, 8), 256, 0, (const float*)partial, (const float*)bias, (const float*)bias_rows, (float*)y, (int)M, (int)N, cut);
+        e = rcu_launch(dev, sum_runs_kernel<T, RESID>, dim3((unsigned)tiles, 8), 256, 0, (const float*)partial, (const float*)bias, (const float*)bias_rows, (const float*)resid, (float*)y, (int)M, (int)N, cut);
         dev->launches++;
     }
     if (partial) rcu_free(dev, partial);          // the pool reuses blocks in stream order
@@ -445,25 +463,44 @@ rcu_status rcu_gemm_parts_f32_group(rcu_device* dev, const LinearGroup& g) {
     const unsigned grid = (unsigned)std::min<uint64_t>(cut.tiles, dev->sm_count);
     auto kern = gemm_parts_kernel<T, true>;
     RCU_CUDA(dev, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(T)));
-    RCU_CUDA(dev, rcu_launch(dev, kern, grid, kThreadsF32, smem_bytes(T), xmap, wmap, (const float*)g.bias[0], (const float*)nullptr, (float*)g.out[0], (float*)nullptr, (int)g.M, (int)g.N,
+    RCU_CUDA(dev, rcu_launch(dev, kern, grid, kThreadsF32, smem_bytes(T), xmap, wmap, (const float*)g.bias[0], (const float*)nullptr, (const float*)nullptr, (float*)g.out[0], (float*)nullptr, (int)g.M, (int)g.N,
                              cut, dev->d_status, group));
     RCU_LAUNCH_CHECK(dev);
     return RCU_OK;
 }
 
-// RCU_ERR_UNSUPPORTED: gemm_tc_f32.cu's kernel is the faster one
-rcu_status rcu_gemm_parts_f32_dispatch(rcu_device* dev, const void* w, const void* x, const void* bias, void* y, uint64_t M, uint64_t N, uint64_t K, uint64_t batches,
-                                       const void* bias_rows) {
-    // Up to 64 tokens, and wherever the tiles leave room on the SMs.  With more tiles than that the 128 x 128 tiles of the split-TF32 kernel
-    // need fewer bytes of shared memory per product (us here / there: 1500 x 1536 x 384, 288 tiles, 20.2 / 16.3; 512 x 3072 x 3072, 192, 74 / 66;
-    // 1500 x 384 x 1536, 72, 21.3 / 23.3; 128 x 3072 x 3072, 48, 25.1 / 26.2; 64 x 10240 x 2560 33 / 49).  Rows that do not start on four columns
-    // come here at any size: the FMA pipe, which they would go to otherwise, is as exact as this and the split-TF32 kernel is not.
+namespace {
+// Up to 64 tokens, and wherever the tiles leave room on the SMs.  With more tiles than that the 128 x 128 tiles of the split-TF32 kernel
+// need fewer bytes of shared memory per product (us here / there: 1500 x 1536 x 384, 288 tiles, 20.2 / 16.3; 512 x 3072 x 3072, 192, 74 / 66;
+// 1500 x 384 x 1536, 72, 21.3 / 23.3; 128 x 3072 x 3072, 48, 25.1 / 26.2; 64 x 10240 x 2560 33 / 49).  Rows that do not start on four columns
+// come here at any size: the FMA pipe, which they would go to otherwise, is as exact as this and the split-TF32 kernel is not.
+bool takes(rcu_device* dev, uint64_t M, uint64_t N, uint64_t batches) {
     const uint64_t tiles = batches * ((M + 63) / 64) * ((N + kRowsW - 1) / kRowsW);
-    if (M > 64 && N % 4 == 0 && tiles > (uint64_t)dev->sm_count) return RCU_ERR_UNSUPPORTED;
+    return M <= 64 || N % 4 != 0 || tiles <= (uint64_t)dev->sm_count;
+}
+rcu_status dispatch(rcu_device* dev, const void* w, const void* x, const void* bias, void* y, uint64_t M, uint64_t N, uint64_t K, uint64_t batches, const void* bias_rows,
+                    const void* resid) {
+#define RCU_PARTS(T_) (resid ? launch_f32<T_, true>(dev, w, x, bias, bias_rows, y, M, N, K, batches, resid) : launch_f32<T_, false>(dev, w, x, bias, bias_rows, y, M, N, K, batches))
     // Tiles of 32 tokens where they leave room on the SMs too and K is short: a CTA's chain of units is what counts then, and theirs are shorter
     // (33 x 64 x 256: 9.8 us with tiles of 64)
     const bool narrow = K <= 8 * kUnitK && batches * ((M + 31) / 32) * ((N + kRowsW - 1) / kRowsW) <= (uint64_t)dev->sm_count;
-    if (M <= 16) return launch_f32<16>(dev, w, x, bias, bias_rows, y, M, N, K, batches);
-    if (M <= 32 || narrow) return launch_f32<32>(dev, w, x, bias, bias_rows, y, M, N, K, batches);
-    return launch_f32<64>(dev, w, x, bias, bias_rows, y, M, N, K, batches);
+    if (M <= 16) return RCU_PARTS(16);
+    if (M <= 32 || narrow) return RCU_PARTS(32);
+    return RCU_PARTS(64);
+#undef RCU_PARTS
+}
+}  // namespace
+
+// RCU_ERR_UNSUPPORTED: gemm_tc_f32.cu's kernel is the faster one
+rcu_status rcu_gemm_parts_f32_dispatch(rcu_device* dev, const void* w, const void* x, const void* bias, void* y, uint64_t M, uint64_t N, uint64_t K, uint64_t batches,
+                                       const void* bias_rows) {
+    return takes(dev, M, N, batches) ? dispatch(dev, w, x, bias, y, M, N, K, batches, bias_rows, nullptr) : RCU_ERR_UNSUPPORTED;
+}
+
+bool rcu_gemm_parts_f32_takes(rcu_device* dev, uint64_t M, uint64_t N, uint64_t K) { return rcu_gemm_tc_f32_eligible(RCU_F32, RCU_F32, M, N, K, 1) && takes(dev, M, N, 1); }
+rcu_status rcu_gemm_parts_f32_resid(rcu_device* dev, const void* w, const void* x, const void* bias, const void* resid, void* y, uint64_t M, uint64_t N, uint64_t K) {
+    if (!rcu_gemm_parts_f32_takes(dev, M, N, K)) return RCU_ERR_UNSUPPORTED;
+    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(bias)) & 15) return RCU_ERR_UNSUPPORTED;
+    DevGuard g(dev->ordinal);
+    return dispatch(dev, w, x, bias, y, M, N, K, 1, nullptr, resid);
 }

@@ -8,7 +8,7 @@
 //   attention32  permute(softmax((dk q)(dk k)^T) v) in f32 (the same with f32 activations, whose casts are no nodes)
 //   heads        cast(rope(cast(permute(view(slice))))), and permute(view(slice)) in front of a cache: straight into the cache's rows
 //   linear       a product with its bias's cast, gelu or silu between casts or the addition to the residual behind it; the product of a glu
-//                (bf16's too)
+//                (bf16's too); the addition to the residual behind an f32 product as well
 //   norm         cast(norm(cast x));   act: cast(gelu or silu(cast x));   glu: up * cast(silu(cast gate)) of the halves of one tensor
 // A subgraph whose sizes or alignment a kernel does not take stays as it is.
 #pragma once
@@ -34,6 +34,7 @@ struct Op {
     uint32_t H = 0, T = 0, L = 0, D = 0, E = 0;
     rcu_lazy *w = nullptr, *x = nullptr, *bias = nullptr, *bias32 = nullptr, *resid = nullptr;      // LINEAR
     int act = -1, glu = -1;
+    bool full = false;                  // f32 (with a residual)
     uint32_t x_col = 0;
     uint64_t M = 0, N = 0, K = 0;
 };
@@ -413,6 +414,36 @@ struct Pass {
         return give(root, std::move(op), seen);
     }
 
+    // an f32 product in front of an addition.  Prompts only: up to 64 tokens a product's time is its weights', and the launches of such a block stay one per
+    // op and sum, as its callers count them.
+    bool linear32(rcu_lazy* root) {
+        if (root->op != RCU_ADD || root->dt != RCU_F32) return false;
+        for (int i = 0; i < 2; ++i) {
+            rcu_lazy *g = root->srcs[i], *r = root->srcs[1 - i];
+            if (!inner(g, K_MATMUL, RCU_F32) || g == r || r->dt != RCU_F32 || r->rank != g->rank || root->rank != g->rank || !std::equal(g->shape, g->shape + g->rank, r->shape)) continue;
+            if (g->flags[0] || !g->flags[1] || !g->flags[2]) continue;
+            Op op;
+            op.kind = LINEAR;
+            op.full = true;
+            op.w = g->srcs[0];
+            op.x = g->srcs[1];
+            op.resid = r;
+            if (op.w->rank != 2 || (op.w->dt != RCU_F32 && op.w->dt != RCU_Q8_0F) || op.x->dt != RCU_F32 || op.x->rank < 2) continue;
+            op.N = op.w->shape[0];
+            op.K = op.w->shape[1];
+            op.M = op.x->numel() / op.x->shape[op.x->rank - 1];
+            if (op.x->shape[op.x->rank - 1] != op.K || g->numel() != op.M * op.N || !aligned(op.w) || !aligned(op.x) || op.M <= 64 || !rcu_gemm_parts_f32_takes(dev, op.M, op.N, op.K)) continue;
+            op.srcs = {op.w, op.x, r};
+            if (g->srcs.size() > 2) {
+                op.bias = g->srcs[2];
+                if (op.bias->dt != RCU_F32 || op.bias->numel() != op.N || !aligned(op.bias)) continue;      // rcu_matmul has the say
+                op.srcs.push_back(op.bias);
+            }
+            return give(root, std::move(op), {g});
+        }
+        return false;
+    }
+
     // glu of a bf16 product that nothing else reads
     bool glu_rows(rcu_lazy* root) {
         rcu_lazy* l = root->srcs[0];
@@ -506,7 +537,7 @@ struct Pass {
             if (t->resolved() || absorbed(t) || find(t)) continue;
             if (t->kind == K_PERMUTE) attention(t) || attention32(t);
             else if (t->kind == K_CAST) heads(t) || norm(t) || linear(t) || act(t);
-            else if (t->kind == K_BINARY) glu(t) || linear(t);
+            else if (t->kind == K_BINARY) glu(t) || linear(t) || linear32(t);
             else if (t->kind == K_MATMUL) linear(t);
             else if (t->kind == K_GLU) glu_rows(t);
         }
@@ -599,6 +630,19 @@ rcu_status run(rcu_device* dev, rcu_lazy* t, const Op& op, RopeTables* tables, v
             return rcu_glu_half(dev, t->srcs[1]->srcs[0]->op, data(op.srcs[0]), t->storage->ptr, t->numel() / F, F);
         }
         case LINEAR: {
+            if (op.full) {
+                const void* w = converted ? converted : op.w->dt == RCU_F32 ? op.w->storage->ptr : nullptr;
+                rcu_status st = w ? rcu_gemm_parts_f32_resid(dev, w, op.x->storage->ptr, data(op.bias), op.resid->storage->ptr, t->storage->ptr, op.M, op.N, op.K) : RCU_ERR_UNSUPPORTED;
+                if (st != RCU_ERR_UNSUPPORTED) return st;
+                rcu_tensor l = op.w->desc(), x = op.x->desc(), y = t->desc(), r = op.resid->desc(), b;
+                if (converted) {
+                    l.dt = RCU_F32;
+                    l.data = converted;
+                }
+                if (op.bias) b = op.bias->desc();
+                st = rcu_matmul(dev, &l, &x, op.bias ? &b : nullptr, false, true, true, &y);
+                return st == RCU_OK ? rcu_binary(dev, RCU_ADD, &y, &r, &y) : st;
+            }
             LinearChain c;
             c.bias = data(op.bias);
             c.bias32 = (const float*)data(op.bias32);

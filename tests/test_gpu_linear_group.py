@@ -61,3 +61,22 @@ def test_an_output_that_takes_over_a_members_input_stays_apart(dev):
     want = resolved_apart(ws, [b[0].add(b[1]).resolve(), None, None], x)
     y = nn.Linear(ws[0], b[0].add(b[1])).schedule(x).mul(nn.Linear(ws[1]).schedule(x).mul(nn.Linear(ws[2]).schedule(x)))
     assert np.array_equal(y.resolve().to_numpy(), want[0] * (want[1] * want[2]))
+
+
+# an f32 product and the addition behind it: whole tiles of 32 and of 64 tokens, tiles that are cut into runs, one row too few or many; a product that
+# another kernel runs (apart)
+@pytest.mark.parametrize("M,N,K", [(16, 136, 256), (33, 128, 512), (64, 2560, 2048), (65, 260, 96), (1500, 384, 384), (1501, 384, 1536), (70, 61, 128), (1500, 1536, 384), (2, 64, 64)])
+@pytest.mark.parametrize("left", [False, True])
+@pytest.mark.parametrize("quantised", [False, True])
+def test_the_addition_behind_an_f32_product(dev, M, N, K, left, quantised):
+    from oracle import oracle as orc
+    g = np.random.Generator(np.random.PCG64(M + N + K))
+    w, x, r = (g.standard_normal((N, K)) * 0.05).astype(np.float32), g.standard_normal((1, M, K)).astype(np.float32), g.standard_normal((1, M, N)).astype(np.float32)
+    x[0, 0, 0], r[0, M - 1, N - 1] = np.inf, np.nan
+    w = Tensor.from_quantized(orc.quantize_q8(w), capi.Q8_0F, (N, K), dev) if quantised else Tensor.from_data(w, device=dev)
+    x, r = Tensor.from_data(x, device=dev), Tensor.from_data(r, device=dev)
+    b = None if left else Tensor.from_data(g.standard_normal(N).astype(np.float32), device=dev)
+    lin = nn.Linear(w, b)
+    want = lin.schedule(x).resolve().to_numpy() + r.to_numpy()
+    got = r.add(lin.schedule(x)) if left else lin.schedule(x).add(r)
+    assert np.array_equal(got.resolve().to_numpy(), want, equal_nan=True)
