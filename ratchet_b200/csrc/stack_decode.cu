@@ -809,8 +809,10 @@ __global__ void __launch_bounds__(kThreads) latent_step_kernel(const float* __re
 // [heads, features] . [features, positions], the features split over the warps and summed in shared memory; online softmax, a
 // thread per (head, position); the weighted latents as [heads, positions] . [positions, features], each warp owning a run
 // of features.  Queries and weights enter as bf16 value plus remainder.
-constexpr int kMmaHeads = 16;
-template <int PC>
+// CL: eight runs are one cluster, which adds its results up through distributed shared memory and leaves one; the kernel that
+// merges the partial results read 64 of them (132 KB) in each of its 128 CTAs, 7 us at a window of 1024.
+constexpr int kMmaHeads = 16, kLatentCluster = 8;
+template <int PC, bool CL>
 __global__ void __launch_bounds__(kThreads) latent_step_mma_kernel(const float* __restrict__ qa, const lm::bf16* __restrict__ ring, int ring_rows, int window,
                                                                    const uint32_t* d_pos, float* __restrict__ partial, int H, int C, int R, bool ahead) {
     using lm::bf16;
@@ -952,6 +954,61 @@ __global__ void __launch_bounds__(kThreads) latent_step_mma_kernel(const float* 
         }
     }
     const int pitch = partial_pitch(C);
+    if constexpr (CL) {
+        namespace cg = cooperative_groups;
+        cg::cluster_group cluster = cg::this_cluster();
+        __shared__ float m_s[kMmaHeads], l_s[kMmaHeads];
+        float* sums = reinterpret_cast<float*>(tiles);      // [kMmaHeads][quads * 4], over queries and rows that every warp is done with
+        const int quads = (C + 3) / 4, ld_s = quads * 4;
+        __syncthreads();
+#pragma unroll
+        for (int c = 0; c < PC; ++c)
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int e = 0; e < 4; e += 2) {
+                    const int col = (warp + c * kWarps) * 16 + 8 * x + 2 * t, r = g + (e >> 1) * 8;
+                    if (col < ld_s) *reinterpret_cast<float2*>(sums + r * ld_s + col) = make_float2(o[c][x][e], o[c][x][e + 1]);
+                }
+        if (sp == 0) {
+            m_s[sh] = m;
+            l_s[sh] = l;
+        }
+        cluster.sync();
+        for (int i = (int)cluster.block_rank() * kThreads + threadIdx.x; i < kMmaHeads * quads; i += kLatentCluster * kThreads) {
+            const int r = i / quads, col = (i - r * quads) * 4;
+            if (h0 + r >= H) break;
+            float ms[kLatentCluster], ls[kLatentCluster], M = -INFINITY;
+            float4 v[kLatentCluster];
+#pragma unroll
+            for (int j = 0; j < kLatentCluster; ++j) {
+                ms[j] = *cluster.map_shared_rank(m_s + r, j);
+                ls[j] = *cluster.map_shared_rank(l_s + r, j);
+                v[j] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(sums + r * ld_s + col, j));
+            }
+#pragma unroll
+            for (int j = 0; j < kLatentCluster; ++j) M = fmaxf(M, ms[j]);
+            float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
+            float total = 0.f;
+#pragma unroll
+            for (int j = 0; j < kLatentCluster; ++j) {
+                const float f = ms[j] == -INFINITY ? 0.f : expf(ms[j] - M);      // a run without a position
+                total = fmaf(f, ls[j], total);
+                w.x = fmaf(f, v[j].x, w.x);
+                w.y = fmaf(f, v[j].y, w.y);
+                w.z = fmaf(f, v[j].z, w.z);
+                w.w = fmaf(f, v[j].w, w.w);
+            }
+            float* dst = partial + ((size_t)(blockIdx.x / kLatentCluster) * H + h0 + r) * pitch;
+            *reinterpret_cast<float4*>(dst + col) = w;       // columns beyond C: of the padded pitch, zero
+            if (col == 0) {
+                dst[pitch - 2] = M;
+                dst[pitch - 1] = total;
+            }
+        }
+        cluster.sync();                       // no CTA leaves while its shared memory is being read
+        return;
+    }
     float* dst = partial + ((size_t)blockIdx.x * H + h0) * pitch;
 #pragma unroll
     for (int c = 0; c < PC; ++c)
@@ -1135,6 +1192,13 @@ namespace {
 
 int latent_splits(const rcu_stack_run& r) { return (int)std::min<uint32_t>(kMaxSplits, std::max<uint32_t>(1, (std::min(r.window, r.ring_rows) + kSub - 1) / kSub)); }
 
+// Partial results of a run's attention: its splits, or the clusters that they form where what the merging kernel would read of a head is long enough to
+// pay for a cluster's two barriers (us per token, splits x rank 32 x 256: 178.7 without / 188.2 with; 64 x 512: 332.6 / 322.6 and 385.8 / 379.8)
+bool latent_clusters(const rcu_stack_run& r, int dt) {
+    return dt == RCU_BF16 && latent_splits(r) >= kLatentCluster && (uint64_t)latent_splits(r) * r.kv_rank >= 16384;
+}
+int latent_partials(const rcu_stack_run& r, int dt) { return latent_clusters(r, dt) ? (latent_splits(r) + kLatentCluster - 1) / kLatentCluster : latent_splits(r); }
+
 uint64_t grouped_seen(const rcu_stack_run& r) {      // rows a token can see at most
     const uint64_t most = r.chunk ? r.chunk : r.window ? r.window : r.ring_rows;
     return std::min<uint64_t>(most, r.ring_rows);
@@ -1198,28 +1262,35 @@ template <class T> rcu_status launch_rows(rcu_device* dev, RowsArgs a) {
 
 rcu_status launch_latent_step(rcu_device* dev, const rcu_stack* s, const rcu_stack_run& r, int dt) {
     const int H = (int)r.heads, C = (int)r.kv_rank, R = (int)r.rot_dim, splits = latent_splits(r);
-#define RCU_LS(KERN_, GRID_, T_, ...)                                                                                                                 \
+#define RCU_LS(KERN_, GRID_, T_, CLUSTER_, ...)                                                                                                                 \
     do {                                                                                                                                         \
         RCU_CUDA(dev, cudaFuncSetAttribute(KERN_, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(smem, (size_t)(48 * 1024))));       \
-        RCU_CUDA(dev, rcu_launch(dev, KERN_, GRID_, kThreads, smem, s->qa, (const T_*)r.state, (int)r.ring_rows, (int)r.window, s->d_pos, s->partial, H, C, R, ##__VA_ARGS__)); \
+        RCU_CUDA(dev, rcu_launch_cluster(dev, KERN_, GRID_, kThreads, smem, CLUSTER_, s->qa, (const T_*)r.state, (int)r.ring_rows, (int)r.window, s->d_pos, s->partial, H, C, R, ##__VA_ARGS__)); \
     } while (0)
     if (dt == RCU_BF16) {
         const int wp = (C + R + 15) & ~15;
         const size_t smem = (size_t)(2 * kMmaHeads + kSub) * (wp + 8) * sizeof(lm::bf16);
-        const dim3 grid(splits, (H + kMmaHeads - 1) / kMmaHeads);
-        if (wp <= 256) RCU_LS(latent_step_mma_kernel<2>, grid, lm::bf16, s->ahead);
-        else if (wp <= 640) RCU_LS(latent_step_mma_kernel<5>, grid, lm::bf16, s->ahead);
-        else RCU_LS(latent_step_mma_kernel<10>, grid, lm::bf16, s->ahead);
+        const bool cl = latent_clusters(r, dt);
+        const dim3 grid(cl ? latent_partials(r, dt) * kLatentCluster : splits, (H + kMmaHeads - 1) / kMmaHeads);
+#define RCU_LS_C(PC_)                                                                                                       \
+    do {                                                                                                                    \
+        if (cl) RCU_LS((latent_step_mma_kernel<PC_, true>), grid, lm::bf16, kLatentCluster, s->ahead);                      \
+        else RCU_LS((latent_step_mma_kernel<PC_, false>), grid, lm::bf16, 0, s->ahead);                                     \
+    } while (0)
+        if (wp <= 256) RCU_LS_C(2);
+        else if (wp <= 640) RCU_LS_C(5);
+        else RCU_LS_C(10);
+#undef RCU_LS_C
     } else {
         const int WP = (C + R + 7) & ~7;
         const size_t smem = (size_t)kHeads * WP * 4 + (size_t)kSub * WP * sizeof(float);
         const dim3 grid(splits, (H + kHeads - 1) / kHeads);
         switch ((WP + 255) / 256) {
-            case 1: RCU_LS((latent_step_kernel<float, 1>), grid, float); break;
-            case 2: RCU_LS((latent_step_kernel<float, 2>), grid, float); break;
-            case 3: RCU_LS((latent_step_kernel<float, 3>), grid, float); break;
-            case 4: RCU_LS((latent_step_kernel<float, 4>), grid, float); break;
-            default: RCU_LS((latent_step_kernel<float, 5>), grid, float); break;
+            case 1: RCU_LS((latent_step_kernel<float, 1>), grid, float, 0); break;
+            case 2: RCU_LS((latent_step_kernel<float, 2>), grid, float, 0); break;
+            case 3: RCU_LS((latent_step_kernel<float, 3>), grid, float, 0); break;
+            case 4: RCU_LS((latent_step_kernel<float, 4>), grid, float, 0); break;
+            default: RCU_LS((latent_step_kernel<float, 5>), grid, float, 0); break;
         }
     }
 #undef RCU_LS
@@ -1320,7 +1391,7 @@ template <class T> rcu_status run_step(rcu_stack* s, const int32_t* token, float
             RCU_LAUNCH_CHECK(dev);
             STACK_TRY(launch_latent_step(dev, s, r, c.weight_dt));
             const int per = 2 * kWarps, quads = (C + 3) / 4, groups = std::max(1, kThreads / quads);
-            RCU_CUDA(dev, rcu_launch(dev, latent_values_kernel<T>, dim3(H, (E + per - 1) / per), kThreads, (size_t)groups * quads * 16, s->partial, latent_splits(r),
+            RCU_CUDA(dev, rcu_launch(dev, latent_values_kernel<T>, dim3(H, (E + per - 1) / per), kThreads, (size_t)groups * quads * 16, s->partial, latent_partials(r, c.weight_dt),
                                      (const T*)r.ukv + (size_t)H * D * C, s->y, H, C, E, per));
             RCU_LAUNCH_CHECK(dev);
             out.pro = PRO_CONCAT; out.x = s->y;

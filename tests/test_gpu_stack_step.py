@@ -1,5 +1,5 @@
 """The fused decode step where the staging of a product's inputs changes its form: vectors that do not start on sixteen bytes, second inputs
-of more than one batch of loads, and the token's latent written beside the query expansion."""
+of more than one batch of loads, the token's latent written beside the query expansion, and latent attention merged in clusters."""
 import numpy as np
 import pytest
 
@@ -15,6 +15,9 @@ MODELS = {
     # a gate that starts at 2 * 63 + 64 floats: rows of whole blocks behind unaligned vectors
     "unaligned": B.config(128, 64, [B.lightning(1, 63, 64, (0.9,), ff=192), B.latent(2, 30, 6, 32, 64, 64, 5, 0.2, ff=64)]),
     # 8256 = 8192 + 64 activations of a feed-forward: one more than a batch takes
+    # runs of positions in clusters of eight: 17 splits (the last cluster's others without a position), ranks that are no multiple of 16, a window of which
+    # only the first runs have positions
+    "clusters": B.config(64, 64, [B.latent(3, 16, 8, 16, 64, 1000, 272, 0.2, scaling=B.YARN), B.latent(17, 8, 4, 8, 64, 512, 1024, 0.25, scaling=B.YARN)]),
     "long": B.config(64, 64, [B.lightning(2, 32, 32, (0.8, 0.99), ff=8256), B.latent(4, 16, 8, 16, 128, 192, 21, 0.25, scaling=B.YARN, ff=8192)]),
 }
 
@@ -25,7 +28,7 @@ def test_tokens_agree_with_the_restatement(name, tmp_path):
     from ratchet_b200.models import load_model
     cfg = MODELS[name]
     W = B.weights(cfg, seed=5)
-    tokens = np.random.Generator(np.random.PCG64(3)).integers(0, cfg["vocab"], 40).tolist()
+    tokens = np.random.Generator(np.random.PCG64(3)).integers(0, cfg["vocab"], 300 if name == "clusters" else 40).tolist()
     want = dz.forward(cfg, W, tokens)
     dev = Device(0)
     try:
