@@ -9,13 +9,14 @@
 //   heads        cast(rope(cast(permute(view(slice))))), and permute(view(slice)) in front of a cache: straight into the cache's rows
 //   linear       a product with its bias's cast, gelu or silu between casts or the addition to the residual behind it; the product of a glu
 //                (bf16's too); the addition to the residual behind an f32 product as well
+//   rows         [cast](permute(gelu or silu(x)) + positions) in f32, a convolution's [1, C, T] on its way to rows of tokens (whisper/encoder.rs:108-122)
 //   norm         cast(norm(cast x));   act: cast(gelu or silu(cast x));   glu: up * cast(silu(cast gate)) of the halves of one tensor
 // A subgraph whose sizes or alignment a kernel does not take stays as it is.
 #pragma once
 
 namespace fusion {
 
-enum Kind { NONE = 0, ATTENTION, ATTENTION32, HEADS, APPEND, NORM, ACT, GLU, LINEAR };
+enum Kind { NONE = 0, ATTENTION, ATTENTION32, HEADS, APPEND, NORM, ACT, GLU, LINEAR, ROWS };
 
 // element (position t, head h, feature d) of a [1, heads, T, D] operand at base[offset + h * head + t * row + d]
 struct Heads {
@@ -490,6 +491,35 @@ struct Pass {
         return give(root, std::move(op), seen);
     }
 
+    bool rows(rcu_lazy* root) {
+        std::vector<rcu_lazy*> seen;
+        rcu_lazy* sum = root;
+        if (root->kind == K_CAST) {
+            sum = root->srcs[0];
+            if (root->dt != RCU_F16 || !inner(sum, K_BINARY, RCU_F32)) return false;
+            seen.push_back(sum);
+        }
+        if (sum->kind != K_BINARY || sum->dt != RCU_F32 || sum->op != RCU_ADD || sum->rank != 3) return false;
+        for (int i = 0; i < 2; ++i) {
+            rcu_lazy *p = sum->srcs[i], *e = sum->srcs[1 - i];
+            if (!inner(p, K_PERMUTE, RCU_F32) || p->rank != 3 || p->u[0] != 0 || p->u[1] != 2 || p->u[2] != 1 || p->shape[0] != 1 || p == e) continue;
+            rcu_lazy* a = p->srcs[0];
+            const uint64_t T = p->shape[1], C = p->shape[2];
+            if (!inner(a, K_UNARY, RCU_F32) || (a->op != RCU_GELU && a->op != RCU_SILU) || T < 2 || T > 0x7fffffffull || (C + 31) / 32 > 65535) continue;
+            if (e->dt != RCU_F32 || e->rank < 2 || e->numel() != T * C || e->shape[e->rank - 1] != C || e->shape[e->rank - 2] != T || sum->numel() != T * C) continue;
+            Op op;
+            op.kind = ROWS;
+            op.act = a->op;
+            op.full = root->dt == RCU_F32;
+            op.M = T;
+            op.N = C;
+            op.srcs = {a->srcs[0], e};
+            seen.insert(seen.end(), {p, a});
+            return give(root, std::move(op), seen);
+        }
+        return false;
+    }
+
     // up * cast(silu(cast gate)), gate and up the halves of one tensor's last dimension
     bool glu(rcu_lazy* root) {
         if (root->kind != K_BINARY || root->op != RCU_MUL || root->dt != RCU_F16) return false;
@@ -536,8 +566,8 @@ struct Pass {
             rcu_lazy* t = o.nodes[i];
             if (t->resolved() || absorbed(t) || find(t)) continue;
             if (t->kind == K_PERMUTE) attention(t) || attention32(t);
-            else if (t->kind == K_CAST) heads(t) || norm(t) || linear(t) || act(t);
-            else if (t->kind == K_BINARY) glu(t) || linear(t) || linear32(t);
+            else if (t->kind == K_CAST) heads(t) || norm(t) || linear(t) || act(t) || rows(t);
+            else if (t->kind == K_BINARY) glu(t) || linear(t) || linear32(t) || rows(t);
             else if (t->kind == K_MATMUL) linear(t);
             else if (t->kind == K_GLU) glu_rows(t);
         }
@@ -545,7 +575,7 @@ struct Pass {
 };
 
 inline const char* name_of(Kind k) {
-    static const char* names[] = {"", "attention", "attention", "heads", "cache", "norm chain", "act chain", "glu chain", "linear chain"};
+    static const char* names[] = {"", "attention", "attention", "heads", "cache", "norm chain", "act chain", "glu chain", "linear chain", "rows chain"};
     return names[k];
 }
 
@@ -629,6 +659,7 @@ rcu_status run(rcu_device* dev, rcu_lazy* t, const Op& op, RopeTables* tables, v
             const uint64_t F = t->shape[t->rank - 1];
             return rcu_glu_half(dev, t->srcs[1]->srcs[0]->op, data(op.srcs[0]), t->storage->ptr, t->numel() / F, F);
         }
+        case ROWS: return rcu_act_rows(dev, op.act, (const float*)data(op.srcs[0]), (const float*)data(op.srcs[1]), t->storage->ptr, !op.full, op.M, op.N);
         case LINEAR: {
             if (op.full) {
                 const void* w = converted ? converted : op.w->dt == RCU_F32 ? op.w->storage->ptr : nullptr;

@@ -14,6 +14,9 @@ __device__ __forceinline__ float chain_act(int act, float x) {
 rcu_status rcu_norm_half(rcu_device* dev, int kind, const void* x, const void* scale, const void* bias, float eps, void* out, uint64_t rows, uint64_t N);
 // out = f16(act(f32(x)))
 rcu_status rcu_act_half(rcu_device* dev, int act, const void* x, void* out, uint64_t n);
+// out[t, c] = act(x[c, t]) + add[t, c], x [C, T] and add [T, C] f32, out f32 or (half) rounded to f16: what a convolution's output goes through on its way to
+// rows of tokens
+rcu_status rcu_act_rows(rcu_device* dev, int act, const float* x, const float* add, void* out, bool half, uint64_t T, uint64_t C);
 // out = up * f16(act(f32(gate))) of rows that hold gate, then up
 rcu_status rcu_glu_half(rcu_device* dev, int act, const void* x, void* out, uint64_t rows, uint64_t F);
 // Heads out of rows: out[h, t, :] = src[t, h, :], rotated as rcu_rope does between casts to f32 and back (rope_dim 0: as they are)

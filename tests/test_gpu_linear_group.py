@@ -80,3 +80,31 @@ def test_the_addition_behind_an_f32_product(dev, M, N, K, left, quantised):
     want = lin.schedule(x).resolve().to_numpy() + r.to_numpy()
     got = r.add(lin.schedule(x)) if left else lin.schedule(x).add(r)
     assert np.array_equal(got.resolve().to_numpy(), want, equal_nan=True)
+
+
+# an activation, a permute, positions and a cast in one kernel, against the ops by themselves (each result held): pieces of 32 in both directions, ragged
+@pytest.mark.parametrize("T,C", [(501, 384), (32, 64), (33, 31), (2, 1), (100, 97)])
+@pytest.mark.parametrize("act", ["gelu", "silu"])
+@pytest.mark.parametrize("half", [False, True])
+@pytest.mark.parametrize("left", [False, True])
+def test_a_convolutions_output_to_rows(dev, T, C, act, half, left):
+    g = np.random.Generator(np.random.PCG64(T + C))
+    x = Tensor.from_data((g.standard_normal((1, C, T)) * 2).astype(np.float32), device=dev)
+    e = Tensor.from_data(g.standard_normal((1, T, C) if left else (T, C)).astype(np.float32), device=dev)
+
+    def schedule(keep):
+        a = getattr(x, act)()
+        p = a.permute([0, 2, 1])
+        s = e.add(p) if left else p.add(e)
+        keep.extend([a, p, s])
+        return s.cast(capi.F16) if half else s
+
+    held = []
+    want = schedule(held).resolve().to_numpy()
+    launches = dev.launches
+    handles = []
+    out = schedule(handles)
+    handles.clear()                              # nothing holds the ops between
+    got = out.resolve().to_numpy()
+    assert dev.launches - launches == 1
+    assert got.dtype == (np.float16 if half else np.float32) and np.array_equal(got, want)
