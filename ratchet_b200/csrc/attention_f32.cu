@@ -84,7 +84,6 @@ struct Args {
 template <bool CARE>
 __global__ void __launch_bounds__(kThreadsA, 1)
 attention_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, const Args a) {
-    rcu_kernel_entry_wait_only();
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* qs = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);      // [tile][part]
     unsigned char* ks = qs + 6 * kBlockQ;               // [stage][part]
@@ -121,6 +120,7 @@ attention_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    rcu_kernel_entry_wait_only();        // nothing before this touches global memory
     // per query tile 256 columns: S of the leading parts 64, S of the small products 64 (the weights' parts, 32 columns each, take their
     // place), O of the leading parts 64, O of the small products 64
     const uint32_t tmem = tmem_slot;

@@ -45,7 +45,6 @@ template <int NB, int EB, bool MASK>
 __global__ void __launch_bounds__(kThreadsA, 1)
 attention_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
                  const __grid_constant__ CUtensorMap mmap, const Args a) {
-    rcu_kernel_entry_wait_only();
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* qs = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
     unsigned char* ks = qs + 2 * NB * kBlockQ;
@@ -87,6 +86,7 @@ attention_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    rcu_kernel_entry_wait_only();        // nothing before this touches global memory
     const uint32_t tmem = tmem_slot;       // per query tile 256 columns: two buffers of 64 (S, then P), 128 for O
 
     if (warp == 0) {

@@ -61,7 +61,6 @@ __global__ void __launch_bounds__(WK == WK_F16 ? kThreadsTc : kThreadsTc + conv_
 gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const QuantArgs qa,
                GemmEpilogue<Out, MODE> epi, Out* out, int M, int N, int K, int* status, int splits, float* __restrict__ partial, uint32_t idesc,
                const __grid_constant__ TcGroup<GROUP> group) {
-    rcu_kernel_entry_wait_only();
     constexpr int A_BYTES = TM * TK * 2;          // 16 KiB
     constexpr int B_BYTES = BN * TK * 2;
     constexpr int STAGE = A_BYTES + B_BYTES;
@@ -117,6 +116,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    rcu_kernel_entry_wait_only();        // nothing before this touches global memory
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {

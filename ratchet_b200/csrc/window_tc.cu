@@ -56,7 +56,6 @@ template <int NB>
 __global__ void __launch_bounds__(kThreadsW, 1)
 window_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap qrmap, const __grid_constant__ CUtensorMap kmap,
                  const __grid_constant__ CUtensorMap krmap, const __grid_constant__ CUtensorMap vmap, const TcArgs a) {
-    rcu_kernel_entry_wait_only();
     extern __shared__ unsigned char smem_dyn[];
     constexpr int nb = NB;
     const int nd = (a.D + 63) / 64, eb = (a.E + 63) / 64;      // 64-column blocks
@@ -100,6 +99,7 @@ window_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    rcu_kernel_entry_wait_only();        // nothing before this touches global memory
     const uint32_t tmem = tmem_slot;
 
     if (warp == 0) {
