@@ -38,3 +38,24 @@ def test_tokens_agree_with_the_restatement(name, tmp_path):
     finally:
         dev.close()
     assert np.sqrt(((got - want) ** 2).mean(-1) / (want ** 2).mean()).max() < LIMIT
+
+
+def test_runs_that_share_a_state(tmp_path):
+    """Two layers over one state: the second's step must see what the first's has written (states are otherwise read ahead of the kernel before)."""
+    from ratchet_b200 import Device
+    from ratchet_b200.models import load_model
+    cfg = B.config(64, 64, [B.lightning(2, 32, 32, (0.8, 0.99), ff=64), B.lightning(2, 32, 32, (0.8, 0.99), ff=64)])
+    W = B.weights(cfg, seed=6)
+    dev = Device(0)
+    try:
+        m = load_model(B.write_model(str(tmp_path / "shared"), cfg, W), dev, "bfloat16")
+        tokens = [5, 9, 60, 2, 33, 7, 7, 1]
+        got = []
+        for step in (lambda st, t: m.prefill([t], st, [0]), lambda st, t: m.decode(st, t)[0].to_numpy()):      # op by op, and the fused step
+            st = m.new_state(len(tokens))
+            st.runs[1] = st.runs[0]
+            got.append(np.concatenate([step(st, t) for t in tokens]))
+    finally:
+        dev.close()
+    assert np.sqrt(((got[1] - got[0]) ** 2).mean(-1) / (got[0] ** 2).mean()).max() < LIMIT
+    assert np.sqrt(((got[0][1:] - got[0][:-1]) ** 2).mean()) > LIMIT
