@@ -59,3 +59,22 @@ def test_runs_that_share_a_state(tmp_path):
         dev.close()
     assert np.sqrt(((got[1] - got[0]) ** 2).mean(-1) / (got[0] ** 2).mean()).max() < LIMIT
     assert np.sqrt(((got[0][1:] - got[0][:-1]) ** 2).mean()) > LIMIT
+
+
+@pytest.mark.parametrize("vocab", [3, 4097, 33000])
+def test_the_picked_token_is_the_first_maximum(tmp_path, vocab):
+    """Vocabularies of less and more than a round of the cluster's threads; equal logits: the lowest id."""
+    from ratchet_b200 import Device
+    from ratchet_b200.models import load_model
+    cfg = B.config(64, vocab, [B.lightning(2, 32, 32, (0.8, 0.99), ff=64)])
+    W = B.weights(cfg, seed=vocab)
+    W["head"][vocab // 2:] = W["head"][:vocab - vocab // 2]              # every logit of the first half comes again
+    dev = Device(0)
+    try:
+        m = load_model(B.write_model(str(tmp_path / "v"), cfg, W), dev, "bfloat16")
+        st = m.new_state(8)
+        for t in (0, 1, 2, 1):
+            logits, picked = m.decode(st, t)
+            assert int(picked.to_numpy()[0]) == int(np.argmax(logits.to_numpy().reshape(-1)))
+    finally:
+        dev.close()
