@@ -428,8 +428,8 @@ static bool converts_once(uint64_t M) {
 }
 
 // Whether the pair kernel converts the tiles itself (gemm_tc2.cu; K of whole groups of 256).  A conversion costs 8.4 ns (Q8_0H; Q4_KH 7) for each
-// 256 weight rows and 64 of K; in the kernel every round of tiles takes some 0.16 us (0.17) longer per 64 of K, the codes passing through
-// shared memory.  us converted / in the kernel, Q8_0H 9216 x 3072: 300 rows 35.8 / 30.5, 512 36.6 / 31.0, 768 (a second round) 51.0 / 53.3, 1000 56.3 /
+// 256 weight rows and 64 of K; in the kernel every round of tiles takes some 0.16 us (0.17) longer per 64 of K, the hand-overs of the
+// converting warps.  us converted / in the kernel, Q8_0H 9216 x 3072: 300 rows 35.8 / 30.5, 512 36.6 / 31.0, 768 (a second round) 51.0 / 53.3, 1000 56.3 /
 // 57.8, 2048 96.4 / 120.1; 16384 x 3072: 512 74.1 / 63.3, 1000 104.7 / 119.9; 5120 x 8192: 512 66.8 / 63.7; 3072 x 8192: 1000 57.1 / 63.2; Q4_KH
 // 9216 x 3072: 300 36.5 / 31.1; 16384 x 3072: 512 69.4 / 60.6; 5120 x 8192: 512 65.9 / 68.8; 32064 x 3072: 300 126.7 / 111.9.
 static bool pair_converts(rcu_device* dev, int dt, uint64_t M, uint64_t N, uint64_t K) {

@@ -25,8 +25,9 @@
 //   warp 19            the scales: plain loads, sixteen bytes a row for four steps (requested by the converting warps themselves, codes and
 //                      scales took 2000 cycles a step: 1500 sectors in flight per SM).
 // The converting warps arrive in CTA scope: the tensor cores read behind a proxy fence; arriving in cluster scope waited 0.65 us a step for L2.
-// 512 x 8192 x 3072 Q4_KH: 38.2 us with the conversion beside it -> 33.3; 512 x 9216 x 3072 Q8_0H: 36.6 -> 31.0 (pair_converts in gemm_tc.cu has more).
-// What bounds it: shared memory, 72 (Q4_K) to 80 KB a step at 128 bytes a cycle, and the chain of hand-overs above.
+// 512 x 8192 x 3072 Q4_KH: 38.2 us with the conversion in front of it -> 33.3; 512 x 9216 x 3072 Q8_0H: 36.6 -> 31.0 (pair_converts in gemm_tc.cu has more).
+// What bounds it: the chain of hand-overs - a step takes some 1000 cycles with the tensor pipe 42 to 45 % busy, issue slots 34 % - and with Q8_0 the codes' and the
+// converted tile's way through shared memory as well (51 % of its wavefronts are the converting warps').
 //
 // The kernel is persistent: a pair walks over tiles pair, pair + n_pairs, ...; the accumulator is
 // double-buffered (2 x 256 of the 512 tensor-memory columns), so the epilogue of tile i overlaps the
