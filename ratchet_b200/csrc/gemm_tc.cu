@@ -417,8 +417,8 @@ bool rcu_gemm_tc2_eligible(rcu_device* dev, uint64_t M, uint64_t N, uint64_t K);
 rcu_status rcu_gemm_tc2_launch(rcu_device* dev, const void* w, const void* x, const void* bias, void* y, uint64_t M, uint64_t N, uint64_t K,
                                const TcLinear& t);
 
-// Quantised weights.  The one-CTA kernel converts a weight tile once per 128-row token tile, i.e. M/128 times over the whole problem.  Beyond
-// kFusedMaxM token rows the pair kernel converts its tiles itself where that pays (pair_converts); otherwise the matrix is converted once into pooled
+// Quantised weights.  The one-CTA kernel converts a weight tile once per 128-row token tile, i.e. M/128 times over the whole problem.  Where it
+// pays the pair kernel converts its tiles itself (pair_converts); beyond kFusedMaxM token rows otherwise the matrix is converted once into pooled
 // f16 scratch (which stays in L2) for the f16 kernels (M = 512, N = 8192, K = 3072, Q4_K: 34 us against 46 us in the one-CTA kernel).
 // RCU_GEMM_FUSED=0/1 forces the conversion or the one-CTA kernel.
 constexpr uint64_t kFusedMaxM = 256;
@@ -433,9 +433,16 @@ static bool converts_once(uint64_t M) {
 // 57.8, 2048 96.4 / 120.1; 16384 x 3072: 512 74.1 / 63.3, 1000 104.7 / 119.9; 5120 x 8192: 512 66.8 / 63.7; 3072 x 8192: 1000 57.1 / 63.2; Q4_KH
 // 9216 x 3072: 300 36.5 / 31.1; 16384 x 3072: 512 69.4 / 60.6; 5120 x 8192: 512 65.9 / 68.8; 32064 x 3072: 300 126.7 / 111.9.
 static bool pair_converts(rcu_device* dev, int dt, uint64_t M, uint64_t N, uint64_t K) {
-    if (K % 256 != 0 || !rcu_gemm_tc2_eligible(dev, M, N, K)) return false;
+    if (K % 256 != 0 || !rcu_gemm_tc2_eligible(dev, std::max<uint64_t>(M, 1 << 20), N, K)) return false;
     const uint64_t tiles_n = (N + 255) / 256, pairs = dev->sm_count / 2, rounds = ((M + 255) / 256 * tiles_n + pairs - 1) / pairs;
-    return tiles_n > (dt == RCU_Q8_0H ? 19 : 24) * rounds;
+    if (M > kFusedMaxM) return rcu_gemm_tc2_eligible(dev, M, N, K) && tiles_n > (dt == RCU_Q8_0H ? 19 : 24) * rounds;
+    // One row of tiles, against the one-CTA kernel, which converts too: as long as its 128 x 64 tiles do not outnumber the SMs it cuts K and is the
+    // faster one (M = 160, 3072 x 3072: 16 us / 29 here), beyond that its two CTAs an SM share the converting warps' issue slots (us there / here, Q8_0H;
+    // Q4_KH is alike: 160 x 5120 x 3072 31.6 / 29.1, 256 x 9216 x 3072 33.4 / 29.8, 256 x 16384 x 3072 50.2 / 31.4, 160 x 32064 x 3072 99.8 / 55.0, 160 x 8192 x
+    // 1024 15.1 / 15.6, 160 x 16384 x 1024 21.3 / 16.6).  Up to 128 rows that is so in one round of tiles only (128 x 9728 x 3072 32.4 / 29.7, 96 x 10240 x 8192
+    // 78.0 / 63.6, 128 x 9216 x 3072 20.6 / 29.6, 128 x 20480 x 3072 50.0 / 52.4, 96 x 16384 x 1024 15.8 / 16.9).
+    if (M <= 32 || (M + TM - 1) / TM * ((N + 63) / 64) <= (uint64_t)dev->sm_count) return false;
+    return M > TM ? K >= 2048 || N >= 16384 : rounds == 1 && K >= 2048;
 }
 
 // The Linear of an f16 graph with what follows it (TcLinear: chained, or glu): whether the tensor-core kernels take it.  A gate and its up
@@ -446,7 +453,9 @@ bool rcu_gemm_tc_chain_takes(rcu_device* dev, int w_dt, uint64_t M, uint64_t N, 
     if (w_dt == RCU_BF16) return glu && N % 16 == 0 && rcu_gemm_tc2_eligible(dev, M, N, K) && M <= 0x7fffffffull && N <= 0x7fffffffull && K <= 0x7fffffffull;
     if (!rcu_gemm_tc_eligible(w_dt, RCU_F16, M, N, K) || N % 8 != 0) return false;
     if (!glu && !act) return M > 32;               // fewer rows: gemm_rows.cu
-    return N % 16 == 0 && (w_dt == RCU_F16 || converts_once(M)) && rcu_gemm_tc2_eligible(dev, M, N, K);
+    if (N % 16 != 0) return false;
+    if (w_dt != RCU_F16 && !getenv("RCU_GEMM_FUSED") && pair_converts(dev, w_dt, M, N, K)) return true;
+    return (w_dt == RCU_F16 || converts_once(M)) && rcu_gemm_tc2_eligible(dev, M, N, K);
 }
 
 rcu_status rcu_gemm_tc_dispatch(rcu_device* dev, int lhs_dt, const void* w, int act_dt, const void* x, const void* bias, void* y,
@@ -455,7 +464,7 @@ rcu_status rcu_gemm_tc_dispatch(rcu_device* dev, int lhs_dt, const void* w, int 
     if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(w)) & 15) return RCU_ERR_UNSUPPORTED;
     DevGuard g(dev->ordinal);
     if (lhs_dt == RCU_F16 && rcu_gemm_tc2_eligible(dev, M, N, K)) return rcu_gemm_tc2_launch(dev, w, x, bias, y, M, N, K, t);
-    if (lhs_dt != RCU_F16 && converts_once(M) && !getenv("RCU_GEMM_FUSED") && pair_converts(dev, lhs_dt, M, N, K)) {
+    if (lhs_dt != RCU_F16 && !getenv("RCU_GEMM_FUSED") && pair_converts(dev, lhs_dt, M, N, K)) {
         size_t at[4];
         rcu_dtype_segments(lhs_dt, N * K, at);
         TcLinear q = t;

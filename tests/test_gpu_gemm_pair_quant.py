@@ -52,7 +52,27 @@ def test_equals_the_product_over_the_converted_matrix(dev, monkeypatch, kind, M,
     assert np.isfinite(want).all() and np.array_equal(got.view(np.uint16), want.view(np.uint16))
 
 
-@pytest.mark.parametrize("kind,M,F,K", [("q8_0h", 500, 2608, 512), ("q4_kh", 470, 4912, 768)])
+# one row of tiles: the first and last rows of a CTA of the pair, none in the second; against the one-CTA kernel that converts, which does not cut K at
+# these sizes either (the last two are on the other side of the rule) but for 18944 columns: 148 tiles of 128, two slices of K.  There f32 sums of K products
+# come in another order (2^-24 each, random signs), and an output may round to f16's neighbour.
+@pytest.mark.parametrize("kind", ["q8_0h", "q4_kh"])
+@pytest.mark.parametrize("M,N,K", [(129, 5120, 2048), (256, 4801, 2304), (200, 16384, 256), (33, 9728, 2048), (128, 18944, 2048), (128, 19200, 2048), (256, 8192, 1024)])
+def test_one_row_of_tiles(dev, monkeypatch, kind, M, N, K):
+    g = np.random.Generator(np.random.PCG64(M + N + K))
+    raw, dt = codes(g, kind, N, K)
+    w, x, b = dev.from_quantized(raw, dt, (N, K)), dev.from_numpy(g.standard_normal((M, K)).astype(F16)), dev.from_numpy(g.standard_normal(N).astype(F16))
+    got = dev.matmul(w, x, b, False, True, True).to_numpy()
+    monkeypatch.setenv("RCU_GEMM_FUSED", "1")
+    want = dev.matmul(w, x, b, False, True, True).to_numpy()
+    assert np.isfinite(want).all()
+    if N == 18944:
+        got, want = got.astype(np.float64), want.astype(np.float64)
+        assert (np.abs(got - want) <= 2.0 ** -10 * np.abs(want) + 4 * 2.0 ** -24 * np.sqrt(K) * np.sqrt((want ** 2).mean())).all()
+    else:
+        assert np.array_equal(got.view(np.uint16), want.view(np.uint16))
+
+
+@pytest.mark.parametrize("kind,M,F,K", [("q8_0h", 500, 2608, 512), ("q4_kh", 470, 4912, 768), ("q8_0h", 200, 5120, 2048), ("q4_kh", 130, 5600, 2048)])
 @pytest.mark.parametrize("what", ["gate", "gelu", "resid"])
 def test_epilogues(dev, monkeypatch, kind, M, F, K, what):
     g = np.random.Generator(np.random.PCG64(F))
