@@ -16,8 +16,9 @@
 //                      output feature), add bias, round to f16, store rows.
 // Quantised weights (Q8_0H, Q4_KH) are dequantised inside the kernel (up to 256 token rows): TMA
 // brings the packed bytes of the weight tile into shared memory, further warps convert them to f16
-// with the CPU dequantiser's arithmetic and write the swizzled tile the MMA reads.  Larger M takes the
-// pair kernel, which converts on the way too, or - too few tiles for it - dequantises once into pooled scratch.
+// with the CPU dequantiser's arithmetic and write the swizzled tile the MMA reads.  Where these tiles
+// outnumber the SMs (pair_converts has the line), and for larger M, the pair kernel converts on the way
+// too; a larger M with too many rounds of its tiles is dequantised once into pooled scratch.
 //
 // Every mbarrier wait is bounded; a wait that gives up sets RCU_DEVFLAG_TIMEOUT and an abort word in
 // shared memory that ends all other waits of the CTA, and the CTA still frees its tensor memory.
