@@ -58,11 +58,13 @@ constexpr int kAccCols = 256;                      // f32 accumulator columns pe
 constexpr int kConvWarps = 8;                      // converting warps of a CTA (quantised weights)
 constexpr int kTeams = 4, kTeamWarps = kConvWarps / kTeams, kFeedWarps = 2;
 constexpr int kGroup = 4;                          // steps whose scales travel together: 256 of K
-constexpr int kRawSlots = 6, kScaleSlots = 2;      // steps of codes, groups of scales in flight
+constexpr int kScaleSlots = 2;                     // groups of scales in flight
 constexpr int stages2(int wk) { return wk == WK_F16 ? kStages2 : wk == WK_Q8 ? 4 : 5; }
+constexpr int raw_slots(int wk) { return wk == WK_F16 ? 0 : 4; }                // steps of codes in flight
+constexpr int free_slots(int wk) { return wk == WK_Q4K ? 8 : 0; }               // stages that are handed on (RawRings); 0: the teams wait for them themselves
 constexpr int raw_row(int wk) { return wk == WK_Q8 ? TK : TK / 2; }             // bytes of a row's codes in a step
 constexpr int scale_row(int wk) { return wk == WK_Q8 ? 16 : 32; }               // of its scales in a group: eight f16; eight multipliers and minima
-constexpr int raw_bytes(int wk) { return wk == WK_F16 ? 0 : TM * (kRawSlots * raw_row(wk) + kScaleSlots * scale_row(wk)); }
+constexpr int raw_bytes(int wk) { return wk == WK_F16 ? 0 : TM * (raw_slots(wk) * raw_row(wk) + kScaleSlots * scale_row(wk)); }
 constexpr int threads2(int wk) { return kThreads2 + (wk == WK_F16 ? 0 : (kConvWarps + kFeedWarps) * 32); }
 constexpr size_t smem2(int wk) { return 1024 + (size_t)stages2(wk) * kStageBytes2 + raw_bytes(wk) + 512; }
 
@@ -111,12 +113,15 @@ __device__ __forceinline__ void umma2_commit_both(uint64_t* bar) {
                  : "memory");
 }
 
-// What the converting warps of a CTA work from.  A barrier's parity tells a use from the one before it, not from one further back; so each ring
-// is filled by one warp, in order, and a team has every fourth step (K is whole groups: a tile does not shift the teams) - whoever waits for
-// a use of a slot has seen, by its own last wait, that the use before the previous one is over.
+// What the converting warps of a CTA work from.  A barrier's parity tells a use of a slot from the one before it, not from one further back, and
+// neither loads nor commits on different barriers need arrive in the order that they were asked for.  So whoever waits for a use of a slot must be who waited
+// for the use before it.  A team has every fourth step (K is whole groups: a tile does not shift the teams), so the ring of codes is a multiple of
+// four slots.  (Of six slots a team met every second fill only, whose parity it had seen already: a load that the one behind it overtook was not waited
+// for.)  So are Q8_0's stages.  Q4_K's five are not - with four 512 x 8192 x 3072 takes 39.0 us, not 33.4 - so the warp that brings the activations, which waits for
+// every use of every stage, hands each on through a ring of eight: more than it can be ahead.
 struct RawRings {
-    unsigned char *codes, *scales;              // [kRawSlots][128][raw_row], [kScaleSlots][128][scale_row]
-    uint64_t *full, *empty, *scale_full, *scale_empty;
+    unsigned char *codes, *scales;              // [raw_slots][128][raw_row], [kScaleSlots][128][scale_row]
+    uint64_t *full, *empty, *scale_full, *scale_empty, *stage_free;
 };
 // The first row of W that this CTA has of tile t
 template <bool GLU> __device__ __forceinline__ int tile_row(int t, int tiles_m, uint32_t rank, int N) {
@@ -126,6 +131,7 @@ template <bool GLU> __device__ __forceinline__ int tile_row(int t, int tiles_m, 
 template <int WK, bool GLU>
 __device__ __forceinline__ void feed_codes(const CUtensorMap* wmap, const RawRings& raw, uint32_t rank, int pair, int n_pairs, int n_tiles, int tiles_m, int N, int nk,
                                            volatile int* abort_flag, int* status) {
+    constexpr int SLOTS = raw_slots(WK);
     if ((threadIdx.x & 31) != 0) return;
     int it = 0, rs = 0, phase = 1;            // a fresh barrier's odd phase counts as done
     for (int t = pair; t < n_tiles; t += n_pairs) {
@@ -133,13 +139,13 @@ __device__ __forceinline__ void feed_codes(const CUtensorMap* wmap, const RawRin
         for (int k = 0; k < nk; ++k, ++it) {
             if (!mbar_wait(&raw.empty[rs], (unsigned)phase, abort_flag, status)) {
                 // given up: the codes in flight get another chance to land before the CTA leaves
-                for (int i = 1; i <= min(it, kRawSlots); ++i)
-                    for (int n = 0; n < (1 << 16) && !gemvq8::mbar_test_wait(&raw.full[(it - i) % kRawSlots], ((it - i) / kRawSlots) & 1); ++n) {}
+                for (int i = 1; i <= min(it, SLOTS); ++i)
+                    for (int n = 0; n < (1 << 16) && !gemvq8::mbar_test_wait(&raw.full[(it - i) % SLOTS], ((it - i) / SLOTS) & 1); ++n) {}
                 return;
             }
             mbar_expect_tx(&raw.full[rs], TM * raw_row(WK));
             tma_load_2d(raw.codes + rs * TM * raw_row(WK), wmap, k * raw_row(WK), row, &raw.full[rs]);
-            if (++rs == kRawSlots) { rs = 0; phase ^= 1; }
+            if (++rs == SLOTS) { rs = 0; phase ^= 1; }
         }
     }
 }
@@ -215,17 +221,18 @@ __device__ __forceinline__ void feed_scales(const QuantArgs& qa, const RawRings&
 template <int WK>
 __device__ __forceinline__ void convert_tiles(const RawRings& raw, unsigned char* smem, uint64_t* full, uint64_t* empty, int steps, volatile int* abort_flag, int* status) {
     using namespace rcu_dequant;
+    constexpr int SLOTS = raw_slots(WK), FREE = free_slots(WK), S = stages2(WK);
     static_assert(kTeams == kGroup, "a team has one step of every group: its index is the step's place there");
+    static_assert(SLOTS % kTeams == 0 && (FREE ? FREE % kTeams == 0 && FREE > S : S % kTeams == 0), "a slot belongs to one team");
     constexpr int PER_ROW = WK == WK_Q8 ? 4 : 2, TASKS = TM / kTeamWarps * PER_ROW / 32, ROWS = 32 / PER_ROW;      // lanes per row; rows of a lane, so far apart
-    constexpr int S = stages2(WK);
     const int lane = threadIdx.x & 31, cw = (threadIdx.x - kThreads2) >> 5, team = cw / kTeamWarps;
     const int r0 = cw % kTeamWarps * (TM / kTeamWarps) + lane / PER_ROW, part = lane % PER_ROW;
     const uint32_t full_leader = map_to_cta(smem_u32(full), 0);
     auto wait = [&](uint64_t* bar, int parity) { return (bool)__all_sync(0xffffffffu, mbar_wait(bar, (unsigned)parity, abort_flag, status)); };
     int gs = 0, scale_phase = 0;
     for (int it = team; it < steps; it += kTeams) {
-        const int s = it % S, rs = it % kRawSlots;
-        if (!wait(&raw.scale_full[gs], scale_phase) || !wait(&raw.full[rs], (it / kRawSlots) & 1)) return;
+        const int s = it % S, rs = it % SLOTS;
+        if (!wait(&raw.scale_full[gs], scale_phase) || !wait(&raw.full[rs], (it / SLOTS) & 1)) return;
         const unsigned char *codes = raw.codes + rs * TM * raw_row(WK), *scales = raw.scales + gs * TM * scale_row(WK);
         uint4 q[TASKS], o[TASKS][WK == WK_Q8 ? 2 : 4];
         uint2 sc[TASKS];
@@ -258,7 +265,11 @@ __device__ __forceinline__ void convert_tiles(const RawRings& raw, unsigned char
             mbar_arrive(&raw.scale_empty[gs]);
         }
         if (++gs == kScaleSlots) { gs = 0; scale_phase ^= 1; }
-        if (!wait(&empty[s], (it / S + 1) & 1)) return;         // a fresh barrier's odd phase counts as done
+        if constexpr (FREE > 0) {
+            if (!wait(&raw.stage_free[it % FREE], (it / FREE) & 1)) return;
+        } else {
+            if (!wait(&empty[s], (it / S + 1) & 1)) return;     // a fresh barrier's odd phase counts as done
+        }
         unsigned char* tile = smem + s * kStageBytes2 + TM * TK * 2;
 #pragma unroll
         for (int i = 0; i < TASKS; ++i) {
@@ -292,7 +303,7 @@ template <class Out, int MODE, bool GLU, int WK>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(threads2(WK), 1)
 gemm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const GemmEpilogue<Out, MODE> epi,
                 Out* out, int M, int N, int K, int tiles_m, int n_tiles, int* status, uint32_t idesc, int glu_act, const QuantArgs qa, bool lead) {
-    constexpr int STAGES = stages2(WK), RAW = raw_bytes(WK);
+    constexpr int STAGES = stages2(WK), RAW = raw_bytes(WK), SLOTS = raw_slots(WK), FREE = free_slots(WK);
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * kStageBytes2 + RAW);   // leader's are the ones in use
@@ -302,8 +313,8 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     uint64_t* raw_bars = reinterpret_cast<uint64_t*>(tmem_slot + 2);
-    const RawRings raw{smem + STAGES * kStageBytes2, smem + STAGES * kStageBytes2 + (WK == WK_F16 ? 0 : kRawSlots * TM * raw_row(WK)), raw_bars, raw_bars + kRawSlots,
-                       raw_bars + 2 * kRawSlots, raw_bars + 2 * kRawSlots + kScaleSlots};
+    const RawRings raw{smem + STAGES * kStageBytes2, smem + STAGES * kStageBytes2 + SLOTS * TM * raw_row(WK), raw_bars, raw_bars + SLOTS,
+                       raw_bars + 2 * SLOTS, raw_bars + 2 * SLOTS + kScaleSlots, raw_bars + 2 * SLOTS + 2 * kScaleSlots};
 
     __shared__ float4 turn[kEpilogueWarps][kTurnQuads];      // one piece of an accumulator per epilogue warp
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -321,7 +332,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
             mbar_init(&acc_empty[b], 2 * kEpilogueWarps);       // both CTAs'
         }
         if (WK != WK_F16) {
-            for (int i = 0; i < kRawSlots; ++i) {
+            for (int i = 0; i < SLOTS; ++i) {
                 mbar_init(&raw.full[i], 1);
                 mbar_init(&raw.empty[i], kTeamWarps);
             }
@@ -329,6 +340,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
                 mbar_init(&raw.scale_full[i], 1);
                 mbar_init(&raw.scale_empty[i], kConvWarps);
             }
+            for (int i = 0; i < FREE; ++i) mbar_init(&raw.stage_free[i], 1);
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -354,6 +366,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
                 for (int k = 0; k < nk; ++k, ++it) {
                     const int s = it % STAGES;
                     if (it >= STAGES && !mbar_wait(&empty[s], ((it / STAGES) - 1) & 1, abort_flag, status)) { ok = false; break; }
+                    if constexpr (FREE > 0) mbar_arrive(&raw.stage_free[it % FREE]);
                     unsigned char* st = smem + s * kStageBytes2;
                     if (rank == 0) mbar_expect_tx(&full[s], WK == WK_F16 ? 2 * kStageBytes2 : kStageBytes2);      // both CTAs' bytes
                     const uint32_t bar = map_to_cta(smem_u32(&full[s]), 0);
@@ -394,11 +407,11 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
             }
         }
     } else if (WK != WK_F16 && warp == 2 + kEpilogueWarps + kConvWarps) {
-        feed_codes<WK, GLU>(&wmap, raw, rank, pair, n_pairs, n_tiles, tiles_m, N, nk, abort_flag, status);
+        if constexpr (WK != WK_F16) feed_codes<WK, GLU>(&wmap, raw, rank, pair, n_pairs, n_tiles, tiles_m, N, nk, abort_flag, status);
     } else if (WK != WK_F16 && warp == 3 + kEpilogueWarps + kConvWarps) {
         feed_scales<WK, GLU>(qa, raw, rank, pair, n_pairs, n_tiles, tiles_m, GLU ? 2 * N : N, N, K, abort_flag, status);
     } else if (WK != WK_F16 && warp >= 2 + kEpilogueWarps) {
-        convert_tiles<WK>(raw, smem, full, empty, pair < n_tiles ? (n_tiles - pair + n_pairs - 1) / n_pairs * nk : 0, abort_flag, status);
+        if constexpr (WK != WK_F16) convert_tiles<WK>(raw, smem, full, empty, pair < n_tiles ? (n_tiles - pair + n_pairs - 1) / n_pairs * nk : 0, abort_flag, status);
     } else {
         // epilogue warps 2..9: tensor-memory lane quarter = warp index modulo 4
         const int q = warp & 3, c0 = (warp - 2) / 4 * (kTileN2 / 2);
