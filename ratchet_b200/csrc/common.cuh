@@ -28,6 +28,10 @@ struct rcu_pool {
     std::unordered_map<void*, uint64_t> live;      // ptr -> block size
     std::unordered_map<void*, uint64_t> all;       // every block owned by the pool
     uint64_t in_use = 0, reserved = 0;
+    uint64_t limit = ~0ull;                        // of `reserved` (RCU_POOL_LIMIT in the environment at creation, in bytes): beyond it memory counts as exhausted
+    // memory that is held for speed alone, given back when an allocation finds none (the resolver's, for the length of a resolve)
+    void (*give_back)(void*) = nullptr;
+    void* giver = nullptr;
 };
 
 struct rcu_device {
@@ -57,6 +61,8 @@ struct rcu_device {
 };
 
 rcu_status rcu_fail(rcu_device* dev, rcu_status st, const char* fmt, ...);
+// A block for speed alone: RCU_ERR_OOM where rcu_alloc would first drop what the pool has cached
+rcu_status rcu_alloc_spare(rcu_device* dev, uint64_t nbytes, void** dptr);
 
 #define RCU_CUDA(dev, expr)                                                                     \
     do {                                                                                        \

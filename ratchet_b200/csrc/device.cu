@@ -46,6 +46,7 @@ static rcu_status create_common(int ordinal, cudaStream_t stream, bool own, rcu_
     }
     if (const char* e = std::getenv("RCU_NO_REUSE")) dev->debug_flags |= std::atoi(e) ? RCU_DEBUG_NO_REUSE : 0;
     if (const char* e = std::getenv("RCU_PROFILE")) dev->debug_flags |= std::atoi(e) ? RCU_DEBUG_PROFILE : 0;
+    if (const char* e = std::getenv("RCU_POOL_LIMIT")) dev->pool.limit = std::strtoull(e, nullptr, 10);
     if (const char* e = std::getenv("RCU_LOG")) dev->debug_flags |= std::atoi(e) ? RCU_DEBUG_LOG : 0;
     cudaMemsetAsync(dev->d_status, 0, kStatusBlockBytes, dev->stream);
     cudaMemcpyAsync(reinterpret_cast<char*>(dev->d_status) + 8, &dev->wait_limit_ns, 8, cudaMemcpyHostToDevice, dev->stream);
@@ -89,22 +90,24 @@ static uint64_t size_class(uint64_t n) {
     return (n + mib - 1) / mib * mib;
 }
 
-rcu_status rcu_alloc(rcu_device* dev, uint64_t nbytes, void** dptr) {
-    if (!dev || !dptr) return RCU_ERR_INVALID_ARG;
+static rcu_status take_block(rcu_device* dev, uint64_t nbytes, void** dptr, bool spare) {
     DevGuard g(dev->ordinal);
     uint64_t sz = size_class(nbytes);
+    auto grow = [&](void** p) { return dev->pool.reserved + sz > dev->pool.limit ? cudaErrorMemoryAllocation : cudaMalloc(p, sz); };
     auto it = dev->pool.free_blocks.find(sz);
     void* p = nullptr;
     if (it != dev->pool.free_blocks.end()) {
         p = it->second;
         dev->pool.free_blocks.erase(it);
     } else {
-        cudaError_t e = cudaMalloc(&p, sz);
+        cudaError_t e = grow(&p);
         if (e != cudaSuccess) {
             // release cached blocks and retry once
             cudaGetLastError();
+            if (spare) return RCU_ERR_OOM;
+            if (dev->pool.give_back) dev->pool.give_back(dev->pool.giver);
             rcu_pool_trim(dev);
-            e = cudaMalloc(&p, sz);
+            e = grow(&p);
             if (e != cudaSuccess) {
                 cudaGetLastError();
                 return rcu_fail(dev, RCU_ERR_OOM, "cudaMalloc(%llu) failed: %s", (unsigned long long)sz, cudaGetErrorString(e));
@@ -118,6 +121,8 @@ rcu_status rcu_alloc(rcu_device* dev, uint64_t nbytes, void** dptr) {
     *dptr = p;
     return RCU_OK;
 }
+
+rcu_status rcu_alloc(rcu_device* dev, uint64_t nbytes, void** dptr) { return dev && dptr ? take_block(dev, nbytes, dptr, false) : RCU_ERR_INVALID_ARG; }
 
 rcu_status rcu_free(rcu_device* dev, void* dptr) {
     if (!dev) return RCU_ERR_INVALID_ARG;
@@ -147,6 +152,12 @@ void rcu_pool_stats(rcu_device* dev, uint64_t* in_use, uint64_t* reserved) {
     if (in_use) *in_use = dev ? dev->pool.in_use : 0;
     if (reserved) *reserved = dev ? dev->pool.reserved : 0;
 }
+
+}  // extern "C"
+
+rcu_status rcu_alloc_spare(rcu_device* dev, uint64_t nbytes, void** dptr) { return take_block(dev, nbytes, dptr, true); }
+
+extern "C" {
 
 // ---------------------------------------------------------------------------------- transfers
 rcu_status rcu_h2d(rcu_device* dev, void* dst, const void* src, uint64_t nbytes) {

@@ -529,12 +529,19 @@ struct ConvertedBeside {
     size_t at = 0;                                 // the item whose product comes next
     bool ready = false;                            // its weights are converted, or on their way
     void* block[2] = {nullptr, nullptr};
+    uint32_t started = 0;                          // conversions beside a product so far
+    int held = -1;                                 // the block that the product being launched reads
     rcu_device::NextConversion next;
     explicit ConvertedBeside(rcu_device* d) : dev(d) {}
     ~ConvertedBeside() {
         dev->next_conversion = nullptr;
-        for (void* b : block)
-            if (b) rcu_free(dev, b);               // the pool reuses blocks in stream order
+        dev->pool.give_back = nullptr;
+        drop(0);
+        drop(1);
+    }
+    void drop(int i) {
+        if (block[i]) rcu_free(dev, block[i]);     // the pool reuses blocks in stream order
+        block[i] = nullptr;
     }
     void plan(const std::vector<rcu_lazy*>& order, const fusion::Pass& fused) {
         uint64_t most = 0;
@@ -545,7 +552,20 @@ struct ConvertedBeside {
             items.push_back({i, w});
             most = std::max(most, w->numel() * 2);
         }
-        if (items.size() < 2 || rcu_alloc(dev, most, &block[0]) != RCU_OK || rcu_alloc(dev, most, &block[1]) != RCU_OK) items.clear();      // no room: each beside its own
+        if (items.size() < 2 || rcu_alloc_spare(dev, most, &block[0]) != RCU_OK || rcu_alloc_spare(dev, most, &block[1]) != RCU_OK) {
+            items.clear();                         // no room: each product converts its own, in scratch that is free again behind it
+            drop(0);
+            return;
+        }
+        dev->pool.give_back = [](void* self) { ((ConvertedBeside*)self)->give_back(); };
+        dev->pool.giver = this;
+    }
+    // Something else of the resolve finds no memory: the products to come convert their own.  A product that is being launched keeps its weights.
+    void give_back() {
+        dev->next_conversion = nullptr;
+        items.clear();
+        for (int i = 0; i < 2; ++i)
+            if (i != held) drop(i);
     }
     bool has(size_t node) const { return at < items.size() && items[at].node == node; }
     // The converted weights of the next product; with it the conversion for the one after is launched.
@@ -558,7 +578,8 @@ struct ConvertedBeside {
             const rcu_status st = rcu_dequantize(dev, &src, &dst);
             if (st != RCU_OK) return st;
         }
-        *w = block[at & 1];
+        held = (int)(at & 1);
+        *w = block[held];
         if (++at < items.size()) {
             uint64_t off[4];
             const rcu_lazy* n = items[at].w;
@@ -569,8 +590,11 @@ struct ConvertedBeside {
         return RCU_OK;
     }
     void end() {
+        if (items.empty()) drop(held);             // given back meanwhile
+        held = -1;
         if (dev->next_conversion) {
             ready = next.started;
+            started += ready;
             dev->next_conversion = nullptr;
         } else {
             ready = false;
@@ -783,8 +807,8 @@ rcu_status resolve(rcu_lazy* out) {
     dev->last_resolve.naive_bytes = naive;
     (void)launched;
     if (log)
-        std::fprintf(stderr, "[rcu] resolve: %zu nodes, %u launches, %u in place, %zu buffers, %llu bytes planned (%llu unshared)\n", n,
-                     dev->last_resolve.launched, n_inplace, objects.size(), (unsigned long long)planned, (unsigned long long)naive);
+        std::fprintf(stderr, "[rcu] resolve: %zu nodes, %u launches, %u in place, %zu buffers, %llu bytes planned (%llu unshared), %u weights converted beside a product\n", n,
+                     dev->last_resolve.launched, n_inplace, objects.size(), (unsigned long long)planned, (unsigned long long)naive, beside.started);
     return RCU_OK;
 }
 
