@@ -1207,9 +1207,17 @@ namespace {
 int latent_splits(const rcu_stack_run& r) { return (int)std::min<uint32_t>(kMaxSplits, std::max<uint32_t>(1, (std::min(r.window, r.ring_rows) + kSub - 1) / kSub)); }
 
 // Partial results of a run's attention: its splits, or the clusters that they form where what the merging kernel would read of a head is long enough to
-// pay for a cluster's two barriers (us per token, splits x rank 32 x 256: 178.7 without / 188.2 with; 64 x 512: 332.6 / 322.6 and 385.8 / 379.8)
+// pay for a cluster's two barriers.  Us per token of six latent layers, width 1024, heads x rank x window, apart / in clusters:
+//   splits x rank up to 16384: 16 x 256 x 512 151.3 / 158.6, 16 x 192 x 1024 146.5 / 165.8, 16 x 256 x 1024 152.7 / 159.4, 64 x 256 x 1024 172.8 / 195.0
+//   17408 to 24576: 16 x 272 x 1024 164.5 / 159.9, 32 x 272 x 1024 173.3 / 164.1, 16 x 320 x 1024 169.9 / 164.0, 48 x 384 x 1024 191.6 / 185.0,
+//     128 x 320 x 1024 290.7 / 284.5; of fewer splits 16 x 1024 x 272 181.1 / 188.1, 32 x 640 x 512 187.2 / 190.3
+//   32768: 16 x 512 x 1024 185.4 / 175.2, 32 x 1024 x 512 223.0 / 214.1;  65536: 16 x 1024 x 1024 228.9 / 192.8
+// Four rows of heads are the exception, why is not known: 64 x 320 x 1024 188.2 / 198.6, 64 x 1024 x 512 239.4 / 249.8, 64 x 512 x 1024 212.7 / 211.4; from 40960
+// on they gain too, 64 x 640 x 1024 253.9 / 229.9.
 bool latent_clusters(const rcu_stack_run& r, int dt) {
-    return dt == RCU_BF16 && latent_splits(r) >= kLatentCluster && (uint64_t)latent_splits(r) * r.kv_rank >= 16384;
+    const uint64_t size = (uint64_t)latent_splits(r) * r.kv_rank;
+    const bool four_rows = (r.heads + kMmaHeads - 1) / kMmaHeads == 4;
+    return dt == RCU_BF16 && latent_splits(r) >= 4 * kLatentCluster && size > (four_rows ? 32768 : 16384);
 }
 int latent_partials(const rcu_stack_run& r, int dt) { return latent_clusters(r, dt) ? (latent_splits(r) + kLatentCluster - 1) / kLatentCluster : latent_splits(r); }
 
