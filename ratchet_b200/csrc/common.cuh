@@ -84,10 +84,19 @@ rcu_status rcu_alloc_spare(rcu_device* dev, uint64_t nbytes, void** dptr);
         RCU_CUDA((dev), cudaGetLastError());                                                    \
     } while (0)
 
-// Every kernel of the library begins with this: wait for the kernel before it in the stream (a no-op unless this
-// one was launched as its programmatic dependent), then let the next kernel's blocks be scheduled.  Launched through
-// rcu_launch, consecutive kernels overlap their launch and start-up with the predecessor's tail; nothing of a kernel's
-// own work precedes the wait, so stream order is what the memory sees.
+// The rule of kernels that are launched through rcu_launch: as programmatic dependents, consecutive kernels overlap their launch and start-up with the
+// predecessor's tail, so each waits for the kernel before it (a no-op unless it was launched as its dependent) ahead of any access to memory that is not constant,
+// and every kernel has waited, in at least one of its blocks, before it ends.  So the end of a kernel is the end of all before it, and whoever has waited sees
+// what they wrote.  Most kernels begin with rcu_kernel_entry().  What does not:
+//   kernels with set-up that touches no global memory (barriers, tensor memory): the wait behind it;
+//   kernels that request constants ahead of the wait: GEMVs and gemm_rows.cu the weights, on the host's or the resolver's word that nobody writes them,
+//     the decode step's kernels weights and norm scales;
+//   a decode step's mixers (stack_decode.cu, grouped_step.cuh): rings, states and the position that earlier steps wrote.  The step's first kernel
+//     triggers behind its wait, so those are complete when any other one begins; `ahead` is off where two runs share a state;
+//   dequant_q8_beside_kernel (quant.cu): writes without a wait, and its first block waits at its end.  The product before it triggers behind its own wait, and the
+//     destination's last reader is before that product.
+// A kernel that triggers at its entry lets the next one start before what precedes it has ended: what may be read ahead of a wait is decided by all
+// kernels in front of it.
 __device__ __forceinline__ void rcu_kernel_entry() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -99,7 +108,7 @@ __device__ __forceinline__ void rcu_kernel_entry() {
 __device__ __forceinline__ void rcu_kernel_entry_wait_only() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // kern<<<grid, block, smem, dev->stream>>>(args...) as a programmatic dependent of the kernel before it
-// (RCU_NO_PDL in the environment launches it plainly).  The kernel must call rcu_kernel_entry() first.  cluster_x > 0: clusters of
+// (RCU_NO_PDL in the environment launches it plainly).  The kernel keeps to the rule above.  cluster_x > 0: clusters of
 // that many CTAs along x.
 template <class... P, class... A>
 inline cudaError_t rcu_launch_cluster(rcu_device* dev, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, int cluster_x, A&&... args) {

@@ -432,8 +432,11 @@ rcu_status launch_f32(rcu_device* dev, const void* w, const void* x, const void*
 
 }  // namespace
 
-// Products over the same rows as tiles of one launch, whole ones: short K (longer ones are cut into runs by themselves) and a product's tiles less than
-// the SMs.  Whisper-tiny's three of 1500 x 384 x 384 take one of them 10 us, the encoder with its four layers 605 us before and 563 with them together.
+// Products over the same rows as tiles of one launch, whole ones: short K (longer ones are cut into runs by themselves: their sums' order would change) and a
+// product's tiles no more than the SMs (beyond that the split-TF32 kernel has them).  Whisper-tiny's three of 1500 x 384 x 384 take one of them 10 us, the encoder with its
+// four layers 605 us before and 563 with them together.  Us for four such groups and the products of their results, apart / together: 2 x 200 x 384 x 384 87.5 / 57.8,
+// 3 x 750 x 512 x 512 161 / 79, 3 x 2000 x 512 x 384 (128 tiles) 174 / 134.  Beyond the limit on K whole tiles would pay further, up to where
+// cutting does: 3 x 300 x 1024 x 1024 190 / 110, 2 x 400 x 512 x 2048 135 / 162.
 bool rcu_gemm_tc_f32_eligible(int lhs_dt, int act_dt, uint64_t M, uint64_t N, uint64_t K, uint64_t batches);
 rcu_status rcu_gemm_parts_f32_group(rcu_device* dev, const LinearGroup& g) {
     constexpr int T = 64;
@@ -480,14 +483,13 @@ bool takes(rcu_device* dev, uint64_t M, uint64_t N, uint64_t batches) {
 }
 rcu_status dispatch(rcu_device* dev, const void* w, const void* x, const void* bias, void* y, uint64_t M, uint64_t N, uint64_t K, uint64_t batches, const void* bias_rows,
                     const void* resid) {
-#define RCU_PARTS(T_) (resid ? launch_f32<T_, true>(dev, w, x, bias, bias_rows, y, M, N, K, batches, resid) : launch_f32<T_, false>(dev, w, x, bias, bias_rows, y, M, N, K, batches))
     // Tiles of 32 tokens where they leave room on the SMs too and K is short: a CTA's chain of units is what counts then, and theirs are shorter
     // (33 x 64 x 256: 9.8 us with tiles of 64)
     const bool narrow = K <= 8 * kUnitK && batches * ((M + 31) / 32) * ((N + kRowsW - 1) / kRowsW) <= (uint64_t)dev->sm_count;
-    if (M <= 16) return RCU_PARTS(16);
-    if (M <= 32 || narrow) return RCU_PARTS(32);
-    return RCU_PARTS(64);
-#undef RCU_PARTS
+    if (resid) return narrow ? launch_f32<32, true>(dev, w, x, bias, bias_rows, y, M, N, K, batches, resid) : launch_f32<64, true>(dev, w, x, bias, bias_rows, y, M, N, K, batches, resid);
+    if (M <= 16) return launch_f32<16, false>(dev, w, x, bias, bias_rows, y, M, N, K, batches);
+    if (M <= 32 || narrow) return launch_f32<32, false>(dev, w, x, bias, bias_rows, y, M, N, K, batches);
+    return launch_f32<64, false>(dev, w, x, bias, bias_rows, y, M, N, K, batches);
 }
 }  // namespace
 

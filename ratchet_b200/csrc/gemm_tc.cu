@@ -414,13 +414,15 @@ bool rcu_gemm_tc_eligible(int lhs_dt, int act_dt, uint64_t M, uint64_t N, uint64
 }
 
 // gemm_tc2.cu: the CTA-pair kernel for f16 weights
+bool rcu_gemm_tc2_on();
 bool rcu_gemm_tc2_eligible(rcu_device* dev, uint64_t M, uint64_t N, uint64_t K);
 rcu_status rcu_gemm_tc2_launch(rcu_device* dev, const void* w, const void* x, const void* bias, void* y, uint64_t M, uint64_t N, uint64_t K,
                                const TcLinear& t);
 
 // Quantised weights.  The one-CTA kernel converts a weight tile once per 128-row token tile, i.e. M/128 times over the whole problem.  Where it
 // pays the pair kernel converts its tiles itself (pair_converts); beyond kFusedMaxM token rows otherwise the matrix is converted once into pooled
-// f16 scratch (which stays in L2) for the f16 kernels (M = 512, N = 8192, K = 3072, Q4_K: 34 us against 46 us in the one-CTA kernel).
+// f16 scratch (which stays in L2) for the f16 kernels (us in the pair kernel / converted first / in the one-CTA kernel, 512 rows: 8192 x 3072 Q4_KH 33.9 / 35.5 /
+// 52.0, 9216 x 3072 Q8_0H 31.5 / 37.4 / 49.7).
 // RCU_GEMM_FUSED=0/1 forces the conversion or the one-CTA kernel.
 constexpr uint64_t kFusedMaxM = 256;
 static bool converts_once(uint64_t M) {
@@ -430,11 +432,11 @@ static bool converts_once(uint64_t M) {
 
 // Whether the pair kernel converts the tiles itself (gemm_tc2.cu; K of whole groups of 256).  A conversion costs 8.4 ns (Q8_0H; Q4_KH 7) for each
 // 256 weight rows and 64 of K; in the kernel every round of tiles takes some 0.16 us (0.17) longer per 64 of K, the hand-overs of the
-// converting warps.  us converted / in the kernel, Q8_0H 9216 x 3072: 300 rows 35.8 / 30.5, 512 36.6 / 31.0, 768 (a second round) 51.0 / 53.3, 1000 56.3 /
-// 57.8, 2048 96.4 / 120.1; 16384 x 3072: 512 74.1 / 63.3, 1000 104.7 / 119.9; 5120 x 8192: 512 66.8 / 63.7; 3072 x 8192: 1000 57.1 / 63.2; Q4_KH
-// 9216 x 3072: 300 36.5 / 31.1; 16384 x 3072: 512 69.4 / 60.6; 5120 x 8192: 512 65.9 / 68.8; 32064 x 3072: 300 126.7 / 111.9.
+// converting warps.  us converted / in the kernel, Q8_0H 9216 x 3072: 300 rows 36.2 / 30.6, 512 37.4 / 31.5, 768 (a second round) 51.0 / 53.3, 1000 56.3 /
+// 57.8, 2048 96.4 / 120.1; 16384 x 3072: 512 68.7 / 55.1, 1000 104.7 / 119.9; 5120 x 8192: 512 75.8 / 63.5; 3072 x 8192: 1000 57.1 / 63.2; Q4_KH
+// 9216 x 3072: 300 36.7 / 32.7; 16384 x 3072: 512 67.0 / 58.6; 5120 x 8192: 512 65.9 / 68.8; 32064 x 3072: 300 122.8 / 104.2.
 static bool pair_converts(rcu_device* dev, int dt, uint64_t M, uint64_t N, uint64_t K) {
-    if (K % 256 != 0 || !rcu_gemm_tc2_eligible(dev, std::max<uint64_t>(M, 1 << 20), N, K)) return false;
+    if (K % 256 != 0 || N < 256 || !rcu_gemm_tc2_on()) return false;
     const uint64_t tiles_n = (N + 255) / 256, pairs = dev->sm_count / 2, rounds = ((M + 255) / 256 * tiles_n + pairs - 1) / pairs;
     if (M > kFusedMaxM) return rcu_gemm_tc2_eligible(dev, M, N, K) && tiles_n > (dt == RCU_Q8_0H ? 19 : 24) * rounds;
     // One row of tiles, against the one-CTA kernel, which converts too: as long as its 128 x 64 tiles do not outnumber the SMs it cuts K and is the
@@ -608,7 +610,9 @@ rcu_status rcu_gemm_tc_chain(rcu_device* dev, int w_dt, const void* w, const voi
 
 // Three products of 501 x 384 x 384, 24 tiles each: 7.7 us and a launch of the host's 4 us apiece (Whisper-tiny's encoder of 1001 frames, Q8_0H:
 // 292 us apart, 244 with its four layers' q, k and v together).  Sizes whose tiles fill the device, or that
-// take other kernels or slices of K alone, stay apart.
+// take other kernels or slices of K alone (their sums' order would change), stay apart.  Us for four such groups and the products of their results, apart / together:
+// 2 x 65 x 64 x 64 63 / 34, 2 x 501 x 384 x 384 52 / 35, 3 x 500 x 512 x 960 101 / 51, 2 x 1500 x 768 x 768 (144 tiles) 65 / 47, 3 x as two and one 100 / 84.
+// Beyond the limits one launch would pay further: 3 x 1500 x 1024 x 512 (192 tiles) 98 / 78, 3 x 300 x 1024 x 1024 102 / 53, 3 x 400 x 512 x 2048 111 / 65.
 rcu_status rcu_gemm_tc_group(rcu_device* dev, const LinearGroup& g) {
     constexpr int BN = 64, STAGES = (100 * 1024) / (TM * TK * 2 + BN * TK * 2);
     if (g.n < 2 || g.n > kGroupLinears || g.M <= 32 || g.N % 8 != 0 || g.K >= 16 * TK || !rcu_gemm_tc_eligible(RCU_F16, RCU_F16, g.M, g.N, g.K)) return RCU_ERR_UNSUPPORTED;

@@ -25,7 +25,7 @@
 //   warp 19            the scales: plain loads, sixteen bytes a row for four steps (requested by the converting warps themselves, codes and
 //                      scales took 2000 cycles a step: 1500 sectors in flight per SM).
 // The converting warps arrive in CTA scope: the tensor cores read behind a proxy fence; arriving in cluster scope waited 0.65 us a step for L2.
-// 512 x 8192 x 3072 Q4_KH: 38.2 us with the conversion in front of it -> 33.3; 512 x 9216 x 3072 Q8_0H: 36.6 -> 31.0 (pair_converts in gemm_tc.cu has more).
+// 512 x 8192 x 3072 Q4_KH: 35.1 us with the conversion in front of it -> 33.7; 512 x 9216 x 3072 Q8_0H: 37.3 -> 31.4 (pair_converts in gemm_tc.cu has more).
 // What bounds it: the chain of hand-overs - a step takes some 1000 cycles with the tensor pipe 42 to 45 % busy, issue slots 34 % - and with Q8_0 the codes' and the
 // converted tile's way through shared memory as well (51 % of its wavefronts are the converting warps').
 //
@@ -511,10 +511,14 @@ bool make_map_f16_sw128_rows(CUtensorMap* map, const void* base, uint64_t rows, 
 
 }  // namespace
 
-// f16 x f16 problems with at least `min_tiles` 256 x 256 tiles take the CTA-pair kernel
-bool rcu_gemm_tc2_eligible(rcu_device* dev, uint64_t M, uint64_t N, uint64_t K) {
+// RCU_GEMM_PAIR=0 in the environment turns the CTA-pair kernel off
+bool rcu_gemm_tc2_on() {
     static const int mode = [] { const char* e = getenv("RCU_GEMM_PAIR"); return e ? atoi(e) : 1; }();
-    if (mode == 0) return false;
+    return mode != 0;
+}
+// f16 x f16 problems with at least a quarter as many 256 x 256 tiles as SMs take the CTA-pair kernel
+bool rcu_gemm_tc2_eligible(rcu_device* dev, uint64_t M, uint64_t N, uint64_t K) {
+    if (!rcu_gemm_tc2_on()) return false;
     if (M < 256 || N < 256 || K < 64 || K % 8 != 0) return false;
     const uint64_t tiles = ((M + 255) / 256) * ((N + 255) / 256);
     return tiles >= (uint64_t)dev->sm_count / 4;

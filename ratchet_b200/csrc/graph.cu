@@ -520,8 +520,8 @@ struct Grouped {
 
 // The large weights that the products of a resolve have converted: each but the first beside the product before its own (rcu_dequantize_beside), into
 // the other of two blocks.  A conversion is a pass over memory and a product bound by the tensor cores; one after the other, as a call
-// by itself has them, the conversions of a Phi-3 prompt of eight layers were 440 us (us a prompt alone / beside, 520 tokens 2323 / 2283, 1000
-// 2989 / 2748, 1250 3618 / 3433, 1500 4003 / 3908: the products' own reads are slower meanwhile).
+// by itself has them, the conversions of a Phi-3 prompt of eight layers were 440 us.  Us a prompt alone / beside, in turns over the same weights: 520 tokens
+// 2305 / 2245, 700 2458 / 2383, 1000 2988 / 2757, 1250 3573 / 3438, 1500 4018 / 3961: the products' own reads are slower meanwhile.
 struct ConvertedBeside {
     struct Item { size_t node; const rcu_lazy* w; };
     rcu_device* dev;

@@ -46,7 +46,8 @@ rcu_status rcu_gemm_tc_chain(rcu_device* dev, int w_dt, const void* w, const voi
 bool rcu_gemm_parts_f32_takes(rcu_device* dev, uint64_t M, uint64_t N, uint64_t K);
 rcu_status rcu_gemm_parts_f32_resid(rcu_device* dev, const void* w, const void* x, const void* bias, const void* resid, void* y, uint64_t M, uint64_t N, uint64_t K);
 
-// Linears of the same sizes over the same rows, in one launch: the projections of an attention, each too small to fill the device.
+// Linears of the same sizes over the same rows, in one launch: the projections of an attention, each too small to fill the device.  q, k and v; a fourth
+// Linear over the same rows runs by itself (every member's tensor map is 128 bytes of each launch's arguments).
 constexpr int kGroupLinears = 3;
 struct LinearGroup {
     int n = 0;

@@ -1000,7 +1000,7 @@ __global__ void __launch_bounds__(kThreads) latent_step_mma_kernel(const float* 
                 w.w = fmaf(f, v[j].w, w.w);
             }
             float* dst = partial + ((size_t)(blockIdx.x / kLatentCluster) * H + h0 + r) * pitch;
-            *reinterpret_cast<float4*>(dst + col) = w;       // columns beyond C: of the padded pitch, zero
+            *reinterpret_cast<float4*>(dst + col) = w;       // columns beyond C lie in the padded pitch: sums of rotated features, which nothing reads
             if (col == 0) {
                 dst[pitch - 2] = M;
                 dst[pitch - 1] = total;
@@ -1331,6 +1331,8 @@ template <class T> rcu_status run_step(rcu_stack* s, const int32_t* token, float
     const rcu_stack_config& c = s->cfg;
     const int W = (int)c.width;
     float *x = s->xa, *other = s->xb;
+    // First of a step's kernels, and it has to be: the others read what earlier steps wrote ahead of their own waits, which is complete only because this
+    // one triggers them behind its wait.
     RCU_CUDA(dev, rcu_launch(dev, embed_kernel<T>, (W + kThreads - 1) / kThreads + s->n_angles, kThreads, 0, token, (const T*)s->embed, (int)c.vocab, W, s->x0, x,
                              (const AngleTable*)s->angle_tables, s->n_angles, s->d_pos, dev->d_status));
     RCU_LAUNCH_CHECK(dev);

@@ -14,10 +14,10 @@ LIMIT = 4e-2
 MODELS = {
     # a gate that starts at 2 * 63 + 64 floats: rows of whole blocks behind unaligned vectors
     "unaligned": B.config(128, 64, [B.lightning(1, 63, 64, (0.9,), ff=192), B.latent(2, 30, 6, 32, 64, 64, 5, 0.2, ff=64)]),
-    # 8256 = 8192 + 64 activations of a feed-forward: one more than a batch takes
     # runs of positions in clusters of eight: 17 splits (the last cluster's others without a position), ranks that are no multiple of 16, a window of which
     # only the first runs have positions
     "clusters": B.config(64, 64, [B.latent(3, 16, 8, 16, 64, 1000, 272, 0.2, scaling=B.YARN), B.latent(17, 8, 4, 8, 64, 512, 1024, 0.25, scaling=B.YARN)]),
+    # 8256 = 8192 + 64 activations of a feed-forward: more than a batch takes
     "long": B.config(64, 64, [B.lightning(2, 32, 32, (0.8, 0.99), ff=8256), B.latent(4, 16, 8, 16, 128, 192, 21, 0.25, scaling=B.YARN, ff=8192)]),
 }
 
