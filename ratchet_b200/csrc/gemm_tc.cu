@@ -423,29 +423,40 @@ rcu_status rcu_gemm_tc2_launch(rcu_device* dev, const void* w, const void* x, co
 // pays the pair kernel converts its tiles itself (pair_converts); beyond kFusedMaxM token rows otherwise the matrix is converted once into pooled
 // f16 scratch (which stays in L2) for the f16 kernels (us in the pair kernel / converted first / in the one-CTA kernel, 512 rows: 8192 x 3072 Q4_KH 33.9 / 35.5 /
 // 52.0, 9216 x 3072 Q8_0H 31.5 / 37.4 / 49.7).
-// RCU_GEMM_FUSED=0/1 forces the conversion or the one-CTA kernel.
+// RCU_GEMM_FUSED=0/1/2 forces the conversion, the one-CTA kernel or the pair kernel, where it can.
 constexpr uint64_t kFusedMaxM = 256;
 static bool converts_once(uint64_t M) {
     const char* force = getenv("RCU_GEMM_FUSED");
     return force ? atoi(force) == 0 : M > kFusedMaxM;
 }
 
-// Whether the pair kernel converts the tiles itself (gemm_tc2.cu; K of whole groups of 256).  A conversion costs 8.4 ns (Q8_0H; Q4_KH 7) for each
-// 256 weight rows and 64 of K; in the kernel every round of tiles takes some 0.16 us (0.17) longer per 64 of K, the hand-overs of the
-// converting warps.  us converted / in the kernel, Q8_0H 9216 x 3072: 300 rows 36.2 / 30.6, 512 37.4 / 31.5, 768 (a second round) 51.0 / 53.3, 1000 56.3 /
-// 57.8, 2048 96.4 / 120.1; 16384 x 3072: 512 68.7 / 55.1, 1000 104.7 / 119.9; 5120 x 8192: 512 75.8 / 63.5; 3072 x 8192: 1000 57.1 / 63.2; Q4_KH
-// 9216 x 3072: 300 36.7 / 32.7; 16384 x 3072: 512 67.0 / 58.6; 5120 x 8192: 512 65.9 / 68.8; 32064 x 3072: 300 122.8 / 104.2.
+// Whether the pair kernel converts the tiles itself (gemm_tc2.cu; K of whole groups of 256).  Above 256 rows the alternative is a conversion in front: 8.4 ns
+// (Q8_0H; Q4_KH 7) for each 256 weight rows and 64 of K.  In the kernel every round of tiles takes some 0.16 us longer per 64 of K, the hand-overs of the
+// converting warps, and with short K its longer start is not made up for: Q8_0H's once a round, Q4_KH's once a launch.  Both lines lie where neither weights
+// from memory nor weights in L2 lose more than 2 to 3 % (720 and 378 products of 257 to 1000 rows, 4864 to 32064 columns, K 256 to 8192; what is taken is 1.11
+// and 1.08 times as fast in the geometric mean; with a line at 19 and 24 columns of tiles a round some lost up to 10 and 17 %).  us converted / in the kernel,
+// weights from memory, Q8_0H 512 rows: 5120 x 2048 23.4 / 24.4 (left), 6656 x 2048 24.2 / 24.1, 9216 x 3072 36.8 / 31.6, 16384 x 3072 68.2 / 55.5, 5120 x 8192
+// 67.0 / 64.0; 600 rows (a round more): 11008 x 2048 38.0 / 40.3 (left); Q4_KH 512 rows: 8192 x 1024 18.4 / 19.9 (left), 8192 x 3072 35.3 / 35.6 (from L2 35.1
+// / 32.7), 16384 x 3072 65.1 / 58.3, 7168 x 8192 76.9 / 70.7.
 static bool pair_converts(rcu_device* dev, int dt, uint64_t M, uint64_t N, uint64_t K) {
     if (K % 256 != 0 || N < 256 || !rcu_gemm_tc2_on()) return false;
+    if (const char* force = getenv("RCU_GEMM_FUSED")) return atoi(force) == 2 && M > 32 && (M <= kFusedMaxM || rcu_gemm_tc2_eligible(dev, M, N, K));
+    const bool q8 = dt == RCU_Q8_0H;
     const uint64_t tiles_n = (N + 255) / 256, pairs = dev->sm_count / 2, rounds = ((M + 255) / 256 * tiles_n + pairs - 1) / pairs;
-    if (M > kFusedMaxM) return rcu_gemm_tc2_eligible(dev, M, N, K) && tiles_n > (dt == RCU_Q8_0H ? 19 : 24) * rounds;
-    // One row of tiles, against the one-CTA kernel, which converts too: as long as its 128 x 64 tiles do not outnumber the SMs it cuts K and is the
-    // faster one (M = 160, 3072 x 3072: 16 us / 29 here), beyond that its two CTAs an SM share the converting warps' issue slots (us there / here, Q8_0H;
-    // Q4_KH is alike: 160 x 5120 x 3072 31.6 / 29.1, 256 x 9216 x 3072 33.4 / 29.8, 256 x 16384 x 3072 50.2 / 31.4, 160 x 32064 x 3072 99.8 / 55.0, 160 x 8192 x
-    // 1024 15.1 / 15.6, 160 x 16384 x 1024 21.3 / 16.6).  Up to 128 rows that is so in one round of tiles only (128 x 9728 x 3072 32.4 / 29.7, 96 x 10240 x 8192
-    // 78.0 / 63.6, 128 x 9216 x 3072 20.6 / 29.6, 128 x 20480 x 3072 50.0 / 52.4, 96 x 16384 x 1024 15.8 / 16.9).
-    if (M <= 32 || (M + TM - 1) / TM * ((N + 63) / 64) <= (uint64_t)dev->sm_count) return false;
-    return M > TM ? K >= 2048 || N >= 16384 : rounds == 1 && K >= 2048;
+    if (M > kFusedMaxM) {
+        if (!rcu_gemm_tc2_eligible(dev, M, N, K)) return false;
+        return q8 ? tiles_n * K >= rounds * (20 * K + 12288) : K >= 1024 && tiles_n * K >= rounds * 20 * K + 32768;
+    }
+    // One row of tiles, against the one-CTA kernel, which converts too: as long as its tiles do not outnumber the SMs it cuts K and is the faster one (M = 160,
+    // 3072 x 3072: 16 us / 29 here; in tiles of 128 x 128 that is so once more where these are as many as the SMs: 40 x 18944 x 3072 35.9 / 37.3, of two rows
+    // with Q4_KH 0.87 to 1.0 for K of 2048 to 4096, with Q8_0H 1.0 to 1.07 times as fast here), beyond that its two CTAs an SM share the converting warps'
+    // issue slots (us there / here, Q8_0H; Q4_KH is alike: 160 x 5120 x 3072 31.6 / 29.1, 256 x 9216 x 3072 33.4 / 29.8, 256 x 16384 x 3072 50.2 / 31.4, 160 x
+    // 32064 x 3072 99.8 / 55.0, 160 x 8192 x 1024 15.1 / 15.6, 160 x 16384 x 1024 21.3 / 16.6, x 256 11.2 / 11.9).  Up to 128 rows that is so in one round of
+    // tiles only (128 x 9728 x 3072 32.4 / 29.7, 96 x 10240 x 8192 78.0 / 63.6, 128 x 9216 x 3072 20.6 / 29.6, 128 x 20480 x 3072 50.0 / 52.4, 96 x 16384 x
+    // 1024 15.8 / 16.9).
+    const uint64_t tiles_m = (M + TM - 1) / TM, sms = dev->sm_count;
+    if (M <= 32 || tiles_m * ((N + 63) / 64) <= sms || (tiles_m * ((N + 127) / 128) == sms && (M <= TM || !q8))) return false;
+    return M > TM ? K >= 2048 || (N >= 16384 && K >= (q8 ? 512 : 768)) : rounds == 1 && K >= 2048;
 }
 
 // The Linear of an f16 graph with what follows it (TcLinear: chained, or glu): whether the tensor-core kernels take it.  A gate and its up
@@ -457,7 +468,7 @@ bool rcu_gemm_tc_chain_takes(rcu_device* dev, int w_dt, uint64_t M, uint64_t N, 
     if (!rcu_gemm_tc_eligible(w_dt, RCU_F16, M, N, K) || N % 8 != 0) return false;
     if (!glu && !act) return M > 32;               // fewer rows: gemm_rows.cu
     if (N % 16 != 0) return false;
-    if (w_dt != RCU_F16 && !getenv("RCU_GEMM_FUSED") && pair_converts(dev, w_dt, M, N, K)) return true;
+    if (w_dt != RCU_F16 && pair_converts(dev, w_dt, M, N, K)) return true;
     return (w_dt == RCU_F16 || converts_once(M)) && rcu_gemm_tc2_eligible(dev, M, N, K);
 }
 
@@ -467,7 +478,7 @@ rcu_status rcu_gemm_tc_dispatch(rcu_device* dev, int lhs_dt, const void* w, int 
     if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(w)) & 15) return RCU_ERR_UNSUPPORTED;
     DevGuard g(dev->ordinal);
     if (lhs_dt == RCU_F16 && rcu_gemm_tc2_eligible(dev, M, N, K)) return rcu_gemm_tc2_launch(dev, w, x, bias, y, M, N, K, t);
-    if (lhs_dt != RCU_F16 && !getenv("RCU_GEMM_FUSED") && pair_converts(dev, lhs_dt, M, N, K)) {
+    if (lhs_dt != RCU_F16 && pair_converts(dev, lhs_dt, M, N, K)) {
         size_t at[4];
         rcu_dtype_segments(lhs_dt, N * K, at);
         TcLinear q = t;
@@ -644,7 +655,7 @@ rcu_status rcu_gemm_tc_group(rcu_device* dev, const LinearGroup& g) {
 
 bool rcu_linear_converts_beside(rcu_device* dev, uint64_t M, uint64_t N, uint64_t K) {
     return M > kFusedMaxM && converts_once(M) && rcu_gemm_tc_eligible(RCU_Q8_0H, RCU_F16, M, N, K) && rcu_gemm_tc2_eligible(dev, M, N, K) &&
-           (getenv("RCU_GEMM_FUSED") || !pair_converts(dev, RCU_Q8_0H, M, N, K));
+           !pair_converts(dev, RCU_Q8_0H, M, N, K);
 }
 bool rcu_gemm_tc_f32_eligible(int lhs_dt, int act_dt, uint64_t M, uint64_t N, uint64_t K, uint64_t batches = 1);
 bool rcu_linear_converts(int w_dt, int act_dt, uint64_t M, uint64_t N, uint64_t K) {

@@ -35,6 +35,16 @@ def codes(g, kind, n, k):
     return raw, dt
 
 
+# the rule, and the pair kernel at sizes that the rule leaves to the others: None and "2" of RCU_GEMM_FUSED
+ROUTES = [None, "2"]
+
+
+def force(monkeypatch, route):
+    monkeypatch.delenv("RCU_GEMM_FUSED", raising=False)
+    if route is not None:
+        monkeypatch.setenv("RCU_GEMM_FUSED", route)
+
+
 # one group of steps, rings that wrap, one tile per pair and several; ragged rows, columns and columns that are no multiple of four; three
 # rows of tiles, and the other side of the rule: too few columns for the rounds, a K of other than whole groups (converted both times)
 SIZES = [("q8_0h", 257, 5120, 256), ("q8_0h", 512, 5125, 512), ("q8_0h", 300, 16384, 3072), ("q8_0h", 400, 40000, 768), ("q8_0h", 700, 16384, 256), ("q8_0h", 700, 9728, 512), ("q8_0h", 300, 4992, 288),
@@ -42,12 +52,17 @@ SIZES = [("q8_0h", 257, 5120, 256), ("q8_0h", 512, 5125, 512), ("q8_0h", 300, 16
 
 
 @pytest.mark.parametrize("kind,M,N,K", SIZES)
-def test_equals_the_product_over_the_converted_matrix(dev, monkeypatch, kind, M, N, K):
+@pytest.mark.parametrize("route", ROUTES)
+def test_equals_the_product_over_the_converted_matrix(dev, monkeypatch, kind, M, N, K, route):
     g = np.random.Generator(np.random.PCG64(M + N + K))
     raw, dt = codes(g, kind, N, K)
     w, x, b = dev.from_quantized(raw, dt, (N, K)), dev.from_numpy(g.standard_normal((M, K)).astype(F16)), dev.from_numpy(g.standard_normal(N).astype(F16))
+    force(monkeypatch, route)
+    launches = dev.launches
     got = dev.matmul(w, x, b, False, True, True).to_numpy()
-    monkeypatch.setenv("RCU_GEMM_FUSED", "0")
+    if route == "2":
+        assert dev.launches - launches == 1                # no conversion in front
+    force(monkeypatch, "0")
     want = dev.matmul(w, x, b, False, True, True).to_numpy()
     assert np.isfinite(want).all() and np.array_equal(got.view(np.uint16), want.view(np.uint16))
 
@@ -56,13 +71,15 @@ def test_equals_the_product_over_the_converted_matrix(dev, monkeypatch, kind, M,
 # these sizes either (the last two are on the other side of the rule) but for 18944 columns: 148 tiles of 128, two slices of K.  There f32 sums of K products
 # come in another order (2^-24 each, random signs), and an output may round to f16's neighbour.
 @pytest.mark.parametrize("kind", ["q8_0h", "q4_kh"])
+@pytest.mark.parametrize("route", ROUTES)
 @pytest.mark.parametrize("M,N,K", [(129, 5120, 2048), (256, 4801, 2304), (200, 16384, 256), (33, 9728, 2048), (128, 18944, 2048), (128, 19200, 2048), (256, 8192, 1024)])
-def test_one_row_of_tiles(dev, monkeypatch, kind, M, N, K):
+def test_one_row_of_tiles(dev, monkeypatch, kind, M, N, K, route):
     g = np.random.Generator(np.random.PCG64(M + N + K))
     raw, dt = codes(g, kind, N, K)
     w, x, b = dev.from_quantized(raw, dt, (N, K)), dev.from_numpy(g.standard_normal((M, K)).astype(F16)), dev.from_numpy(g.standard_normal(N).astype(F16))
+    force(monkeypatch, route)
     got = dev.matmul(w, x, b, False, True, True).to_numpy()
-    monkeypatch.setenv("RCU_GEMM_FUSED", "1")
+    force(monkeypatch, "1")
     want = dev.matmul(w, x, b, False, True, True).to_numpy()
     assert np.isfinite(want).all()
     if N == 18944:
@@ -74,7 +91,8 @@ def test_one_row_of_tiles(dev, monkeypatch, kind, M, N, K):
 
 @pytest.mark.parametrize("kind,M,F,K", [("q8_0h", 500, 2608, 512), ("q4_kh", 470, 4912, 768), ("q8_0h", 200, 5120, 2048), ("q4_kh", 130, 5600, 2048)])
 @pytest.mark.parametrize("what", ["gate", "gelu", "resid"])
-def test_epilogues(dev, monkeypatch, kind, M, F, K, what):
+@pytest.mark.parametrize("route", ROUTES)
+def test_epilogues(dev, monkeypatch, kind, M, F, K, what, route):
     g = np.random.Generator(np.random.PCG64(F))
     raw, dt = codes(g, kind, 2 * F, K)
     x, r = g.standard_normal((1, M, K)).astype(F16), g.standard_normal((1, M, 2 * F)).astype(F16)
@@ -87,6 +105,7 @@ def test_epilogues(dev, monkeypatch, kind, M, F, K, what):
             return h.add(Tensor.from_data(r, device=dev)).resolve().to_numpy()
         return h.slice([(0, 1), (0, M), (F, 2 * F)]).mul(h.slice([(0, 1), (0, M), (0, F)]).full().silu().cast(capi.F16)).resolve().to_numpy()
 
+    force(monkeypatch, route)
     got = run()
-    monkeypatch.setenv("RCU_GEMM_FUSED", "0")
+    force(monkeypatch, "0")
     assert np.array_equal(got.view(np.uint16), run().view(np.uint16))
