@@ -105,7 +105,8 @@ uint64_t rcu_profile_report(rcu_device* dev, char* buf, uint64_t capacity, int r
 
 /* ------------------------------------------------------------------ storage (storage/gpu_buffer.rs) */
 /* BufferAllocator / BufferPool: pooled device memory (gpu/pools/buffer_pool.rs:80-94 rounds sizes
- * up to 4 B with a 16 B minimum; this pool rounds to 256 B size classes and caches freed blocks). */
+ * up to 4 B with a 16 B minimum; this pool rounds to 256 B size classes and caches freed blocks).
+ * RCU_POOL_LIMIT in the environment when the device is created, in bytes: beyond it memory counts as exhausted. */
 rcu_status rcu_alloc(rcu_device* dev, uint64_t nbytes, void** dptr);
 rcu_status rcu_free(rcu_device* dev, void* dptr);
 /* Return cached blocks to the driver (WgpuDevice::begin_pass garbage collection analogue). */

@@ -26,8 +26,8 @@
 //                      scales took 2000 cycles a step: 1500 sectors in flight per SM).
 // The converting warps arrive in CTA scope: the tensor cores read behind a proxy fence; arriving in cluster scope waited 0.65 us a step for L2.
 // 512 x 8192 x 3072 Q4_KH: 35.1 us with the conversion in front of it -> 33.7; 512 x 9216 x 3072 Q8_0H: 37.3 -> 31.4 (pair_converts in gemm_tc.cu has more).
-// What bounds it: the chain of hand-overs - a step takes some 1000 cycles with the tensor pipe 42 to 45 % busy, issue slots 34 % - and with Q8_0 the codes' and the
-// converted tile's way through shared memory as well (51 % of its wavefronts are the converting warps').
+// What bounds it: the chain of hand-overs - a step takes some 1000 cycles with the tensor pipe 40 to 45 % busy, issue slots 33 % - and with Q8_0 the codes' and the
+// converted tile's way through shared memory as well (52 % of its wavefronts are the converting warps').
 //
 // The kernel is persistent: a pair walks over tiles pair, pair + n_pairs, ...; the accumulator is
 // double-buffered (2 x 256 of the 512 tensor-memory columns), so the epilogue of tile i overlaps the
