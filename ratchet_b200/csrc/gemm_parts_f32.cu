@@ -254,14 +254,21 @@ gemm_parts_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
                     }
                     const float bn = bs ? bs[n] : 0.f;
                     float* o = ys + (size_t)m0 * N + n;
-                    if constexpr (RESID) {           // all of a thread's are requested before the first is added
+                    if constexpr (RESID) {
+                        // in batches of sixteen: all 32 of a tile of 64 tokens at once, beside its sums, spilled 188 bytes of a thread beyond its 72 registers
+                        // (four of 65 x 9216 x 256 and three products of their results: 77 us, 56 now); eight at a time wait for memory twice as often (69)
+                        constexpr int B = 16;
+                        static_assert(C % B == 0, "");
                         const float* rs = resid + (size_t)m0 * N + n;
-                        float r[C];
 #pragma unroll
-                        for (int j = 0; j < C; ++j) r[j] = m0 + j < M ? rs[(size_t)j * N] : 0.f;
+                        for (int j0 = 0; j0 < C; j0 += B) {
+                            float r[B];
 #pragma unroll
-                        for (int j = 0; j < C; ++j)
-                            if (m0 + j < M) o[(size_t)j * N] = (acc[j] + bn) + r[j];
+                            for (int j = 0; j < B; ++j) r[j] = m0 + j0 + j < M ? rs[(size_t)(j0 + j) * N] : 0.f;
+#pragma unroll
+                            for (int j = 0; j < B; ++j)
+                                if (m0 + j0 + j < M) o[(size_t)(j0 + j) * N] = (acc[j0 + j] + bn) + r[j];
+                        }
                     } else {
 #pragma unroll
                         for (int j = 0; j < C; ++j)
@@ -391,6 +398,16 @@ bool make_map_f32_sw128(CUtensorMap* map, const void* base, uint64_t batches, ui
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Whole tiles (0), or the line of units cut into a run per SM: in units of the longest CTA, the sums of cut tiles (a launch, their partial
+// sums out and in again) counted as kSumUnits
+int cut_runs(uint64_t sms, uint64_t tiles, uint64_t nk) {
+    constexpr uint64_t kSumUnits = 7;
+    const uint64_t units = tiles * nk, whole = (tiles + sms - 1) / sms * nk;
+    // no more than sixteen runs of a tile: one thread adds an output's up (64 x 64 x 8192, one tile: 28 us with 128 runs)
+    const uint64_t runs = std::min({sms, units, 16 * tiles}), even = (units + runs - 1) / runs + kSumUnits;
+    return tiles % sms != 0 && even < whole ? (int)runs : 0;
+}
+
 template <int T, bool RESID>
 rcu_status launch_f32(rcu_device* dev, const void* w, const void* x, const void* bias, const void* bias_rows, void* y, uint64_t M, uint64_t N, uint64_t K, uint64_t batches, const void* resid = nullptr) {
     CUtensorMap xmap, wmap;
@@ -404,16 +421,11 @@ rcu_status launch_f32(rcu_device* dev, const void* w, const void* x, const void*
     const uint64_t tiles = batches * cut.tiles_m * (uint64_t)cut.tiles_n;
     if (tiles > 0x3fffffffull) return RCU_ERR_UNSUPPORTED;
     cut.tiles = (int)tiles;
-    // Whole tiles, or the line of units cut into a run per SM: in units of the longest CTA, the sums of cut tiles (a launch, their partial
-    // sums out and in again) counted as kSumUnits
-    const uint64_t sms = dev->sm_count, units = tiles * cut.nk, whole = (tiles + sms - 1) / sms * cut.nk;
-    constexpr uint64_t kSumUnits = 7;
-    // no more than sixteen runs of a tile: one thread adds an output's up (64 x 64 x 8192, one tile: 28 us with 128 runs)
-    const uint64_t runs = std::min({sms, units, 16 * tiles}), even = (units + runs - 1) / runs + kSumUnits;
-    cut.runs = tiles % sms != 0 && even < whole ? (int)runs : 0;
+    const uint64_t sms = dev->sm_count;
+    cut.runs = cut_runs(sms, tiles, cut.nk);
     void* partial = nullptr;
     if (cut.runs) {
-        if (rcu_alloc(dev, (runs + tiles) * (uint64_t)(T * kRowsW) * 4, &partial) != RCU_OK) cut.runs = 0;      // no room: whole tiles need none
+        if (rcu_alloc(dev, (cut.runs + tiles) * (uint64_t)(T * kRowsW) * 4, &partial) != RCU_OK) cut.runs = 0;      // no room: whole tiles need none
     }
     const unsigned grid = cut.runs ? (unsigned)cut.runs : (unsigned)std::min(tiles, sms);
     auto kern = gemm_parts_kernel<T, false, RESID>;
@@ -499,7 +511,13 @@ rcu_status rcu_gemm_parts_f32_dispatch(rcu_device* dev, const void* w, const voi
     return takes(dev, M, N, batches) ? dispatch(dev, w, x, bias, y, M, N, K, batches, bias_rows, nullptr) : RCU_ERR_UNSUPPORTED;
 }
 
-bool rcu_gemm_parts_f32_takes(rcu_device* dev, uint64_t M, uint64_t N, uint64_t K) { return rcu_gemm_tc_f32_eligible(RCU_F32, RCU_F32, M, N, K, 1) && takes(dev, M, N, 1); }
+// The residual too, where that is no slower than an addition behind the product: tiles that are cut into runs (whose sums are a pass over the output anyway) and short
+// K.  Whole tiles of longer K wait for it with their SM to themselves (us for four of them and three products, apart / in: 65 x 768 x 768 52.1 / 45.1, 1500 x 384 x 384
+// 54.2 / 49.4, 1500 x 512 x 512 72.2 / 70.5, 65 x 9216 x 256 55.8 / 55.8, 750 x 768 x 768 86.2 / 86.2, 750 x 1024 x 1024 105.0 / 107.6, 129 x 4096 x 1024 104.2 / 108.5).
+bool rcu_gemm_parts_f32_takes(rcu_device* dev, uint64_t M, uint64_t N, uint64_t K) {
+    if (!rcu_gemm_tc_f32_eligible(RCU_F32, RCU_F32, M, N, K, 1) || !takes(dev, M, N, 1)) return false;
+    return K <= 8 * kUnitK || cut_runs(dev->sm_count, (M + 63) / 64 * ((N + kRowsW - 1) / kRowsW), (K + kUnitK - 1) / kUnitK) > 0;
+}
 rcu_status rcu_gemm_parts_f32_resid(rcu_device* dev, const void* w, const void* x, const void* bias, const void* resid, void* y, uint64_t M, uint64_t N, uint64_t K) {
     if (!rcu_gemm_parts_f32_takes(dev, M, N, K)) return RCU_ERR_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(bias)) & 15) return RCU_ERR_UNSUPPORTED;

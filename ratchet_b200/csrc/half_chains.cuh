@@ -42,7 +42,7 @@ struct LinearChain {
 bool rcu_gemm_tc_chain_takes(rcu_device* dev, int w_dt, uint64_t M, uint64_t N, uint64_t K, bool glu, bool act);
 rcu_status rcu_gemm_tc_chain(rcu_device* dev, int w_dt, const void* w, const void* x, void* y, uint64_t M, uint64_t N, uint64_t K, const LinearChain& c);
 
-// The addition to a residual behind an f32 Linear that gemm_parts_f32.cu runs: y = (x W^T + bias) + resid, each rounded as the ops by themselves do
+// The addition to a residual behind an f32 Linear that gemm_parts_f32.cu runs, where that pays: y = (x W^T + bias) + resid, each rounded as the ops by themselves do
 bool rcu_gemm_parts_f32_takes(rcu_device* dev, uint64_t M, uint64_t N, uint64_t K);
 rcu_status rcu_gemm_parts_f32_resid(rcu_device* dev, const void* w, const void* x, const void* bias, const void* resid, void* y, uint64_t M, uint64_t N, uint64_t K);
 

@@ -64,8 +64,9 @@ def test_an_output_that_takes_over_a_members_input_stays_apart(dev):
 
 
 # an f32 product and the addition behind it: whole tiles of 32 and of 64 tokens, tiles that are cut into runs, one row too few or many; a product that
-# another kernel runs (apart)
-@pytest.mark.parametrize("M,N,K", [(16, 136, 256), (33, 128, 512), (64, 2560, 2048), (65, 260, 96), (1500, 384, 384), (1501, 384, 1536), (70, 61, 128), (1500, 1536, 384), (2, 64, 64)])
+# another kernel runs (apart); whole tiles of 64 tokens with short K, and with a longer one (apart)
+@pytest.mark.parametrize("M,N,K", [(16, 136, 256), (33, 128, 512), (64, 2560, 2048), (65, 260, 96), (1500, 384, 384), (1501, 384, 1536), (70, 61, 128), (1500, 1536, 384), (2, 64, 64),
+                                   (65, 9216, 256), (1500, 512, 512), (750, 768, 768)])
 @pytest.mark.parametrize("left", [False, True])
 @pytest.mark.parametrize("quantised", [False, True])
 def test_the_addition_behind_an_f32_product(dev, M, N, K, left, quantised):
@@ -79,7 +80,11 @@ def test_the_addition_behind_an_f32_product(dev, M, N, K, left, quantised):
     lin = nn.Linear(w, b)
     want = lin.schedule(x).resolve().to_numpy() + r.to_numpy()
     got = r.add(lin.schedule(x)) if left else lin.schedule(x).add(r)
-    assert np.array_equal(got.resolve().to_numpy(), want, equal_nan=True)
+    launches = dev.launches
+    got = got.resolve()
+    if not quantised and N >= 512:
+        assert dev.launches - launches == (1 if M > 64 and K <= 512 and N != 1536 else 3 if M == 64 else 2)        # 64 tokens: cut into runs
+    assert np.array_equal(got.to_numpy(), want, equal_nan=True)
 
 
 # an activation, a permute, positions and a cast in one kernel, against the ops by themselves (each result held): pieces of 32 in both directions, ragged
