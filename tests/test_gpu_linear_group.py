@@ -88,7 +88,8 @@ def test_the_addition_behind_an_f32_product(dev, M, N, K, left, quantised):
 
 
 # an activation, a permute, positions and a cast in one kernel, against the ops by themselves (each result held): pieces of 32 in both directions, ragged
-@pytest.mark.parametrize("T,C", [(501, 384), (32, 64), (33, 31), (2, 1), (100, 97)])
+# in the last two, many pieces that are mostly empty (apart)
+@pytest.mark.parametrize("T,C", [(501, 384), (32, 64), (33, 31), (2, 1), (100, 97), (2, 131105), (131105, 3)])
 @pytest.mark.parametrize("act", ["gelu", "silu"])
 @pytest.mark.parametrize("half", [False, True])
 @pytest.mark.parametrize("left", [False, True])
@@ -111,5 +112,5 @@ def test_a_convolutions_output_to_rows(dev, T, C, act, half, left):
     out = schedule(handles)
     handles.clear()                              # nothing holds the ops between
     got = out.resolve().to_numpy()
-    assert dev.launches - launches == 1
+    assert dev.launches - launches == (1 if T * C < 1 << 18 else 4 if half else 3)
     assert got.dtype == (np.float16 if half else np.float32) and np.array_equal(got, want)
