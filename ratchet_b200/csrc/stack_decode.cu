@@ -120,7 +120,7 @@ template <bool VEC> __device__ __forceinline__ float4 load4(const float* p, int 
 }
 
 constexpr int kKept = 4;                // quads of a vector that a thread keeps in registers
-constexpr int kBatch = 8;               // quads of a vector that is only copied, in flight at a time
+constexpr int kBatch = 8;               // quads of a vector that is only copied, in flight at a time (VEC)
 
 // The norm scales of a product's input, requested before the wait for the kernel before it (they are constant).
 template <bool VEC> struct StagedScales {
@@ -259,18 +259,22 @@ template <bool VEC, class Put> __device__ __forceinline__ void stage_input(const
         }
         return;                                         // both pieces come from the norm
     }
-    // the second input's first quads travel with the first input
-    float4 second[kBatch];
+    // The second input's first quads travel with the first input.  Without VEC there are no batches: they cost rows_kernel 22 registers, and with
+    // 102 an SM holds two of its CTAs, not three (us per token, six layers, before / with / without: 64 heads of 64, width 512, f32 368 / 396 / 368; 16 latent
+    // heads of rank 1024, width 1536, f32 509 / 532 / 466; width 96, bf16 198 / 219 / 198).
+    float4 second[VEC ? kBatch : 1];
+    if constexpr (VEC) {
 #pragma unroll
-    for (int i = 0; i < kBatch; ++i) second[i] = load4<VEC>(a.x2 + j0 + i * step, a.split ? 0 : a.kb - (j0 + i * step));
+        for (int i = 0; i < kBatch; ++i) second[i] = load4<VEC>(a.x2 + j0 + i * step, a.split ? 0 : a.kb - (j0 + i * step));
+    }
     if (a.pro == PRO_GATED_RMS) {
-        float4 v[kKept], g[kKept];
+        float4 v[kKept], g[VEC ? kKept : 1];
         float q = 0.f;
         auto square = [&](const float4& w) { q += (w.x * w.x + w.y * w.y) + (w.z * w.z + w.w * w.w); };
 #pragma unroll
         for (int i = 0; i < kKept; ++i) {
             v[i] = load4<VEC>(a.x + j0 + i * step, a.ka - (j0 + i * step));
-            g[i] = load4<VEC>(a.gate + j0 + i * step, a.ka - (j0 + i * step));
+            if constexpr (VEC) g[i] = load4<VEC>(a.gate + j0 + i * step, a.ka - (j0 + i * step));
         }
 #pragma unroll
         for (int i = 0; i < kKept; ++i) square(v[i]);
@@ -281,7 +285,10 @@ template <bool VEC, class Put> __device__ __forceinline__ void stage_input(const
             put(0, j, make_float4(w.x * rstd * s.x * g.x, w.y * rstd * s.y * g.y, w.z * rstd * s.z * g.z, w.w * rstd * s.w * g.w));
         };
 #pragma unroll
-        for (int i = 0; i < kKept; ++i) emit(v[i], j0 + i * step, sc.s1[i], g[i]);
+        for (int i = 0; i < kKept; ++i) {
+            if constexpr (VEC) emit(v[i], j0 + i * step, sc.s1[i], g[i]);
+            else emit(v[i], j0 + i * step, sc.s1[i], load4(a.gate + j0 + i * step, a.ka - (j0 + i * step)));
+        }
         for (int j = j0 + kKept * step; j < padded(a.ka); j += step)
             emit(load4<VEC>(a.x + j, a.ka - j), j, load4<VEC>(a.s1 + j, a.ka - j), load4<VEC>(a.gate + j, a.ka - j));
     } else {
@@ -292,40 +299,50 @@ template <bool VEC, class Put> __device__ __forceinline__ void stage_input(const
             auto one = [&](int i) { return i >= a.ka ? 0.f : i < a.split ? a.x[i] : a.x2[i - a.split]; };
             return make_float4(one(j), one(j + 1), one(j + 2), one(j + 3));
         };
-        for (int j = j0; j < padded(a.ka); j += kBatch * step) {
-            float4 v[kBatch];
+        if constexpr (VEC) {
+            for (int j = j0; j < padded(a.ka); j += kBatch * step) {
+                float4 v[kBatch];
 #pragma unroll
-            for (int i = 0; i < kBatch; ++i) v[i] = at(j + i * step);
+                for (int i = 0; i < kBatch; ++i) v[i] = at(j + i * step);
 #pragma unroll
-            for (int i = 0; i < kBatch; ++i)
-                if (j + i * step < padded(a.ka)) put(0, j + i * step, v[i]);
+                for (int i = 0; i < kBatch; ++i)
+                    if (j + i * step < padded(a.ka)) put(0, j + i * step, v[i]);
+            }
+        } else {
+#pragma unroll 4
+            for (int j = j0; j < padded(a.ka); j += step) put(0, j, at(j));
         }
     }
-    for (int j = j0; j < padded(a.kb); j += kBatch * step) {
-        if (j != j0) {
+    if constexpr (VEC) {
+        for (int j = j0; j < padded(a.kb); j += kBatch * step) {
+            if (j != j0) {
 #pragma unroll
-            for (int i = 0; i < kBatch; ++i) second[i] = load4<VEC>(a.x2 + j + i * step, a.kb - (j + i * step));
+                for (int i = 0; i < kBatch; ++i) second[i] = load4<VEC>(a.x2 + j + i * step, a.kb - (j + i * step));
+            }
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i)
+                if (j + i * step < padded(a.kb)) put(1, j + i * step, second[i]);
         }
-#pragma unroll
-        for (int i = 0; i < kBatch; ++i)
-            if (j + i * step < padded(a.kb)) put(1, j + i * step, second[i]);
+    } else {
+#pragma unroll 4
+        for (int j = j0; j < padded(a.kb); j += step) put(1, j, load4(a.x2 + j, a.kb - j));
     }
 }
 
-// What a row's epilogue adds: its bias or residual.  Asked for before the product, a trip to L2 (0.8 us) does not follow it.
+// What a row's epilogue adds: its bias or residual.  Asked for before the product (rows_mma_kernel), a trip to L2 (0.8 us) does not follow it.
 __device__ __forceinline__ float addend(const RowsArgs& a, int row) {
     if (row >= a.na) return 0.f;
     return a.epi == EPI_BIAS ? a.bias[row] : a.epi == EPI_RESIDUAL ? a.resid[row] : 0.f;
 }
-__device__ __forceinline__ void finish_row(const RowsArgs& a, int row, float v, float add) {
+template <class Add> __device__ __forceinline__ void finish_row(const RowsArgs& a, int row, float v, Add add) {
     if (row >= a.na) return;
     if (a.epi == EPI_MIXER_IN) {
         if (row < a.n_silu) v = lm::silu(v);
         else if (row >= a.n_sigmoid) v = lm::sigmoid(v);
     } else if (a.epi == EPI_RESIDUAL) {
-        v = fmaf(a.alpha, v, add);
+        v = fmaf(a.alpha, v, add());
     } else if (a.epi == EPI_BIAS) {
-        v += add;
+        v += add();
     } else if (a.epi == EPI_RELU_SQUARED) {
         v = v > 0.f ? v * v : 0.f;
     } else if (a.epi == EPI_SOFTCAP) {
@@ -334,8 +351,10 @@ __device__ __forceinline__ void finish_row(const RowsArgs& a, int row, float v, 
     a.out[row] = v;
 }
 
-// Any type and row length: two rows per unit in FFMA, a team of warps splitting the columns.
-template <class T>
+// Any type and row length: two rows per unit in FFMA, a team of warps splitting the columns.  LATENT: of a model that has latent
+// runs; one of its products has the CTA that writes the token's latent row (a.C > 0).  A form of its own for that product alone took turns with the other one in a step: 198
+// and 184 us (64 latent heads, width 256, f32); without any of it a model of grouped heads gains 1 to 2 %.
+template <class T, bool LATENT>
 __global__ void __launch_bounds__(kThreads) rows_kernel(const RowsArgs a) {
     rcu_kernel_entry();
     extern __shared__ __align__(16) float xs[];        // input A, input B
@@ -344,10 +363,12 @@ __global__ void __launch_bounds__(kThreads) rows_kernel(const RowsArgs a) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int parts = a.parts, teams = kWarps / parts, team = warp / parts, part = warp % parts;
     const int ua = (a.na + kRows - 1) / kRows, units = ua + (a.dual ? 0 : a.pairs);
-    const int xb = padded(a.ka), grid = (int)gridDim.x - (a.C > 0);
-    if ((int)blockIdx.x == grid) {
-        append_latent<T>(a, scratch);
-        return;
+    const int xb = padded(a.ka), grid = (int)gridDim.x - (LATENT && a.C > 0);
+    if constexpr (LATENT) {
+        if ((int)blockIdx.x == grid) {
+            append_latent<T>(a, scratch);
+            return;
+        }
     }
     StagedScales<false> sc;
     sc.request(a);
@@ -386,8 +407,8 @@ __global__ void __launch_bounds__(kThreads) rows_kernel(const RowsArgs a) {
         }
         if (part == 0 && lane == 0) {
             if (a.dual || u < ua) {
-                finish_row(a, u * kRows, acc[0], addend(a, u * kRows));
-                finish_row(a, u * kRows + 1, acc[1], addend(a, u * kRows + 1));
+                finish_row(a, u * kRows, acc[0], [&] { return addend(a, u * kRows); });
+                finish_row(a, u * kRows + 1, acc[1], [&] { return addend(a, u * kRows + 1); });
             } else {
                 a.out2[u - ua] = lm::gelu_tanh(acc[0]) * acc[1];
             }
@@ -535,8 +556,8 @@ __global__ void __launch_bounds__(kThreads) rows_mma_kernel(const __grid_constan
         }
         if (mine) {
             if (a.dual || u < ua) {
-                finish_row(a, u * kUnit + g, lo, add_lo);
-                finish_row(a, u * kUnit + g + 8, hi, add_hi);
+                finish_row(a, u * kUnit + g, lo, [&] { return add_lo; });
+                finish_row(a, u * kUnit + g + 8, hi, [&] { return add_hi; });
             } else {
                 const int p = (u - ua) * (kUnit / 2) + g;
                 if (p < a.pairs) a.out2[p] = lm::gelu_tanh(lo) * hi;
@@ -1192,6 +1213,7 @@ struct rcu_stack {
     float *angle_pool, *angle_tables, *arrived;      // (cos, sin) pairs; AngleTable[n_angles]; counters of the grouped attention
     std::vector<float2*> run_angles;                 // per run: its pairs (null: a lightning mixer)
     int n_angles = 0;
+    bool latent = false;                // has latent runs
     bool ahead = true;                  // no two runs share memory of their states: kernels may read theirs ahead of the wait
     uint32_t* d_pos = nullptr;
     uint32_t position = 0, kernels_per_step = 0;
@@ -1247,7 +1269,8 @@ int plan_parts(int grid, int units, int items) {
     return best;
 }
 
-template <class T> rcu_status launch_rows(rcu_device* dev, RowsArgs a) {
+template <class T> rcu_status launch_rows(const rcu_stack* s, RowsArgs a) {
+    rcu_device* dev = s->dev;
     a.status = dev->d_status;
     const bool has_b = a.kb > 0 && a.wb;
     const size_t inputs = ((size_t)padded(a.ka) + (size_t)padded(a.kb)) * 4, per_slot = (size_t)kWarps * kSlotBytes;
@@ -1275,8 +1298,9 @@ template <class T> rcu_status launch_rows(rcu_device* dev, RowsArgs a) {
         a.parts = plan_parts(dev->sm_count, units, a.dual ? nca + ncb : std::max(nca, ncb));
         const int teams = kWarps / a.parts, grid = std::max(1, std::min(4 * dev->sm_count, (units + teams - 1) / teams)) + (a.C > 0);
         if (inputs > most) return rcu_fail(dev, RCU_ERR_UNSUPPORTED, "stack: input vectors of %d + %d do not fit shared memory", a.ka, a.kb);
-        RCU_CUDA(dev, cudaFuncSetAttribute(rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
-        RCU_CUDA(dev, rcu_launch(dev, rows_kernel<T>, grid, kThreads, inputs, a));
+        auto kern = s->latent ? rows_kernel<T, true> : rows_kernel<T, false>;
+        RCU_CUDA(dev, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+        RCU_CUDA(dev, rcu_launch(dev, kern, grid, kThreads, inputs, a));
     }
     RCU_LAUNCH_CHECK(dev);
     return RCU_OK;
@@ -1355,7 +1379,7 @@ template <class T> rcu_status run_step(rcu_stack* s, const int32_t* token, float
             RowsArgs in = {};
             stream_input(in);
             in.wa = r.mix_in; in.na = (H + G) * D + G * E; in.epi = r.mix_bias ? EPI_BIAS : EPI_STORE; in.bias = (const float*)r.mix_bias; in.out = s->mix;
-            STACK_TRY(launch_rows<T>(dev, in));
+            STACK_TRY(launch_rows<T>(s, in));
             const gstep::Args at{s->mix, (const float*)r.mix_norm, (const float*)r.kv_norm, s->run_angles[k], (const float*)r.sink, r.state, s->d_pos, s->y, s->partial,
                                  (uint32_t*)s->arrived, H, G, D, E, (int)r.rot_pairs, (int)r.ring_rows,
                                  r.window ? (int)std::min<uint32_t>(r.window, 1u << 30) : 1 << 30, (int)std::min<uint32_t>(r.chunk, 1u << 30), c.eps, r.scale, s->ahead};
@@ -1363,16 +1387,16 @@ template <class T> rcu_status run_step(rcu_stack* s, const int32_t* token, float
             RowsArgs o = {};
             o.wa = r.out; o.na = W; o.ka = H * E; o.pro = PRO_CONCAT; o.x = s->y; o.out = s->sub;
             o.epi = r.out_bias ? EPI_BIAS : EPI_STORE; o.bias = (const float*)r.out_bias;
-            STACK_TRY(launch_rows<T>(dev, o));
+            STACK_TRY(launch_rows<T>(s, o));
             after = (const float*)r.norm1; after_shift = (const float*)r.norm1_shift;
             if (r.ff) {
                 RowsArgs up = {};
                 stream_input(up);
                 up.wa = r.gate_up; up.na = (int)r.ff; up.epi = EPI_RELU_SQUARED; up.out = s->act;
-                STACK_TRY(launch_rows<T>(dev, up));
+                STACK_TRY(launch_rows<T>(s, up));
                 RowsArgs down = {};
                 down.wa = r.down; down.na = W; down.ka = (int)r.ff; down.pro = PRO_CONCAT; down.x = s->act; down.out = s->sub;
-                STACK_TRY(launch_rows<T>(dev, down));
+                STACK_TRY(launch_rows<T>(s, down));
                 after = (const float*)r.norm2; after_shift = (const float*)r.norm2_shift;
             }
             continue;
@@ -1383,7 +1407,7 @@ template <class T> rcu_status run_step(rcu_stack* s, const int32_t* token, float
             a.pro = PRO_CONCAT; a.epi = EPI_BIAS;
             a.x = x; a.x2 = s->x0; a.split = W;
             a.bias = (const float*)r.enter_bias; a.out = other;
-            STACK_TRY(launch_rows<T>(dev, a));
+            STACK_TRY(launch_rows<T>(s, a));
             std::swap(x, other);
         }
         const int H = (int)r.heads, D = (int)r.dim, E = (int)r.vdim, ff = (int)r.ff;
@@ -1397,7 +1421,7 @@ template <class T> rcu_status run_step(rcu_stack* s, const int32_t* token, float
         if (r.mixer == RCU_MIXER_LIGHTNING) {
             in.na = 2 * H * D + 2 * H * E;
             in.epi = EPI_MIXER_IN; in.n_silu = 2 * H * D + H * E; in.n_sigmoid = in.n_silu;
-            STACK_TRY(launch_rows<T>(dev, in));
+            STACK_TRY(launch_rows<T>(s, in));
             RCU_CUDA(dev, rcu_launch(dev, lightning_step_kernel, dim3(H, (E + 31) / 32), kThreads, 0, s->mix, (const float*)r.decay, (float*)r.state, s->y, H, D, E, s->ahead));
             RCU_LAUNCH_CHECK(dev);
             out.pro = PRO_GATED_RMS; out.x = s->y; out.s1 = (const float*)r.mix_norm; out.gate = s->mix + 2 * H * D + H * E;
@@ -1405,12 +1429,12 @@ template <class T> rcu_status run_step(rcu_stack* s, const int32_t* token, float
             const int Q = (int)r.q_rank, C = (int)r.kv_rank, R = (int)r.rot_dim, nf = (int)r.rot_pairs;
             in.na = Q + C + R;
             in.epi = EPI_STORE;
-            STACK_TRY(launch_rows<T>(dev, in));
+            STACK_TRY(launch_rows<T>(s, in));
             RowsArgs uq = {};
             uq.wa = r.uq; uq.na = H * (D + R); uq.ka = Q; uq.pro = PRO_RMS; uq.x = s->mix; uq.s1 = (const float*)r.mix_norm; uq.eps = c.eps; uq.out = s->q;
             uq.low = s->mix + Q; uq.c_scale = (const float*)r.kv_norm; uq.angles = s->run_angles[k]; uq.ring = r.state; uq.C = C; uq.R = R; uq.n_freq = nf;
             uq.ring_rows = (int)r.ring_rows; uq.d_pos = s->d_pos;
-            STACK_TRY(launch_rows<T>(dev, uq));
+            STACK_TRY(launch_rows<T>(s, uq));
             RCU_CUDA(dev, rcu_launch(dev, absorb_kernel<T>, dim3(H, (C + 31) / 32), kThreads, 0, s->q, (const T*)r.ukv, s->run_angles[k], nf, s->qa, D, R, C, r.scale));
             RCU_LAUNCH_CHECK(dev);
             STACK_TRY(launch_latent_step(dev, s, r, c.weight_dt));
@@ -1420,7 +1444,7 @@ template <class T> rcu_status run_step(rcu_stack* s, const int32_t* token, float
             RCU_LAUNCH_CHECK(dev);
             out.pro = PRO_CONCAT; out.x = s->y;
         }
-        STACK_TRY(launch_rows<T>(dev, out));
+        STACK_TRY(launch_rows<T>(s, out));
     }
     RowsArgs head = {};
     if (after) {
@@ -1432,7 +1456,7 @@ template <class T> rcu_status run_step(rcu_stack* s, const int32_t* token, float
     }
     head.wa = s->head; head.na = (int)c.vocab; head.out = logits;
     if (c.logit_softcap > 0.f) { head.epi = EPI_SOFTCAP; head.alpha = c.logit_softcap; }
-    STACK_TRY(launch_rows<T>(dev, head));
+    STACK_TRY(launch_rows<T>(s, head));
     RCU_CUDA(dev, rcu_launch_cluster(dev, argmax_next_kernel, kArgmaxCtas, kArgmaxThreads, 0, kArgmaxCtas, logits, (int)c.vocab, argmax, s->d_pos));
     RCU_LAUNCH_CHECK(dev);
     return RCU_OK;
@@ -1527,6 +1551,7 @@ rcu_status rcu_stack_create(rcu_device* dev, const rcu_stack_config* cfg, const 
     }
     for (uint32_t i = 0; i < cfg->n_runs; ++i) s->run_angles.push_back(table_of[i] < 0 ? nullptr : tables[table_of[i]].out);
     s->n_angles = (int)n_tables;
+    for (const rcu_stack_run& r : s->runs) s->latent = s->latent || r.mixer == RCU_MIXER_LATENT;
     std::vector<std::pair<uintptr_t, uintptr_t>> held;
     for (const rcu_stack_run& r : s->runs) {
         const uint64_t e = dt_esize(cfg->weight_dt);
